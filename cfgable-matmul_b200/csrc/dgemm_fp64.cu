@@ -58,6 +58,14 @@ struct ColMask {
   int blk;
 };
 
+// A kernel of one of two forms that both are enqueued: it runs when the device
+// word (the choice made earlier on the stream) is zero / nonzero as wanted.
+struct Gate {
+  const int* word;  // null: always runs
+  int want;
+  __device__ __forceinline__ bool closed() const { return word && (*word != 0) != (want != 0); }
+};
+
 template <bool kRowsContig>
 struct TileCopier {
   const double* src;     // element i = 0 of the current K step
@@ -295,7 +303,8 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 __global__ void __launch_bounds__(THREADS, 1)
 dgemm_tma_kernel(double* __restrict__ c, int m, int n, int k, size_t ldc,
                  const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 TailSplit tail) {
+                 TailSplit tail, Gate gate) {
+  if (gate.closed()) return;
   extern __shared__ uint8_t tsmem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tsmem_raw) + 1023) &
                                            ~uintptr_t(1023));
@@ -585,7 +594,8 @@ dgemm_tma_act_kernel(double* __restrict__ c, int m, int n, int k, size_t ldc,
 // K-contiguous operand.  A warp per row, 256 columns per block.
 __global__ void __launch_bounds__(256)
 pack_rows(double* __restrict__ dst, const double* __restrict__ src, size_t ld, int rows, int k,
-          int kpad) {
+          int kpad, Gate gate) {
+  if (gate.closed()) return;
   const int r = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;
   const double* srow = src + size_t(r) * ld;
@@ -601,7 +611,8 @@ pack_rows(double* __restrict__ dst, const double* __restrict__ src, size_t ld, i
 // a mask, element (p, j) is zero unless tab[p * ldtab + j / blk].
 __global__ void __launch_bounds__(256)
 pack_transpose(double* __restrict__ dst, const double* __restrict__ src, size_t ld, int cols,
-               int k, int kpad, const uint8_t* __restrict__ tab, size_t ldtab, int blk) {
+               int k, int kpad, const uint8_t* __restrict__ tab, size_t ldtab, int blk, Gate gate) {
+  if (gate.closed()) return;
   __shared__ double t[32][33];
   const int j0 = blockIdx.x * 32, p0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -653,7 +664,8 @@ bool make_operand_map(CUtensorMap* map, const double* base, int rows, int kpad) 
 // C[tile] += the splits' partial tiles, added in split order (deterministic).
 __global__ void __launch_bounds__(256)
 dgemm_tail_reduce(double* __restrict__ c, const double* __restrict__ ws, int m, int n,
-                  size_t ldc, int full, int splits) {
+                  size_t ldc, int full, int splits, Gate gate) {
+  if (gate.closed()) return;
   const int tiles_m = (m + BM - 1) / BM, tiles_n = (n + BN - 1) / BN;
   const int tile = full + blockIdx.x;
   const int per_group = GROUP_M * tiles_n;
@@ -715,8 +727,8 @@ cudaError_t launch_t(double* c, const double* a, const double* b, int m, int n, 
   err = cudaGetLastError();
   if (ts.splits) {
     if (err == cudaSuccess) {
-      dgemm_tail_reduce<<<unsigned(tiles - ts.full), 256, 0, stream>>>(c, ts.ws, m, n, ldc,
-                                                                       ts.full, ts.splits);
+      dgemm_tail_reduce<<<unsigned(tiles - ts.full), 256, 0, stream>>>(
+          c, ts.ws, m, n, ldc, ts.full, ts.splits, Gate{nullptr, 0});
       err = cudaGetLastError();
     }
     const cudaError_t e2 = cudaFreeAsync(ts.ws, stream);
@@ -728,7 +740,7 @@ cudaError_t launch_t(double* c, const double* a, const double* b, int m, int n, 
 // The TMA form: pack A and B, build their tensor maps, run, release.
 cudaError_t launch_packed(double* c, const double* a, const double* b, int m, int n, int k,
                           size_t lda, size_t ldb, size_t ldc, bool transa, bool transb,
-                          ColMask mask, cudaStream_t stream) {
+                          ColMask mask, cudaStream_t stream, Gate gate = Gate{nullptr, 0}) {
   const int kpad = (k + 7) / 8 * 8;
   double* ws = nullptr;
   cudaError_t err = cudaMallocAsync(reinterpret_cast<void**>(&ws),
@@ -737,15 +749,17 @@ cudaError_t launch_packed(double* c, const double* a, const double* b, int m, in
   double* ap = ws;
   double* bp = ws + size_t(m) * kpad;
   if (!transa)
-    pack_rows<<<dim3((kpad + 255) / 256, (m + 7) / 8), 256, 0, stream>>>(ap, a, lda, m, k, kpad);
+    pack_rows<<<dim3((kpad + 255) / 256, (m + 7) / 8), 256, 0, stream>>>(ap, a, lda, m, k, kpad,
+                                                                          gate);
   else
     pack_transpose<<<dim3((m + 31) / 32, (kpad + 31) / 32), 256, 0, stream>>>(
-        ap, a, lda, m, k, kpad, nullptr, 0, 1);
+        ap, a, lda, m, k, kpad, nullptr, 0, 1, gate);
   if (transb)
-    pack_rows<<<dim3((kpad + 255) / 256, (n + 7) / 8), 256, 0, stream>>>(bp, b, ldb, n, k, kpad);
+    pack_rows<<<dim3((kpad + 255) / 256, (n + 7) / 8), 256, 0, stream>>>(bp, b, ldb, n, k, kpad,
+                                                                          gate);
   else
     pack_transpose<<<dim3((n + 31) / 32, (kpad + 31) / 32), 256, 0, stream>>>(
-        bp, b, ldb, n, k, kpad, mask.tab, mask.ldtab, mask.blk);
+        bp, b, ldb, n, k, kpad, mask.tab, mask.ldtab, mask.blk, gate);
   err = cudaGetLastError();
   CUtensorMap tmA, tmB;
   if (err == cudaSuccess &&
@@ -771,11 +785,12 @@ cudaError_t launch_packed(double* c, const double* a, const double* b, int m, in
   }
   if (err == cudaSuccess) {
     const long long grid = ts.splits ? ts.full + (tiles - ts.full) * ts.splits : tiles;
-    dgemm_tma_kernel<<<unsigned(grid), THREADS, TMA_SMEM, stream>>>(c, m, n, k, ldc, tmA, tmB, ts);
+    dgemm_tma_kernel<<<unsigned(grid), THREADS, TMA_SMEM, stream>>>(c, m, n, k, ldc, tmA, tmB, ts,
+                                                                    gate);
     err = cudaGetLastError();
     if (err == cudaSuccess && ts.splits) {
       dgemm_tail_reduce<<<unsigned(tiles - ts.full), 256, 0, stream>>>(c, ts.ws, m, n, ldc,
-                                                                       ts.full, ts.splits);
+                                                                       ts.full, ts.splits, gate);
       err = cudaGetLastError();
     }
   }
@@ -899,25 +914,74 @@ cudaError_t dgemm_fp64(double* c, const double* a, const double* b, int m, int n
   return launch_t<true, true>(c, a, b, m, n, k, lda, ldb, ldc, none, stream);
 }
 
+cudaError_t dgemm_pack_kmajor(double* dst, const double* a, size_t lda, int m, int k, int pitch,
+                              bool transa, const int* run, cudaStream_t stream) {
+  const Gate gate{run, 1};
+  if (transa)
+    pack_rows<<<dim3((pitch + 255) / 256, (k + 7) / 8), 256, 0, stream>>>(dst, a, lda, k, m, pitch,
+                                                                         gate);
+  else
+    pack_transpose<<<dim3((k + 31) / 32, (pitch + 31) / 32), 256, 0, stream>>>(
+        dst, a, lda, k, m, pitch, nullptr, 0, 1, gate);
+  return cudaGetLastError();
+}
+
 cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int m, int n, int k,
                                size_t lda, size_t ldb, size_t ldc, bool transa,
                                const uint8_t* tab, size_t ldtab, int blk, cudaStream_t stream) {
   if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
   const ColMask mask{tab, ldtab, blk};
-  if (use_packed(m, n, k))
-    return launch_packed(c, a, b, m, n, k, lda, ldb, ldc, transa, false, mask, stream);
-  if (!transa) return launch_t<false, false>(c, a, b, m, n, k, lda, ldb, ldc, mask, stream);
-  return launch_t<true, false>(c, a, b, m, n, k, lda, ldb, ldc, mask, stream);
+  const bool packed = use_packed(m, n, k);
+  if (!dgemm_mask_applies(m, n, k, blk)) {
+    if (packed)
+      return launch_packed(c, a, b, m, n, k, lda, ldb, ldc, transa, false, mask, stream);
+    if (!transa) return launch_t<false, false>(c, a, b, m, n, k, lda, ldb, ldc, mask, stream);
+    return launch_t<true, false>(c, a, b, m, n, k, lda, ldb, ldc, mask, stream);
+  }
+  // Where the dense form can be the faster one, both are enqueued and the device
+  // picks by the share of present tiles: the host does not know it without
+  // waiting for the mask.  Below the packed sizes the dense form's single wave
+  // of 128 x 128 tiles is not faster (600 x 1500 x 600, 90 % present: 129 us
+  // against 97).
+  const double share = packed ? dgemm_mask_max_share(n, blk) : 1.0;
+  const size_t wsb = dgemm_mask_workspace(a, b, m, n, k, lda, ldb, transa, blk);
+  int* compact = nullptr;  // the choice, outliving the compacted form's scratch
+  void* ws = nullptr;
+  cudaError_t err = cudaSuccess;
+  if (share < 1.0) {
+    if ((err = cudaMallocAsync(reinterpret_cast<void**>(&compact), 256, stream)) != cudaSuccess)
+      return err;
+    err = cudaMallocAsync(&ws, wsb, stream);
+  } else {
+    err = cudaMallocAsync(&ws, wsb + 256, stream);
+  }
+  if (err == cudaSuccess) {
+    err = dgemm_mask_compact(
+        c, a, b, m, n, k, lda, ldb, ldc, transa, tab, ldtab, blk, share,
+        compact ? compact : reinterpret_cast<int*>(static_cast<char*>(ws) + wsb), ws, stream);
+    const cudaError_t e2 = cudaFreeAsync(ws, stream);
+    if (err == cudaSuccess) err = e2;
+  }
+  if (compact) {
+    if (err == cudaSuccess)
+      err = launch_packed(c, a, b, m, n, k, lda, ldb, ldc, transa, false, mask, stream,
+                          Gate{compact, 0});
+    const cudaError_t e3 = cudaFreeAsync(compact, stream);
+    if (err == cudaSuccess) err = e3;
+  }
+  return err;
 }
 
 cudaError_t dgemm_reset_error(cudaStream_t stream) {
   static const int zero = 0;
-  return cudaMemcpyToSymbolAsync(g_dgemm_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice,
-                                 stream);
+  const cudaError_t err = cudaMemcpyToSymbolAsync(g_dgemm_error, &zero, sizeof(int), 0,
+                                                  cudaMemcpyHostToDevice, stream);
+  return err != cudaSuccess ? err : dgemm_mask_reset_error(stream);
 }
 
 cudaError_t dgemm_read_error(int* code) {
-  return cudaMemcpyFromSymbol(code, g_dgemm_error, sizeof(int));
+  const cudaError_t err = cudaMemcpyFromSymbol(code, g_dgemm_error, sizeof(int));
+  return err != cudaSuccess || *code != 0 ? err : dgemm_mask_read_error(code);
 }
 
 }  // namespace cfgmm

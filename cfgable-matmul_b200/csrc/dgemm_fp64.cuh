@@ -16,6 +16,29 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
                                size_t lda, size_t ldb, size_t ldc, bool transa,
                                const uint8_t* tab, size_t ldtab, int blk, cudaStream_t stream);
 
+// The masked GEMM on each column block's compacted rows (dgemm_mask.cu).
+// dgemm_mask_applies: the shapes it takes; dgemm_mask_max_share: the share of
+// present tiles up to which it is faster than the dense form (>= 1: always).
+// dgemm_mask_compact enqueues the lists, the choice and the kernel: where more
+// than max_share (< 1) of the tiles is present nothing is added to C and the
+// device word *compact is 0 (the caller then enqueues the dense form gated on
+// it), otherwise it is 1.
+bool dgemm_mask_applies(int m, int n, int k, int blk);
+double dgemm_mask_max_share(int n, int blk);
+size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,
+                            size_t ldb, bool transa, int blk);
+cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int m, int n, int k,
+                               size_t lda, size_t ldb, size_t ldc, bool transa,
+                               const uint8_t* tab, size_t ldtab, int blk, double max_share,
+                               int* compact, void* workspace, cudaStream_t stream);
+cudaError_t dgemm_mask_reset_error(cudaStream_t stream);
+cudaError_t dgemm_mask_read_error(int* code);
+
+// dst[p*pitch + i] = opA(i, p) for p < k, i < m, 0 for m <= i < pitch; with
+// `run`, only when *run != 0 on the device.
+cudaError_t dgemm_pack_kmajor(double* dst, const double* a, size_t lda, int m, int k, int pitch,
+                              bool transa, const int* run, cudaStream_t stream);
+
 // Fock-build contraction of one density set on `stream`: V[u*ldv + v] +=
 // sum over g with tab[u][g/blk] and tab[v][g/blk] of ao_lhs[u][g] w[g]
 // ao_rhs[v][g].  `workspace` holds fock_fp64_workspace(nao, ngrid) bytes,

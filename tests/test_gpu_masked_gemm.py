@@ -116,3 +116,47 @@ def test_large_masked_host_call_in_blocks(cm, wl, prec):
                              prec)
         torch.cuda.synchronize()
         assert np.array_equal(dc.cpu().numpy(), c)
+
+
+@pytest.mark.parametrize("transa,m,n,k,blk,density,pad", [
+    (False, 128, 256, 65, 32, 0.5, 0),     # one row tile
+    (False, 129, 257, 80, 32, 0.6, 0),     # one row past it; odd rows of B are copied
+    (True, 130, 130, 90, 64, 0.4, 0),      # A and B in place
+    (True, 131, 457, 133, 65, 0.4, 1),     # odd BLKSIZE, two pieces per block
+    (False, 40, 1400, 250, 200, 0.2, 2),   # five pieces of 40 columns
+    (False, 5, 33, 70, 48, 1.0, 0),        # a block wider than C, every tile present
+    (False, 300, 320, 96, 80, 0.0, 0),     # no tile present: C is untouched
+    (False, 128, 256, 64, 32, 0.5, 0),     # two K steps and one wave: the direct form
+    (False, 1000, 1600, 640, 33, 0.65, 0),  # both forms enqueued, compacted runs
+    (False, 1000, 1600, 640, 33, 0.9, 0),  # both forms enqueued, dense runs
+])
+def test_non0tab_compacted_rows_vs_dense(cm, wl, transa, m, n, k, blk, density, pad):
+    """Edges of the compacted form's tiles (128 rows, 16 list rows, pieces of up
+    to 64 columns) and its alignment cases; masked entries of B are nonzero, and
+    row strides are padded by `pad`.  Empty blocks leave C bit for bit."""
+    import torch
+    rng = np.random.default_rng(1000 * blk + n)
+    a = rng.uniform(-1, 1, (k, m + pad) if transa else (m, k + pad))
+    b = rng.uniform(-1, 1, (k, n + pad))
+    nblk = -(-n // blk)
+    tab = (rng.random((k, nblk)) < density).astype(np.uint8)
+    if density < 1.0:
+        tab[:, 0] = 0
+    if 0.0 < density < 1.0:  # lists of one row, of a full stage of 16, of one more
+        for blk_i, rows in zip(range(1, nblk), (1, 16, 17)):
+            tab[:, blk_i] = 0
+            tab[rng.choice(k, rows, replace=False), blk_i] = 1
+    c0 = rng.uniform(-1, 1, (m, n + pad))
+    bm = np.where(wl.expand_mask(tab, n, blk), b[:, :n], 0.0)
+    ref = c0.copy()
+    ref[:, :n] += (a[:, :m].T if transa else a[:, :k]) @ bm
+    t = lambda x: torch.from_numpy(x.copy()).cuda()
+    c = t(c0)
+    cm.matmul_non0tab_ex(c, t(a), t(b), m, n, k, a.shape[1], n + pad, n + pad, transa, False,
+                         t(tab), nblk, blk)
+    torch.cuda.synchronize()
+    c = c.cpu().numpy()
+    assert normwise(c, ref) < TOL
+    assert np.array_equal(c[:, n:], c0[:, n:])
+    if density < 1.0:
+        assert np.array_equal(c[:, :min(blk, n)], c0[:, :min(blk, n)])
