@@ -776,11 +776,10 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   const size_t o_pairs = o_items + a256(slots * sizeof(int4));
   const size_t o_ctr = o_pairs + a256(cnt_n * gsub * sizeof(int2));
   const size_t o_part = o_ctr + a256((nset_max + 2) * sizeof(int));  // + total, asymmetry flag
-  const size_t o_maps = o_part + a256(slots * nset_max * TG * sizeof(double));
   // split precision keeps only the active lists here (its own layout follows)
   const size_t bytes = precision == CFGMM_PREC_OZAKI_INT8
                            ? o_batch
-                           : o_maps + nbatch * sizeof(CUtensorMap);
+                           : o_part + slots * nset_max * TG * sizeof(double);
   cudaError_t err = cudaMallocAsync(&plan->mem, bytes, s);
   if (err != cudaSuccess) return cleanup(cuda_fail(err, "cudaMalloc(plan)"));
   char* base = static_cast<char*>(plan->mem);
@@ -819,6 +818,10 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   }
 
   // ---- 2. descriptors and the global work list, heaviest first ----
+  const bool pipe_ok = cfgmm::aodm_pipe_enabled();
+  // the half contraction needs D = D^T and, in every batch, phi_lhs = phi_rhs;
+  // a row tile then contracts the list from its own first column on
+  const bool sym = pipe_ok && cfgmm::aodm_sym_enabled() && same_phi(batches, nbatch);
   std::vector<cfgmm::AodmBatch> hb(nbatch);
   std::vector<int4> items;
   std::vector<int2> pairs;
@@ -842,16 +845,10 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   }
   std::stable_sort(items.begin(), items.end(),
                    [](const int4& x, const int4& y) { return x.w > y.w; });
-  // ao_rhs gather maps of the pipelined form (batches whose rows TMA cannot
-  // address are gathered by cp.async)
-  const bool pipe_ok = cfgmm::aodm_pipe_enabled();
-  std::vector<CUtensorMap> maps(nbatch);
-  std::memset(maps.data(), 0, nbatch * sizeof(CUtensorMap));
+  // ao_rhs rows by bulk copies where they are aligned, by cp.async otherwise
   for (size_t i = 0; i < nbatch && pipe_ok; ++i)
-    hb[i].rhs_tma = cfgmm::aodm_rhs_map(&maps[i], batches[i].ao_rhs, batches[i].stride_grid,
-                                        int(nao), int(batches[i].ngrid), int(blksize))
-                        ? 1
-                        : 0;
+    hb[i].rhs_bulk =
+        cfgmm::aodm_rhs_bulk(batches[i].ao_rhs, batches[i].stride_grid, int(blksize)) ? 1 : 0;
   plan->nitems = int(items.size());
   plan->npairs = int(pairs.size());
   plan->rpairs = reinterpret_cast<int2*>(base + o_pairs);
@@ -862,9 +859,6 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
                           cudaMemcpyHostToDevice, s);
   if (err == cudaSuccess && !pairs.empty())
     err = cudaMemcpyAsync(plan->rpairs, pairs.data(), pairs.size() * sizeof(int2),
-                          cudaMemcpyHostToDevice, s);
-  if (err == cudaSuccess && pipe_ok)
-    err = cudaMemcpyAsync(base + o_maps, maps.data(), nbatch * sizeof(CUtensorMap),
                           cudaMemcpyHostToDevice, s);
   if (err != cudaSuccess) return cleanup(cuda_fail(err, "plan upload"));
 
@@ -878,11 +872,8 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   a.max_utiles = max_ut;
   a.nset_max = int(nset_max);
   a.batches = reinterpret_cast<const cfgmm::AodmBatch*>(base + o_batch);
-  a.rhs_maps = pipe_ok ? reinterpret_cast<const CUtensorMap*>(base + o_maps) : nullptr;
   a.items = reinterpret_cast<const int4*>(base + o_items);
   a.counters = reinterpret_cast<int*>(base + o_ctr);
-  // the half contraction needs D = D^T and, in every batch, phi_lhs = phi_rhs
-  const bool sym = pipe_ok && cfgmm::aodm_sym_enabled() && same_phi(batches, nbatch);
   // reset, symmetry check of D, main kernel (the reduction follows in a run)
   auto launch = [&](const cfgmm::AodmConfig& c, cudaStream_t st) -> cudaError_t {
     a.asym = sym && c.tk == 0 ? a.counters + a.ngroups + 1 : nullptr;

@@ -27,7 +27,7 @@
 //      The active list of the current block is staged in shared memory, so
 //      the gather addresses never wait on global loads.
 //   3b. aodm_fp64_pipe_kernel: the same items with producer warps (D by
-//      cp.async; ao_rhs rows by TMA gather4 where the rows are 16-byte
+//      cp.async; ao_rhs rows by one bulk copy each where the rows are 16-byte
 //      aligned and BLKSIZE is even, by cp.async otherwise) and consumer warps
 //      (DMMA m16n8k8) meeting on mbarriers; with a symmetric-D mode.  The
 //      form used; form 3 remains for CFGMM_AODM_PIPE=0.
@@ -35,9 +35,6 @@
 //      fixed order, so results are deterministic run to run (unlike the
 //      reference, whose lock order varies).
 #include <cstdlib>
-#include <mutex>
-
-#include <cudaTypedefs.h>
 
 #include "common.cuh"
 #include "aodmao2rho_fp64.cuh"
@@ -338,9 +335,13 @@ __global__ void __launch_bounds__(THREADS, 1) aodm_fp64_kernel(AodmArgs p) {
 // 3b. pipelined main kernel: the same work items and partial sums as (3), with
 //     the roles split.  Four producer warps gather D_s[I_rows, I(k0..k0+15)]
 //     with 8-byte cp.async (lanes along consecutive compacted columns, so a
-//     warp's reads coalesce over the runs of active AOs) and one producer lane
-//     fetches the ao_rhs rows I(k0..k0+15) x 64 points with TMA gather4 (four
-//     arbitrary rows per instruction).  Both complete on the stage's mbarrier;
+//     warp's reads coalesce over the runs of active AOs) and sixteen producer
+//     lanes fetch the ao_rhs rows I(k0..k0+15) x 64 points, a bulk copy each,
+//     into rows of 68 doubles: a quarter warp's 16-byte fragment loads (rows
+//     k = q, points 2g and 2g + 1) then meet 8 distinct 16-byte bank groups.
+//     (Rows of 64 doubles laid down by TMA gather4 put all four k rows into the
+//     same banks: 55 M of the 101 M shared-load wavefronts of a taxol-size call
+//     were conflicts.)  Both complete on the stage's mbarrier;
 //     eight consumer warps run DMMA m16n8k8 from the stages and release them
 //     through a second mbarrier, so the gather of later stages -- and of the
 //     next work item -- overlaps the tensor-core work.  The roles meet only on
@@ -357,7 +358,8 @@ constexpr int NCONS = 256;     // consumer threads (8 warps, 2 x 4 over rows x p
 constexpr int PTHREADS = NPROD + NCONS;
 constexpr int RING = 4;        // work items in flight between the roles
 constexpr int D_BYTES = TU * TK * 8;      // one density matrix's tile per stage
-constexpr int PHI_BYTES = TK * TG * 8;    // ao_rhs rows, 64 points each, no swizzle
+constexpr int PHI_PITCH = TG + 4;          // ao_rhs row pitch (doubles), see above
+constexpr int PHI_BYTES = TK * PHI_PITCH * 8;
 constexpr int RSTEP = NPROD / TK;              // rows apart of one thread's gathers
 constexpr int ROWS_PER_THREAD = TU / RSTEP;     // 16
 
@@ -388,16 +390,6 @@ constexpr size_t smem_bytes() {
 __device__ __forceinline__ int d_off(int r, int k) {
   const int slot = ((k >> 3) << 2) | (k & 3);
   return r * TK + ((slot ^ swz_key(r)) << 1) + ((k >> 2) & 1);
-}
-
-__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, uint64_t* bar, int x,
-                                            int r0, int r1, int r2, int r3) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(tc::smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_u32(bar)), "r"(x), "r"(r0), "r"(r1),
-      "r"(r2), "r"(r3)
-      : "memory");
 }
 
 // The mbarrier tracks the completion of all cp.async this thread issued before.
@@ -436,6 +428,12 @@ __device__ __forceinline__ Item decode(const AodmArgs& p, int4 w, int set0) {
   return t;
 }
 
+// Point of the tile that accumulator column 2q + e of n8 tile nt holds, in the
+// consumer warps' point group wn.
+__device__ __forceinline__ int point_of(int wn, int nt, int q, int e) {
+  return wn * 8 * NT + (nt >> 1) * 16 + 4 * q + 2 * e + (nt & 1);
+}
+
 // Weight of D[u0 + r][u0 + c] in the diagonal tile of the symmetric mode.
 __device__ __forceinline__ double sym_factor(int r, int c) {
   return c < r ? 0.0 : (c == r ? 0.5 : 1.0);
@@ -451,8 +449,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* e
 
 template <int NS>
 __global__ void __launch_bounds__(pipe::PTHREADS, 1)
-aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
-                      const __grid_constant__ CUtensorMap rhs_map) {
+aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
   using namespace pipe;
   constexpr int SB = stage_bytes<NS>();
   extern __shared__ uint8_t pipe_smem_raw[];
@@ -476,7 +473,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
 
   if (tid == 0) {
     for (int s = 0; s < PSTAGES; ++s) {
-      tc::mbar_init(&full[s], NPROD + 1);     // NPROD cp.async arrivals + the TMA's expect_tx
+      tc::mbar_init(&full[s], NPROD + 1);     // NPROD cp.async arrivals + the bulk copies' expect_tx
       tc::mbar_init(&empty[s], NCONS / 32);   // one per consumer warp
     }
     for (int r = 0; r < RING; ++r) {
@@ -512,7 +509,11 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
       if (it >= total) break;
       const int4 w = p.items[it];
       const Item t = decode<NS>(p, w, set0);
-      const CUtensorMap* map = p.batches ? &p.rhs_maps[w.x] : &rhs_map;
+      // points of the tile that the table holds: none where a wide block's later
+      // tiles start past the grid's end; an odd number (the last tile of an odd
+      // grid) is no whole number of 16-byte pieces
+      const int pts = max(0, min(TG, t.B->ngrid - t.g0));
+      const bool bulk = t.B->rhs_bulk && pts % 2 == 0;
       int prow[ROWS_PER_THREAD];  // AO of each gathered row, -1 past the item's rows
 #pragma unroll
       for (int i = 0; i < ROWS_PER_THREAD; ++i) {
@@ -548,7 +549,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
             cp_async_8(dst + s * (D_BYTES / 8), valid ? src + s * p.dm_stride : src, valid);
         }
         uint8_t* phi = st + NS * D_BYTES;
-        if (!t.B->rhs_tma) {
+        if (!bulk) {
           // ao_rhs rows [TK][TG] by cp.async: lanes along points; the row of
           // stage column j comes from lane j of this warp (kcol = lane & 15)
           const int pt = tid & (TG - 1);
@@ -557,39 +558,35 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
           for (int i = 0; i < TK / (NPROD / TG); ++i) {
             const int j = (tid / TG) + (NPROD / TG) * i;
             const int row = __shfl_sync(0xffffffffu, v, j);
-            cp_async_8(reinterpret_cast<double*>(phi) + j * TG + pt,
+            cp_async_8(reinterpret_cast<double*>(phi) + j * PHI_PITCH + pt,
                        pv ? t.B->ao_rhs + size_t(row) * t.B->stride_grid + t.g0 + pt
                           : t.B->ao_rhs,
                        pv);
           }
         }
         cp_async_arrive_noinc(&full[stage]);
-        // test hook: the first stage's last arrival (the TMA's expect_tx, or
-        // its stand-in) is never made, so the consumers' bounded wait runs out
+        // test hook: the first stage's last arrival (the bulk copies' expect_tx,
+        // or its stand-in) is never made, so the consumers' bounded wait runs out
         const bool withhold = p.inject && fill == 0;
-        if (t.B->rhs_tma) {
+        if (bulk) {
           if (tid < 32 && !withhold) {
             // ao_rhs rows of the stage columns, from the lanes that gather them
-            // (lane j of warp 0 holds column j; D is zero past the list's end)
-            int rows[TK];
-#pragma unroll
-            for (int j = 0; j < TK; ++j) rows[j] = __shfl_sync(0xffffffffu, v, j);
-            if (tid == 0) {
-              tc::mbar_arrive_expect_tx(&full[stage], PHI_BYTES);
-#pragma unroll
-              for (int j = 0; j < TK / 4; ++j)
-                tma_gather4(phi + j * 4 * TG * 8, map, &full[stage], t.g0, rows[4 * j],
-                            rows[4 * j + 1], rows[4 * j + 2], rows[4 * j + 3]);
-            }
+            // (lane j < 16 of warp 0 holds column j; D is zero past the list's end)
+            if (tid == 0) tc::mbar_arrive_expect_tx(&full[stage], TK * pts * 8);
+            __syncwarp();
+            if (tid < TK && pts > 0)
+              tc::bulk_load(phi + tid * PHI_PITCH * 8,
+                            t.B->ao_rhs + size_t(v) * t.B->stride_grid + t.g0, pts * 8,
+                            &full[stage]);
           }
         } else if (tid == 0 && !withhold) {
-          tc::mbar_arrive(&full[stage]);  // the arrival the TMA's expect_tx makes otherwise
+          tc::mbar_arrive(&full[stage]);  // the arrival the expect_tx makes otherwise
         }
       }
     }
     cp_async_wait_all();
     if (tid == 0) {
-      // let every TMA this thread issued land before the CTA exits
+      // let every bulk copy of the CTA land before the CTA exits
       for (uint32_t f = fill > PSTAGES ? fill - PSTAGES : 0; f < fill; ++f)
         tc::mbar_wait(&full[f % PSTAGES], (f / PSTAGES) & 1, err, kErrTeardown, true, lim);
     }
@@ -611,7 +608,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
       const Item t = decode<NS>(p, p.items[it], set0);
 
       // the phi_lhs rows of this thread's epilogue (rows wm*16*MT + mt*16 + g + 8h,
-      // points wn*8*NT + nt*8 + 2q + e) are brought into L2 now, so that the
+      // points point_of(wn, nt, q, e)) are brought into L2 now, so that the
       // epilogue's loads hit while the tensor pipe waits for them
       int urow[MT][2];
 #pragma unroll
@@ -653,12 +650,14 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
         const bool diag = sym && kc < kc0 + TU / TK;
 #pragma unroll
         for (int kk = 0; kk < TK; kk += 8) {
-          double b0[NT], b1[NT];
+          // tiles 2j and 2j + 1 take the even and the odd points of a group of
+          // 16: column x of tile 2j + e is point 2x + e of the group
+          double2 b0[NT / 2], b1[NT / 2];
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            const int col = wn * 8 * NT + nt * 8 + g;
-            b0[nt] = phi[(kk + q) * TG + col];
-            b1[nt] = phi[(kk + q + 4) * TG + col];
+          for (int j = 0; j < NT / 2; ++j) {
+            const double* at = phi + (kk + q) * PHI_PITCH + wn * 8 * NT + j * 16 + 2 * g;
+            b0[j] = *reinterpret_cast<const double2*>(at);
+            b1[j] = *reinterpret_cast<const double2*>(at + 4 * PHI_PITCH);
           }
           const int slot8 = ((kk >> 3) << 2) | q;
 #pragma unroll
@@ -679,8 +678,10 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
                 hi.y *= sym_factor(r + 8, c + 4);
               }
 #pragma unroll
-              for (int nt = 0; nt < NT; ++nt)
-                dmma_16x8x8(acc[s][mt][nt], lo.x, hi.x, lo.y, hi.y, b0[nt], b1[nt]);
+              for (int j = 0; j < NT / 2; ++j) {
+                dmma_16x8x8(acc[s][mt][2 * j], lo.x, hi.x, lo.y, hi.y, b0[j].x, b1[j].x);
+                dmma_16x8x8(acc[s][mt][2 * j + 1], lo.x, hi.x, lo.y, hi.y, b0[j].y, b1[j].y);
+              }
             }
           }
         }
@@ -702,7 +703,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
           for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int j = wn * 8 * NT + nt * 8 + 2 * q + e;
+              const int j = point_of(wn, nt, q, e);
               lhs[mt][h][nt][e] = (row && j < t.gw) ? row[t.g0 + j] : 0.0;
             }
         }
@@ -722,7 +723,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p,
             v += __shfl_xor_sync(0xffffffffu, v, 4);
             v += __shfl_xor_sync(0xffffffffu, v, 8);
             v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (g == 0) rb[(s * CWM + wm) * TG + wn * 8 * NT + nt * 8 + 2 * q + e] = v;
+            if (g == 0) rb[(s * CWM + wm) * TG + point_of(wn, nt, q, e)] = v;
           }
       tc::mbar_arrive(&epi[n & 1]);
       // The buffer is written again two items later, after every consumer has
@@ -824,8 +825,7 @@ cudaError_t launch_main_t(const AodmArgs& a, cudaStream_t stream, bool attrs_onl
 }
 
 template <int NS>
-cudaError_t launch_pipe_t(const AodmArgs& a, const CUtensorMap& map, cudaStream_t stream,
-                          bool attrs_only) {
+cudaError_t launch_pipe_t(const AodmArgs& a, cudaStream_t stream, bool attrs_only) {
   constexpr size_t smem = pipe::smem_bytes<NS>();
   static_assert(smem <= 227 * 1024, "shared memory budget");
   cudaError_t err = cudaFuncSetAttribute(aodm_fp64_pipe_kernel<NS>,
@@ -835,22 +835,8 @@ cudaError_t launch_pipe_t(const AodmArgs& a, const CUtensorMap& map, cudaStream_
   if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
   if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return err;
-  aodm_fp64_pipe_kernel<NS><<<dim3(nsm, a.ngroups), pipe::PTHREADS, smem, stream>>>(a, map);
+  aodm_fp64_pipe_kernel<NS><<<dim3(nsm, a.ngroups), pipe::PTHREADS, smem, stream>>>(a);
   return cudaGetLastError();
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) ==
-            cudaSuccess &&
-        qr == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-  });
-  return fn;
 }
 
 // The pipelined form is used unless CFGMM_AODM_PIPE=0.
@@ -866,29 +852,16 @@ bool pipe_enabled() {
 
 bool aodm_pipe_enabled() { return pipe_enabled(); }
 
-bool aodm_rhs_map(CUtensorMap* map, const double* ao_rhs, size_t stride_grid, int nao, int ngrid,
-                  int blk) {
-  // TMA: 16-byte aligned base and row pitch; the x coordinate of every load
-  // (a 64-point tile start b*blk + 64*gt) must be even, so blk must be even.
-  if (nao <= 0 || ngrid <= 0 || blk % 2 != 0 ||
-      reinterpret_cast<uintptr_t>(ao_rhs) % 16 != 0 || (stride_grid * sizeof(double)) % 16 != 0)
-    return false;
-  auto enc = encode_tiled();
-  if (!enc) return false;
-  cuuint64_t dims[2] = {cuuint64_t(ngrid), cuuint64_t(nao)};
-  cuuint64_t strides[1] = {cuuint64_t(stride_grid) * sizeof(double)};
-  cuuint32_t box[2] = {cuuint32_t(TG), 1};  // gather4: one row per box, four rows per load
-  cuuint32_t estr[2] = {1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(ao_rhs), dims, strides,
-             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+bool aodm_rhs_bulk(const double* ao_rhs, size_t stride_grid, int blk) {
+  // every 64-point tile starts at the even point b*blk + 64*gt of a 16-byte
+  // aligned row
+  return blk % 2 == 0 && reinterpret_cast<uintptr_t>(ao_rhs) % 16 == 0 && stride_grid % 2 == 0;
 }
 
-cudaError_t aodm_launch_pipe(const AodmArgs& a, int ns, const CUtensorMap& map,
-                             cudaStream_t stream, bool attrs_only) {
-  if (ns == 1) return launch_pipe_t<1>(a, map, stream, attrs_only);
-  if (ns == 2) return launch_pipe_t<2>(a, map, stream, attrs_only);
-  if (ns == 3) return launch_pipe_t<3>(a, map, stream, attrs_only);
+cudaError_t aodm_launch_pipe(const AodmArgs& a, int ns, cudaStream_t stream, bool attrs_only) {
+  if (ns == 1) return launch_pipe_t<1>(a, stream, attrs_only);
+  if (ns == 2) return launch_pipe_t<2>(a, stream, attrs_only);
+  if (ns == 3) return launch_pipe_t<3>(a, stream, attrs_only);
   return cudaErrorInvalidValue;
 }
 
@@ -950,9 +923,8 @@ AodmConfig aodm_default_config(int nset) {
 
 cudaError_t aodm_launch_main(const AodmArgs& a, const AodmConfig& cfg, cudaStream_t stream,
                              bool attrs_only) {
-  if (cfg.tk == 0) {  // pipelined form over the batches' maps
-    if (!a.batches || !a.rhs_maps) return cudaErrorInvalidValue;
-    return aodm_launch_pipe(a, cfg.ns, CUtensorMap{}, stream, attrs_only);
+  if (cfg.tk == 0) {  // pipelined form
+    return aodm_launch_pipe(a, cfg.ns, stream, attrs_only);
   }
   if (cfg.tk == 32) {
     if (cfg.ns == 1) return launch_main_t<1, 32>(a, stream, attrs_only);
@@ -1058,9 +1030,8 @@ cudaError_t aodmao2rho_fp64(double* rhos, const double* dms, const double* ao_lh
   a.counters = counters;
   a.ngroups = ngroups;
   a.partial = partial;
-  CUtensorMap map{};
   if (pipe_enabled()) {
-    a.one.rhs_tma = aodm_rhs_map(&map, ao_rhs, stride_grid, nao, ngrid, blk) ? 1 : 0;
+    a.one.rhs_bulk = aodm_rhs_bulk(ao_rhs, stride_grid, blk) ? 1 : 0;
     // the half contraction needs D = D^T and phi_lhs = phi_rhs (one array)
     if (aodm_sym_enabled() && ao_lhs == ao_rhs) {
       a.asym = counters + ngroups + 1;
@@ -1073,7 +1044,7 @@ cudaError_t aodmao2rho_fp64(double* rhos, const double* dms, const double* ao_lh
       a.inject = 1;
       a.wait_ns = ns;
     }
-    err = aodm_launch_pipe(a, cfg.ns, map, stream);
+    err = aodm_launch_pipe(a, cfg.ns, stream);
   }
   else
     err = aodm_launch_main(a, cfg, stream);

@@ -2,7 +2,6 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace cfgmm {
@@ -18,7 +17,7 @@ struct AodmBatch {
   int ngrid;
   int nset;                // density matrices used by this batch (<= nset_max)
   long long partial_off;   // first partial-sum slot of this batch
-  int rhs_tma;             // pipelined form: ao_rhs rows by TMA (its map is valid), else cp.async
+  int rhs_bulk;            // pipelined form: ao_rhs rows by bulk copies, else cp.async
 };
 
 // Kernel arguments: density matrices shared by all batches, and either a
@@ -30,7 +29,6 @@ struct AodmArgs {
   int max_utiles;               // partial slots per (batch, block tile)
   int nset_max;
   const AodmBatch* batches;     // null: use `one`
-  const CUtensorMap* rhs_maps;  // with batches: ao_rhs gather map of each batch (pipelined form)
   AodmBatch one;
   const int4* items;            // work list: (batch, block tile, row tile, 0)
   int* counters;                // [ngroups] work counters, the item total, the asymmetry flag
@@ -51,8 +49,7 @@ bool take_wait_injection(int kind, unsigned long long* wait_ns);
 
 // Tile configuration of the main kernel (the autotuner's search space):
 // `ns` density matrices share one ao_rhs tile (1..3), `tk` compacted AOs per
-// pipeline stage of form 3 (16 or 32), or tk = 0 for the pipelined form
-// (which then takes the ao_rhs maps from AodmArgs::rhs_maps).
+// pipeline stage of form 3 (16 or 32), or tk = 0 for the pipelined form.
 struct AodmConfig {
   int ns;
   int tk;
@@ -94,18 +91,15 @@ cudaError_t aodm_launch_main(const AodmArgs& a, const AodmConfig& cfg, cudaStrea
 cudaError_t aodm_launch_reduce(const AodmArgs& a, const int2* rpairs, int npairs,
                                cudaStream_t stream);
 
-// Pipelined form of the main kernel (warp-specialised; ao_rhs rows by TMA
-// gather4 where AodmBatch::rhs_tma is set, by the producers' cp.async
-// otherwise).  aodm_rhs_map builds the gather map of one ao_rhs table and
-// returns false where TMA does not apply (base or row pitch not 16-byte
-// aligned, odd BLKSIZE).  `map` is used when a.batches is null, a.rhs_maps
-// (a 64-byte aligned device array, one map per batch) otherwise.
-// aodm_pipe_enabled() is false when CFGMM_AODM_PIPE=0 (form 3 then runs).
+// Pipelined form of the main kernel (warp-specialised; ao_rhs rows by bulk
+// copies where AodmBatch::rhs_bulk is set, by the producers' cp.async
+// otherwise).  aodm_rhs_bulk: whether bulk copies apply to a table (base and row
+// pitch 16-byte aligned, even BLKSIZE).  aodm_pipe_enabled() is false when
+// CFGMM_AODM_PIPE=0 (form 3 then runs).
 bool aodm_pipe_enabled();
-bool aodm_rhs_map(CUtensorMap* map, const double* ao_rhs, size_t stride_grid, int nao, int ngrid,
-                  int blk);
-cudaError_t aodm_launch_pipe(const AodmArgs& a, int ns, const CUtensorMap& map,
-                             cudaStream_t stream, bool attrs_only = false);
+bool aodm_rhs_bulk(const double* ao_rhs, size_t stride_grid, int blk);
+cudaError_t aodm_launch_pipe(const AodmArgs& a, int ns, cudaStream_t stream,
+                             bool attrs_only = false);
 // Code of the first timed-out wait of the pipelined kernel since the last
 // call's setup kernel (0: none).
 cudaError_t aodm_read_error(int* code);
