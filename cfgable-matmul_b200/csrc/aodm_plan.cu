@@ -837,7 +837,7 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
       for (int gt = 0; gt < gsub; ++gt) {
         const int bg = int(blk) * gsub + gt;
         if (nt > 0) pairs.push_back(make_int2(int(i), bg));
-        for (int u = 0; u < nt; ++u) items.push_back(make_int4(int(i), bg, u, nb));
+        for (int u = 0; u < nt; ++u) items.push_back(make_int4(int(i), bg, u, sym ? nb - u * TU : nb));
       }
       work += double(b.nset) * nb * nb;
     }

@@ -89,47 +89,67 @@ aodm_block_lists(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nbl
 
 // ---------------------------------------------------------------------------
 // 2. work list: items[i] = (0, b * gsub + gt, utile) for every row tile of every
-//    non-empty (block, grid tile), in block order; counters[g] = 0.
+//    non-empty (block, grid tile); counters[g] = 0.  The items come in order of
+//    the row tiles from theirs to the list's end, most first (within one number
+//    in no fixed order): in the symmetric mode an item's work is proportional
+//    to that number, so the last items drawn are the shortest and the SMs end
+//    together.  In block order a taxol-size call's SMs were busy 93 % of the
+//    kernel's time, the longest items (129 k cycles) starting at any point.
+//    Every item has its own partial-sum slot, so the order changes no result.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
 aodm_build_items(const int* __restrict__ counts, int nblk, int gsub, int4* __restrict__ items,
                  int* __restrict__ counters, int ncounters) {
+  constexpr int RANKS = 1024;           // longer lists share the first rank
+  __shared__ int start[RANKS + 1];      // by tiles left: blocks, then the next free item
   __shared__ int warp_tot[32];
-  __shared__ int base_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    base_s = 0;
-    g_aodm_error = 0;
-  }
+  if (tid == 0) g_aodm_error = 0;
   // [ncounters] = total, [ncounters + 1] = asymmetry flag
   for (int i = tid; i <= ncounters + 1; i += 1024) counters[i] = 0;
+  for (int r = tid; r <= RANKS; r += 1024) start[r] = 0;
   __syncthreads();
-  for (int b0 = 0; b0 < nblk; b0 += 1024) {
-    const int b = b0 + tid;
-    const int nt = (b < nblk) ? (counts[b] + TU - 1) / TU : 0;
-    const int mine = nt * gsub;
-    // block-wide exclusive scan of `mine`
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    int before = base_s;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    before += incl - mine;
-    for (int j = 0; j < mine; ++j) items[before + j] = make_int4(0, b * gsub + j / nt, j % nt, 0);
-    __syncthreads();
-    if (tid == 0) {
-      int t = 0;
-      for (int w = 0; w < 32; ++w) t += warp_tot[w];
-      base_s += t;
-    }
-    __syncthreads();
+  // items with r tiles left: one of every block with at least r of them; rank
+  // RANKS takes all above it too
+  for (int b = tid; b < nblk; b += 1024) {
+    const int nt = (counts[b] + TU - 1) / TU;
+    if (nt > 0) atomicAdd(&start[min(nt, RANKS)], 1);
   }
-  if (tid == 0) counters[ncounters] = base_s;
+  __syncthreads();
+  // thread t: rank RANKS - t, scanned from the highest rank down
+  const int rank = RANKS - tid;
+  int blocks = start[rank];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, blocks, o);
+    if (lane >= o) blocks += v;
+  }
+  if (lane == 31) warp_tot[warp] = blocks;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) blocks += warp_tot[w];  // blocks with >= rank tiles
+  int mine = blocks;
+  if (tid == 0)  // rank RANKS: every tile from the RANKS-th on
+    for (int b = 0; mine && b < nblk; ++b) mine += max(0, (counts[b] + TU - 1) / TU - RANKS);
+  int incl = mine;
+  __syncthreads();
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) incl += warp_tot[w];
+  start[rank] = (incl - mine) * gsub;
+  if (tid == 1023) counters[ncounters] = incl * gsub;  // rank 1: the total
+  __syncthreads();
+  for (int b = tid; b < nblk; b += 1024) {
+    const int nt = (counts[b] + TU - 1) / TU;
+    for (int u = 0; u < nt; ++u) {
+      const int at = atomicAdd(&start[min(nt - u, RANKS)], gsub);
+      for (int gt = 0; gt < gsub; ++gt) items[at + gt] = make_int4(0, b * gsub + gt, u, 0);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -77,7 +77,7 @@ cudaError_t aodm_block_lists_launch(const uint8_t* tab, size_t ldtab, int nao, i
                                     int* lists, int* counts, cudaStream_t stream);
 
 // Work list of one grid batch: items[i] = (0, block tile, row tile of 64 active
-// AOs, 0) in block order; counters[0..ncounters) = 0, counters[ncounters] = the
+// AOs, 0), those with the most row tiles of their list left first; counters[0..ncounters) = 0, counters[ncounters] = the
 // item count, counters[ncounters + 1] = 0.
 cudaError_t aodm_build_items_launch(const int* counts, int nblk, int gsub, int4* items,
                                     int* counters, int ncounters, cudaStream_t stream);
