@@ -215,20 +215,23 @@ int check_split_gemm(size_t k) {
 
 // Reads the sticky error words of the tcgen05 kernels after a synchronised call.
 int check_device_waits() {
-  int code = 0, code2 = 0, code3 = 0, code4 = 0;
+  int code = 0, code2 = 0, code3 = 0, code4 = 0, code5 = 0;
   CFGMM_CUDA(cfgmm::gemm_i8_read_error(&code));
   CFGMM_CUDA(cfgmm::aodmao2rho_split_read_error(&code2));
   CFGMM_CUDA(cfgmm::dgemm_read_error(&code3));
   CFGMM_CUDA(cfgmm::aodm_read_error(&code4));
+  CFGMM_CUDA(cfgmm::fock_read_error(&code5));
   if (code == 0) code = code2;
   if (code == 0) code = code3;
   if (code == 0) code = code4;
+  if (code == 0) code = code5;
   if (code != 0) {
     // reported once: the words start over for the next call
     cudaError_t e = cfgmm::gemm_i8_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::aodmao2rho_split_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::dgemm_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::aodm_reset_error(nullptr);
+    if (e == cudaSuccess) e = cfgmm::fock_reset_error(nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "resetting the device wait words");
     char msg[128];

@@ -412,14 +412,6 @@ __device__ __forceinline__ int d_off(int r, int k) {
   return r * TK + ((slot ^ swz_key(r)) << 1) + ((k >> 2) & 1);
 }
 
-// The mbarrier tracks the completion of all cp.async this thread issued before.
-__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // wait-site codes recorded in g_aodm_error
 enum : int { kErrItemEmpty = 0x4101, kErrItemFull, kErrStageEmpty, kErrStageFull, kErrEpilogue,
              kErrTeardown };
@@ -584,7 +576,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
                        pv);
           }
         }
-        cp_async_arrive_noinc(&full[stage]);
+        tc::cp_async_arrive_noinc(&full[stage]);
         // test hook: the first stage's last arrival (the bulk copies' expect_tx,
         // or its stand-in) is never made, so the consumers' bounded wait runs out
         const bool withhold = p.inject && fill == 0;
@@ -604,7 +596,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
         }
       }
     }
-    cp_async_wait_all();
+    tc::cp_async_wait_all();
     if (tid == 0) {
       // let every bulk copy of the CTA land before the CTA exits
       for (uint32_t f = fill > PSTAGES ? fill - PSTAGES : 0; f < fill; ++f)

@@ -5,48 +5,59 @@
 // the transpose of the AO-DM-AO contraction (aodmao2rho_fp64.cu) on its layouts
 // and mask: where that one gathers D[I(b), I(b)] as an input, this one scatters
 // V[I(b), I(b)] as an output.  Work item = (block, 64-point tile, 64 rows of the
-// active list I(b)) for one weight vector w_s, the same items as the AO-DM-AO
-// kernels.  The CTA stages A = phi_lhs[I rows, tile] diag(w_s) once, walks the
-// compacted columns in chunks of 64 (phi_rhs rows by 8-byte cp.async into a
-// double buffer), forms the 64 x 64 product over the 64 points on DMMA
-// m16n8k8 and adds it into V[I rows][I chunk] with FP64 atomics (red.add): the
-// same (u, v) receives one addition per block in which both are active.  Only
-// the masked products are formed (a dense product over all AO pairs runs ~10x
-// their number on the taxol-size mask).  When phi_lhs and phi_rhs are the same
-// array the block's contribution is symmetric in (u, v): row tile a then walks
-// the chunks from its own (chunk a) on and adds each product of a later chunk
-// to V[u][v] and V[v][u], half the products.  Sums over blocks arrive in
-// completion order, so the last bits of V vary from run to run.
+// active list I(b)) for up to 4 weight vectors w_s, the same items as the
+// AO-DM-AO kernels.  Only the masked products are formed (a dense product over
+// all AO pairs runs ~10x their number on the taxol-size mask).  When phi_lhs and
+// phi_rhs are the same array the block's contribution is symmetric in (u, v):
+// row tile a then walks the chunks from its own (chunk a) on and adds each
+// product of a later chunk to V[u][v] and V[v][u], half the products.  Sums over
+// blocks arrive in completion order, so the last bits of V vary from run to run.
+//
+// One producer warp and eight consumer warps per CTA, two CTAs per SM:
+//   * The producer fetches the item's 64 rows of phi_lhs and its weights once,
+//     then the compacted columns in chunks of 64 rows of phi_rhs into a ring of
+//     two, one bulk copy per row (8-byte cp.async where the rows are not 16-byte
+//     aligned).  The columns serve all weight vectors of the item.
+//   * Consumer warps (16 rows x 32 columns each) multiply the weights into the
+//     phi_lhs fragments, run DMMA m16n8k8 over the tile's points and add the
+//     products into V with FP64 atomics (red.add), each warp at its own pace: a
+//     warp's atomics overlap the others' DMMAs.
+//   * The 16 x 8 fragments are permuted so that a warp's atomics fall into few
+//     32-byte sectors: row (column) x of a tile stands for row (column)
+//     4 (x % 2) + x / 2 of its 8, and one exchange between lane pairs turns 8
+//     rows x 4 columns per instruction into 4 rows x 8 adjacent list columns.
+//     A model of the sectors at taxol size: 193 M -> 139 M per call.
+//   * Warps whose rows or columns lie past the list's end, and those below the
+//     diagonal in the symmetric mode's diagonal tile, skip their products.
+// Measured at 2228 AOs x 16384 points x 3 weight vectors (symmetric mode): 1.03 ms;
+// 1.52 ms with chunks copied by the computing warps behind CTA barriers, one
+// weight vector per item and unpermuted atomics; 1.12 ms before the skips.  What
+// bounds it: the FP64 tensor pipe (DMMA; its floor is 0.6 ms), then the L2's atomic
+// units (without the atomics the kernel takes 0.15 ms less).
+#include <type_traits>
+
 #include "common.cuh"
 #include "aodmao2rho_fp64.cuh"
 #include "fock.cuh"
+#include "tcgen05.cuh"
 
 namespace cfgmm {
 namespace {
 
-constexpr int FT = 64;         // rows per item = columns per chunk = points per tile
-constexpr int THREADS = 256;   // 8 warps: 4 along rows (16 each) x 2 along columns (32 each)
-constexpr int TILE = FT * FT;  // doubles per staged tile
+__device__ int g_fock_error;
 
-// Offset (doubles) of element (row, point k) of a 64 x 64 tile: the 16-byte slot
-// k/2 of a row holds points k and k+1, contiguous in phi, so one 16-byte copy
-// fills it; the slots of a row are XOR-swizzled by swz_key(row), so a fragment
-// load's phases of 8 lanes meet 8 distinct slots.  A k step of 8 points gives
-// the m16n8k8 index j (0..3) the points 2j and 2j+1 as its k = j and k = j + 4,
-// on both operands alike: the products summed are the same, and a fragment
-// pair (a0, a2) of A (rows = u) or (b0, b1) of B (rows = v) is one 16-byte load.
-__device__ __forceinline__ int f_off(int r, int k) {
-  return r * FT + (((k >> 1) ^ swz_key(r)) << 1) + (k & 1);
-}
-
-// 16-byte asynchronous copy of which the first `bytes` (0, 8 or 16) are read
-// from `src`; the rest of the destination is zero-filled.
-__device__ __forceinline__ void cp_async_16_n(void* smem_dst, const void* gmem_src, int bytes) {
-  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem_src),
-               "r"(bytes)
-               : "memory");
-}
+constexpr int FT = 64;        // rows per item = columns per chunk = points per tile
+constexpr int CONS = 8;       // consumer warps: 4 along rows (16 each) x 2 along columns (32 each)
+constexpr int THREADS = 32 * (CONS + 1);
+constexpr int NS = 4;         // weight vectors per item at most
+constexpr int STAGES = 2;     // chunks of phi_rhs in flight
+// Row pitch of a staged tile (doubles): 33 16-byte groups, so the 8 lanes of a
+// quarter warp's fragment load (rows r and r + 4, point pairs q = 0..3) meet 8
+// distinct groups modulo 8.
+constexpr int PITCH = FT + 2;
+constexpr int TILE = FT * PITCH;
+constexpr size_t FOCK_SMEM =
+    (size_t(1 + STAGES) * TILE + NS * FT) * 8 + (2 + 2 * STAGES) * 8 + 8 * sizeof(int);
 
 struct FockArgs {
   double* v;
@@ -57,151 +68,281 @@ struct FockArgs {
   size_t stride_grid;
   const int* lists;  // [nblk][nao]
   const int* counts;
-  int nao, ngrid, blk, gsub;
+  int nao, ngrid, nset, blk, gsub;
   int sym;  // ao_lhs == ao_rhs: chunks from the row tile's own on, mirrored
-  int vec;  // phi rows and w 16-byte aligned at every tile: pairs of points per copy
+  int vec;  // phi rows and w 16-byte aligned at every tile
   const int4* items;
-  int* counters;  // [nset] work counters, [nset] = item total
+  int* counters;  // [groups] work counters, [groups] = item total
+};
+
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int code) {
+  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_fock_error, code));
+}
+
+// One item as the producer decodes it for the consumers; bg < 0: no more items.
+struct FockItem {
+  int bg, nb, u0, gw, b;
 };
 
 __global__ void __launch_bounds__(THREADS, 2)
 fock_compact_kernel(const __grid_constant__ FockArgs p) {
-  __shared__ __align__(16) double As[TILE];
-  extern __shared__ __align__(16) double Bs[];  // [2][TILE]
-  __shared__ int item_s;
-  const int set = blockIdx.y;
+  extern __shared__ __align__(128) double fock_smem[];
+  double* As = fock_smem;                 // [64][PITCH] phi_lhs rows
+  double* Bs = As + TILE;                 // [STAGES][64][PITCH] phi_rhs rows
+  double* Ws = Bs + STAGES * TILE;        // [NS][64]
+  uint64_t* afull = reinterpret_cast<uint64_t*>(Ws + NS * FT);
+  uint64_t* aempty = afull + 1;
+  uint64_t* full = aempty + 1;            // [STAGES]
+  uint64_t* empty = full + STAGES;        // [STAGES]
+  FockItem* item = reinterpret_cast<FockItem*>(empty + STAGES);
+
+  const int set0 = blockIdx.y * NS;
+  const int ns = min(NS, p.nset - set0);
   const int total = p.counters[gridDim.y];
-  int* counter = p.counters + set;
-  const double* w = p.w + size_t(set) * p.stride_grid;
-  double* V = p.v + size_t(set) * p.v_stride;
-
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int g = lane >> 2, q = lane & 3;
-
-  for (;;) {
-    if (tid == 0) item_s = atomicAdd(counter, 1);
-    __syncthreads();  // also: the previous item's last reads of As / Bs are done
-    const int it = item_s;
-    if (it >= total) break;
-    const int4 wi = p.items[it];
-    const int bg = wi.y, a = wi.z;
-    const int b = bg / p.gsub, gt = bg % p.gsub;
-    const int nb = p.counts[b];
-    const int* I = p.lists + size_t(b) * p.nao;
-    const int u0 = a * FT;
-    const int mu = min(FT, nb - u0);
-    const int g0 = b * p.blk + gt * FT;
-    const int gw = min(min((b + 1) * p.blk, p.ngrid), g0 + FT) - g0;
-
-    auto issue = [&](int ch) {
-      double* B = Bs + (ch & 1) * TILE;
-      const int c0 = ch * FT;
-      if (p.vec) {
-        // one 16-byte copy per pair of points; a pair past ngrid is zero-filled
-        // (one of its points, or both)
-#pragma unroll
-        for (int e = tid; e < TILE / 2; e += THREADS) {
-          const int c = e >> 5, k = 2 * (e & 31);
-          const int left = p.ngrid - (g0 + k);
-          const int bytes = c0 + c < nb ? (left >= 2 ? 16 : (left == 1 ? 8 : 0)) : 0;
-          const double* src =
-              bytes ? p.ao_rhs + size_t(I[c0 + c]) * p.stride_grid + g0 + k : p.ao_rhs;
-          cp_async_16_n(B + f_off(c, k), src, bytes);
-        }
-      } else {
-#pragma unroll 4
-        for (int e = tid; e < TILE; e += THREADS) {
-          const int c = e >> 6, k = e & 63;
-          const bool valid = c0 + c < nb && g0 + k < p.ngrid;
-          const double* src =
-              valid ? p.ao_rhs + size_t(I[c0 + c]) * p.stride_grid + g0 + k : p.ao_rhs;
-          cp_async_8(B + f_off(c, k), src, valid);
-        }
-      }
-      cp_async_commit();
-    };
-    const int nch = (nb + FT - 1) / FT;
-    const int ch0 = p.sym ? a : 0;
-    issue(ch0);  // the first chunk's copies fly while A is staged
-    // A = phi_lhs[I[u0 + r]][g0 + k] * w[g0 + k], zero past the rows and points
-    if (p.vec) {
-      // pairs of points (k even): the partner of the tile's last point lies
-      // inside the row (stride_grid is even, so ngrid < stride_grid when odd)
-#pragma unroll
-      for (int e = tid; e < TILE / 2; e += THREADS) {
-        const int r = e >> 5, k = 2 * (e & 31);
-        double2 x = make_double2(0.0, 0.0);
-        if (r < mu && k < gw) {
-          const double2 f = *reinterpret_cast<const double2*>(
-              p.ao_lhs + size_t(I[u0 + r]) * p.stride_grid + g0 + k);
-          const double2 ww = *reinterpret_cast<const double2*>(w + g0 + k);
-          x.x = f.x * ww.x;
-          if (k + 1 < gw) x.y = f.y * ww.y;
-        }
-        *reinterpret_cast<double2*>(As + f_off(r, k)) = x;
-      }
-    } else {
-#pragma unroll 4
-      for (int e = tid; e < TILE; e += THREADS) {
-        const int r = e >> 6, k = e & 63;
-        double x = 0.0;
-        if (r < mu && k < gw)
-          x = p.ao_lhs[size_t(I[u0 + r]) * p.stride_grid + g0 + k] * w[g0 + k];
-        As[f_off(r, k)] = x;
-      }
+  if (tid == 0) {
+    // the producer's 32 lanes and one more arrival: the bulk copies' expect_tx
+    tc::mbar_init(afull, 33);
+    tc::mbar_init(aempty, CONS);
+    for (int s = 0; s < STAGES; ++s) {
+      tc::mbar_init(&full[s], 33);
+      tc::mbar_init(&empty[s], CONS);
     }
-    const int r_lo = wm * 16 + g, r_hi = r_lo + 8;
-    const int u_lo = r_lo < mu ? I[u0 + r_lo] : -1;
-    const int u_hi = r_hi < mu ? I[u0 + r_hi] : -1;
-    for (int ch = ch0; ch < nch; ++ch) {
-      if (ch + 1 < nch) {
-        issue(ch + 1);
-        cp_async_wait<1>();
+    tc::mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (warp == CONS) {
+    // ------------------------------- producer -------------------------------
+    int* counter = p.counters + blockIdx.y;
+    int it = 0;
+    if (lane == 0) it = atomicAdd(counter, 1);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    int fill = 0, n = 0;
+    bool ok = true;
+    // rows lane and lane + 32 of `rows` table rows (lane r, r + 32: AOs v0, v1)
+    // into a staged tile: `gw` points from g0, none past the rows
+    auto rows_in = [&](double* dst, const double* ao, int v0, int v1, int rows, int g0, int gw,
+                       uint64_t* bar, bool bulk, uint32_t extra) {
+      if (bulk) {
+        if (lane == 0) tc::mbar_arrive_expect_tx(bar, uint32_t(rows) * gw * 8 + extra);
+        __syncwarp();
+        if (lane < rows)
+          tc::bulk_load(dst + lane * PITCH, ao + size_t(v0) * p.stride_grid + g0, gw * 8, bar);
+        if (lane + 32 < rows)
+          tc::bulk_load(dst + (lane + 32) * PITCH, ao + size_t(v1) * p.stride_grid + g0, gw * 8,
+                        bar);
       } else {
-        cp_async_wait<0>();
+        for (int r = 0; r < rows; ++r) {
+          const int v = __shfl_sync(0xffffffffu, r < 32 ? v0 : v1, r & 31);
+          const double* src = ao + size_t(v) * p.stride_grid + g0;
+#pragma unroll
+          for (int k = lane; k < FT; k += 32)
+            cp_async_8(dst + r * PITCH + k, k < gw ? src + k : ao, k < gw);
+        }
+        if (lane == 0) tc::mbar_arrive(bar);  // in the expect_tx's place
       }
-      __syncthreads();  // chunk ch (and A) visible to every warp
-      const double* B = Bs + (ch & 1) * TILE;
-      double acc[4][4];
+    };
+    while (ok && it < total) {
+      int next = 0;  // drawn now, needed after this item's copies
+      if (lane == 0) next = atomicAdd(counter, 1);
+      const int4 wi = p.items[it];
+      const int b = wi.y / p.gsub, gt = wi.y % p.gsub, a = wi.z;
+      const int nb = p.counts[b];
+      const int* I = p.lists + size_t(b) * p.nao;
+      const int u0 = a * FT, mu = min(FT, nb - u0);
+      const int g0 = b * p.blk + gt * FT;
+      const int gw = min(min((b + 1) * p.blk, p.ngrid), g0 + FT) - g0;
+      if (gw > 0) {  // a wide block's later tiles may start past the grid's end
+        const bool bulk = p.vec && gw % 2 == 0;
+        const int nch = (nb + FT - 1) / FT, ch0 = p.sym ? a : 0;
+        const int ua = I[min(u0 + lane, nb - 1)], ub = I[min(u0 + lane + 32, nb - 1)];
+        int va = I[min(ch0 * FT + lane, nb - 1)], vb = I[min(ch0 * FT + lane + 32, nb - 1)];
+        for (int ch = ch0; ch < nch && ok; ++ch, ++fill) {
+          const int v0 = va, v1 = vb, c1 = (ch + 1) * FT + lane;
+          va = I[min(c1, nb - 1)];
+          vb = I[min(c1 + 32, nb - 1)];
+          const int s = fill % STAGES;
+          if (fill >= STAGES && !wait_all(&empty[s], ((fill / STAGES) - 1) & 1, 0x6101)) {
+            ok = false;
+            break;
+          }
+          rows_in(Bs + s * TILE, p.ao_rhs, v0, v1, min(FT, nb - ch * FT), g0, gw, &full[s], bulk,
+                  0);
+          if (bulk)
+            tc::mbar_arrive(&full[s]);
+          else
+            tc::cp_async_arrive_noinc(&full[s]);
+          if (ch == ch0) {  // the item's own rows, behind its first chunk
+            if (n > 0 && !wait_all(aempty, (n - 1) & 1, 0x6102)) {
+              ok = false;
+              ++fill;
+              break;
+            }
+            if (lane == 0) *item = FockItem{wi.y, nb, u0, gw, b};
+            rows_in(As, p.ao_lhs, ua, ub, mu, g0, gw, afull, bulk, uint32_t(ns) * gw * 8);
+            if (bulk) {
+              if (lane < ns)
+                tc::bulk_load(Ws + lane * FT, p.w + size_t(set0 + lane) * p.stride_grid + g0,
+                              gw * 8, afull);
+              tc::mbar_arrive(afull);
+            } else {
+              for (int s2 = 0; s2 < ns; ++s2)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[nt][e] = 0.0;
-#pragma unroll
-      for (int kk = 0; kk < FT; kk += 8) {
-        const int slot = ((kk >> 3) << 2) | q;
-        const double2 lo =
-            *reinterpret_cast<const double2*>(As + r_lo * FT + ((slot ^ swz_key(r_lo)) << 1));
-        const double2 hi =
-            *reinterpret_cast<const double2*>(As + r_hi * FT + ((slot ^ swz_key(r_hi)) << 1));
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const int c = wn * 32 + nt * 8 + g;
-          const double2 bv =
-              *reinterpret_cast<const double2*>(B + c * FT + ((slot ^ swz_key(c)) << 1));
-          dmma_16x8x8(acc[nt], lo.x, hi.x, lo.y, hi.y, bv.x, bv.y);
+                for (int k = lane; k < FT; k += 32)
+                  cp_async_8(Ws + s2 * FT + k,
+                             k < gw ? p.w + size_t(set0 + s2) * p.stride_grid + g0 + k : p.w,
+                             k < gw);
+              tc::cp_async_arrive_noinc(afull);
+            }
+            ++n;
+          }
         }
       }
-      // V[u][v] += the chunk's products (and V[v][u] past the diagonal tile)
-      const int c0 = ch * FT;
-      const bool mirror = p.sym && ch != a;
+      it = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (ok && (n == 0 || wait_all(aempty, (n - 1) & 1, 0x6102))) {  // the end mark
+      if (lane == 0) {
+        item->bg = -1;
+        tc::mbar_arrive(afull);
+      }
+      __syncwarp();
+      tc::mbar_arrive(afull);
+      ++n;
+    }
+    // every copy lands before the CTA exits
+    tc::cp_async_wait_all();
+    if (lane == 0) {
+      for (int f = max(0, fill - STAGES); f < fill; ++f)
+        tc::mbar_wait(&full[f % STAGES], (f / STAGES) & 1, &g_fock_error, 0x6105, true);
+      if (n > 0) tc::mbar_wait(afull, (n - 1) & 1, &g_fock_error, 0x6106, true);
+    }
+    return;
+  }
+
+  // ------------------------------- consumers -------------------------------
+  const int wm = warp >> 1;
+  const int g = lane >> 2, q = lane & 3;
+  const int rg = 4 * (g & 1) + (g >> 1);  // row (column) of its 8 that index g stands for
+  const bool odd = g & 1;
+  const int r_lo = wm * 16 + rg;
+  int use = 0;
+  for (int n = 0;; ++n) {
+    if (!wait_all(afull, n & 1, 0x6103)) break;
+    const FockItem t = *item;
+    if (t.bg < 0) break;
+    // the columns' halves change sides with every item: the warps that have less
+    // to do (a list's ragged end, the diagonal tile) are not always on the same
+    // two of the SM's four schedulers
+    const int wn = (warp ^ n) & 1;
+    const int* I = p.lists + size_t(t.b) * p.nao;
+    // this lane's rows (u), and those of its pair of lanes (g even, g odd)
+    int u_own[2], u_ev[2], u_od[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = t.u0 + r_lo + 8 * h;
+      u_own[h] = r < t.nb ? I[r] : -1;
+      u_ev[h] = __shfl_sync(0xffffffffu, u_own[h], lane & ~4);
+      u_od[h] = __shfl_sync(0xffffffffu, u_own[h], lane | 4);
+    }
+    const int ksteps = (t.gw + 7) / 8;
+    const int nch = (t.nb + FT - 1) / FT, a = t.u0 / FT, ch0 = p.sym ? a : 0;
+    const double* A = As + r_lo * PITCH + 2 * q;
+    bool ok = true;
+    for (int ch = ch0; ch < nch; ++ch, ++use) {
+      // in the symmetric mode's diagonal tile the products of rows 32..63 with
+      // columns 0..31 are those of rows 0..31 with columns 32..63, mirrored
+      const bool diag = p.sym && ch == a;
+      const bool mirror = p.sym && (!diag || (wm < 2 && wn == 1));
+      const int cols = t.nb - (ch * FT + wn * 32);  // of the list, in this warp's 32
+      const bool idle = cols <= 0 || t.u0 + wm * 16 >= t.nb || (diag && wm >= 2 && wn == 0);
+      // list columns of accumulator columns 2q + e of n8 tile nt: e * 4 + q
+      int vc[4][2];
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = c0 + wn * 32 + nt * 8 + 2 * q + e;
-          if (c >= nb) continue;
-          const size_t vcol = size_t(I[c]);
-          if (u_lo >= 0) atomicAdd(V + size_t(u_lo) * p.stride_ao + vcol, acc[nt][e]);
-          if (u_hi >= 0) atomicAdd(V + size_t(u_hi) * p.stride_ao + vcol, acc[nt][2 + e]);
-          if (mirror) {
-            if (u_lo >= 0) atomicAdd(V + vcol * p.stride_ao + u_lo, acc[nt][e]);
-            if (u_hi >= 0) atomicAdd(V + vcol * p.stride_ao + u_hi, acc[nt][2 + e]);
+          const int c = nt * 8 + 4 * e + q;
+          vc[nt][e] = !idle && c < cols ? I[ch * FT + wn * 32 + c] : -1;
+        }
+      const int s = use % STAGES;
+      if (!wait_all(&full[s], (use / STAGES) & 1, 0x6104)) {
+        ok = false;
+        break;
+      }
+      const double* B = Bs + s * TILE + (wn * 32 + rg) * PITCH + 2 * q;
+      auto release = [&] {  // the staged rows are read (the item's own with its last chunk)
+        __syncwarp();
+        if (lane == 0) {
+          tc::mbar_arrive(&empty[s]);
+          if (ch == nch - 1) tc::mbar_arrive(aempty);
+        }
+      };
+      // the products of the warp's 16 rows with its first 8 ntv columns, into V
+      auto products = [&](auto ntv) {
+        constexpr int N8 = decltype(ntv)::value;
+        for (int set = 0; set < ns; ++set) {
+          const double* W = Ws + set * FT + 2 * q;
+          double acc[N8][4];
+#pragma unroll
+          for (int nt = 0; nt < N8; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[nt][e] = 0.0;
+#pragma unroll 4
+          for (int ks = 0; ks < ksteps; ++ks) {
+            const double2 w = *reinterpret_cast<const double2*>(W + ks * 8);
+            double2 lo = *reinterpret_cast<const double2*>(A + ks * 8);
+            double2 hi = *reinterpret_cast<const double2*>(A + 8 * PITCH + ks * 8);
+            double2 bv[N8];
+#pragma unroll
+            for (int nt = 0; nt < N8; ++nt)
+              bv[nt] = *reinterpret_cast<const double2*>(B + nt * 8 * PITCH + ks * 8);
+            lo.x *= w.x;
+            lo.y *= w.y;
+            hi.x *= w.x;
+            hi.y *= w.y;
+            if (ks * 8 + 8 > t.gw && ks * 8 + 2 * q >= t.gw) {  // points past the tile's end
+              lo = hi = make_double2(0.0, 0.0);
+#pragma unroll
+              for (int nt = 0; nt < N8; ++nt) bv[nt] = make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int nt = 0; nt < N8; ++nt)
+              dmma_16x8x8(acc[nt], lo.x, hi.x, lo.y, hi.y, bv[nt].x, bv[nt].y);
+          }
+          if (set == ns - 1) release();
+          // V[u][v] += the products, and V[v][u] where they stand for both
+          double* V = p.v + size_t(set0 + set) * p.v_stride;
+#pragma unroll
+          for (int nt = 0; nt < N8; ++nt) {
+            const int vd = odd ? vc[nt][1] : vc[nt][0];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const double x0 = acc[nt][2 * h], x1 = acc[nt][2 * h + 1];
+              // lane pair (g, g ^ 1): the even row's 8 columns, then the odd row's
+              const double other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 4);
+              if (vd >= 0) {
+                if (u_ev[h] >= 0)
+                  atomicAdd(V + size_t(u_ev[h]) * p.stride_ao + vd, odd ? other : x0);
+                if (u_od[h] >= 0)
+                  atomicAdd(V + size_t(u_od[h]) * p.stride_ao + vd, odd ? x1 : other);
+              }
+              if (mirror && u_own[h] >= 0) {
+                if (vc[nt][0] >= 0) atomicAdd(V + size_t(vc[nt][0]) * p.stride_ao + u_own[h], x0);
+                if (vc[nt][1] >= 0) atomicAdd(V + size_t(vc[nt][1]) * p.stride_ao + u_own[h], x1);
+              }
+            }
           }
         }
-      __syncthreads();  // chunk ch's buffer is refilled by chunk ch + 2
+      };
+      if (idle)
+        release();
+      else if (cols > 16)
+        products(std::integral_constant<int, 4>());
+      else
+        products(std::integral_constant<int, 2>());
     }
+    if (!ok) break;
   }
 }
 
@@ -246,7 +387,8 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   int* counters = reinterpret_cast<int*>(wsp + L.counters);
   cudaError_t err = aodm_block_lists_launch(tab, ldtab, nao, nblk, lists, counts, stream);
   if (err != cudaSuccess) return err;
-  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, nset, stream)) !=
+  const int groups = (nset + NS - 1) / NS;
+  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, groups, stream)) !=
       cudaSuccess)
     return err;
   FockArgs a{};
@@ -261,26 +403,37 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   a.counts = counts;
   a.nao = nao;
   a.ngrid = ngrid;
+  a.nset = nset;
   a.blk = blk;
   a.gsub = gsub;
   a.sym = ao_lhs == ao_rhs;
-  // 16-byte copies need every tile's first point (b * blk + 64 t) 16-byte
-  // aligned in phi and w: an even BLKSIZE and row stride, aligned bases
+  // bulk copies need every tile's first point (b * blk + 64 t) 16-byte aligned
+  // in phi and w: an even BLKSIZE and row stride, aligned bases
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   a.vec = blk % 2 == 0 && stride_grid % 2 == 0 && al16(ao_lhs) && al16(ao_rhs) && al16(ws);
   a.items = items;
   a.counters = counters;
-  const size_t dyn = 2 * TILE * sizeof(double);
+  static_assert(2 * (FOCK_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
   if ((err = cudaFuncSetAttribute(fock_compact_kernel,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn))) !=
-      cudaSuccess)
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(FOCK_SMEM))) != cudaSuccess)
     return err;
   int dev = 0, nsm = 0;
   if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
   if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return err;
-  fock_compact_kernel<<<dim3(2 * nsm, nset), THREADS, dyn, stream>>>(a);
+  fock_compact_kernel<<<dim3(2 * nsm, groups), THREADS, FOCK_SMEM, stream>>>(a);
   return cudaGetLastError();
+}
+
+cudaError_t fock_reset_error(cudaStream_t stream) {
+  static const int zero = 0;
+  return cudaMemcpyToSymbolAsync(g_fock_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice,
+                                 stream);
+}
+
+cudaError_t fock_read_error(int* code) {
+  return cudaMemcpyFromSymbol(code, g_fock_error, sizeof(int));
 }
 
 }  // namespace cfgmm

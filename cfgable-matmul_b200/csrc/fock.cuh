@@ -18,4 +18,8 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
                               int nao, int ngrid, int nset, const uint8_t* tab, size_t ldtab,
                               int blk, void* workspace, cudaStream_t stream);
 
+// Sticky error word of the kernel's bounded waits (0 = none).
+cudaError_t fock_reset_error(cudaStream_t stream);
+cudaError_t fock_read_error(int* code);
+
 }  // namespace cfgmm

@@ -105,6 +105,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
       : "memory");
 }
 
+// The mbarrier tracks the completion of all cp.async this thread issued before
+// (one arrival, counted in the barrier's initial count).
+__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Orders this thread's generic-proxy shared-memory writes before later
 // async-proxy reads (tcgen05.mma operands written by threads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
