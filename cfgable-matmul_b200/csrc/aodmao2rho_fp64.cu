@@ -606,7 +606,7 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
     // ------------------------------- consumers -------------------------------
     const int ct = tid - NPROD;
     const int warp = ct >> 5;
-    const int wm = warp / CWN, wn = warp % CWN;  // warp tile: rows wm*16*MT.., points wn*8*NT..
+    const int wn = warp % CWN;  // warp tile: rows wm*16*MT.., points wn*8*NT..
     const int g = lane >> 2, q = lane & 3;
     uint32_t use = 0;
     for (int n = 0;; ++n) {
@@ -618,6 +618,10 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
       if (lane == 0) tc::mbar_arrive(&iempty[slot]);
       if (it >= total) break;
       const Item t = decode<NS>(p, p.items[it], set0);
+      // the row groups change warps with every item: those with less to do (the
+      // diagonal tile's upper rows below, a list's ragged end) are not always on
+      // the same schedulers, and the ring of stages lets warps drift apart
+      const int wm = (warp / CWN + n) % CWM;
 
       // the phi_lhs rows of this thread's epilogue (rows wm*16*MT + mt*16 + g + 8h,
       // points point_of(wn, nt, q, e)) are brought into L2 now, so that the
@@ -658,10 +662,15 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
         }
         const uint8_t* st = sm + stage * SB;
         const double* phi = reinterpret_cast<const double*>(st + NS * D_BYTES);
-        // symmetric D, diagonal tile: D' = strict upper triangle + half diagonal
+        // symmetric D, diagonal tile: D' = strict upper triangle + half diagonal;
+        // a stage left of all of the warp's rows holds only zeros of it
         const bool diag = sym && kc < kc0 + TU / TK;
+        const bool none =
+            (diag && (kc - kc0 + 1) * TK <= wm * 16 * MT) || wm * 16 * MT >= t.mu;
+        const int kend = none ? 0 : (t.nb - kc * TK > 8 ? TK : 8);
 #pragma unroll
         for (int kk = 0; kk < TK; kk += 8) {
+          if (kk >= kend) break;
           // tiles 2j and 2j + 1 take the even and the odd points of a group of
           // 16: column x of tile 2j + e is point 2x + e of the group
           double2 b0[NT / 2], b1[NT / 2];
