@@ -26,6 +26,15 @@ __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src
                : "memory");
 }
 
+// 16-byte asynchronous copy of which the first `bytes` (0, 8 or 16) are read
+// from `src`; the rest of the destination is zero-filled.
+__device__ __forceinline__ void cp_async_16_n(void* smem_dst, const void* gmem_src, int bytes) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem_src),
+               "r"(bytes)
+               : "memory");
+}
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 template <int N>

@@ -50,7 +50,11 @@ cudaError_t fock_fp64(double* v, size_t ldv, const double* w, const double* ao_l
                       const uint8_t* tab, size_t ldtab, int blk, bool pack_rhs, void* workspace,
                       cudaStream_t stream);
 
-// Sticky error word of the TMA form's bounded waits (0 = none).
+cudaError_t fock_dense_reset_error(cudaStream_t stream);
+cudaError_t fock_dense_read_error(int* code);
+
+// Sticky error words of the bounded waits of the masked GEMM's compacted form and
+// the dense Fock form (0 = none).
 cudaError_t dgemm_reset_error(cudaStream_t stream);
 cudaError_t dgemm_read_error(int* code);
 

@@ -14,7 +14,7 @@
 //
 // Measured at 2228 x 16384 x 2228, BLKSIZE 48, 30 % of the tiles present: 1.60 ms
 // (30.5 TFLOP/s of present products; the floor at the DMMA peak of 37 is 1.32),
-// where the dense form took 5.60 ms; every tile present: 5.11 against 5.60 ms.
+// where the dense form takes 5.04 ms; every tile present: 5.11 against 5.06 ms.
 //
 // dgemm_mask_kernel: work item = (column block piece of up to 64 columns, 128
 // rows of C).  One producer warp fetches 16 list rows per stage with untiled
@@ -363,25 +363,27 @@ bool dgemm_mask_applies(int m, int n, int k, int blk) {
   const long long items = nblk * nsub * ((m + TM - 1) / TM);
   // narrow blocks fill too little of a tile
   if (width < 32) return false;
-  // one wave of at most two K steps of the direct form is over before the lists
-  // are made: 1 x 48 x 17 takes 13 us there and 21 here, 129 x 64 x 64 29 in both,
-  // 200 x 1000 x 200 58 there and 30 here
-  const long long tiles = ((m + 127ll) / 128) * ((n + 127ll) / 128);
-  if (k <= 64 && tiles <= 148) return false;
+  // up to here the dense form over zero-filled tiles is over before the lists are
+  // made and their items run: 200 x 1000 x 200 takes 18 us against 24 to 34 here
+  // (15 % to all tiles present), 300 x 2000 x 300 36 against 25 to 43,
+  // 600 x 1500 x 600 68 against 39 to 107, 500 x 8000 x 500 174 against 56 to 164
+  if (2.0 * m * n * k <= 4e8) return false;
   // index and grid limits
   return items < (1ll << 30) && nblk < (1 << 24) &&
          nblk * (blk + 1ll) < (1ll << 31) && k <= 500000 && m <= 2000000;
 }
 
-// A piece costs the time of its padded width.  Measured at 2228 x 16384 x 2228:
-// 31.4 TFLOP/s of present products where no column is padded (BLKSIZE 48 and
-// 64; the dense form 29.1 of all products), and at 79 % present tiles BLKSIZE 33
-// (33 of 48 columns used) 6.1 ms against 5.6 dense, BLKSIZE 40 4.9.  So the
-// compacted form is the faster one up to a share of 1.07 times the used part of
-// the padded width.
+// A piece costs the time of its padded width.  Measured at 2228 x 8000 x 2228 (the
+// dense form takes 2.51 ms there whatever is present): BLKSIZE 33, 33 of 48 columns
+// used, 2.35 ms at 60 % present and 2.89 at 75 %; BLKSIZE 40 (of 48) 2.31 at 75 %
+// and 2.77 at 90 %; 56 (of 64) 2.22 and 2.64.  So the compacted form is the faster
+// one up to a share of 0.96 times the used part of the padded width.  Where the
+// whole width is used (BLKSIZE 48, 64) it always runs: with every tile present it
+// loses 1 to 5 %, less than a dense form that is enqueued and mostly not run.
 double dgemm_mask_max_share(int n, int blk) {
   const int width = std::min(blk, n);
-  return 1.07 * width / padded(width, pieces(width));
+  const double used = double(width) / padded(width, pieces(width));
+  return used == 1.0 ? 1.0 : 0.96 * used;
 }
 
 size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,

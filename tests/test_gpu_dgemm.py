@@ -107,3 +107,34 @@ def test_matmul_full_size_sampled(cm, wl, ta, tb):
     B = b.T if tb else b
     ref = np.einsum("sk,ks->s", A[i, :], B[:, j])
     assert normwise(c[i, j], ref) < TOL
+
+
+@pytest.mark.parametrize("transa,transb", [(False, False), (False, True), (True, False),
+                                           (True, True)])
+@pytest.mark.parametrize("m,n,k,pad", [
+    (64, 64, 16, 0),      # one tile, one K step; rows 16-byte aligned
+    (65, 63, 17, 1),      # one past, one short of a tile; odd rows: 8-byte copies
+    (1, 1, 1, 0),         # odd rows of one element
+    (2, 130, 33, 0),      # two parts of K, the second one shorter
+    (66, 62, 1000, 0),    # eight parts of K in a cluster, odd and even tile edges
+    (129, 200, 515, 3),   # eight parts, a last K step of three
+    (1600, 1552, 66, 0),  # more tiles than a wave, a last group of one tile row
+    (1543, 1601, 801, 0), # operands copied into aligned rows first
+])
+def test_dgemm_tiles_and_k_parts(cm, transa, transb, m, n, k, pad):
+    """Edges of the 64 x 64 tiles, of the K steps of 16, of the parts of K that a
+    cluster shares, and of the copies of one and of two elements; padded rows,
+    accumulation into a nonzero C whose padding stays untouched."""
+    import torch
+    g = torch.Generator().manual_seed(m + 3 * n + 7 * k)
+    u = lambda *s: torch.rand(*s, generator=g, dtype=torch.float64) * 2 - 1
+    a = u(k, m + pad) if transa else u(m, k + pad)
+    b = u(n, k + pad) if transb else u(k, n + pad)
+    c0 = u(m, n + pad)
+    ref = c0.clone()
+    ref[:, :n] += (a[:, :m].t() if transa else a[:, :k]) @ (b[:, :k].t() if transb else b[:, :n])
+    c = c0.cuda()
+    cm.matmul_ex(c, a.cuda(), b.cuda(), m, n, k, a.shape[1], b.shape[1], n + pad, transa, transb)
+    torch.cuda.synchronize()
+    assert normwise(c.cpu().numpy(), ref.numpy()) < TOL
+    assert torch.equal(c.cpu()[:, n:], c0[:, n:])
