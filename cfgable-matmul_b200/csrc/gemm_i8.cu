@@ -44,6 +44,28 @@ struct TileIdx {
   int l, m0, n0;
 };
 
+// packed[w] = the bytes of v[4w..4w+3] mods m, for |v| <= 2^30 and mul =
+// rint(2^38 / m): q = (v mul + 2^37) >> 38 is rint(v / m) exactly, because the
+// error of v mul 2^-38 is at most 2^30 / 2 * 2^-38 = 2^-9, below the least
+// distance 1/(2m) >= 1/510 of v / m from a half-integer for odd m, and zero for
+// m = 256 (where a half rounds up, to the residue -128).  A wide multiply-add, a
+// shift and a multiply-add per value.
+__device__ __forceinline__ void mods32(const uint32_t (&v)[32], int m, int mul,
+                                       uint32_t (&packed)[8]) {
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    uint32_t r[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int a = int(v[4 * w + e]);
+      const long long t = static_cast<long long>(a) * mul + (1ll << 37);
+      r[e] = uint32_t(a - (int(t >> 32) >> 6) * m);
+    }
+    packed[w] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040),
+                            0x5410);
+  }
+}
+
 __device__ __forceinline__ TileIdx tile_of(int t, int tiles_m, int tiles_n) {
   const int per_l = tiles_m * tiles_n;
   TileIdx r;
@@ -180,8 +202,7 @@ gemm_i8_mod_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       ++buse[buf];
       tc::fence_after_sync();
       const int m = p.mod[ti.l];
-      const float inv = p.inv[ti.l];
-      const int hi = (m - 1) >> 1, lo = -(m >> 1);
+      const int mul = p.mul[ti.l];
       const int row = ti.m0 + 32 * quarter + lane;
       int8_t* out = p.out + (size_t(ti.l) * p.rows_a + row) * p.ldr;
 #pragma unroll 1
@@ -190,22 +211,7 @@ gemm_i8_mod_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         tc::tmem_ld_32x32b_x32(tmem_base + uint32_t(buf * BN + c) + lane_off, v);
         tc::tmem_ld_wait();
         uint32_t packed[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-          uint32_t word = 0;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int a = int(v[4 * w + e]);
-            const int q = __float2int_rn(__int2float_rn(a) * inv);
-            int r = a - q * m;  // q is within 2 of the exact quotient for |a| < 2^30
-            if (r > hi) r -= m;
-            if (r > hi) r -= m;
-            if (r < lo) r += m;
-            if (r < lo) r += m;
-            word |= (uint32_t(r) & 0xffu) << (8 * e);
-          }
-          packed[w] = word;
-        }
+        mods32(v, m, mul, packed);
         const int col = ti.n0 + c;
         if (row < p.rows_a && col < p.rows_b) {
           if (col + 32 <= p.rows_b) {
@@ -239,14 +245,25 @@ gemm_i8_mod_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 // reads 8 KB of operands per MMA from shared memory instead of 12 KB.  One
 // thread of CTA 0 issues the MMAs; its stage barrier counts the TMA bytes of
 // both CTAs, the MMA commits arrive on both CTAs' barriers, and the epilogue
-// warps of both CTAs release an accumulator on CTA 0's barrier.  Every role
+// warps of both CTAs release an accumulator on CTA 0's barrier.  The epilogue has
+// eight warps per CTA (32 rows x 128 columns each): a wide multiply-add gives the
+// exact quotient (mods32), and a warp's residues leave through shared memory by one
+// TMA store.  With four warps, a quotient through float conversions and corrections,
+// and 16-byte stores 32 rows apart, the epilogue took 6.5 us per tile, longer than
+// the MMAs of short contractions: 14 products of 4096 x 4096 x 1024 317 -> 182 us (147
+// with no epilogue work at all), of 3527 x 9583 x 6581 2125 -> 1939 (1898).  Every role
 // leaves its loop on a bounded wait's timeout and meets the other CTA at the
 // final cluster barrier.
 // ---------------------------------------------------------------------------
 constexpr int P_BM = 256, P_BN = 256, P_STAGES = 6;
+constexpr int P_EPI = 8;                      // epilogue warps per CTA: TMEM quarters x halves
+constexpr int P_THREADS = 32 * (2 + P_EPI);
 constexpr uint32_t P_A_STAGE = (P_BM / 2) * BK, P_B_STAGE = (P_BN / 2) * BK;  // per CTA
 constexpr uint32_t P_STAGE_BYTES = P_A_STAGE + P_B_STAGE;
-constexpr size_t P_SMEM_BYTES = size_t(P_STAGES) * P_STAGE_BYTES + 1024 + 256;
+constexpr uint32_t P_OUT_WARP = 32 * 128;      // bytes of an epilogue warp's 32 x 128 residues
+constexpr size_t P_SMEM_BYTES =
+    size_t(P_STAGES) * P_STAGE_BYTES + P_EPI * P_OUT_WARP + 1024 + 256;
+static_assert(P_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
 __device__ __forceinline__ TileIdx pair_tile_of(int t, int tiles_m, int tiles_n) {
   const int per_l = tiles_m * tiles_n;
@@ -263,19 +280,22 @@ __device__ __forceinline__ TileIdx pair_tile_of(int t, int tiles_m, int tiles_n)
   return r;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_i8_mod_pair_kernel(const __grid_constant__ CUtensorMap tmA,
-                        const __grid_constant__ CUtensorMap tmB, GemmI8Args p) {
+                        const __grid_constant__ CUtensorMap tmB,
+                        const __grid_constant__ CUtensorMap tmR,
+                        const __grid_constant__ GemmI8Args p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + P_STAGES * P_A_STAGE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES);
+  uint8_t* sOut = smem + P_STAGES * P_STAGE_BYTES;  // [P_EPI][32 rows][128], 128-byte swizzle
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + P_EPI * P_OUT_WARP);
   uint64_t* full = bars;                      // [P_STAGES] TMA -> MMA (CTA 0's counts both)
   uint64_t* empty = bars + P_STAGES;          // [P_STAGES] MMA -> each CTA's producer
   uint64_t* tfull = bars + 2 * P_STAGES;      // [2] MMA -> each CTA's epilogue
-  uint64_t* tempty = bars + 2 * P_STAGES + 2;  // [2] (CTA 0's) 8 epilogue warps -> MMA
+  uint64_t* tempty = bars + 2 * P_STAGES + 2;  // [2] (CTA 0's) both CTAs' epilogue warps -> MMA
   uint64_t* drain = bars + 2 * P_STAGES + 4;   // MMA completion at teardown (CTA 0)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * P_STAGES + 5);
 
@@ -290,12 +310,13 @@ gemm_i8_mod_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(&tfull[b], 1);
-      tc::mbar_init(&tempty[b], 8);
+      tc::mbar_init(&tempty[b], 2 * P_EPI);
     }
     tc::mbar_init(drain, 1);
     tc::mbar_fence_init();
     tc::prefetch_tensormap(&tmA);
     tc::prefetch_tensormap(&tmB);
+    tc::prefetch_tensormap(&tmR);
   }
   if (warp == 1) {
     tc::tmem_alloc_pair(tmem_slot, TMEM_COLS);
@@ -316,13 +337,14 @@ gemm_i8_mod_pair_kernel(const __grid_constant__ CUtensorMap tmA,
     // ---------------- TMA producer (both CTAs) ----------------
     if (lane == 0) {
       const uint32_t full0 = tc::mapa_shared(tc::smem_u32(full), 0);  // CTA 0's full[0]
+      uint32_t fill = 0;  // stage fills issued so far
       int stage = 0;
-      uint32_t uses[P_STAGES] = {0, 0, 0, 0, 0, 0};
+      uint32_t phase = 1;  // parity of the wait for the stage's last use
       bool ok = true;
       for (int t = cid; t < ntiles && ok; t += nclusters) {
         const TileIdx ti = pair_tile_of(t, tiles_m, tiles_n);
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (uses[stage] > 0 && !tc::mbar_wait(&empty[stage], (uses[stage] - 1) & 1, err, 21)) {
+          if (fill >= P_STAGES && !tc::mbar_wait(&empty[stage], phase, err, 21)) {
             ok = false;
             break;
           }
@@ -332,36 +354,36 @@ gemm_i8_mod_pair_kernel(const __grid_constant__ CUtensorMap tmA,
                                ti.m0 + int(rank) * (P_BM / 2), ti.l);
           tc::tma_load_3d_pair(sB + stage * P_B_STAGE, &tmB, fb, kb * BK,
                                ti.n0 + int(rank) * (P_BN / 2), ti.l);
-          ++uses[stage];
-          stage = (stage + 1) % P_STAGES;
+          ++fill;
+          if (++stage == P_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
       // teardown: CTA 0's stage barriers count both CTAs' bytes
       if (rank == 0)
-        for (int s = 0; s < P_STAGES; ++s)
-          if (uses[s] > 0) tc::mbar_wait(&full[s], (uses[s] - 1) & 1, err, 22, true);
+        for (uint32_t f = fill > P_STAGES ? fill - P_STAGES : 0; f < fill; ++f)
+          tc::mbar_wait(&full[f % P_STAGES], (f / P_STAGES) & 1, err, 22, true);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (CTA 0) ----------------
     if (rank == 0 && lane == 0) {
       const uint32_t idesc = tc::idesc_i8(P_BM, P_BN);
       int stage = 0;
-      uint32_t fuse[P_STAGES] = {0, 0, 0, 0, 0, 0};
-      uint32_t buse[2] = {0, 0};
-      int buf = 0;
+      uint32_t phase = 0;
+      int n = 0;  // tiles issued: accumulator n % 2, its use n / 2
       bool ok = true;
-      for (int t = cid; t < ntiles && ok; t += nclusters) {
-        if (buse[buf] > 0 &&
-            !tc::mbar_wait_cluster(&tempty[buf], (buse[buf] - 1) & 1, err, 23))
-          break;
+      for (int t = cid; t < ntiles && ok; t += nclusters, ++n) {
+        const int buf = n & 1;
+        if (n >= 2 && !tc::mbar_wait_cluster(&tempty[buf], ((n >> 1) - 1) & 1, err, 23)) break;
         tc::fence_after_sync();
         const uint32_t dtmem = tmem_base + uint32_t(buf * P_BN);
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!tc::mbar_wait_cluster(&full[stage], fuse[stage] & 1, err, 24)) {
+          if (!tc::mbar_wait_cluster(&full[stage], phase, err, 24)) {
             ok = false;
             break;
           }
-          ++fuse[stage];
           tc::fence_after_sync();
           const uint32_t a0 = tc::smem_u32(sA + stage * P_A_STAGE);
           const uint32_t b0 = tc::smem_u32(sB + stage * P_B_STAGE);
@@ -370,73 +392,71 @@ gemm_i8_mod_pair_kernel(const __grid_constant__ CUtensorMap tmA,
             tc::mma_i8_pair(dtmem, tc::smem_desc_k128(a0 + 32 * ks),
                             tc::smem_desc_k128(b0 + 32 * ks), idesc, kb > 0 || ks > 0);
           tc::mma_commit_pair(&empty[stage]);
-          stage = (stage + 1) % P_STAGES;
+          if (++stage == P_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
         if (!ok) break;
         tc::mma_commit_pair(&tfull[buf]);
-        ++buse[buf];
-        buf ^= 1;
       }
       // teardown: every issued MMA has completed
       tc::mma_commit_pair_local(drain);
       tc::mbar_wait(drain, 0, err, 25, true);
     }
   } else {
-    // ---------------- epilogue (warps 2..5, both CTAs) ----------------
-    const int quarter = warp & 3;  // TMEM lanes this warp may access
+    // ---------------- epilogue (warps 2..9, both CTAs) ----------------
+    const int quarter = warp & 3;            // TMEM lanes this warp may access
+    const int col0 = ((warp - 2) >> 2) * (P_BN / 2);  // its half of the columns
     const uint32_t lane_off = uint32_t(32 * quarter) << 16;
     const uint32_t tempty0 = tc::mapa_shared(tc::smem_u32(tempty), 0);  // CTA 0's tempty[0]
-    uint32_t buse[2] = {0, 0};
-    int buf = 0;
-    for (int t = cid; t < ntiles; t += nclusters) {
+    uint8_t* mine = sOut + (warp - 2) * P_OUT_WARP;
+    int n = 0;
+    for (int t = cid; t < ntiles; t += nclusters, ++n) {
       const TileIdx ti = pair_tile_of(t, tiles_m, tiles_n);
-      if (!tc::mbar_wait_cluster(&tfull[buf], buse[buf] & 1, err, 26)) break;
-      ++buse[buf];
+      const int buf = n & 1;
+      if (!tc::mbar_wait_cluster(&tfull[buf], (n >> 1) & 1, err, 26)) break;
       tc::fence_after_sync();
-      const int m = p.mod[ti.l];
-      const float inv = p.inv[ti.l];
-      const int hi = (m - 1) >> 1, lo = -(m >> 1);
-      const int row = ti.m0 + int(rank) * (P_BM / 2) + 32 * quarter + lane;
-      int8_t* out = p.out + (size_t(ti.l) * p.rows_a + row) * p.ldr;
-#pragma unroll 1
-      for (int c = 0; c < P_BN; c += 32) {
-        uint32_t v[32];
-        tc::tmem_ld_32x32b_x32(tmem_base + uint32_t(buf * P_BN + c) + lane_off, v);
-        tc::tmem_ld_wait();
+      const int m = p.mod[ti.l], mul = p.mul[ti.l];
+      const uint32_t src = tmem_base + uint32_t(buf * P_BN + col0) + lane_off;
+      // columns c .. c + 31 of this lane's row: 16-byte pieces c / 16 and the next
+      auto keep = [&](const uint32_t (&v)[32], int c) {
         uint32_t packed[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-          uint32_t word = 0;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int a = int(v[4 * w + e]);
-            const int q = __float2int_rn(__int2float_rn(a) * inv);
-            int r = a - q * m;  // q is within 2 of the exact quotient for |a| < 2^30
-            if (r > hi) r -= m;
-            if (r > hi) r -= m;
-            if (r < lo) r += m;
-            if (r < lo) r += m;
-            word |= (uint32_t(r) & 0xffu) << (8 * e);
-          }
-          packed[w] = word;
-        }
-        const int col = ti.n0 + c;
-        if (row < p.rows_a && col < p.rows_b) {
-          if (col + 32 <= p.rows_b) {
-            uint4* dst = reinterpret_cast<uint4*>(out + col);
-            dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-          } else {
-            for (int e = 0; e < p.rows_b - col; ++e)
-              out[col + e] = int8_t((packed[e >> 2] >> (8 * (e & 3))) & 0xffu);
-          }
-        }
-      }
-      tc::fence_before_sync();
+        mods32(v, m, mul, packed);
+        uint8_t* at = mine + lane * 128;
+        *reinterpret_cast<uint4*>(at + (((c >> 4) ^ (lane & 7)) << 4)) =
+            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        *reinterpret_cast<uint4*>(at + ((((c >> 4) + 1) ^ (lane & 7)) << 4)) =
+            make_uint4(packed[4], packed[5], packed[6], packed[7]);
+      };
+      // the next 32 columns are on their way while the last ones are reduced; the
+      // accumulator goes back to the MMAs before its last columns are
+      uint32_t v0[32], v1[32];
+      tc::tmem_ld_32x32b_x32(src, v0);
+      if (lane == 0) tc::bulk_wait_read();  // the last tile's store has read `mine`
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(tempty0 + uint32_t(buf) * 8u);
-      buf ^= 1;
+#pragma unroll
+      for (int c = 0; c < P_BN / 2; c += 64) {
+        tc::tmem_ld_wait_for(v0);
+        tc::tmem_ld_32x32b_x32(src + uint32_t(c + 32), v1);
+        keep(v0, c);
+        tc::tmem_ld_wait_for(v1);
+        if (c + 64 < P_BN / 2) {
+          tc::tmem_ld_32x32b_x32(src + uint32_t(c + 64), v0);
+        } else {
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive_cluster(tempty0 + uint32_t(buf) * 8u);
+        }
+        keep(v1, c + 32);
+      }
+      // 32 rows x 128 columns by one TMA store, clipped at the matrix's edges
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      const int row = ti.m0 + int(rank) * (P_BM / 2) + 32 * quarter, col = ti.n0 + col0;
+      if (lane == 0 && row < p.rows_a && col < p.rows_b) tc::tma_store_3d(&tmR, mine, col, row, ti.l);
     }
+    if (lane == 0) tc::bulk_wait_all();
   }
 
   tc::fence_before_sync();
@@ -460,8 +480,8 @@ int gemm_i8_tile_rows_a() { return BM; }
 int gemm_i8_tile_rows_b() { return pair_enabled() ? P_BN / 2 : BN; }
 int gemm_i8_k_block() { return BK; }
 
-cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmI8Args& args,
-                        cudaStream_t stream) {
+cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmR,
+                        const GemmI8Args& args, cudaStream_t stream) {
   if (pair_enabled()) {
     cudaError_t err = cudaFuncSetAttribute(gemm_i8_mod_pair_kernel,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -474,7 +494,7 @@ cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const Ge
     static int max_clusters = [] {
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3(2, 1, 1);
-      cfg.blockDim = dim3(THREADS, 1, 1);
+      cfg.blockDim = dim3(P_THREADS, 1, 1);
       cfg.dynamicSmemBytes = P_SMEM_BYTES;
       int n = 0;
       if (cudaOccupancyMaxActiveClusters(&n, gemm_i8_mod_pair_kernel, &cfg) != cudaSuccess)
@@ -483,8 +503,8 @@ cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const Ge
     }();
     if (max_clusters <= 0) return cudaErrorLaunchOutOfResources;
     const long long clusters = tiles < max_clusters ? tiles : max_clusters;
-    gemm_i8_mod_pair_kernel<<<unsigned(2 * clusters), THREADS, P_SMEM_BYTES, stream>>>(tmA, tmB,
-                                                                                     args);
+    gemm_i8_mod_pair_kernel<<<unsigned(2 * clusters), P_THREADS, P_SMEM_BYTES, stream>>>(
+        tmA, tmB, tmR, args);
     return cudaGetLastError();
   }
   cudaError_t err = cudaFuncSetAttribute(gemm_i8_mod_kernel,

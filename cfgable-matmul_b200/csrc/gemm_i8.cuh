@@ -17,7 +17,7 @@ struct GemmI8Args {
   int8_t* out;     // residues [nmod][rows_a][ldr]
   size_t ldr;      // row stride of `out` (multiple of 16)
   int mod[kMaxModuli];
-  float inv[kMaxModuli];
+  int mul[kMaxModuli];  // rint(2^38 / mod), see mods32
 };
 
 // Tile geometry (A rows per tile, B rows per tile, K bytes per stage).
@@ -26,9 +26,10 @@ int gemm_i8_tile_rows_b();
 int gemm_i8_k_block();
 
 // tmA / tmB: 3-D tensor maps over INT8 planes (K, rows, nmod), 128-byte
-// swizzle, boxes (128, 128, 1) and (128, 256, 1).
-cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmI8Args& args,
-                        cudaStream_t stream);
+// swizzle, boxes (128, 128, 1) and (128, 256, 1).  tmR: the map of args.out
+// (rows_b, rows_a, nmod), 128-byte swizzle, box (128, 32, 1).
+cudaError_t gemm_i8_mod(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmR,
+                        const GemmI8Args& args, cudaStream_t stream);
 
 // Sticky per-device error word of the kernel (0 = ok; else the code of the
 // wait that timed out).  reset enqueues a clear; read is synchronous.

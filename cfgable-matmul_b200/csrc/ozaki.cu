@@ -517,12 +517,14 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-bool make_plane_map(CUtensorMap* map, void* base, int k, int rows, int nplanes, size_t kpad,
+// Planes of `rows` rows of `cols` bytes at stride `pitch`, boxes of 128 bytes x
+// box_rows rows, 128-byte swizzle.
+bool make_plane_map(CUtensorMap* map, void* base, int cols, int rows, int nplanes, size_t pitch,
                     int box_rows) {
   auto enc = encode_fn();
   if (!enc) return false;
-  cuuint64_t dims[3] = {cuuint64_t(k), cuuint64_t(rows), cuuint64_t(nplanes)};
-  cuuint64_t strides[2] = {cuuint64_t(kpad), cuuint64_t(rows) * kpad};
+  cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(nplanes)};
+  cuuint64_t strides[2] = {cuuint64_t(pitch), cuuint64_t(rows) * pitch};
   cuuint32_t box[3] = {128, cuuint32_t(box_rows), 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr,
@@ -704,8 +706,9 @@ cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int 
   if ((err = side.join()) != cudaSuccess) return err;
 
   mark(1);
-  CUtensorMap tmA, tmB;
-  if (!make_plane_map(&tmA, a_res, k, m, plan.nmod, L.kpad, gemm_i8_tile_rows_a()) ||
+  CUtensorMap tmA, tmB, tmR;
+  if (!make_plane_map(&tmR, r, n, m, plan.nmod, L.ldr, 32) ||
+      !make_plane_map(&tmA, a_res, k, m, plan.nmod, L.kpad, gemm_i8_tile_rows_a()) ||
       !make_plane_map(&tmB, b_res, k, n, plan.nmod, L.kpad, gemm_i8_tile_rows_b()))
     return cudaErrorInvalidValue;
   GemmI8Args g{};
@@ -717,9 +720,9 @@ cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int 
   g.ldr = L.ldr;
   for (int l = 0; l < plan.nmod; ++l) {
     g.mod[l] = plan.mod[l];
-    g.inv[l] = plan.inv_f[l];
+    g.mul[l] = int((2 * (1ll << 38) / plan.mod[l] + 1) / 2);  // rint(2^38 / mod)
   }
-  if ((err = gemm_i8_mod(tmA, tmB, g, stream)) != cudaSuccess) return err;
+  if ((err = gemm_i8_mod(tmA, tmB, tmR, g, stream)) != cudaSuccess) return err;
   mark(2);
 
   ReconArgs rc{};
