@@ -738,6 +738,14 @@ int matmul_f32_run(float* c, const float* a, const float* b, size_t m, size_t n,
                    size_t lda, size_t ldb, size_t ldc, bool ta, bool tb, const GemmExtents& ex,
                    int precision, cudaStream_t s) {
   StreamScratch sc(s);
+  if (precision == CFGMM_PREC_OZAKI_INT8) {
+    const int nmod = cfgmm::ozaki_moduli_for_bits(int(k), kF32OperandBits);
+    void* ws = nullptr;
+    CFGMM_CUDA(sc.get(&ws, cfgmm::ozaki_dgemm_workspace(int(m), int(n), int(k), nmod)));
+    CFGMM_CUDA(cfgmm::ozaki_dgemm(c, a, b, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, nmod, ws,
+                                  s));
+    return CFGMM_OK;
+  }
   double *da = nullptr, *db = nullptr, *dc = nullptr;
   CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&da), ex.a * 8));
   CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&db), ex.b * 8));
@@ -745,15 +753,7 @@ int matmul_f32_run(float* c, const float* a, const float* b, size_t m, size_t n,
   CFGMM_CUDA(cfgmm::widen_f32(a, da, ex.a, s));
   CFGMM_CUDA(cfgmm::widen_f32(b, db, ex.b, s));
   CFGMM_CUDA(cfgmm::widen_f32(c, dc, ex.c, s));
-  if (precision == CFGMM_PREC_OZAKI_INT8) {
-    const int nmod = cfgmm::ozaki_moduli_for_bits(int(k), kF32OperandBits);
-    void* ws = nullptr;
-    CFGMM_CUDA(sc.get(&ws, cfgmm::ozaki_dgemm_workspace(int(m), int(n), int(k), nmod)));
-    CFGMM_CUDA(cfgmm::ozaki_dgemm(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, nmod,
-                                  ws, s));
-  } else {
-    CFGMM_CUDA(cfgmm::dgemm_fp64(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, s));
-  }
+  CFGMM_CUDA(cfgmm::dgemm_fp64(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, s));
   CFGMM_CUDA(cfgmm::narrow_f64(dc, c, ex.c, s));
   return CFGMM_OK;
 }

@@ -29,11 +29,15 @@
 #include <cstring>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "gemm_i8.cuh"
 #include "ozaki.cuh"
 #include "side_stream.cuh"
 
 namespace cfgmm {
+
+namespace cg = cooperative_groups;
 
 // Pairwise coprime moduli, largest first (256 = 2^8, 255 = 3*5*17,
 // 253 = 11*23, 247 = 13*19, 217 = 7*31, the rest prime).
@@ -122,41 +126,38 @@ OzakiPlan ozaki_plan(int k, int nmod, int min_bits) {
 namespace {
 
 constexpr int kNonFinite = INT_MAX;  // exponent sentinel of a row holding Inf/NaN
+constexpr size_t kScanBytes = size_t(40) << 20;  // operands read twice from L2, see residues_cols
 
 // ---------------------------------------------------------------------------
-// exponents: e[r] = bits - E_r with max_p |x(r,p)| < 2^E_r  (0 for a zero row)
-// Computed in two steps: Emax[r] = max over chunks of the binary exponent of
-// the chunk maximum (INT_MAX for Inf/NaN, INT_MIN for all-zero), then e[r].
+// exponents: e[r] = bits - E_r with max_p |x(r,p)| < 2^E_r (0 for a zero row,
+// kNonFinite for one holding Inf/NaN).  The maximum is taken over the elements'
+// magnitude bits, which order as the values do and put Inf and NaN last.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int exponent_of(double amax) {
-  if (!(amax <= 1.7976931348623157e308)) return INT_MAX;  // Inf or NaN
-  if (amax == 0.0) return INT_MIN;
+template <class T>
+struct Magnitude;
+template <>
+struct Magnitude<double> {
+  using Bits = unsigned long long;
+  static __device__ __forceinline__ Bits of(double x) {
+    return static_cast<Bits>(__double_as_longlong(x)) & 0x7fffffffffffffffull;
+  }
+  static __device__ __forceinline__ double value(Bits b) {
+    return __longlong_as_double(static_cast<long long>(b));
+  }
+};
+template <>
+struct Magnitude<float> {
+  using Bits = unsigned;
+  static __device__ __forceinline__ Bits of(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+  static __device__ __forceinline__ double value(Bits b) { return __uint_as_float(b); }
+};
+
+__device__ __forceinline__ int row_exponent(double amax, int bits) {
+  if (!(amax <= 1.7976931348623157e308)) return kNonFinite;  // Inf or NaN
+  if (amax == 0.0) return 0;
   int E;
   frexp(amax, &E);  // amax = f 2^E, f in [0.5, 1): amax < 2^E
-  return E;
-}
-
-__global__ void fill_int(int* __restrict__ v, int n, int value) {
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i < n) v[i] = value;
-}
-
-// element (r, p) at x[r*ld + p]: one CTA per row
-__global__ void __launch_bounds__(256)
-emax_rows(const double* __restrict__ x, size_t ld, int rows, int k, int* __restrict__ emax) {
-  const int r = blockIdx.x;
-  if (r >= rows) return;
-  const double* row = x + size_t(r) * ld;
-  int E = INT_MIN;
-  for (int p = threadIdx.x; p < k; p += 256) E = max(E, exponent_of(fabs(row[p])));
-  for (int o = 16; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
-  __shared__ int red[8];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = E;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) E = max(E, red[w]);
-    emax[r] = max(E, red[0]);
-  }
+  return bits - E;
 }
 
 // Optional mask of the masked GEMM: element (r, p) of op(B)^T takes part only
@@ -169,32 +170,6 @@ struct Mask {
     return !tab || tab[size_t(p) * ldtab + r / blk] != 0;
   }
 };
-
-// element (r, p) at x[p*ld + r]: thread per r (coalesced), CTA rows of p chunks
-constexpr int kColChunk = 128;
-__global__ void __launch_bounds__(256)
-emax_cols(const double* __restrict__ x, size_t ld, int rows, int k, int* __restrict__ emax,
-          Mask mask) {
-  const int r = blockIdx.x * 256 + threadIdx.x;
-  const int p0 = blockIdx.y * kColChunk;
-  if (r >= rows) return;
-  const int p1 = min(k, p0 + kColChunk);
-  double mx = 0.0;
-  bool bad = false;
-  for (int p = p0; p < p1; ++p) {
-    const double v = mask.on(r, p) ? fabs(x[size_t(p) * ld + r]) : 0.0;
-    bad |= !(v <= 1.7976931348623157e308);
-    mx = fmax(mx, v);
-  }
-  atomicMax(&emax[r], bad ? INT_MAX : exponent_of(mx));
-}
-
-__global__ void finalize_exps(const int* __restrict__ emax, int rows, int bits, int* __restrict__ e) {
-  const int r = blockIdx.x * 256 + threadIdx.x;
-  if (r >= rows) return;
-  const int E = emax[r];
-  e[r] = (E == INT_MAX) ? kNonFinite : (E == INT_MIN ? 0 : bits - E);
-}
 
 // ---------------------------------------------------------------------------
 // residues: Y[l][r][p] = rint(x(r,p) 2^e[r]) mods m_l  (int8), p < k
@@ -368,57 +343,204 @@ __device__ __forceinline__ void write_residues8(const ResidueArgs& a, int8_t* Y,
   }
 }
 
-// element (r, p) at x[r*ld + p]: CTA per row, thread per 8 consecutive p
-template <int kForm>
+// The largest magnitude bits of row r (element (r, p) at x[r*ld + p]) by kThreads
+// threads, to all of them; every thread of the CTA calls it.
+template <int kThreads, class T>
+__device__ __forceinline__ typename Magnitude<T>::Bits row_max(const T* __restrict__ row, int k) {
+  using Mag = Magnitude<T>;
+  __shared__ typename Mag::Bits red[8];
+  typename Mag::Bits mx = 0;
+#pragma unroll 4
+  for (int p = threadIdx.x % kThreads; p < k; p += kThreads) mx = max(mx, Mag::of(row[p]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) red[warp] = mx;
+  __syncthreads();
+  const int w0 = warp / (kThreads / 32) * (kThreads / 32);
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) mx = max(mx, red[w0 + w]);
+  return mx;
+}
+
+// top[r] = the largest magnitude bits of row r, a CTA per row.
+template <class T>
+__global__ void __launch_bounds__(256)
+maxima_rows(const T* __restrict__ x, size_t ld, int k, typename Magnitude<T>::Bits* __restrict__ top) {
+  const auto mx = row_max<256>(x + size_t(blockIdx.x) * ld, k);
+  if (threadIdx.x == 0) top[blockIdx.x] = mx;
+}
+
+// element (r, p) at x[r*ld + p]: kThreads threads per row, 8 consecutive p each.
+// kScan: they take the row's maximum first and read it again from the caches, one
+// launch instead of two; operands past kScanBytes have their maxima from
+// maxima_rows, whose reads then overlap the other operand's arithmetic.
+template <int kForm, int kThreads, bool kScan, class T>
 __global__ void __launch_bounds__(256, 5)
-residues_rows(const double* __restrict__ x, size_t ld, int rows, int k, size_t kpad,
-              const int* __restrict__ e, int8_t* __restrict__ Y, ResidueArgs a) {
-  const int r = blockIdx.x;
+residues_rows(const T* __restrict__ x, size_t ld, int rows, int k, size_t kpad, int bits,
+              int* __restrict__ e, int8_t* __restrict__ Y, const __grid_constant__ ResidueArgs a,
+              const typename Magnitude<T>::Bits* __restrict__ top) {
+  const int t = threadIdx.x % kThreads;
+  const int r = blockIdx.x * (256 / kThreads) + threadIdx.x / kThreads;
+  const T* row = x + size_t(min(r, rows - 1)) * ld;
+  typename Magnitude<T>::Bits mx;
+  if constexpr (kScan)
+    mx = row_max<kThreads>(row, k);
+  else
+    mx = top[min(r, rows - 1)];
   if (r >= rows) return;
-  const int er = e[r];
-  const double* row = x + size_t(r) * ld;
+  const int er = row_exponent(Magnitude<T>::value(mx), bits);
+  if (t == 0) e[r] = er;
   const size_t plane = size_t(rows) * kpad;
-  for (int p = 8 * threadIdx.x; p < k; p += 8 * 256) {
+  for (int p = 8 * t; p < k; p += 8 * kThreads) {
     double v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      v[j] = (p + j < k) ? scaled<kForm>(row[p + j], er) : scaled_zero<kForm>();
+      v[j] = (p + j < k) ? scaled<kForm>(double(row[p + j]), er) : scaled_zero<kForm>();
     write_residues8<kForm>(a, Y, plane, size_t(r) * kpad + p, v);
   }
 }
 
-// element (r, p) at x[p*ld + r]: 32 (r) x 64 (p) tiles transposed through shared
-// memory.  Element (p, r) sits in column r ^ 2 (p / 8) of row p: a row is written
-// by one warp (a permutation of its 32 columns), and each half-warp of the
-// read side (two r, eight groups of p) meets 16 distinct 8-byte bank pairs.
-__device__ __forceinline__ int tile_col(int p, int r) { return r ^ ((p >> 2) & 14); }
-
-template <int kForm>
-__global__ void __launch_bounds__(256, 5)
-residues_cols(const double* __restrict__ x, size_t ld, int rows, int k, size_t kpad,
-              const int* __restrict__ e, int8_t* __restrict__ Y, ResidueArgs a, Mask mask) {
-  __shared__ double tile[64][32];
-  const int r0 = blockIdx.x * 32, p0 = blockIdx.y * 64;
-  const int tr = threadIdx.x & 31, tp = threadIdx.x >> 5;  // 8 rows of p per pass
-#pragma unroll
-  for (int pp = tp; pp < 64; pp += 8) {
-    const int p = p0 + pp, r = r0 + tr;
-    tile[pp][tile_col(pp, tr)] =
-        (p < k && r < rows && mask.on(r, p)) ? x[size_t(p) * ld + r] : 0.0;
+// The largest magnitude of each of CW adjacent r (element (r, p) at x[p*ld + r]) over
+// p in [p0, p1), to every thread of the first CW of the CTA; 256 threads.
+template <int CW, class T>
+__device__ __forceinline__ typename Magnitude<T>::Bits
+column_max(const T* __restrict__ x, size_t ld, int rows, int r0, int p0, int p1, Mask mask) {
+  using Mag = Magnitude<T>;
+  using Bits = typename Mag::Bits;
+  __shared__ Bits red[256 / CW][CW];
+  const int c = threadIdx.x % CW, pr = threadIdx.x / CW;
+  Bits mx = 0;
+  if (r0 + c < rows) {
+    const T* col = x + r0 + c;
+    if (mask.tab) {
+      for (int p = p0 + pr; p < p1; p += 256 / CW)
+        if (mask.on(r0 + c, p)) mx = max(mx, Mag::of(col[size_t(p) * ld]));
+    } else {
+#pragma unroll 8
+      for (int p = p0 + pr; p < p1; p += 256 / CW) mx = max(mx, Mag::of(col[size_t(p) * ld]));
+    }
   }
+  red[pr][c] = mx;
   __syncthreads();
-  const size_t plane = size_t(rows) * kpad;
-  // 32 rows x 8 groups of 8 p: one unit per thread
-  const int rr = threadIdx.x >> 3, pg = (threadIdx.x & 7) * 8;
-  const int r = r0 + rr, p = p0 + pg;
-  if (r >= rows || p >= k) return;
-  const int er = e[r];
-  double v[8];
+  if (threadIdx.x < CW)
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
-    v[j] = (p + j < k) ? scaled<kForm>(tile[pg + j][tile_col(pg + j, rr)], er)
-                       : scaled_zero<kForm>();
-  write_residues8<kForm>(a, Y, plane, size_t(r) * kpad + p, v);
+    for (int w = 0; w < 256 / CW; ++w) mx = max(mx, red[w][c]);
+  return mx;
+}
+
+// The maxima of a cluster's CTAs (each with a part of p), combined through
+// distributed shared memory, as exponents to exps[] of every CTA.
+template <int CW, class T>
+__device__ __forceinline__ void cluster_exponents(typename Magnitude<T>::Bits mx, int parts,
+                                                  int bits, int* exps) {
+  using Mag = Magnitude<T>;
+  __shared__ typename Mag::Bits part_max[CW];
+  const cg::cluster_group cluster = cg::this_cluster();
+  if (threadIdx.x < CW) part_max[threadIdx.x] = mx;
+  cluster.sync();
+  if (threadIdx.x < CW) {
+    for (int s = 0; s < parts; ++s)
+      mx = max(mx, *cluster.map_shared_rank(&part_max[threadIdx.x], s));
+    exps[threadIdx.x] = row_exponent(Mag::value(mx), bits);
+  }
+  cluster.sync();  // the maxima are read, the exponents visible
+}
+
+// The maxima of op(X) alone, for the residues of large operands: top[r] (zeroed
+// before) = the largest magnitude bits of element (r, p) at x[p*ld + r].  Thread per
+// r, CTA = 256 r x 128 p: 79 us for 6581 x 9583 doubles, the time of reading them
+// (in clusters of 8, 64 r each, 132: 1200 CTAs are a wave of 1184 and a rest).
+template <class T>
+__global__ void __launch_bounds__(256)
+maxima_cols(const T* __restrict__ x, size_t ld, int rows, int k,
+            typename Magnitude<T>::Bits* __restrict__ top, Mask mask) {
+  using Mag = Magnitude<T>;
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  const int p0 = blockIdx.y * 128, p1 = min(k, p0 + 128);
+  if (r >= rows) return;
+  typename Mag::Bits mx = 0;
+  if (mask.tab) {
+    for (int p = p0; p < p1; ++p)
+      if (mask.on(r, p)) mx = max(mx, Mag::of(x[size_t(p) * ld + r]));
+  } else {
+#pragma unroll 8
+    for (int p = p0; p < p1; ++p) mx = max(mx, Mag::of(x[size_t(p) * ld + r]));
+  }
+  atomicMax(top + r, mx);
+}
+
+// element (r, p) at x[p*ld + r]: CTA = CR r, a part of the tiles of CP p, transposed
+// through shared memory.
+// kScan: the CTAs of a cluster (the `parts` of the same r) first take their parts'
+// maxima and share them, then read their tiles again, from L2: one launch instead
+// of four.  That holds while x stays in L2 (1024 x 1024 x 1024: both operands 52 ->
+// 30 us); at 6581 x 9583 only 18 % of the second reads hit and the kernel took 432
+// us, so operands past kScanBytes have their maxima from maxima_cols.
+// The tile is 16 r x 128 p with the scan (more CTAs for a small operand) and 32 r x
+// 64 p without (256 bytes per row read: 295 us for the 6581 x 9583 doubles, 340 with
+// 128).  Element (p, r) sits in column tile_col(p, r) of row p: a row is written as
+// a permutation of its columns, and a half-warp of the read side (two r and eight
+// groups of 8 p, or one r and 16) meets 16 distinct 8-byte bank pairs.
+template <int CR>
+__device__ __forceinline__ int tile_col(int p, int r) {
+  return CR == 32 ? r ^ ((p >> 2) & 14) : r ^ ((p >> 3) & 15);
+}
+
+template <int kForm, bool kScan, class T>
+__global__ void __launch_bounds__(256, 5)
+residues_cols(const T* __restrict__ x, size_t ld, int rows, int k, size_t kpad, int bits,
+              int* __restrict__ e, int8_t* __restrict__ Y, const __grid_constant__ ResidueArgs a,
+              Mask mask, int parts, const typename Magnitude<T>::Bits* __restrict__ top) {
+  constexpr int CR = kScan ? 16 : 32, CP = 2048 / CR;
+  constexpr int G = CP / 8;  // groups of 8 p: G x CR units, one per thread
+  __shared__ T tile[CP][CR];
+  __shared__ int exps[CR];
+  const int part = blockIdx.x % parts, r0 = blockIdx.x / parts * CR;
+  // with the scan each CTA has a share of the tiles, without one tile
+  const int ntiles = kScan ? (k + CP - 1) / CP : 0;
+  const int t0 = kScan ? int((long long)part * ntiles / parts) : part;
+  const int t1 = kScan ? int((long long)(part + 1) * ntiles / parts) : part + 1;
+  const int c = threadIdx.x % CR, pr = threadIdx.x / CR;  // 256 / CR rows of p per pass
+  const bool rin = r0 + c < rows;
+  const T* col = x + r0 + c;
+  if constexpr (kScan) {
+    const auto mx = column_max<CR>(x, ld, rows, r0, t0 * CP, min(k, t1 * CP), mask);
+    cluster_exponents<CR, T>(mx, parts, bits, exps);
+    if (part == 0 && threadIdx.x < CR && rin) e[r0 + c] = exps[c];
+  } else {
+    if (threadIdx.x < CR) {
+      exps[c] = rin ? row_exponent(Magnitude<T>::value(top[r0 + c]), bits) : 0;
+      if (part == 0 && rin) e[r0 + c] = exps[c];
+    }
+  }
+  const size_t plane = size_t(rows) * kpad;
+  const int rr = threadIdx.x / G, pg = threadIdx.x % G * 8;
+  for (int t = t0; t < t1; ++t) {
+    const int p0 = t * CP;
+    T in[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int p = p0 + pr + (256 / CR) * i;
+      in[i] = (p < k && rin && mask.on(r0 + c, p)) ? col[size_t(p) * ld] : T(0);
+    }
+    __syncthreads();  // the last tile's elements are read
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int p = pr + (256 / CR) * i;
+      tile[p][tile_col<CR>(p, c)] = in[i];
+    }
+    __syncthreads();
+    if (r0 + rr < rows && p0 + pg < k) {
+      const int er = exps[rr];
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = (p0 + pg + j < k) ? scaled<kForm>(double(tile[pg + j][tile_col<CR>(pg + j, rr)]), er)
+                                 : scaled_zero<kForm>();
+      write_residues8<kForm>(a, Y, plane, size_t(r0 + rr) * kpad + p0 + pg, v);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -440,9 +562,11 @@ struct ReconArgs {
 // operations, is within ~1e-12 of sum_l r_l w_l / M (|X 2^T / M| <= 128 N);
 // |C'| <= M/8 keeps that exact value within 1/8 of the integer q, so
 // q = rint(t) is the one of exact arithmetic.
+template <class T>
 __global__ void __launch_bounds__(256)
-reconstruct(double* __restrict__ c, size_t ldc, int m, int n, const int8_t* __restrict__ R,
-            size_t ldr, const int* __restrict__ ea, const int* __restrict__ eb, ReconArgs a) {
+reconstruct(T* __restrict__ c, size_t ldc, int m, int n, const int8_t* __restrict__ R,
+            size_t ldr, const int* __restrict__ ea, const int* __restrict__ eb,
+            const __grid_constant__ ReconArgs a) {
   const int bpr = (n + 1023) / 1024;  // CTAs per row of C
   const int i = blockIdx.x / bpr;
   const int j0 = ((blockIdx.x % bpr) * 256 + threadIdx.x) * 4;
@@ -455,13 +579,13 @@ reconstruct(double* __restrict__ c, size_t ldc, int m, int n, const int8_t* __re
   for (int l = 0; l < kMaxModuli; ++l)
     if (l < a.nmod) rv[l] = __ldg(reinterpret_cast<const uint32_t*>(Ri + size_t(l) * plane));
   // C and the column scales are requested with the residues (one round trip)
-  double* ci = c + size_t(i) * ldc;
+  T* ci = c + size_t(i) * ldc;
   double c_old[4];
   int fj[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const bool in = j0 + u < n;
-    c_old[u] = in ? ci[j0 + u] : 0.0;
+    c_old[u] = in ? double(ci[j0 + u]) : 0.0;
     fj[u] = in ? __ldg(eb + j0 + u) : 0;
   }
   constexpr double kBias = 4503599627370624.0;  // 2^52 + 128
@@ -496,7 +620,7 @@ reconstruct(double* __restrict__ c, size_t ldc, int m, int n, const int8_t* __re
       val = cp * __longlong_as_double(static_cast<long long>(sc + 1023) << 52);
     else
       val = ldexp(cp, sc);
-    ci[j] = c_old[u] + val;
+    ci[j] = T(c_old[u] + val);  // f32: rounded once
   }
 }
 
@@ -536,7 +660,7 @@ bool make_plane_map(CUtensorMap* map, void* base, int cols, int rows, int nplane
 size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct DgemmLayout {
-  size_t kpad, ldr, a_res, b_res, r, ea, eb, emax_a, emax_b, total;
+  size_t kpad, ldr, a_res, b_res, r, ea, eb, top_a, top_b, total;
 };
 
 DgemmLayout dgemm_layout(int m, int n, int k, int nmod) {
@@ -548,9 +672,9 @@ DgemmLayout dgemm_layout(int m, int n, int k, int nmod) {
   L.r = L.b_res + a256(size_t(nmod) * n * L.kpad);
   L.ea = L.r + a256(size_t(nmod) * m * L.ldr);
   L.eb = L.ea + a256(size_t(m) * sizeof(int));
-  L.emax_a = L.eb + a256(size_t(n) * sizeof(int));
-  L.emax_b = L.emax_a + a256(size_t(m) * sizeof(int));
-  L.total = L.emax_b + a256(size_t(n) * sizeof(int));
+  L.top_a = L.eb + a256(size_t(n) * sizeof(int));
+  L.top_b = L.top_a + a256(size_t(m) * sizeof(double));
+  L.total = L.top_b + a256(size_t(n) * sizeof(double));
   return L;
 }
 
@@ -583,36 +707,67 @@ ResidueArgs residue_args(const OzakiPlan& p) {
   return a;
 }
 
-// Scales, rounds and splits op(X) into residue planes Y[nmod][rows][kpad];
-// `emax` is scratch for rows ints.
-cudaError_t prepare(const double* x, size_t ld, bool rows_contig, int rows, int k, size_t kpad,
-                    int bits, int* emax, int* e, int8_t* Y, const ResidueArgs& ra,
-                    cudaStream_t s, Mask mask = Mask{nullptr, 0, 1}) {
-  const int rb = (rows + 255) / 256;
+template <int kForm, class T>
+cudaError_t prepare_form(const T* x, size_t ld, bool rows_contig, int rows, int k, size_t kpad,
+                         int bits, void* top, int* e, int8_t* Y, const ResidueArgs& ra,
+                         cudaStream_t s, Mask mask) {
+  using Bits = typename Magnitude<T>::Bits;
+  Bits* maxima = static_cast<Bits*>(top);
+  const bool scan = size_t(rows) * k * sizeof(T) <= kScanBytes;
   if (rows_contig) {
-    emax_rows<<<rows, 256, 0, s>>>(x, ld, rows, k, emax);
-  } else {
-    fill_int<<<rb, 256, 0, s>>>(emax, rows, INT_MIN);
-    emax_cols<<<dim3(rb, (k + kColChunk - 1) / kColChunk), 256, 0, s>>>(x, ld, rows, k, emax,
-                                                                         mask);
+    if (!scan) {
+      maxima_rows<T><<<rows, 256, 0, s>>>(x, ld, k, maxima);
+      residues_rows<kForm, 256, false, T>
+          <<<rows, 256, 0, s>>>(x, ld, rows, k, kpad, bits, e, Y, ra, maxima);
+    } else if (k <= 512) {  // short rows share a CTA
+      residues_rows<kForm, 64, true, T>
+          <<<(rows + 3) / 4, 256, 0, s>>>(x, ld, rows, k, kpad, bits, e, Y, ra, nullptr);
+    } else {
+      residues_rows<kForm, 256, true, T>
+          <<<rows, 256, 0, s>>>(x, ld, rows, k, kpad, bits, e, Y, ra, nullptr);
+    }
+    return cudaGetLastError();
   }
-  finalize_exps<<<rb, 256, 0, s>>>(emax, rows, bits, e);
+  int parts = 8;
+  while (parts > (k + 127) / 128) parts /= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned((rows + 15) / 16) * parts);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = unsigned(parts);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (scan)
+    return cudaLaunchKernelEx(&cfg, residues_cols<kForm, true, T>, x, ld, rows, k, kpad, bits, e,
+                              Y, ra, mask, parts, static_cast<const Bits*>(nullptr));
+  cudaError_t err = cudaMemsetAsync(maxima, 0, size_t(rows) * sizeof(Bits), s);
+  if (err != cudaSuccess) return err;
+  maxima_cols<T><<<dim3((rows + 255) / 256, (k + 127) / 128), 256, 0, s>>>(x, ld, rows, k, maxima,
+                                                                          mask);
+  if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  const int ntiles = (k + 63) / 64;
+  residues_cols<kForm, false, T><<<unsigned((rows + 31) / 32) * ntiles, 256, 0, s>>>(
+      x, ld, rows, k, kpad, bits, e, Y, ra, mask, ntiles, maxima);
+  return cudaGetLastError();
+}
+
+// Scales, rounds and splits op(X) into residue planes Y[nmod][rows][kpad], the
+// rows' exponents into e; `top` is scratch for rows doubles.
+template <class T>
+cudaError_t prepare(const T* x, size_t ld, bool rows_contig, int rows, int k, size_t kpad,
+                    int bits, void* top, int* e, int8_t* Y, const ResidueArgs& ra, cudaStream_t s,
+                    Mask mask = Mask{nullptr, 0, 1}) {
   // scaled elements up to 2^47 take three 16-bit digits, up to 2^50 the
   // biased form of four 14-bit digits, the rest the plain form
-  const int form = bits <= 47 ? kBiased16 : (bits <= 50 ? kBiased14 : kPlain);
-  if (rows_contig) {
-    auto kern = form == kBiased16 ? residues_rows<kBiased16>
-                                  : (form == kBiased14 ? residues_rows<kBiased14>
-                                                       : residues_rows<kPlain>);
-    kern<<<rows, 256, 0, s>>>(x, ld, rows, k, kpad, e, Y, ra);
-  } else {
-    dim3 grid((rows + 31) / 32, (k + 63) / 64);
-    auto kern = form == kBiased16 ? residues_cols<kBiased16>
-                                  : (form == kBiased14 ? residues_cols<kBiased14>
-                                                       : residues_cols<kPlain>);
-    kern<<<grid, 256, 0, s>>>(x, ld, rows, k, kpad, e, Y, ra, mask);
-  }
-  return cudaGetLastError();
+  if (bits <= 47)
+    return prepare_form<kBiased16>(x, ld, rows_contig, rows, k, kpad, bits, top, e, Y, ra, s, mask);
+  if (bits <= 50)
+    return prepare_form<kBiased14>(x, ld, rows_contig, rows, k, kpad, bits, top, e, Y, ra, s, mask);
+  return prepare_form<kPlain>(x, ld, rows_contig, rows, k, kpad, bits, top, e, Y, ra, s, mask);
 }
 
 }  // namespace
@@ -661,7 +816,8 @@ size_t ozaki_dgemm_workspace(int m, int n, int k, int nmod) {
   return dgemm_layout(m, n, k, nmod).total;
 }
 
-cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int n, int k,
+template <class T>
+cudaError_t ozaki_dgemm(T* c, const T* a, const T* b, int m, int n, int k,
                         size_t lda, size_t ldb, size_t ldc, bool transa, bool transb, int nmod,
                         void* workspace, cudaStream_t stream, const cudaEvent_t* events,
                         const uint8_t* tab, size_t ldtab, int blk, cudaEvent_t c_ready,
@@ -684,22 +840,21 @@ cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int 
   mark(0);
   // op(A) rows are i (k contiguous unless transa); op(B) "rows" are j
   // (k contiguous only when transb).
-  int* emax_a = reinterpret_cast<int*>(ws + L.emax_a);
-  int* emax_b = reinterpret_cast<int*>(ws + L.emax_b);
   cudaError_t err = cudaSuccess;
-  // With both operands to prepare, A's kernels run on a side stream beside B's:
-  // the residue kernels are bound by instruction issue and the exponent scans
-  // by DRAM, so the two chains overlap.  The side stream joins back before the
+  // With both operands to prepare, A's kernel runs on a side stream beside B's:
+  // their phases are bound by instruction issue (residues) and by memory (the
+  // scan for the exponents), so the two overlap.  The side stream joins back before the
   // GEMM (the fork and join are events, so a stream capture follows them).
   SideScope side((!reuse_a && !reuse_b) ? side_stream() : nullptr, stream);
   if ((err = side.fork()) != cudaSuccess) return err;
   const cudaStream_t sa = side.stream();
   if (!reuse_a) {
-    err = prepare(a, lda, !transa, m, k, L.kpad, plan.alpha, emax_a, ea, a_res, ra, sa);
+    err = prepare(a, lda, !transa, m, k, L.kpad, plan.alpha, ws + L.top_a, ea,
+                  a_res, ra, sa);
     if (err != cudaSuccess) return err;
   }
   if (!reuse_b) {
-    err = prepare(b, ldb, transb, n, k, L.kpad, plan.beta, emax_b, eb, b_res, ra, stream,
+    err = prepare(b, ldb, transb, n, k, L.kpad, plan.beta, ws + L.top_b, eb, b_res, ra, stream,
                   Mask{tab, ldtab, blk > 0 ? blk : 1});
     if (err != cudaSuccess) return err;
   }
@@ -743,5 +898,14 @@ cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int 
   mark(3);
   return cudaGetLastError();
 }
+
+template cudaError_t ozaki_dgemm<double>(double*, const double*, const double*, int, int, int,
+                                         size_t, size_t, size_t, bool, bool, int, void*,
+                                         cudaStream_t, const cudaEvent_t*, const uint8_t*, size_t,
+                                         int, cudaEvent_t, int, int, bool, bool);
+template cudaError_t ozaki_dgemm<float>(float*, const float*, const float*, int, int, int, size_t,
+                                        size_t, size_t, bool, bool, int, void*, cudaStream_t,
+                                        const cudaEvent_t*, const uint8_t*, size_t, int,
+                                        cudaEvent_t, int, int, bool, bool);
 
 }  // namespace cfgmm

@@ -54,7 +54,10 @@ size_t ozaki_dgemm_workspace(int m, int n, int k, int nmod);
 // `reuse_a` (`reuse_b`) takes the residues and exponents of A (B) that an
 // earlier call on the same stream, workspace, A (B), k and nmod left there
 // instead of forming them again.
-cudaError_t ozaki_dgemm(double* c, const double* a, const double* b, int m, int n, int k,
+// T is double or float: f32 operands are widened exactly as they are read, and each
+// element of an f32 C is rounded once.
+template <class T>
+cudaError_t ozaki_dgemm(T* c, const T* a, const T* b, int m, int n, int k,
                         size_t lda, size_t ldb, size_t ldc, bool transa, bool transb, int nmod,
                         void* workspace, cudaStream_t stream,
                         const cudaEvent_t* events = nullptr, const uint8_t* tab = nullptr,
