@@ -33,7 +33,11 @@
 //      form used; form 3 remains for CFGMM_AODM_PIPE=0.
 //   4. aodm_reduce: adds the per-row-tile partial sums of each grid tile in a
 //      fixed order, so results are deterministic run to run (unlike the
-//      reference, whose lock order varies).
+//      reference, whose lock order varies).  In a small single call the warp that
+//      stores a grid tile's last partial sums does it (3b).
+//   A single call is three launches, or four with 4: lists and symmetry check, work
+//   list, 3b.
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -55,36 +59,119 @@ constexpr int LIST_CAP = 8192;  // active-list entries staged in shared memory
 
 // ---------------------------------------------------------------------------
 // 1. active lists: lists[b*nao + i] = i-th active AO of block b, counts[b]
+//    Each of the CTA's eight warps takes an eighth of up to 16384 AOs: the mask
+//    bytes are requested eight at a time, their ballots kept in shared memory, and
+//    after one barrier each warp writes its part of the list behind the others'.
+//    (256 AOs at a time, each with its own loads and three barriers, took 11 us for
+//    2228 AOs.)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-aodm_block_lists(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nblk,
-                 int* __restrict__ lists, int* __restrict__ counts) {
-  const int b = blockIdx.x;
-  if (b >= nblk) return;
+constexpr int LIST_WORDS = 64;  // ballots per warp and pass
+
+__device__ __forceinline__ void
+block_list(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int b, int* __restrict__ lists,
+           int* __restrict__ counts) {
+  __shared__ uint32_t words[8][LIST_WORDS];
   __shared__ int warp_tot[8];
-  __shared__ int base_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) base_s = 0;
-  __syncthreads();
+  const uint8_t* col = tab + b;
   int* out = lists + size_t(b) * nao;
-  for (int u0 = 0; u0 < nao; u0 += 256) {
-    const int u = u0 + tid;
-    const bool on = (u < nao) && tab[size_t(u) * ldtab + b] != 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, on);
-    if (lane == 0) warp_tot[warp] = __popc(bal);
+  int base = 0;
+  for (int first = 0; first < nao; first += 8 * 32 * LIST_WORDS) {
+    const int left = min(nao - first, 8 * 32 * LIST_WORDS);
+    const int nw = (left + 255) / 256;  // ballots of a warp
+    const int u0 = first + warp * nw * 32;
+    int n = 0;
+    for (int i = 0; i < nw; i += 8) {
+      uint8_t on[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int u = u0 + (i + q) * 32 + lane;
+        on[q] = i + q < nw && u < nao ? col[size_t(u) * ldtab] : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, on[q] != 0);
+        n += __popc(bal);
+        if (lane == 0 && i + q < nw) words[warp][i + q] = bal;
+      }
+    }
+    if (lane == 0) warp_tot[warp] = n;
     __syncthreads();
-    int before = base_s;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (on) out[before + __popc(bal & ((1u << lane) - 1u))] = u;
-    __syncthreads();
-    if (tid == 0) {
-      int t = 0;
-      for (int w = 0; w < 8; ++w) t += warp_tot[w];
-      base_s += t;
+    int at = base;
+    for (int w = 0; w < 8; ++w) {
+      base += warp_tot[w];
+      if (w < warp) at += warp_tot[w];
+    }
+    for (int i = 0; i < nw; ++i) {
+      const uint32_t bal = words[warp][i];
+      if (bal >> lane & 1u) out[at + __popc(bal & ((1u << lane) - 1u))] = u0 + i * 32 + lane;
+      at += __popc(bal);
     }
     __syncthreads();
   }
-  if (tid == 0) counts[b] = base_s;
+  if (tid == 0) counts[b] = base;
+}
+
+__global__ void __launch_bounds__(256)
+aodm_block_lists(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nblk,
+                 int* __restrict__ lists, int* __restrict__ counts) {
+  if (int(blockIdx.x) < nblk) block_list(tab, ldtab, nao, blockIdx.x, lists, counts);
+}
+
+// Whether tile (by, bx) of d (32 x 32, by <= bx) differs from the transpose of tile
+// (bx, by); to every thread of the CTA (256).
+__device__ __forceinline__ bool asym_tile(const double* __restrict__ d, size_t stride_ao, int nao,
+                                          int bx, int by) {
+  __shared__ double tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  // both tiles are requested before the barrier: tile (by, bx) into shared
+  // memory, this thread's elements of tile (bx, by) into registers
+  double mine[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = ty + 8 * k;
+    const int r = by * 32 + i, c = bx * 32 + tx;
+    tile[i][tx] = (r < nao && c < nao) ? d[size_t(r) * stride_ao + c] : 0.0;
+    const int r2 = bx * 32 + i, c2 = by * 32 + tx;
+    mine[k] = (r2 < nao && c2 < nao) ? d[size_t(r2) * stride_ao + c2] : 0.0;
+  }
+  __syncthreads();
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = ty + 8 * k;
+    const int r2 = bx * 32 + i, c2 = by * 32 + tx;
+    if (r2 < nao && c2 < nao) bad |= !(mine[k] == tile[tx][i]);
+  }
+  return __syncthreads_or(bad) != 0;
+}
+
+// A single call's first launch: the block lists (CTAs 0 .. nblk-1) and, beside
+// them, the symmetry check of every D_s (the `ncheck` CTAs after them, each with
+// every ncheck-th of the tile pairs of one s after the other; bad[i] = whether CTA i
+// found one that differs).
+__global__ void __launch_bounds__(256)
+aodm_lists_and_check(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nblk,
+                     int* __restrict__ lists, int* __restrict__ counts,
+                     const double* __restrict__ dms, size_t stride_ao, int nset, int ncheck,
+                     uint8_t* __restrict__ bad) {
+  if (int(blockIdx.x) < nblk) {
+    block_list(tab, ldtab, nao, blockIdx.x, lists, counts);
+    return;
+  }
+  const int me = int(blockIdx.x) - nblk;
+  const unsigned nt = unsigned(nao + 31) / 32;
+  const unsigned pairs = nt * (nt + 1) / 2;  // below 2^32 / nset: D would not fit otherwise
+  bool any = false;
+  for (unsigned t = me; t < pairs * nset && !any; t += ncheck) {
+    const unsigned s = t / pairs, k = t % pairs;  // pair (by <= bx) at bx (bx + 1) / 2 + by
+    unsigned bx = unsigned((sqrtf(8.0f * float(k) + 1.0f) - 1.0f) * 0.5f);
+    while (bx * (bx + 1) / 2 > k) --bx;
+    while ((bx + 1) * (bx + 2) / 2 <= k) ++bx;
+    any = asym_tile(dms + size_t(s) * stride_ao * stride_ao, stride_ao, nao, int(bx),
+                    int(k - bx * (bx + 1) / 2));
+  }
+  if (threadIdx.x == 0) bad[me] = any;
 }
 
 // ---------------------------------------------------------------------------
@@ -96,19 +183,24 @@ aodm_block_lists(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nbl
 //    together.  In block order a taxol-size call's SMs were busy 93 % of the
 //    kernel's time, the longest items (129 k cycles) starting at any point.
 //    Every item has its own partial-sum slot, so the order changes no result.
+//    With `bad` (aodm_lists_and_check's findings) the asymmetry flag is set too.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
 aodm_build_items(const int* __restrict__ counts, int nblk, int gsub, int4* __restrict__ items,
-                 int* __restrict__ counters, int ncounters) {
+                 int* __restrict__ counters, int ncounters, const uint8_t* __restrict__ bad,
+                 int ncheck) {
   constexpr int RANKS = 1024;           // longer lists share the first rank
   __shared__ int start[RANKS + 1];      // by tiles left: blocks, then the next free item
   __shared__ int warp_tot[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) g_aodm_error = 0;
   // [ncounters] = total, [ncounters + 1] = asymmetry flag
-  for (int i = tid; i <= ncounters + 1; i += 1024) counters[i] = 0;
+  for (int i = tid; i <= ncounters; i += 1024) counters[i] = 0;
   for (int r = tid; r <= RANKS; r += 1024) start[r] = 0;
-  __syncthreads();
+  int differs = 0;
+  for (int i = tid; i < ncheck; i += 1024) differs |= bad[i];
+  differs = __syncthreads_or(differs);
+  if (tid == 0) counters[ncounters + 1] = differs != 0;
   // items with r tiles left: one of every block with at least r of them; rank
   // RANKS takes all above it too
   for (int b = tid; b < nblk; b += 1024) {
@@ -145,6 +237,9 @@ aodm_build_items(const int* __restrict__ counts, int nblk, int gsub, int4* __res
   __syncthreads();
   for (int b = tid; b < nblk; b += 1024) {
     const int nt = (counts[b] + TU - 1) / TU;
+    // .w of entry bg: the main kernel's ticket of block tile bg (its own or another
+    // item's entry, zero either way)
+    for (int gt = 0; gt < gsub; ++gt) items[b * gsub + gt].w = 0;
     for (int u = 0; u < nt; ++u) {
       const int at = atomicAdd(&start[min(nt - u, RANKS)], gsub);
       for (int gt = 0; gt < gsub; ++gt) items[at + gt] = make_int4(0, b * gsub + gt, u, 0);
@@ -451,6 +546,31 @@ __device__ __forceinline__ double sym_factor(int r, int c) {
   return c < r ? 0.0 : (c == r ? 0.5 : 1.0);
 }
 
+// rho[j] += sum over u < nt of part[u * step + j], j < width <= 64, by one warp;
+// the partial sums come from other SMs (read past L1), eight in flight per lane.
+__device__ __forceinline__ void reduce_tile(const double* part, size_t step, int nt, double* rho,
+                                            int width, int lane) {
+  double v[2] = {0.0, 0.0};
+  for (int u = 0; u < nt; u += 4) {
+    double x[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        x[i][h] = u + i < nt ? __ldcg(part + size_t(u + i) * step + 32 * h + lane) : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (u + i < nt) v[h] += x[i][h];
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int j = 32 * h + lane;
+    if (j < width) rho[j] = v[h] + rho[j];
+  }
+}
+
 // Bounded wait whose outcome is the same for every lane of the warp.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code,
                                           uint64_t lim) {
@@ -504,12 +624,15 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
     uint32_t fill = 0;                // stage fills issued so far
     for (int n = 0;; ++n) {
       const int slot = n % RING;
-      if (tid == 0) {  // fetch the next item for every warp of the CTA
+      // the next item for every warp of the CTA: the first is the CTA's own, the others
+      // are drawn when they are needed (an item drawn ahead waits behind the one
+      // being loaded while other CTAs are idle: 38 -> 43 us at 512 AOs x 4096 points)
+      if (tid == 0) {
         int it = total;
         if (*reinterpret_cast<volatile int*>(err) == 0 &&
             (n < RING ||
              tc::mbar_wait(&iempty[slot], ((n / RING) - 1) & 1, err, kErrItemEmpty, false, lim)))
-          it = min(atomicAdd(counter, 1), total);
+          it = min(n == 0 ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(counter, 1), total);
         ring[slot] = it;
         tc::mbar_arrive(&ifull[slot]);
       }
@@ -758,6 +881,26 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
         for (int w = 0; w < CWM; ++w) v += rb[(s * CWM + w) * TG + j];
         p.partial[(pslot * p.nset_max + set0 + s) * TG + j] = sym ? 2.0 * v : v;
       }
+      if (p.tickets) {
+        // the warp that stores the block tile's last partial sums adds them all into
+        // rho, in the fixed order of aodm_reduce
+        const int nt = (t.nb + TU - 1) / TU;
+        int ticket = 0;
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          ticket = atomicAdd(&p.tickets[4 * size_t(t.bg)], 1);
+        }
+        ticket = __shfl_sync(0xffffffffu, ticket, 0);
+        if (ticket == nt * (NCONS / 32) * p.ngroups - 1) {
+          __threadfence();
+          const double* part =
+              p.partial + (t.B->partial_off + size_t(t.bg) * p.max_utiles) * p.nset_max * TG;
+          for (int s = 0; s < t.B->nset; ++s)
+            if (t.gw > 0) reduce_tile(part + s * TG, size_t(p.nset_max) * TG, nt,
+                                      t.B->rhos + size_t(s) * t.B->stride_grid + t.g0, t.gw, lane);
+        }
+      }
     }
   }
 }
@@ -796,36 +939,15 @@ __global__ void aodm_reset_counters(int* counters, int ngroups) {
   }
 }
 
-// *asym = 1 if some D_s differs from its transpose.  Block (bx, by, s) with
-// by <= bx compares the 32 x 32 tile (by, bx) with the transpose of (bx, by).
+// *asym = 1 if some D_s differs from its transpose (plans).  Block (bx, by, s)
+// with by <= bx compares the 32 x 32 tile (by, bx) with the transpose of (bx, by).
 __global__ void __launch_bounds__(256)
 aodm_sym_check(const double* __restrict__ dms, size_t stride_ao, size_t dm_stride, int nao,
                int* asym) {
-  const int bx = blockIdx.x, by = blockIdx.y;
-  if (by > bx) return;
-  __shared__ double tile[32][33];
-  const double* d = dms + size_t(blockIdx.z) * dm_stride;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  // both tiles are requested before the barrier: tile (by, bx) into shared
-  // memory, this thread's elements of tile (bx, by) into registers
-  double mine[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int i = ty + 8 * k;
-    const int r = by * 32 + i, c = bx * 32 + tx;
-    tile[i][tx] = (r < nao && c < nao) ? d[size_t(r) * stride_ao + c] : 0.0;
-    const int r2 = bx * 32 + i, c2 = by * 32 + tx;
-    mine[k] = (r2 < nao && c2 < nao) ? d[size_t(r2) * stride_ao + c2] : 0.0;
-  }
-  __syncthreads();
-  bool bad = false;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int i = ty + 8 * k;
-    const int r2 = bx * 32 + i, c2 = by * 32 + tx;
-    if (r2 < nao && c2 < nao) bad |= !(mine[k] == tile[tx][i]);
-  }
-  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(asym, 1);
+  if (blockIdx.y > blockIdx.x) return;
+  if (asym_tile(dms + size_t(blockIdx.z) * dm_stride, stride_ao, nao, blockIdx.x, blockIdx.y) &&
+      threadIdx.x == 0)
+    atomicOr(asym, 1);
 }
 
 template <int NS, int TKT>
@@ -995,7 +1117,8 @@ Layout layout(size_t nao, size_t ngrid, size_t nset, size_t blk) {
 
 cudaError_t aodm_build_items_launch(const int* counts, int nblk, int gsub, int4* items,
                                     int* counters, int ncounters, cudaStream_t stream) {
-  aodm_build_items<<<1, 1024, 0, stream>>>(counts, nblk, gsub, items, counters, ncounters);
+  aodm_build_items<<<1, 1024, 0, stream>>>(counts, nblk, gsub, items, counters, ncounters,
+                                           nullptr, 0);
   return cudaGetLastError();
 }
 
@@ -1030,10 +1153,21 @@ cudaError_t aodmao2rho_fp64(double* rhos, const double* dms, const double* ao_lh
   int* counters = reinterpret_cast<int*>(ws + L.counters);
   double* partial = reinterpret_cast<double*>(ws + L.partial);
 
-  aodm_block_lists<<<nblk, 256, 0, stream>>>(tab, ldtab, nao, nblk, lists, counts);
+  // the half contraction needs D = D^T and phi_lhs = phi_rhs (one array)
+  const bool sym = pipe_enabled() && aodm_sym_enabled() && ao_lhs == ao_rhs;
+  // tile pairs to compare, a CTA each up to 16384; their findings wait in the
+  // partial sums' place, which is written later
+  const long long nt32 = (nao + 31) / 32;
+  const int ncheck =
+      sym ? int(std::min({nt32 * (nt32 + 1) / 2 * nset, 16384ll, (long long)(L.total - L.partial)}))
+          : 0;
+  uint8_t* bad = reinterpret_cast<uint8_t*>(partial);
+  aodm_lists_and_check<<<unsigned(nblk + ncheck), 256, 0, stream>>>(
+      tab, ldtab, nao, nblk, lists, counts, dms, stride_ao, nset, ncheck, bad);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  aodm_build_items<<<1, 1024, 0, stream>>>(counts, nblk, gsub, items, counters, ngroups);
+  aodm_build_items<<<1, 1024, 0, stream>>>(counts, nblk, gsub, items, counters, ngroups, bad,
+                                           ncheck);
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
 
   AodmArgs a{};
@@ -1053,22 +1187,22 @@ cudaError_t aodmao2rho_fp64(double* rhos, const double* dms, const double* ao_lh
   a.partial = partial;
   if (pipe_enabled()) {
     a.one.rhs_bulk = aodm_rhs_bulk(ao_rhs, stride_grid, blk) ? 1 : 0;
-    // the half contraction needs D = D^T and phi_lhs = phi_rhs (one array)
-    if (aodm_sym_enabled() && ao_lhs == ao_rhs) {
-      a.asym = counters + ngroups + 1;
-      if ((err = aodm_launch_sym_check(dms, stride_ao, nao, nset, counters + ngroups + 1,
-                                       stream)) != cudaSuccess)
-        return err;
-    }
+    if (sym) a.asym = counters + ngroups + 1;
+    // The kernel's own reduction saves a launch (2 us and the reduction's 5 to 11) and
+    // costs each item a fence while its CTA's tensor pipe waits: with at most 4096
+    // items (28 per SM) 512 AOs x 4096 points x 1 take 40 us instead of 44; at 8960
+    // possible items 2228 AOs x 16384 points x 3 take 1.03 ms with it and 1.01 without.
+    if ((long long)nblk * gsub * max_utiles <= 4096) a.tickets = &items[0].w;
     unsigned long long ns = 0;
     if (take_wait_injection(0, &ns)) {  // cfgmm_test_arm_wait_timeout
       a.inject = 1;
       a.wait_ns = ns;
     }
     err = aodm_launch_pipe(a, cfg.ns, stream);
-  }
-  else
+    if (a.tickets) return err;  // rho is reduced
+  } else {
     err = aodm_launch_main(a, cfg, stream);
+  }
   if (err != cudaSuccess) return err;
   return aodm_launch_reduce(a, nullptr, nblk * gsub, stream);
 }

@@ -35,6 +35,8 @@ struct AodmArgs {
   int ngroups;
   const int* asym;              // null, or counters + ngroups + 1: 0 when every D_s is symmetric
   double* partial;              // [slot][nset_max][64]
+  int* tickets;                 // null, or 4 ints per block tile of `one`, the first zero: the
+                                // pipelined kernel adds the partial sums into rho itself
   unsigned long long wait_ns;   // bound of the pipelined kernel's waits (0: the default 2 s)
   int inject;                   // test hook: the pipelined kernel's first stage is never published
 };

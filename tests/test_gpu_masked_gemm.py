@@ -126,7 +126,8 @@ def test_large_masked_host_call_in_blocks(cm, wl, prec):
     (False, 40, 1400, 250, 200, 0.2, 2),   # five pieces of 40 columns
     (False, 5, 33, 70, 48, 1.0, 0),        # a block wider than C, every tile present
     (False, 300, 320, 96, 80, 0.0, 0),     # no tile present: C is untouched
-    (False, 128, 256, 64, 32, 0.5, 0),     # two K steps and one wave: the direct form
+    (False, 128, 256, 64, 32, 0.5, 0),     # small: the dense form on zero-filled tiles
+    (False, 120, 96, 20000, 48, 0.3, 0),   # lists of more rows than one pass builds
     (False, 1000, 1600, 640, 33, 0.65, 0),  # both forms enqueued, compacted runs
     (False, 1000, 1600, 640, 33, 0.9, 0),  # both forms enqueued, dense runs
 ])
