@@ -9,7 +9,7 @@
 //   integer round(x' 2^48) (digits_packed below).  The products of the
 //   digits of D and phi whose levels add up to L = i + j <= 6 are summed
 //   EXACTLY in one INT32 accumulator per level:
-//     S_L[u][g] = sum_{i+j=L} sum_v d_i(u,v) p_j(v,g)        (28 INT8 MMAs)
+//     S_L[u][g] = sum_{i+j=L} sum_v d_i(u,v) p_j(v,g)        (28 products)
 //   and X[u][g] = 2^-(tau_u + sigma_g) sum_L 2^(-8L) S_L[u][g] in FP64.  The
 //   dropped levels L >= 7 weigh at most 6 * 2^-54 of the largest scaled
 //   product and the digit remainders 2^-55 each, so X carries about 51 bits
@@ -41,10 +41,10 @@
 //                     along a row read consecutive columns; two shuffle rounds
 //                     turn the 8-byte elements into digit planes, stored
 //                     without bank conflicts) and later run the epilogue;
-//                     warp 12 issues the 28 MMAs of a chunk (M=128, N=64, K=32)
-//                     into 7 TMEM level accumulators (448 columns), grouped by
-//                     D digit so that each D plane is read once and reused
-//                     from the tensor core's collector buffer; warp 13
+//                     warp 12 issues a chunk's 28 digit products (M=128, 64
+//                     points, K=32) into 7 TMEM level accumulators (448
+//                     columns) as 10 MMAs of N up to 256
+//                     (tc::mma_digit_products); warp 13
 //                     bulk-loads the phi digit tiles.  The epilogue rebuilds X
 //                     in FP64, weights it with phi and reduces over the rows
 //                     of each warp; X never leaves the SM.
@@ -584,7 +584,6 @@ __global__ void __launch_bounds__(THREADS, 1) split_main(SplitArgs p) {
   } else if (warp == GATHER_WARPS) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      const uint32_t idesc = tc::idesc_i8(TU, TG);
       uint32_t seq = 0, nitem = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++nitem) {
@@ -605,28 +604,8 @@ __global__ void __launch_bounds__(THREADS, 1) split_main(SplitArgs p) {
           tc::fence_after_sync();
           const uint32_t a0 = tc::smem_u32(smem + stg * STAGE);
           const uint32_t b0 = a0 + A_STAGE;
-          // D digit i meets phi digits 0 .. NSL-1-i (levels i .. NSL-1) in
-          // consecutive MMAs, so its plane is read from shared memory once and
-          // held in the collector buffer for the rest; level L still receives
-          // its products in the order i = 0, 1, ..., L.
-#pragma unroll
-          for (int i = 0; i < NSL; ++i) {
-            const uint64_t ad = tc::smem_desc_k32(a0 + i * A_SLICE);
-            const bool acc = c > kc0 || i > 0;
-#pragma unroll
-            for (int L = i; L < NSL; ++L) {
-              const uint32_t d = tmem + uint32_t(L * TG);
-              const uint64_t bd = tc::smem_desc_k32(b0 + (L - i) * B_SLICE);
-              if (i == NSL - 1)
-                tc::mma_i8(d, ad, bd, idesc, acc);
-              else if (L == i)
-                tc::mma_i8_collect<tc::ACollector::kFill>(d, ad, bd, idesc, acc);
-              else if (L == NSL - 1)
-                tc::mma_i8_collect<tc::ACollector::kLastUse>(d, ad, bd, idesc, acc);
-              else
-                tc::mma_i8_collect<tc::ACollector::kUse>(d, ad, bd, idesc, acc);
-            }
-          }
+          // D digits (the A operand) times phi digits
+          tc::mma_digit_products<NSL, TG>(tmem, a0, A_SLICE, b0, c == kc0);
           tc::mma_commit(&empty[stg]);
         }
         if (!ok) break;

@@ -174,41 +174,6 @@ __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t
       : "memory");
 }
 
-// mma_i8 with the A operand kept in the tensor core's collector buffer across
-// consecutive MMAs that share it: kFill reads A from shared memory and keeps
-// it, kUse reads the kept copy, kLastUse reads it and releases it.  The same A
-// descriptor is passed each time.
-enum class ACollector { kFill, kUse, kLastUse };
-template <ACollector U>
-__device__ __forceinline__ void mma_i8_collect(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                               uint32_t idesc, bool accumulate) {
-  if constexpr (U == ACollector::kFill) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8.collector::a::fill [%0], %1, %2, %3, p;\n\t}" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(uint32_t(accumulate))
-        : "memory");
-  } else if constexpr (U == ACollector::kUse) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8.collector::a::use [%0], %1, %2, %3, p;\n\t}" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(uint32_t(accumulate))
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(uint32_t(accumulate))
-        : "memory");
-  }
-}
-
 // Arrives once on `bar` when all previously issued tcgen05.mma of this thread
 // have completed (their shared-memory operands may then be overwritten).
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -420,6 +385,36 @@ __host__ __device__ constexpr uint32_t idesc_i8(int M, int N) {
          | (1u << 10)                   // B format: signed 8-bit
          | (uint32_t(N >> 3) << 17)     // N / 8
          | (uint32_t(M >> 4) << 24);    // M / 16
+}
+
+// All products of one chunk of two digit-plane operands with i + j < NSL, for one
+// thread to issue: A digit i (a0 + i a_slice: M = 128 rows of 32 bytes, 32-byte
+// swizzle) with B digits 0 .. NSL-1-i (b0 + j TN * 32: TN rows each), level i + j
+// accumulating in the TN columns from tmem + (i + j) TN.  The B planes stand one
+// behind the other, so the planes 0 .. n of one A digit are one operand of (n + 1) TN
+// rows whose products fall into the levels i .. i + n, adjacent columns: one MMA of
+// N = (n + 1) TN up to 256 instead of n + 1 MMAs of N = TN.  (An MMA reads M + N rows
+// of 32 bytes from shared memory; at N = 64 that takes 48 cycles and more, at N = 128
+// and above less than the products: 28 MMAs of N = 64 took 2.1 k cycles per chunk of
+// 7 digits, their products are 0.9 k.)  `first`: the levels start over.
+template <int NSL, int TN>
+__device__ __forceinline__ void mma_digit_products(uint32_t tmem, uint32_t a0, uint32_t a_slice,
+                                                   uint32_t b0, bool first) {
+  constexpr int kMost = 256 / TN;  // planes of one MMA
+#pragma unroll
+  for (int i = 0; i < NSL; ++i) {
+    const uint64_t ad = smem_desc_k32(a0 + uint32_t(i) * a_slice);
+    const int planes = NSL - i;
+    const int pieces = (planes + kMost - 1) / kMost;
+    const bool acc = i > 0 || !first;
+#pragma unroll
+    for (int q = 0; q < pieces; ++q) {
+      const int j0 = (q * planes + pieces - 1) / pieces;        // planes j0 .. j1-1: equal
+      const int j1 = ((q + 1) * planes + pieces - 1) / pieces;  // pieces, the larger ones first
+      mma_i8(tmem + uint32_t((i + j0) * TN), ad, smem_desc_k32(b0 + uint32_t(j0 * TN * 32)),
+             idesc_i8(128, (j1 - j0) * TN), acc);
+    }
+  }
 }
 
 }  // namespace tc
