@@ -27,6 +27,7 @@
 #include "fock.cuh"
 #include "server.cuh"
 #include "gemm_i8.cuh"
+#include "host_stage.cuh"
 #include "ozaki.cuh"
 
 namespace {
@@ -88,6 +89,7 @@ struct DeviceState {
   cudaEvent_t up[kHostBlocks] = {}, done[kHostBlocks] = {};
   void* buf = nullptr;
   size_t cap = 0;
+  cfgmm::HostStage stage;  // pinned buffers of copies from and to pageable memory
 };
 
 std::mutex g_devices_mu;
@@ -305,8 +307,8 @@ int gemm_host_blocked(DeviceState* st, double* c, const double* a, const double*
   cudaError_t err = cudaSuccess;
   if (split) err = cfgmm::gemm_i8_reset_error(st->stream);
   if (err == cudaSuccess)
-    err = by_rows ? cudaMemcpyAsync(db, b, eb * 8, cudaMemcpyHostToDevice, st->copy)
-                  : cudaMemcpyAsync(da, a, ea * 8, cudaMemcpyHostToDevice, st->copy);
+    err = by_rows ? st->stage.upload(db, b, eb * 8, st->copy)
+                  : st->stage.upload(da, a, ea * 8, st->copy);
   if (err == cudaSuccess && dt)  // the mask of the masked GEMM, whole
     err = cudaMemcpyAsync(dt, tab, tab_ext, cudaMemcpyHostToDevice, st->copy);
   size_t done_blocks = 0;
@@ -318,19 +320,16 @@ int gemm_host_blocked(DeviceState* st, double* c, const double* a, const double*
     const size_t i0 = by_rows ? x0 : 0, mk = by_rows ? xk : m;
     const size_t j0 = by_rows ? 0 : x0, nk = by_rows ? n : xk;
     if (by_rows)  // rows of op(A): columns of A when transposed
-      err = transa ? cudaMemcpy2DAsync(da + i0, lda * 8, a + i0, lda * 8, mk * 8, k,
-                                       cudaMemcpyHostToDevice, st->copy)
-                   : cudaMemcpy2DAsync(da + i0 * lda, lda * 8, a + i0 * lda, lda * 8, k * 8, mk,
-                                       cudaMemcpyHostToDevice, st->copy);
+      err = transa ? st->stage.upload(da + i0, lda * 8, a + i0, lda * 8, mk * 8, k, st->copy)
+                   : st->stage.upload(da + i0 * lda, lda * 8, a + i0 * lda, lda * 8, k * 8, mk,
+                                      st->copy);
     else  // columns of op(B): rows of B when transposed
-      err = transb ? cudaMemcpy2DAsync(db + j0 * ldb, ldb * 8, b + j0 * ldb, ldb * 8, k * 8, nk,
-                                       cudaMemcpyHostToDevice, st->copy)
-                   : cudaMemcpy2DAsync(db + j0, ldb * 8, b + j0, ldb * 8, nk * 8, k,
-                                       cudaMemcpyHostToDevice, st->copy);
+      err = transb ? st->stage.upload(db + j0 * ldb, ldb * 8, b + j0 * ldb, ldb * 8, k * 8, nk,
+                                      st->copy)
+                   : st->stage.upload(db + j0, ldb * 8, b + j0, ldb * 8, nk * 8, k, st->copy);
     double* dck = dc + i0 * ldc + j0;
     if (err == cudaSuccess)
-      err = cudaMemcpy2DAsync(dck, ldc * 8, c + i0 * ldc + j0, ldc * 8, nk * 8, mk,
-                              cudaMemcpyHostToDevice, st->copy);
+      err = st->stage.upload(dck, ldc * 8, c + i0 * ldc + j0, ldc * 8, nk * 8, mk, st->copy);
     if (err == cudaSuccess) err = cudaEventRecord(st->up[blk], st->copy);
     if (err == cudaSuccess) err = cudaStreamWaitEvent(st->stream, st->up[blk], 0);
     const double* dak = transa ? da + i0 : da + i0 * lda;
@@ -399,8 +398,8 @@ int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const doub
     return gemm_host_blocked(st, c, a, b, m, n, k, lda, ldb, ldc, transa != 0, transb != 0, split,
                              nmod, da, db, dc, base + ows, by_rows, mk.tab, dt, tab_ext,
                              mk.ldtab, mk.blk);
-  CFGMM_CUDA(cudaMemcpyAsync(da, a, ex.a * 8, cudaMemcpyHostToDevice, st->stream));
-  CFGMM_CUDA(cudaMemcpyAsync(db, b, ex.b * 8, cudaMemcpyHostToDevice, st->stream));
+  CFGMM_CUDA(st->stage.upload(da, a, ex.a * 8, st->stream));
+  CFGMM_CUDA(st->stage.upload(db, b, ex.b * 8, st->stream));
   if (masked) CFGMM_CUDA(cudaMemcpyAsync(dt, mk.tab, tab_ext, cudaMemcpyHostToDevice, st->stream));
   if (split) {
     // C goes up on the copy stream once A and B are in, while the residues
@@ -408,7 +407,7 @@ int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const doub
     if ((rc = ensure_copy_stream(st)) != CFGMM_OK) return rc;
     CFGMM_CUDA(cudaEventRecord(st->ab_done, st->stream));
     CFGMM_CUDA(cudaStreamWaitEvent(st->copy, st->ab_done, 0));
-    CFGMM_CUDA(cudaMemcpyAsync(dc, c, ex.c * 8, cudaMemcpyHostToDevice, st->copy));
+    CFGMM_CUDA(st->stage.upload(dc, c, ex.c * 8, st->copy));
     CFGMM_CUDA(cudaEventRecord(st->c_ready, st->copy));
     cudaError_t err = cfgmm::gemm_i8_reset_error(st->stream);
     if (err == cudaSuccess)
@@ -422,15 +421,15 @@ int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const doub
       return cuda_fail(err, "ozaki_dgemm");
     }
   } else if (masked) {
-    CFGMM_CUDA(cudaMemcpyAsync(dc, c, ex.c * 8, cudaMemcpyHostToDevice, st->stream));
+    CFGMM_CUDA(st->stage.upload(dc, c, ex.c * 8, st->stream));
     CFGMM_CUDA(cfgmm::dgemm_fp64_non0tab(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc,
                                          transa != 0, dt, mk.ldtab, int(mk.blk), st->stream));
   } else {
-    CFGMM_CUDA(cudaMemcpyAsync(dc, c, ex.c * 8, cudaMemcpyHostToDevice, st->stream));
+    CFGMM_CUDA(st->stage.upload(dc, c, ex.c * 8, st->stream));
     CFGMM_CUDA(cfgmm::dgemm_fp64(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc, transa != 0,
                                  transb != 0, st->stream));
   }
-  CFGMM_CUDA(cudaMemcpyAsync(c, dc, ex.c * 8, cudaMemcpyDeviceToHost, st->stream));
+  CFGMM_CUDA(st->stage.download(c, dc, ex.c * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
   return check_device_waits();
 }
@@ -492,6 +491,62 @@ int aodm_device_status(bool split) {
   return CFGMM_OK;
 }
 
+// How the phi tables of a host call go up: from pageable memory only the present
+// tiles, packed by the copying threads (the kernels read no others), when they are at
+// most three quarters of a table of 4 MB or more.  `offsets` empty: whole tables.
+struct PhiUpload {
+  size_t elems = 0;  // of a table's present tiles
+  std::vector<unsigned long long> offsets;
+  bool tiles() const { return !offsets.empty(); }
+  // device scratch: the packed tiles, the rows' offsets
+  size_t bytes() const { return tiles() ? align256(elems * 8) + align256(offsets.size() * 8) : 0; }
+};
+
+PhiUpload plan_phi_upload(const double* ao_lhs, const double* ao_rhs, size_t nao, size_t ngrid,
+                          const uint8_t* tab, size_t ldtab, size_t blksize) {
+  PhiUpload u;
+  if (nao * ngrid * 8 < (size_t(4) << 20) || blksize > (size_t(1) << 17) ||
+      !cfgmm::host_pageable(ao_lhs) || !cfgmm::host_pageable(ao_rhs))
+    return u;
+  try {
+    u.elems = cfgmm::HostStage::tiles_elems(nao, ngrid, tab, ldtab, blksize, &u.offsets);
+  } catch (const std::exception&) {
+    u.offsets.clear();
+  }
+  if (u.elems * 4 > nao * ngrid * 3) u.offsets.clear();
+  return u;
+}
+
+// phi_lhs and, unless it is the same table, phi_rhs, on `s`; the mask is already on
+// its way there (d_tab).
+cudaError_t upload_phi(DeviceState* st, const PhiUpload& u, void* scratch, double* d_lhs,
+                       const double* ao_lhs, double* d_rhs, const double* ao_rhs,
+                       size_t stride_grid, size_t nao, size_t ngrid, size_t ao_len,
+                       const uint8_t* tab, const uint8_t* d_tab, size_t ldtab, size_t blksize,
+                       cudaStream_t s) {
+  for (int side = 0; side < (ao_lhs == ao_rhs ? 1 : 2); ++side) {
+    double* dst = side ? d_rhs : d_lhs;
+    const double* src = side ? ao_rhs : ao_lhs;
+    cudaError_t err = cudaErrorMemoryAllocation;
+    if (u.tiles()) {
+      double* packed = static_cast<double*>(scratch);
+      auto* offs = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) +
+                                                         align256(u.elems * 8));
+      try {
+        err = st->stage.upload_tiles(dst, packed, offs, src, stride_grid, nao, ngrid, tab, d_tab,
+                                     ldtab, blksize, u.offsets, u.elems, s);
+      } catch (const std::exception&) {  // no memory for the list of pieces
+      }
+    }
+    if (err == cudaErrorMemoryAllocation) {  // also: no pinned buffers
+      cudaGetLastError();
+      err = st->stage.upload(dst, src, ao_len * 8, s);
+    }
+    if (err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
+}
+
 // A host-pointer AO-DM-AO contraction whose phi tables exceed 64 MB, in 4
 // blocks of whole grid blocks so that the PCIe transfers of one block overlap
 // the work and the transfers of the others: D, the mask and rho go up first,
@@ -514,18 +569,18 @@ int aodm_host_blocked(DeviceState* st, double* rhos, const double* dms, const do
   const bool same_ao = d_lhs == d_rhs;
   cudaError_t err = split ? cfgmm::aodmao2rho_split_reset_error(st->stream) : cudaSuccess;
   if (err == cudaSuccess)
-    err = cudaMemcpyAsync(d_dms, dms, ex.dms * 8, cudaMemcpyHostToDevice, st->copy);
+    err = st->stage.upload(d_dms, dms, ex.dms * 8, st->copy);
   if (err == cudaSuccess) err = cudaMemcpyAsync(d_tab, tab, ex.tab, cudaMemcpyHostToDevice, st->copy);
   if (err == cudaSuccess)
-    err = cudaMemcpyAsync(d_rho, rhos, ex.rhos * 8, cudaMemcpyHostToDevice, st->copy);
+    err = st->stage.upload(d_rho, rhos, ex.rhos * 8, st->copy);
   for (size_t blk = 0; err == cudaSuccess && blk < kBlocks; ++blk) {
     const size_t g0 = bound[blk], gk = bound[blk + 1] - g0;
     if (gk == 0) continue;
-    err = cudaMemcpy2DAsync(d_lhs + g0, stride_grid * 8, ao_lhs + g0, stride_grid * 8, gk * 8, nao,
-                            cudaMemcpyHostToDevice, st->copy);
+    err = st->stage.upload(d_lhs + g0, stride_grid * 8, ao_lhs + g0, stride_grid * 8, gk * 8, nao,
+                           st->copy);
     if (err == cudaSuccess && !same_ao)
-      err = cudaMemcpy2DAsync(d_rhs + g0, stride_grid * 8, ao_rhs + g0, stride_grid * 8, gk * 8,
-                              nao, cudaMemcpyHostToDevice, st->copy);
+      err = st->stage.upload(d_rhs + g0, stride_grid * 8, ao_rhs + g0, stride_grid * 8, gk * 8,
+                             nao, st->copy);
     if (err == cudaSuccess) err = cudaEventRecord(st->up[blk], st->copy);
     if (err == cudaSuccess) err = cudaStreamWaitEvent(st->stream, st->up[blk], 0);
     const size_t b0 = g0 / blksize;
@@ -579,23 +634,24 @@ int aodm_host(double* rhos, size_t rhos_len, const double* dms, size_t dms_len,
   const size_t o_ws = o_rho + align256(ex.rhos * 8);
   const size_t ws = split ? cfgmm::aodmao2rho_split_workspace(nao, ngrid, nset, blksize)
                           : cfgmm::aodmao2rho_fp64_workspace(nao, ngrid, nset, blksize);
-  if ((rc = reserve(st, o_ws + ws)) != CFGMM_OK) return rc;
+  // the packed tiles lie where the scratch of the contraction comes after them
+  const PhiUpload phi = plan_phi_upload(ao_lhs, ao_rhs, nao, ngrid, tab, ldtab, blksize);
+  if ((rc = reserve(st, o_ws + std::max(ws, phi.bytes()))) != CFGMM_OK) return rc;
   char* base = static_cast<char*>(st->buf);
   double* d_dms = reinterpret_cast<double*>(base + o_dms);
   double* d_lhs = reinterpret_cast<double*>(base + o_lhs);
   double* d_rhs = reinterpret_cast<double*>(base + o_rhs);
   uint8_t* d_tab = reinterpret_cast<uint8_t*>(base + o_tab);
   double* d_rho = reinterpret_cast<double*>(base + o_rho);
-  if (ex.ao * 8 >= (size_t(64) << 20) && ngrid >= 4 * blksize)
+  if (ex.ao * 8 >= (size_t(64) << 20) && ngrid >= 4 * blksize && !phi.tiles())
     return aodm_host_blocked(st, rhos, dms, ao_lhs, ao_rhs, stride_ao, stride_grid, nao, ngrid,
                              nset, tab, ldtab, blksize, split, ex, d_dms, d_lhs,
                              same_ao ? d_lhs : d_rhs, d_tab, d_rho, base + o_ws);
-  CFGMM_CUDA(cudaMemcpyAsync(d_dms, dms, ex.dms * 8, cudaMemcpyHostToDevice, st->stream));
-  CFGMM_CUDA(cudaMemcpyAsync(d_lhs, ao_lhs, ex.ao * 8, cudaMemcpyHostToDevice, st->stream));
-  if (!same_ao)
-    CFGMM_CUDA(cudaMemcpyAsync(d_rhs, ao_rhs, ex.ao * 8, cudaMemcpyHostToDevice, st->stream));
   CFGMM_CUDA(cudaMemcpyAsync(d_tab, tab, ex.tab, cudaMemcpyHostToDevice, st->stream));
-  CFGMM_CUDA(cudaMemcpyAsync(d_rho, rhos, ex.rhos * 8, cudaMemcpyHostToDevice, st->stream));
+  CFGMM_CUDA(upload_phi(st, phi, base + o_ws, d_lhs, ao_lhs, d_rhs, ao_rhs, stride_grid, nao,
+                        ngrid, ex.ao, tab, d_tab, ldtab, blksize, st->stream));
+  CFGMM_CUDA(st->stage.upload(d_dms, dms, ex.dms * 8, st->stream));
+  CFGMM_CUDA(st->stage.upload(d_rho, rhos, ex.rhos * 8, st->stream));
   if (split) {
     CFGMM_CUDA(cfgmm::aodmao2rho_split_reset_error(st->stream));
     CFGMM_CUDA(cfgmm::aodmao2rho_split(d_rho, d_dms, d_lhs, same_ao ? d_lhs : d_rhs, stride_ao,
@@ -606,7 +662,7 @@ int aodm_host(double* rhos, size_t rhos_len, const double* dms, size_t dms_len,
                                       stride_grid, int(nao), int(ngrid), int(nset), d_tab, ldtab,
                                       int(blksize), base + o_ws, st->stream));
   }
-  CFGMM_CUDA(cudaMemcpyAsync(rhos, d_rho, ex.rhos * 8, cudaMemcpyDeviceToHost, st->stream));
+  CFGMM_CUDA(st->stage.download(rhos, d_rho, ex.rhos * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
   if (split) return check_device_waits();
   int code = 0;
@@ -693,23 +749,26 @@ int fock_host(double* vs, size_t vs_len, const double* ws, size_t ws_len, const 
   const size_t o_tab = o_rhs + (same_ao ? 0 : align256(ex.ao * 8));
   const size_t o_v = o_tab + align256(ex.tab);
   const size_t o_ws = o_v + align256(ex.dms * 8);
-  if ((rc = reserve(st, o_ws + fock_workspace(nao, ngrid, nset, blksize))) != CFGMM_OK) return rc;
+  // (the dense form packs whole rows, masked as it goes)
+  const PhiUpload phi = plan_phi_upload(ao_lhs, ao_rhs, nao, ngrid, tab, ldtab, blksize);
+  if ((rc = reserve(st, o_ws + std::max(fock_workspace(nao, ngrid, nset, blksize),
+                                        phi.bytes()))) != CFGMM_OK)
+    return rc;
   char* base = static_cast<char*>(st->buf);
   double* d_w = reinterpret_cast<double*>(base + o_w);
   double* d_lhs = reinterpret_cast<double*>(base + o_lhs);
   double* d_rhs = reinterpret_cast<double*>(base + o_rhs);
   uint8_t* d_tab = reinterpret_cast<uint8_t*>(base + o_tab);
   double* d_v = reinterpret_cast<double*>(base + o_v);
-  CFGMM_CUDA(cudaMemcpyAsync(d_w, ws, ex.rhos * 8, cudaMemcpyHostToDevice, st->stream));
-  CFGMM_CUDA(cudaMemcpyAsync(d_lhs, ao_lhs, ex.ao * 8, cudaMemcpyHostToDevice, st->stream));
-  if (!same_ao)
-    CFGMM_CUDA(cudaMemcpyAsync(d_rhs, ao_rhs, ex.ao * 8, cudaMemcpyHostToDevice, st->stream));
   CFGMM_CUDA(cudaMemcpyAsync(d_tab, tab, ex.tab, cudaMemcpyHostToDevice, st->stream));
-  CFGMM_CUDA(cudaMemcpyAsync(d_v, vs, ex.dms * 8, cudaMemcpyHostToDevice, st->stream));
+  CFGMM_CUDA(upload_phi(st, phi, base + o_ws, d_lhs, ao_lhs, d_rhs, ao_rhs, stride_grid, nao,
+                        ngrid, ex.ao, tab, d_tab, ldtab, blksize, st->stream));
+  CFGMM_CUDA(st->stage.upload(d_w, ws, ex.rhos * 8, st->stream));
+  CFGMM_CUDA(st->stage.upload(d_v, vs, ex.dms * 8, st->stream));
   if ((rc = fock_run(d_v, d_w, d_lhs, same_ao ? d_lhs : d_rhs, stride_ao, stride_grid, nao, ngrid,
                      nset, d_tab, ldtab, blksize, base + o_ws, st->stream)) != CFGMM_OK)
     return rc;
-  CFGMM_CUDA(cudaMemcpyAsync(vs, d_v, ex.dms * 8, cudaMemcpyDeviceToHost, st->stream));
+  CFGMM_CUDA(st->stage.download(vs, d_v, ex.dms * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
   return check_device_waits();
 }
@@ -1166,14 +1225,14 @@ int cfgmm_matmul_f32(float* c, size_t c_len, const float* a, size_t a_len, const
     CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&da), ex.a * 4));
     CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&db), ex.b * 4));
     CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&dc), ex.c * 4));
-    CFGMM_CUDA(cudaMemcpyAsync(da, a, ex.a * 4, cudaMemcpyHostToDevice, s));
-    CFGMM_CUDA(cudaMemcpyAsync(db, b, ex.b * 4, cudaMemcpyHostToDevice, s));
-    CFGMM_CUDA(cudaMemcpyAsync(dc, c, ex.c * 4, cudaMemcpyHostToDevice, s));
+    CFGMM_CUDA(st->stage.upload(da, a, ex.a * 4, s));
+    CFGMM_CUDA(st->stage.upload(db, b, ex.b * 4, s));
+    CFGMM_CUDA(st->stage.upload(dc, c, ex.c * 4, s));
     if (precision == CFGMM_PREC_OZAKI_INT8) CFGMM_CUDA(cfgmm::gemm_i8_reset_error(s));
     if ((rc = matmul_f32_run(dc, da, db, m, n, k, lda, ldb, ldc, transa != 0, transb != 0, ex,
                              precision, s)) != CFGMM_OK)
       return rc;
-    CFGMM_CUDA(cudaMemcpyAsync(c, dc, ex.c * 4, cudaMemcpyDeviceToHost, s));
+    CFGMM_CUDA(st->stage.download(c, dc, ex.c * 4, s));
   }
   CFGMM_CUDA(cudaStreamSynchronize(s));
   return check_device_waits();
@@ -1226,18 +1285,18 @@ int cfgmm_aodmao2rho_f32(float* rhos, size_t rhos_len, const float* dms, size_t 
     CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&d_lhs), ex.ao * 4));
     if (!same_ao) CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&d_rhs), ex.ao * 4));
     CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&d_tab), ex.tab));
-    CFGMM_CUDA(cudaMemcpyAsync(d_rho, rhos, ex.rhos * 4, cudaMemcpyHostToDevice, s));
-    CFGMM_CUDA(cudaMemcpyAsync(d_dms, dms, ex.dms * 4, cudaMemcpyHostToDevice, s));
-    CFGMM_CUDA(cudaMemcpyAsync(d_lhs, ao_lhs, ex.ao * 4, cudaMemcpyHostToDevice, s));
+    CFGMM_CUDA(st->stage.upload(d_rho, rhos, ex.rhos * 4, s));
+    CFGMM_CUDA(st->stage.upload(d_dms, dms, ex.dms * 4, s));
+    CFGMM_CUDA(st->stage.upload(d_lhs, ao_lhs, ex.ao * 4, s));
     if (!same_ao)
-      CFGMM_CUDA(cudaMemcpyAsync(d_rhs, ao_rhs, ex.ao * 4, cudaMemcpyHostToDevice, s));
+      CFGMM_CUDA(st->stage.upload(d_rhs, ao_rhs, ex.ao * 4, s));
     CFGMM_CUDA(cudaMemcpyAsync(d_tab, tab, ex.tab, cudaMemcpyHostToDevice, s));
     if (split) CFGMM_CUDA(cfgmm::aodmao2rho_split_reset_error(s));
     if ((rc = aodm_f32_run(d_rho, d_dms, d_lhs, same_ao ? d_lhs : d_rhs, stride_ao, stride_grid,
                            nao, ngrid, nset, d_tab, ldtab, blksize, ex, precision, s)) !=
         CFGMM_OK)
       return rc;
-    CFGMM_CUDA(cudaMemcpyAsync(rhos, d_rho, ex.rhos * 4, cudaMemcpyDeviceToHost, s));
+    CFGMM_CUDA(st->stage.download(rhos, d_rho, ex.rhos * 4, s));
   }
   CFGMM_CUDA(cudaStreamSynchronize(s));
   if (split) return check_device_waits();
@@ -1276,6 +1335,7 @@ int cfgmm_release_workspace(void) {
   if (st->buf) CFGMM_CUDA(cudaFree(st->buf));
   st->buf = nullptr;
   st->cap = 0;
+  st->stage.release();
   cfgmm::release_pinned_staging();
   return CFGMM_OK;
 }

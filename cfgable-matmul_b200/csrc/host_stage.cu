@@ -1,0 +1,364 @@
+// host_stage.cu -- copies between pageable host memory and the device (host_stage.cuh).
+#include "host_stage.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstring>
+#include <functional>
+#include <mutex>
+#include <system_error>
+#include <thread>
+
+namespace cfgmm {
+namespace {
+
+constexpr size_t kSlot = size_t(1) << 20;      // bytes of a pinned buffer
+constexpr size_t kDirect = size_t(256) << 10;  // smaller copies go the driver's way
+constexpr int kMaxWorkers = 6;  // copying threads, the caller among them
+
+// A few threads that run one job at a time.  They live as long as the process: the
+// object is never destroyed, so none of them meets a destroyed mutex at exit.
+class Workers {
+ public:
+  static Workers& get() {
+    static Workers* w = new Workers;
+    return *w;
+  }
+  int count() const { return 1 + int(threads_); }
+  // fn(worker) on every thread, worker 0 being the caller; returns when all are done.
+  void run(const std::function<void(int)>& fn) {
+    std::lock_guard<std::mutex> one(job_mu_);
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      fn_ = &fn;
+      running_ = int(threads_);
+      ++round_;
+    }
+    start_.notify_all();
+    fn(0);
+    std::unique_lock<std::mutex> lk(mu_);
+    done_.wait(lk, [&] { return running_ == 0; });
+    fn_ = nullptr;
+  }
+
+ private:
+  Workers() {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int want = std::max(1, std::min(kMaxWorkers, int(hw / 2))) - 1;
+    for (int i = 0; i < want; ++i) {
+      try {
+        std::thread([this, i] { loop(i + 1); }).detach();
+      } catch (const std::system_error&) {
+        break;  // fewer threads
+      }
+      ++threads_;
+    }
+  }
+  void loop(int worker) {
+    unsigned long long seen = 0;
+    for (;;) {
+      const std::function<void(int)>* fn;
+      {
+        std::unique_lock<std::mutex> lk(mu_);
+        start_.wait(lk, [&] { return round_ != seen; });
+        seen = round_;
+        fn = fn_;
+      }
+      (*fn)(worker);
+      std::lock_guard<std::mutex> lk(mu_);
+      if (--running_ == 0) done_.notify_one();
+    }
+  }
+  std::mutex job_mu_, mu_;
+  std::condition_variable start_, done_;
+  const std::function<void(int)>* fn_ = nullptr;
+  int running_ = 0;
+  unsigned long long round_ = 0;
+  size_t threads_ = 0;
+};
+
+// A row's present tiles from `packed` (offsets[row] on, one after the other) to their
+// places; CTA per row.
+__global__ void __launch_bounds__(256)
+spread_tiles(double* __restrict__ dst, size_t ld, const double* __restrict__ packed,
+             const unsigned long long* __restrict__ offsets, const uint8_t* __restrict__ tab,
+             size_t ldtab, long long cols, long long blk, int nblk) {
+  __shared__ int warp_tot[8];
+  __shared__ int list[256];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double* src = packed + offsets[blockIdx.x];
+  double* row = dst + size_t(blockIdx.x) * ld;
+  const uint8_t* t = tab + size_t(blockIdx.x) * ldtab;
+  for (int b0 = 0; b0 < nblk; b0 += 256) {
+    const int b = b0 + tid;
+    const bool on = b < nblk && t[b] != 0;
+    const unsigned bal = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) warp_tot[warp] = __popc(bal);
+    __syncthreads();
+    int at = 0, total = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) at += warp_tot[w];
+      total += warp_tot[w];
+    }
+    if (on) list[at + __popc(bal & ((1u << lane) - 1u))] = b;
+    __syncthreads();
+    const long long n = (long long)total * blk;
+    for (long long i = tid; i < n; i += 256) {
+      const long long q = i / blk, col = list[q] * blk + (i - q * blk);
+      if (col < cols) row[col] = src[i];  // only the row's last tile can be short
+    }
+    src += n;
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+bool host_pageable(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+cudaError_t HostStage::ensure() try {
+  const size_t slots = 2 * size_t(Workers::get().count());
+  if (!pinned_) {
+    const cudaError_t err =
+        cudaHostAlloc(reinterpret_cast<void**>(&pinned_), slots * kSlot, cudaHostAllocPortable);
+    if (err != cudaSuccess) {
+      pinned_ = nullptr;
+      return err;
+    }
+  }
+  while (events_.size() < slots) {
+    cudaEvent_t e;
+    const cudaError_t err = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (err != cudaSuccess) return err;
+    events_.push_back(e);
+  }
+  return cudaSuccess;
+} catch (const std::exception&) {  // no memory for the threads or the events
+  return cudaErrorMemoryAllocation;
+}
+
+void HostStage::release() {
+  for (cudaEvent_t e : events_) cudaEventDestroy(e);
+  events_.clear();
+  if (pinned_) cudaFreeHost(pinned_);
+  pinned_ = nullptr;
+}
+
+namespace {
+
+// Runs piece(i, slot) for i < n on the copying threads, with the device current on
+// each and a free pinned buffer; `piece` fills it and enqueues its copy on `stream`,
+// behind which the buffer's event is recorded.
+cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, size_t n,
+                       cudaStream_t stream,
+                       const std::function<cudaError_t(size_t, char*)>& piece) {
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{0};
+  Workers::get().run([&](int worker) {
+    cudaError_t e = worker > 0 ? cudaSetDevice(dev) : cudaSuccess;
+    for (int turn = 0; e == cudaSuccess && failed.load() == 0; turn ^= 1) {
+      const size_t i = next.fetch_add(1);
+      if (i >= n) break;
+      const size_t slot = 2 * size_t(worker) + turn;
+      e = cudaEventSynchronize(events[slot]);  // an event never recorded is complete
+      if (e == cudaSuccess) e = piece(i, pinned + slot * kSlot);
+      if (e == cudaSuccess) e = cudaEventRecord(events[slot], stream);
+    }
+    if (e != cudaSuccess) {
+      int none = 0;
+      failed.compare_exchange_strong(none, int(e));
+    }
+  });
+  return cudaError_t(failed.load());
+}
+
+// Bytes of a piece of a contiguous copy: every thread gets two or more.
+size_t piece_bytes(size_t total) {
+  const size_t each = total / (2 * size_t(Workers::get().count()));
+  return std::min(kSlot, std::max(size_t(128) << 10, (each + 4095) / 4096 * 4096));
+}
+
+}  // namespace
+
+cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t spitch,
+                              size_t width, size_t rows, cudaStream_t stream) {
+  if (rows > 1 && dpitch == width && spitch == width) {
+    width *= rows;
+    dpitch = spitch = width;
+    rows = 1;
+  }
+  if (width * rows < kDirect || !host_pageable(src) || ensure() != cudaSuccess) {
+    cudaGetLastError();
+    return rows == 1 ? cudaMemcpyAsync(dst, src, width, cudaMemcpyHostToDevice, stream)
+                     : cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows,
+                                         cudaMemcpyHostToDevice, stream);
+  }
+  char* d = static_cast<char*>(dst);
+  const char* s = static_cast<const char*>(src);
+  const size_t most = piece_bytes(width * rows);
+  if (width > most) {  // parts of a row
+    const size_t per_row = (width + most - 1) / most;
+    return run_pieces(pinned_, events_, per_row * rows, stream, [&](size_t i, char* slot) {
+      const size_t r = i / per_row, off = i % per_row * most;
+      const size_t n = std::min(most, width - off);
+      std::memcpy(slot, s + r * spitch + off, n);
+      return cudaMemcpyAsync(d + r * dpitch + off, slot, n, cudaMemcpyHostToDevice, stream);
+    });
+  }
+  const size_t some = most / width;  // rows
+  return run_pieces(pinned_, events_, (rows + some - 1) / some, stream, [&](size_t i, char* slot) {
+    const size_t r0 = i * some, n = std::min(some, rows - r0);
+    for (size_t r = 0; r < n; ++r) std::memcpy(slot + r * width, s + (r0 + r) * spitch, width);
+    return cudaMemcpy2DAsync(d + r0 * dpitch, dpitch, slot, width, width, n,
+                             cudaMemcpyHostToDevice, stream);
+  });
+}
+
+cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  if (bytes < kDirect || !host_pageable(dst) || ensure() != cudaSuccess) {
+    cudaGetLastError();
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
+  }
+  // A thread copies a piece out of one of its buffers while the next piece arrives in
+  // the other.
+  char* d = static_cast<char*>(dst);
+  const char* s = static_cast<const char*>(src);
+  const size_t most = piece_bytes(bytes), n = (bytes + most - 1) / most;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{0};
+  Workers::get().run([&](int worker) {
+    cudaError_t e = worker > 0 ? cudaSetDevice(dev) : cudaSuccess;
+    size_t held[2] = {n, n};  // the pieces in this thread's buffers
+    bool more = true;
+    for (int turn = 0; e == cudaSuccess && failed.load() == 0; turn ^= 1) {
+      const size_t slot = 2 * size_t(worker) + turn;
+      char* buf = pinned_ + slot * kSlot;
+      if (held[turn] < n) {
+        e = cudaEventSynchronize(events_[slot]);
+        if (e != cudaSuccess) break;
+        const size_t off = held[turn] * most;
+        std::memcpy(d + off, buf, std::min(most, bytes - off));
+        held[turn] = n;
+      }
+      const size_t i = more ? next.fetch_add(1) : n;
+      if (i < n) {
+        const size_t off = i * most;
+        e = cudaMemcpyAsync(buf, s + off, std::min(most, bytes - off), cudaMemcpyDeviceToHost,
+                            stream);
+        if (e == cudaSuccess) e = cudaEventRecord(events_[slot], stream);
+        held[turn] = i;
+      } else {
+        more = false;
+        if (held[turn ^ 1] >= n) break;
+      }
+    }
+    if (e != cudaSuccess) {
+      int none = 0;
+      failed.compare_exchange_strong(none, int(e));
+    }
+  });
+  return cudaError_t(failed.load());
+}
+
+size_t HostStage::tiles_elems(size_t rows, size_t cols, const uint8_t* tab, size_t ldtab,
+                              size_t blk, std::vector<unsigned long long>* offsets) {
+  const size_t nblk = (cols + blk - 1) / blk;
+  offsets->resize(rows);
+  unsigned long long at = 0;
+  for (size_t r = 0; r < rows; ++r) {
+    (*offsets)[r] = at;
+    const uint8_t* t = tab + r * ldtab;
+    unsigned n = 0;
+    for (size_t b = 0; b < nblk; ++b) n += t[b] != 0;
+    at += (unsigned long long)n * blk;
+    if (t[nblk - 1]) at -= nblk * blk - cols;  // the last tile may be short
+  }
+  return size_t(at);
+}
+
+cudaError_t HostStage::upload_tiles(double* dst, double* packed, unsigned long long* d_offsets,
+                                    const double* src, size_t ld, size_t rows, size_t cols,
+                                    const uint8_t* tab, const uint8_t* d_tab, size_t ldtab,
+                                    size_t blk, const std::vector<unsigned long long>& offsets,
+                                    size_t total, cudaStream_t stream) {
+  cudaError_t err = ensure();
+  if (err != cudaSuccess) return err;
+  const size_t nblk = (cols + blk - 1) / blk;
+  // pieces of at most a buffer: whole rows, or a part of the tiles of a long one
+  struct Piece {
+    size_t row, b, elems;
+    unsigned long long at;
+  };
+  std::vector<Piece> pieces;
+  const size_t most = std::max(piece_bytes(total * 8) / 8, blk);  // blk * 8 <= kSlot: the caller's
+  for (size_t r = 0; r < rows; ++r) {
+    const unsigned long long at = offsets[r];
+    const size_t n = size_t((r + 1 < rows ? offsets[r + 1] : total) - at);
+    if (n == 0) continue;
+    if (n > most) {
+      size_t done = 0;
+      for (size_t b = 0; b < nblk; ++b)
+        if (tab[r * ldtab + b]) {
+          const size_t w = std::min(blk, cols - b * blk);
+          if (done == 0 || pieces.back().elems + w > most) pieces.push_back({r, b, 0, at + done});
+          pieces.back().elems += w;
+          done += w;
+        }
+    } else if (pieces.empty() || pieces.back().elems + n > most) {
+      pieces.push_back({r, 0, n, at});
+    } else {
+      pieces.back().elems += n;
+    }
+  }
+  err = cudaMemcpyAsync(d_offsets, offsets.data(), rows * sizeof(unsigned long long),
+                        cudaMemcpyHostToDevice, stream);
+  if (err != cudaSuccess) return err;
+  err = run_pieces(pinned_, events_, pieces.size(), stream, [&](size_t i, char* slot) {
+    const Piece& p = pieces[i];
+    double* to = reinterpret_cast<double*>(slot);
+    size_t left = p.elems, r = p.row, b = p.b;
+    while (left > 0) {
+      if (b == nblk) {
+        ++r;
+        b = 0;
+        continue;
+      }
+      const uint8_t* t = tab + r * ldtab;
+      if (!t[b]) {
+        ++b;
+        continue;
+      }
+      size_t n = 0;  // a run of present tiles
+      const size_t c0 = b * blk;
+      while (b < nblk && t[b] && n < left) {
+        n += std::min(blk, cols - b * blk);
+        ++b;
+      }
+      std::memcpy(to, src + r * ld + c0, n * 8);
+      to += n;
+      left -= n;
+    }
+    return cudaMemcpyAsync(packed + p.at, slot, p.elems * 8, cudaMemcpyHostToDevice, stream);
+  });
+  if (err != cudaSuccess) return err;
+  if (total == 0) return cudaSuccess;
+  spread_tiles<<<unsigned(rows), 256, 0, stream>>>(dst, ld, packed, d_offsets, d_tab, ldtab,
+                                                   (long long)cols, (long long)blk, int(nblk));
+  return cudaGetLastError();
+}
+
+}  // namespace cfgmm
