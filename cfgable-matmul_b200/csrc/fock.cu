@@ -6,7 +6,9 @@
 // and mask: where that one gathers D[I(b), I(b)] as an input, this one scatters
 // V[I(b), I(b)] as an output.  Work item = (block, 64-point tile, 64 rows of the
 // active list I(b)) for up to 4 weight vectors w_s, the same items as the
-// AO-DM-AO kernels.  Only the masked products are formed (a dense product over
+// AO-DM-AO kernels (fewer vectors where that would leave a CTA under 8 items to
+// draw: 1081 AOs x 3490 points x 4 vectors, 275 items in all, took 189 us with four
+// to an item, 167 before vectors were shared).  Only the masked products are formed (a dense product over
 // all AO pairs runs ~10x their number on the taxol-size mask).  When phi_lhs and
 // phi_rhs are the same array the block's contribution is symmetric in (u, v):
 // row tile a then walks the chunks from its own (chunk a) on and adds each
@@ -72,7 +74,7 @@ struct FockArgs {
   int sym;  // ao_lhs == ao_rhs: chunks from the row tile's own on, mirrored
   int vec;  // phi rows and w 16-byte aligned at every tile
   const int4* items;
-  int* counters;  // [groups] work counters, [groups] = item total
+  int* counters;  // the work counter, the item total
 };
 
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int code) {
@@ -81,7 +83,7 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int cod
 
 // One item as the producer decodes it for the consumers; bg < 0: no more items.
 struct FockItem {
-  int bg, nb, u0, gw, b;
+  int bg, nb, u0, gw, b, set0, ns;
 };
 
 __global__ void __launch_bounds__(THREADS, 2)
@@ -96,9 +98,12 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
   uint64_t* empty = full + STAGES;        // [STAGES]
   FockItem* item = reinterpret_cast<FockItem*>(empty + STAGES);
 
-  const int set0 = blockIdx.y * NS;
-  const int ns = min(NS, p.nset - set0);
-  const int total = p.counters[gridDim.y];
+  // the items once for each group of weight vectors
+  const int items = p.counters[1];
+  const int groups =
+      max((p.nset + NS - 1) / NS, min(p.nset, (8 * int(gridDim.x) + items - 1) / max(items, 1)));
+  const int per_group = (p.nset + groups - 1) / groups;
+  const int total = items * groups;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
     // the producer's 32 lanes and one more arrival: the bulk copies' expect_tx
@@ -114,7 +119,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
 
   if (warp == CONS) {
     // ------------------------------- producer -------------------------------
-    int* counter = p.counters + blockIdx.y;
+    int* counter = p.counters;
     int it = 0;
     if (lane == 0) it = atomicAdd(counter, 1);
     it = __shfl_sync(0xffffffffu, it, 0);
@@ -146,14 +151,18 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
     while (ok && it < total) {
       int next = 0;  // drawn now, needed after this item's copies
       if (lane == 0) next = atomicAdd(counter, 1);
-      const int4 wi = p.items[it];
+      const int4 wi = p.items[it % items];
+      const int set0 = it / items * per_group;
+      const int ns = min(per_group, p.nset - set0);
       const int b = wi.y / p.gsub, gt = wi.y % p.gsub, a = wi.z;
       const int nb = p.counts[b];
       const int* I = p.lists + size_t(b) * p.nao;
       const int u0 = a * FT, mu = min(FT, nb - u0);
       const int g0 = b * p.blk + gt * FT;
       const int gw = min(min((b + 1) * p.blk, p.ngrid), g0 + FT) - g0;
-      if (gw > 0) {  // a wide block's later tiles may start past the grid's end
+      // a wide block's later tiles may start past the grid's end, the last groups past
+      // the vectors' (5 in 4 groups of 2)
+      if (gw > 0 && ns > 0) {
         const bool bulk = p.vec && gw % 2 == 0;
         const int nch = (nb + FT - 1) / FT, ch0 = p.sym ? a : 0;
         const int ua = I[min(u0 + lane, nb - 1)], ub = I[min(u0 + lane + 32, nb - 1)];
@@ -179,7 +188,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
               ++fill;
               break;
             }
-            if (lane == 0) *item = FockItem{wi.y, nb, u0, gw, b};
+            if (lane == 0) *item = FockItem{wi.y, nb, u0, gw, b, set0, ns};
             rows_in(As, p.ao_lhs, ua, ub, mu, g0, gw, afull, bulk, uint32_t(ns) * gw * 8);
             if (bulk) {
               if (lane < ns)
@@ -281,7 +290,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
       // the products of the warp's 16 rows with its first 8 ntv columns, into V
       auto products = [&](auto ntv) {
         constexpr int N8 = decltype(ntv)::value;
-        for (int set = 0; set < ns; ++set) {
+        for (int set = 0; set < t.ns; ++set) {
           const double* W = Ws + set * FT + 2 * q;
           double acc[N8][4];
 #pragma unroll
@@ -310,9 +319,9 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
             for (int nt = 0; nt < N8; ++nt)
               dmma_16x8x8(acc[nt], lo.x, hi.x, lo.y, hi.y, bv[nt].x, bv[nt].y);
           }
-          if (set == ns - 1) release();
+          if (set == t.ns - 1) release();
           // V[u][v] += the products, and V[v][u] where they stand for both
-          double* V = p.v + size_t(set0 + set) * p.v_stride;
+          double* V = p.v + size_t(t.set0 + set) * p.v_stride;
 #pragma unroll
           for (int nt = 0; nt < N8; ++nt) {
             const int vd = odd ? vc[nt][1] : vc[nt][0];
@@ -387,8 +396,7 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   int* counters = reinterpret_cast<int*>(wsp + L.counters);
   cudaError_t err = aodm_block_lists_launch(tab, ldtab, nao, nblk, lists, counts, stream);
   if (err != cudaSuccess) return err;
-  const int groups = (nset + NS - 1) / NS;
-  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, groups, stream)) !=
+  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, 1, stream)) !=
       cudaSuccess)
     return err;
   FockArgs a{};
@@ -422,7 +430,7 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
   if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return err;
-  fock_compact_kernel<<<dim3(2 * nsm, groups), THREADS, FOCK_SMEM, stream>>>(a);
+  fock_compact_kernel<<<2 * nsm, THREADS, FOCK_SMEM, stream>>>(a);
   return cudaGetLastError();
 }
 
