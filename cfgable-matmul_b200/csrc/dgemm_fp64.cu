@@ -375,19 +375,20 @@ cudaError_t launch_t(const GemmArgs& p, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-// CTAs per tile.  An SM's time is taken as its CTAs (at least 2.3: fewer do not
-// fill it) times the K steps of each plus a start and an end worth 1 step, 3 with
-// the exchange in the cluster; the least time wins.  Measured against every
-// choice on 16 shapes (131 x 257 x 300 to 3000 x 3000 x 3000) the model's is within
-// 6 % of the fastest: 800 x 800 x 800 (169 tiles) takes 68, 61, 58, 55 us with 1,
-// 2, 4, 8 parts, 1200 x 1500 x 1000 (456) 166, 154, 142, 148, 2000 x 2000 x 500
-// (1024) 146, 160, 176, 204.
+// CTAs per tile.  An SM's time is taken as its CTAs times the K steps of each plus
+// two for a CTA's start and end; its CTAs are counted between the most that an SM
+// gets and the mean (they do not all start together), half a one more for the last
+// to end, and at least 3 (fewer do not fill an SM).  The least time wins, the fewer
+// parts of equals.  On 70 shapes (tiles 4 to 2500, k 100 to 6500) timed with 1, 2, 4
+// and 8 parts the choice is within 0.8 % of the fastest on average and 9 % at worst;
+// 130 x 130 x 5000 takes 269, 146, 75, 42 us with 1, 2, 4, 8 parts, 1200 x 1500 x 1000
+// 166, 154, 142, 148, 2000 x 2000 x 500 146, 160, 176, 204.
 int choose_splits(long long tiles, int steps, int nsm) {
   int best = 1;
   double least = 0.0;
   for (int s = 1; s <= 8 && (s == 1 || steps >= 2 * s); s *= 2) {
-    const double ctas = double((tiles * s + nsm - 1) / nsm);
-    const double t = std::max(ctas, 2.3) * (double(steps) / s + (s == 1 ? 1.0 : 3.0));
+    const double mean = double(tiles * s) / nsm, most = double((tiles * s + nsm - 1) / nsm);
+    const double t = std::max(0.5 * (most + mean) + 0.5, 3.0) * (double(steps) / s + 2.0);
     if (s == 1 || t < least) {
       best = s;
       least = t;
