@@ -697,7 +697,7 @@ int check_fock(double* vs, size_t vs_len, const double* ws, size_t ws_len, const
 }
 
 // The compacted form (fock.cu) unless CFGMM_FOCK_DENSE=1 selects the dense
-// product with K-step skipping (dgemm_fp64.cu).
+// product with K-step skipping (fock_dense.cu).
 bool fock_dense() {
   static const bool on = [] {
     const char* e = std::getenv("CFGMM_FOCK_DENSE");
@@ -794,8 +794,8 @@ struct StreamScratch {
 constexpr int kF32OperandBits = 26;  // f32 mantissa (24 bits) and two guard bits
 
 int matmul_f32_run(float* c, const float* a, const float* b, size_t m, size_t n, size_t k,
-                   size_t lda, size_t ldb, size_t ldc, bool ta, bool tb, const GemmExtents& ex,
-                   int precision, cudaStream_t s) {
+                   size_t lda, size_t ldb, size_t ldc, bool ta, bool tb, int precision,
+                   cudaStream_t s) {
   StreamScratch sc(s);
   if (precision == CFGMM_PREC_OZAKI_INT8) {
     const int nmod = cfgmm::ozaki_moduli_for_bits(int(k), kF32OperandBits);
@@ -805,15 +805,7 @@ int matmul_f32_run(float* c, const float* a, const float* b, size_t m, size_t n,
                                   s));
     return CFGMM_OK;
   }
-  double *da = nullptr, *db = nullptr, *dc = nullptr;
-  CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&da), ex.a * 8));
-  CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&db), ex.b * 8));
-  CFGMM_CUDA(sc.get(reinterpret_cast<void**>(&dc), ex.c * 8));
-  CFGMM_CUDA(cfgmm::widen_f32(a, da, ex.a, s));
-  CFGMM_CUDA(cfgmm::widen_f32(b, db, ex.b, s));
-  CFGMM_CUDA(cfgmm::widen_f32(c, dc, ex.c, s));
-  CFGMM_CUDA(cfgmm::dgemm_fp64(dc, da, db, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, s));
-  CFGMM_CUDA(cfgmm::narrow_f64(dc, c, ex.c, s));
+  CFGMM_CUDA(cfgmm::dgemm_f32(c, a, b, int(m), int(n), int(k), lda, ldb, ldc, ta, tb, s));
   return CFGMM_OK;
 }
 
@@ -1229,7 +1221,7 @@ int cfgmm_matmul_f32(float* c, size_t c_len, const float* a, size_t a_len, const
     CFGMM_CUDA(st->stage.upload(db, b, ex.b * 4, s));
     CFGMM_CUDA(st->stage.upload(dc, c, ex.c * 4, s));
     if (precision == CFGMM_PREC_OZAKI_INT8) CFGMM_CUDA(cfgmm::gemm_i8_reset_error(s));
-    if ((rc = matmul_f32_run(dc, da, db, m, n, k, lda, ldb, ldc, transa != 0, transb != 0, ex,
+    if ((rc = matmul_f32_run(dc, da, db, m, n, k, lda, ldb, ldc, transa != 0, transb != 0,
                              precision, s)) != CFGMM_OK)
       return rc;
     CFGMM_CUDA(st->stage.download(c, dc, ex.c * 4, s));
@@ -1251,7 +1243,7 @@ int cfgmm_matmul_f32_dev(float* c, const float* a, const float* b, size_t m, siz
   if (precision == CFGMM_PREC_OZAKI_INT8 && (rc = check_split_gemm(k)) != CFGMM_OK) return rc;
   int dev;
   if ((rc = current_device(&dev)) != CFGMM_OK) return rc;
-  return matmul_f32_run(c, a, b, m, n, k, lda, ldb, ldc, transa != 0, transb != 0, ex, precision,
+  return matmul_f32_run(c, a, b, m, n, k, lda, ldb, ldc, transa != 0, transb != 0, precision,
                         static_cast<cudaStream_t>(stream));
 }
 

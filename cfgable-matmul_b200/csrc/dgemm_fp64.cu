@@ -32,6 +32,7 @@
 //     cover about 1536 x 1536 of C and share their rows of A and B in L2.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -43,16 +44,16 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int T = 64;         // tile of C
+constexpr int TILE = 64;      // of C
 constexpr int TK = 16;        // K step
 constexpr int STAGES = 3;
 constexpr int THREADS = 128;
 constexpr int GROUP = 24;     // tile rows of a group (see above)
-constexpr int KP = T + 2;     // pitch of a [k][row] tile
+constexpr int KP = TILE + 2;  // pitch of a [k][row] tile
 constexpr int OP = TK * KP;   // doubles of one staged operand (the larger of both layouts)
-constexpr int CP = T + 2;     // pitch of the partial tile exchanged in a cluster
+constexpr int CP = TILE + 2;  // pitch of the partial tile exchanged in a cluster
 constexpr size_t SMEM = size_t(STAGES) * 2 * OP * 8;
-static_assert(size_t(T) * CP * 8 <= SMEM, "the partial tile fits the stages");
+static_assert(size_t(TILE) * CP * 8 <= SMEM, "the partial tile fits the stages");
 
 // A kernel of one of two forms that both are enqueued: it runs when the device
 // word (the choice made earlier on the stream) is zero / nonzero as wanted.
@@ -62,8 +63,9 @@ struct Gate {
   __device__ __forceinline__ bool closed() const { return word && (*word != 0) != (want != 0); }
 };
 
+template <class T>
 struct GemmArgs {
-  double* c;
+  T* c;
   const double* a;
   const double* b;
   int m, n, k;
@@ -141,9 +143,10 @@ struct Copier {
   }
 };
 
-template <bool TA, bool TB>
+// T: the type of C; an f32 element is widened, added to and rounded once.
+template <bool TA, bool TB, class T>
 __global__ void __launch_bounds__(THREADS, 4)
-dgemm_kernel(const __grid_constant__ GemmArgs p) {
+dgemm_kernel(const __grid_constant__ GemmArgs<T> p) {
   if (p.gate.closed()) return;  // every CTA of the grid alike
   extern __shared__ __align__(128) double gemm_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -153,7 +156,7 @@ dgemm_kernel(const __grid_constant__ GemmArgs p) {
   const int per_group = GROUP * p.tiles_n;
   const int first = tile / per_group * GROUP, in_group = tile % per_group;
   const int rows_g = min(GROUP, p.tiles_m - first);
-  const int m0 = (first + in_group % rows_g) * T, n0 = in_group / rows_g * T;
+  const int m0 = (first + in_group % rows_g) * TILE, n0 = in_group / rows_g * TILE;
   const int steps = (p.k + TK - 1) / TK;
   const int s0 = int((long long)part * steps / p.splits);
   const int s1 = int((long long)(part + 1) * steps / p.splits);
@@ -243,18 +246,18 @@ dgemm_kernel(const __grid_constant__ GemmArgs p) {
       for (int h = 0; h < 2; ++h) {
         const int row = m0 + row_of(mt, h);
         if (row >= p.m) continue;
-        double* crow = p.c + size_t(row) * p.ldc + n0;
+        T* crow = p.c + size_t(row) * p.ldc + n0;
         double old[4][2];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e)
-            old[j][e] = n0 + col_of(j, e) < p.n ? crow[col_of(j, e)] : 0.0;
+            old[j][e] = n0 + col_of(j, e) < p.n ? double(crow[col_of(j, e)]) : 0.0;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e)
-            if (n0 + col_of(j, e) < p.n) crow[col_of(j, e)] = old[j][e] + acc[mt][j][2 * h + e];
+            if (n0 + col_of(j, e) < p.n) crow[col_of(j, e)] = T(old[j][e] + acc[mt][j][2 * h + e]);
       }
     return;
   }
@@ -270,36 +273,38 @@ dgemm_kernel(const __grid_constant__ GemmArgs p) {
         for (int e = 0; e < 2; ++e)
           gemm_smem[row_of(mt, h) * CP + col_of(j, e)] = acc[mt][j][2 * h + e];
   cluster.sync();
-  const int rows = T / p.splits;  // of each CTA
-  for (int i = tid; i < rows * T; i += THREADS) {
-    const int r = part * rows + i / T, cc = i % T;
+  const int rows = TILE / p.splits;  // of each CTA
+  for (int i = tid; i < rows * TILE; i += THREADS) {
+    const int r = part * rows + i / TILE, cc = i % TILE;
     if (m0 + r >= p.m || n0 + cc >= p.n) continue;
     double v = 0.0;
     for (int s = 0; s < p.splits; ++s)
       v += *cluster.map_shared_rank(gemm_smem + r * CP + cc, s);
-    double* dst = p.c + size_t(m0 + r) * p.ldc + n0 + cc;
-    *dst += v;
+    T* dst = p.c + size_t(m0 + r) * p.ldc + n0 + cc;
+    *dst = T(double(*dst) + v);
   }
   cluster.sync();  // a CTA's partial tile is read until here
 }
 
 // dst[r*pitch + c] = src[r*ld + c] (c < cols; with a mask, zero unless
-// tab[r*ldtab + c/blk]): an operand into rows of an even pitch.  1024 columns of a
-// row per pass of a CTA.
+// tab[r*ldtab + c/blk]): an operand into doubles in rows of an even pitch.  1024
+// columns of a row per pass of a CTA.
+template <class T>
 __global__ void __launch_bounds__(256)
-pack_aligned(double* __restrict__ dst, int pitch, const double* __restrict__ src, size_t ld,
+pack_aligned(double* __restrict__ dst, int pitch, const T* __restrict__ src, size_t ld,
              int rows, int cols, const uint8_t* __restrict__ tab, size_t ldtab, int blk,
              Gate gate) {
   if (gate.closed()) return;
   for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-    const double* s = src + size_t(r) * ld;
+    const T* s = src + size_t(r) * ld;
     double* d = dst + size_t(r) * pitch;
     double2 v[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int c = blockIdx.x * 1024 + 512 * i + 2 * threadIdx.x;
-      v[i].x = c < cols && (!tab || tab[size_t(r) * ldtab + c / blk]) ? s[c] : 0.0;
-      v[i].y = c + 1 < cols && (!tab || tab[size_t(r) * ldtab + (c + 1) / blk]) ? s[c + 1] : 0.0;
+      v[i].x = c < cols && (!tab || tab[size_t(r) * ldtab + c / blk]) ? double(s[c]) : 0.0;
+      v[i].y = c + 1 < cols && (!tab || tab[size_t(r) * ldtab + (c + 1) / blk]) ? double(s[c + 1])
+                                                                                : 0.0;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -354,9 +359,9 @@ pack_transpose(double* __restrict__ dst, const double* __restrict__ src, size_t 
 }
 
 
-template <bool TA, bool TB>
-cudaError_t launch_t(const GemmArgs& p, cudaStream_t stream) {
-  auto kern = dgemm_kernel<TA, TB>;
+template <bool TA, bool TB, class T>
+cudaError_t launch_t(const GemmArgs<T>& p, cudaStream_t stream) {
+  auto kern = dgemm_kernel<TA, TB, T>;
   cudaError_t err =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM));
   if (err != cudaSuccess) return err;
@@ -420,17 +425,22 @@ bool pack_pays(int m, int n, int k, double elems) {
   return 0.045 * flops / 32e12 > elems * 16.0 / 5.5e12 + 4e-6;
 }
 
-cudaError_t gemm(double* c, const double* a, const double* b, int m, int n, int k, size_t lda,
-                 size_t ldb, size_t ldc, bool transa, bool transb, const uint8_t* tab,
+// f32 operands are widened into aligned rows of doubles, whatever their size, and the
+// kernel adds to the f32 C itself (64-bit sums, one rounding).  Widening A, B and C
+// and narrowing C in passes of their own: 390 x 200 x 1109 202 -> 34 us (K parts
+// included), 691 x 2668 x 124 72 -> 60, 3448 x 3968 x 840 1008 -> 757.
+template <class T>
+cudaError_t gemm(T* c, const T* a, const T* b, int m, int n, int k, size_t lda, size_t ldb,
+                 size_t ldc, bool transa, bool transb, const uint8_t* tab,
                  size_t ldtab, int blk, Gate gate, cudaStream_t stream) {
-  const long long tiles_m = (m + T - 1) / T, tiles_n = (n + T - 1) / T;
+  const long long tiles_m = (m + TILE - 1) / TILE, tiles_n = (n + TILE - 1) / TILE;
   if (tiles_m * tiles_n > (1ll << 27)) return cudaErrorInvalidConfiguration;
   int dev = 0, nsm = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err == cudaSuccess)
     err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (err != cudaSuccess) return err;
-  GemmArgs p{};
+  GemmArgs<T> p{};
   p.c = c;
   p.m = m;
   p.n = n;
@@ -441,9 +451,15 @@ cudaError_t gemm(double* c, const double* a, const double* b, int m, int n, int 
   p.splits = choose_splits(tiles_m * tiles_n, (k + TK - 1) / TK, nsm);
   p.gate = gate;
   const int ar = transa ? k : m, ac = transa ? m : k, br = transb ? n : k, bc = transb ? k : n;
-  const bool pa = !al16(a, lda) && pack_pays(m, n, k, double(m) * k);
-  const bool pb = (tab || !al16(b, ldb)) && pack_pays(m, n, k, double(n) * k);
+  constexpr bool widen = !std::is_same<T, double>::value;
+  const bool pa = widen || (!al16(a, lda) && pack_pays(m, n, k, double(m) * k));
+  const bool pb = widen || ((tab || !al16(b, ldb)) && pack_pays(m, n, k, double(n) * k));
   const int apitch = (ac + 1) / 2 * 2, bpitch = (bc + 1) / 2 * 2;
+  const double *da = nullptr, *db = nullptr;
+  if constexpr (!widen) {
+    da = a;
+    db = b;
+  }
   double* ws = nullptr;
   if (pa || pb) {
     const size_t an = pa ? size_t(ar) * apitch : 0, bn = pb ? size_t(br) * bpitch : 0;
@@ -453,27 +469,27 @@ cudaError_t gemm(double* c, const double* a, const double* b, int m, int n, int 
     if (pa) {
       pack_aligned<<<dim3((apitch + 1023) / 1024, std::min(ar, 65535)), 256, 0, stream>>>(
           ws, apitch, a, lda, ar, ac, nullptr, 0, 1, gate);
-      a = ws;
+      da = ws;
       lda = apitch;
     }
     if (pb) {
       pack_aligned<<<dim3((bpitch + 1023) / 1024, std::min(br, 65535)), 256, 0, stream>>>(
           ws + an, bpitch, b, ldb, br, bc, tab, ldtab, blk, gate);
-      b = ws + an;
+      db = ws + an;
       ldb = bpitch;
       tab = nullptr;
     }
     err = cudaGetLastError();
   }
-  p.a = a;
-  p.b = b;
+  p.a = da;
+  p.b = db;
   p.lda = lda;
   p.ldb = ldb;
   p.tab = tab;
   p.ldtab = ldtab;
   p.blk = blk;
-  p.avec = al16(a, lda);
-  p.bvec = !tab && al16(b, ldb);
+  p.avec = al16(da, lda);
+  p.bvec = !tab && al16(db, ldb);
   if (err == cudaSuccess) {
     if (!transa)
       err = transb ? launch_t<false, true>(p, stream) : launch_t<false, false>(p, stream);
@@ -492,6 +508,13 @@ cudaError_t gemm(double* c, const double* a, const double* b, int m, int n, int 
 cudaError_t dgemm_fp64(double* c, const double* a, const double* b, int m, int n, int k,
                        size_t lda, size_t ldb, size_t ldc, bool transa, bool transb,
                        cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
+  return gemm(c, a, b, m, n, k, lda, ldb, ldc, transa, transb, nullptr, 0, 1, Gate{nullptr, 0},
+              stream);
+}
+
+cudaError_t dgemm_f32(float* c, const float* a, const float* b, int m, int n, int k, size_t lda,
+                      size_t ldb, size_t ldc, bool transa, bool transb, cudaStream_t stream) {
   if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
   return gemm(c, a, b, m, n, k, lda, ldb, ldc, transa, transb, nullptr, 0, 1, Gate{nullptr, 0},
               stream);

@@ -10,6 +10,11 @@ cudaError_t dgemm_fp64(double* c, const double* a, const double* b, int m, int n
                        size_t lda, size_t ldb, size_t ldc, bool transa, bool transb,
                        cudaStream_t stream);
 
+// The same on f32 data: operands widened exactly, FP64 arithmetic, each element of C
+// rounded once.
+cudaError_t dgemm_f32(float* c, const float* a, const float* b, int m, int n, int k, size_t lda,
+                      size_t ldb, size_t ldc, bool transa, bool transb, cudaStream_t stream);
+
 // Masked GEMM (src/impl_matmul_non0tab.rs:210-306): B is not transposed;
 // element (p, j) of B takes part only when tab[p * ldtab + j / blk] != 0.
 cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int m, int n, int k,

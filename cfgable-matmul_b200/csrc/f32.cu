@@ -2,11 +2,12 @@
 //
 // The reference's MatmulLoops is generic over the element type (structs.rs:3-13)
 // with f64 implementations only (structs.rs:19-20); the f32 entry points of the
-// C ABI take f32 operands, widen them exactly to f64 in device scratch, run the
-// f64 kernels (DMMA, or the Ozaki split with the moduli that 26-bit operands
-// need) and round the accumulated result back to f32 once.  These kernels are
-// the widening and narrowing passes: one read and one write of each array,
-// vectorised where the base pointers allow, grid-stride over the SMs.
+// C ABI take f32 operands, widen them exactly to f64, run the f64 kernels (DMMA, or
+// the Ozaki split with the moduli that 26-bit operands need) and round the
+// accumulated result back to f32 once.  The GEMM reads f32 itself (ozaki.cu,
+// dgemm_fp64.cu); these kernels are the widening and narrowing passes of the
+// AO-DM-AO contraction: one read and one write of each array, vectorised where the
+// base pointers allow, grid-stride over the SMs.
 #include "f32.cuh"
 
 #include <cstdint>

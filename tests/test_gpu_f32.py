@@ -37,6 +37,34 @@ def test_matmul_f32(cm, prec, tol, transa, transb, m, n, k, pad):
     assert np.array_equal(c[:, n:], c0[:, n:])  # padding untouched
 
 
+@pytest.mark.parametrize("transa,transb", [(False, False), (True, True)])
+@pytest.mark.parametrize("m,n,k,pad", [
+    (1, 1, 1, 0),         # odd rows of one element
+    (65, 63, 17, 1),      # one past, one short of a tile; the widened rows padded by one
+    (66, 62, 1000, 0),    # eight parts of K in a cluster
+    (1543, 1601, 101, 0), # whole tiles' epilogue, a K step of five
+])
+def test_matmul_f32_direct(cm, transa, transb, m, n, k, pad):
+    """FP64 arithmetic into an f32 C on the device: each element one rounding of the
+    f64 result (half an ulp, and the f64 sums' own error far below it)."""
+    import torch
+    g = torch.Generator().manual_seed(m + 3 * n + 7 * k)
+    u = lambda *s: torch.rand(*s, generator=g, dtype=torch.float32) * 2 - 1
+    a = u(k, m + pad) if transa else u(m, k + pad)
+    b = u(n, k + pad) if transb else u(k, n + pad)
+    c0 = u(m, n + pad)
+    a64, b64 = a.double(), b.double()
+    ref = c0[:, :n].double() + (a64[:, :m].t() if transa else a64[:, :k]) @ (
+        b64[:, :k].t() if transb else b64[:, :n])
+    c = c0.cuda()
+    cm.matmul_f32(c, a.cuda(), b.cuda(), m, n, k, a.shape[1], b.shape[1], n + pad, transa, transb)
+    torch.cuda.synchronize()
+    got = c.cpu()
+    assert torch.equal(got[:, n:], c0[:, n:])
+    bound = ref.abs() * (2.0 ** -24 * 1.001) + k * 2.0 ** -52
+    assert bool(((got[:, :n].double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("prec,tol", [(0, 1e-7), (1, 2e-7)])
 def test_aodmao2rho_f32(cm, oracle, wl, prec, tol):
     p = wl.small_masked(seed=61, nao=512, ngrid=4000, blksize=64, nset=2)
