@@ -106,7 +106,7 @@ struct PairArgs {
   const int* cbase;       // [pair] first phi chunk
   const PairBatch* batches;  // device array, or null: `one`
   PairBatch one;
-  double* partial;        // [poff[pair] + row tile][nset_max][128]
+  double* partial;        // [poff[pair] + row tile][nset_max][column part][128]
   const int* poff;        // [pair] first partial row tile, or null: pair * max_t
   int nao, blk, gsub, max_t, nset_max;
   const int* asym;        // null, or 0 when every D_s is symmetric (half contraction)
@@ -176,7 +176,7 @@ cudaError_t split_pair_prepare_d(const double* dms, size_t stride_ao, int nao, i
                                  uint2* dsl, int* tau, uint2* dhalf, int* asym,
                                  cudaStream_t stream);
 int split_pair_stages();  // the pair kernel's pipeline depth
-// partial sums per (row tile, DM) of a pair: one per gather group and point
+// partial sums per (row tile, DM) of a pair: one per column part and point
 int split_pair_partial_points();
 // stages: ignored (the pair form's pipeline depth is fixed: split_pair_stages())
 cudaError_t split_pair_launch_main(const PairArgs& a, int nsl, cudaStream_t stream,

@@ -46,22 +46,26 @@
 //                 (points) x 32 bytes in the UMMA 32-byte-swizzled K-major
 //                 layout, so one bulk copy moves a chunk
 //   pair_d_digits D digits (8 bytes per element) and row scales
-//   pair_main     persistent, 14 warps: 12 warps gather the D digits of TN
-//                 rows x 32 union columns in three groups that take turns by
-//                 chunk and run the epilogue; 1 warp issues the MMAs (a chunk's
-//                 28 digit products as 10 MMAs of N up to 256: taxol-size call
-//                 0.89 -> 0.74 ms, tc::mma_digit_products); 1 warp
-//                 draws work items (dynamic, through a ring in shared memory)
-//                 and bulk-loads the phi tiles.  A group copies the item's
-//                 phi_lhs values to shared memory as the item starts, loads
-//                 its first chunk of the next item before the accumulator
-//                 wait and stores it right after reading TMEM, so the MMAs
-//                 resume at once.  The epilogue reads each point's TMEM row
-//                 (lane = point), rebuilds X in FP64, weights it with phi_lhs
-//                 and sums over the row's AOs -- no cross-lane reduction; X
-//                 never leaves the SM.
-//   pair_reduce   adds the partial sums of each point (per row tile and
-//                 gather group) in a fixed order (deterministic).
+//   pair_main     persistent, 23 warps.  12 gather the D digits of TN rows x 32
+//                 union columns, in three groups that take turns by chunk and
+//                 run on over the ends of items; 8 run the epilogue; one thread
+//                 each issues the MMAs (a chunk's 28 digit products as 10 MMAs
+//                 of N up to 256, tc::mma_digit_products), loads the phi tiles
+//                 in bulk, and draws work items (dynamic, through a ring in
+//                 shared memory).  The epilogue warps fetch the item's phi_lhs
+//                 values, row scales and flags while its chunks run, read each
+//                 point's TMEM row (lane = point), rebuild X in FP64, weight it
+//                 with phi_lhs and sum over the row's AOs -- no cross-lane
+//                 reduction; X never leaves the SM.  nao 2228, 16384 points, 3
+//                 matrices: 743 -> 621 us the whole call against gather warps
+//                 that ran the epilogue too (half of their time went to an
+//                 item's prologue and epilogue, with no loads in flight).  The
+//                 MMAs run for 52 % of the kernel's cycles (900 of a chunk); the
+//                 largest part of the rest is the accumulators' read at an
+//                 item's end, 5,000 cycles: seven levels of 64 columns leave no
+//                 TMEM for a second set.
+//   pair_reduce   adds the partial sums of each point (per row tile and part
+//                 of its columns) in a fixed order (deterministic).
 // Every mbarrier wait is bounded (tcgen05.cuh).
 #include <cuda_runtime.h>
 
@@ -84,8 +88,11 @@ constexpr int HT = 64;    // points per block tile (half an item)
 constexpr int TK = 32;    // union AOs per chunk: one INT8 MMA K step
 constexpr int NG = 3;     // gather groups of four warps
 constexpr int GW = 4 * NG;
-constexpr int THREADS = 32 * (GW + 2);
-constexpr int kStages = 3;        // pipeline depth (at least NG: see the row form)
+constexpr int EG = 2;     // epilogue groups of four warps, each a part of the columns
+constexpr int EW = 4 * EG;
+constexpr int MMA_WARP = GW + EW, LOAD_WARP = MMA_WARP + 1, DRAW_WARP = MMA_WARP + 2;
+constexpr int THREADS = 32 * (DRAW_WARP + 1);
+constexpr int kStages = 3;        // pipeline depth
 constexpr int kBadExp = INT_MAX;  // scale of a row / point holding Inf or NaN
 constexpr int kWin = 32;          // pairing candidates on each side in key order
 constexpr int kSortMax = 4096;    // tiles sorted in shared memory (more: caller's order)
@@ -93,7 +100,7 @@ constexpr int kRounds = 8;        // mutual-best matching rounds
 constexpr int kMatchCandMax = 600;  // tiles whose candidate lists the matching stages in shared memory
 constexpr int kRing = 4;          // work items in flight between the kernel's roles
 constexpr int kAhead = 2;         // items drawn ahead of the one being loaded (< kRing)
-static_assert(kStages >= NG, "a group's parity wait needs at least NG stages");
+static_assert(kStages == NG, "a group waits for every phase of its stage in turn");
 
 template <int NSL>
 struct Cfg {
@@ -105,18 +112,18 @@ struct Cfg {
   static constexpr uint32_t STAGE = A_STAGE + B_STAGE;
   static constexpr int WROWS = TN / 4;     // D rows per gather warp
   static constexpr int STEPS = WROWS / 4;  // four rows per step
-  static constexpr int OCTETS = TN / 8;    // TMEM column octets of one level
-  static constexpr int MAXQ = 2 * ((OCTETS + NG - 1) / NG);  // epilogue quartets per group
-  // shared memory of a launch: stages, barriers, the item ring and the
-  // epilogue's phi_lhs values ([warp][column][lane])
+  static constexpr int CW = TN / EG;       // columns of an epilogue warp
+  static constexpr int ROUNDS = (CW + 31) / 32;
+  // shared memory of a launch: stages, barriers, the item ring, the epilogue's
+  // row scales ([warp][column]) and phi_lhs values ([warp][column][lane])
   template <int STAGES>
   static constexpr size_t smem_bytes() {
-    return size_t(STAGES) * STAGE + 1024 + 256 + kRing * (16 + 4) +
-           size_t(GW) * 4 * MAXQ * 32 * 8;
+    return size_t(STAGES) * STAGE + 1024 + 256 + kRing * 32 + size_t(EW) * CW * 8 +
+           size_t(EW) * CW * 32 * 8;
   }
   static_assert(NSL * TN <= 512, "level accumulators exceed the TMEM columns");
   static_assert(STAGE % 256 == 0 && A_STAGE % 256 == 0, "32-byte swizzle atoms");
-  static_assert(WROWS % 4 == 0 && (OCTETS + NG - 1) / NG * 8 <= 32, "epilogue columns per group");
+  static_assert(WROWS % 4 == 0 && TN % (4 * EG) == 0, "rows and columns in fours");
 };
 
 __device__ int g_pair_error;
@@ -720,7 +727,7 @@ pair_phi_tiles(const double* __restrict__ ao, size_t stride_grid,
         uint2 w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const int k = c * TK + q * 4 + t;
+          const int k = c * TK + 8 * t + q;  // K slot 4q + t (see pair_main)
           const bool on = g >= 0 && k < nu && e != kBadExp && ((__ldg(F + k) >> h) & 1u);
           w[t] = on ? digits_of<NSL>(ao[size_t(__ldg(U + k)) * stride_grid + g], e)
                     : make_uint2(0u, 0u);
@@ -834,23 +841,17 @@ pair_d_prep(const double* __restrict__ dms, size_t stride_ao, size_t dm_stride, 
     out[v] = e != kBadExp ? digits_of<NSL>(d[v], e) : make_uint2(0u, 0u);
 }
 
-// Byte selector assembling, from `keep` (bytes 0..3) and `recv` (4..7) of the
-// gather's second shuffle round, the digit word of 4 consecutive columns:
-// column qd from keep.b0, qd^2 from keep.b2, qd^1 from recv.b0, qd^3 from
-// recv.b2 (the lane's second digit plane: +1 on every nibble).
-__device__ __forceinline__ uint32_t gather_selector(int qd) {
-  uint32_t sel = 0;
-#pragma unroll
-  for (int col = 0; col < 4; ++col) {
-    const uint32_t src = col == qd ? 0u : col == (qd ^ 2) ? 2u : col == (qd ^ 1) ? 4u : 6u;
-    sel |= src << (4 * col);
-  }
-  return sel;
-}
-
 // ---------------------------------------------------------------------------
 // main kernel
 // ---------------------------------------------------------------------------
+// A work item as the roles read it from the ring in shared memory.
+struct alignas(16) RingItem {
+  int pi, ut, s, w;  // pair, row tile, DM, batch
+  int nu;            // union size of the pair
+  int live;          // 0: no more items
+  int pad[2];
+};
+
 template <int NSL, int STAGES>
 __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
   using C = Cfg<NSL>;
@@ -865,14 +866,17 @@ __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
   uint64_t* acc_full = bars + 3 * STAGES;
   uint64_t* acc_empty = acc_full + 1;
   uint64_t* drain = acc_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 5);
-  // the work-item ring: the loader thread draws items from the global counter
-  // (dynamic scheduling: the list is pair-major, heaviest pairs first) and
-  // every role reads them from here in the same order
-  uint64_t* ifull = reinterpret_cast<uint64_t*>(smem + STAGES * C::STAGE + 256);  // [kRing]
-  uint64_t* iempty = ifull + kRing;                                   // [kRing]
-  int* ring = reinterpret_cast<int*>(iempty + kRing);                 // [kRing]
-  double* phl_all = reinterpret_cast<double*>(ring + kRing);          // [GW][4 MAXQ][32]
+  uint64_t* started = acc_full + 3;     // [kRing]: the loader began the item
+  uint64_t* ifull = started + kRing;    // [kRing]
+  uint64_t* iempty = ifull + kRing;     // [kRing]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(iempty + kRing);
+  static_assert((3 * STAGES + 3 + 3 * kRing) * 8 + 4 <= 256, "barrier block");
+  // the work-item ring: one thread draws items from the global counter (dynamic
+  // scheduling: the list is pair-major, heaviest pairs first) and every role
+  // reads them from here in the same order
+  RingItem* ring = reinterpret_cast<RingItem*>(smem + STAGES * C::STAGE + 256);
+  double* scale_all = reinterpret_cast<double*>(ring + kRing);  // [EW][CW]
+  double* phl_all = scale_all + EW * C::CW;                     // [EW][CW][32]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* err = &g_pair_error;
@@ -884,15 +888,16 @@ __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
       tc::mbar_init(&empty[s], 1);
     }
     tc::mbar_init(acc_full, 1);
-    tc::mbar_init(acc_empty, GW);
+    tc::mbar_init(acc_empty, EW);
     tc::mbar_init(drain, 1);
     for (int r = 0; r < kRing; ++r) {
+      tc::mbar_init(&started[r], 1);
       tc::mbar_init(&ifull[r], 1);
-      tc::mbar_init(&iempty[r], GW + 2);  // every warp reads every item
+      tc::mbar_init(&iempty[r], GW + EW + 2);  // every warp but the drawing one reads every item
     }
     tc::mbar_fence_init();
   }
-  if (warp == GW) {
+  if (warp == MMA_WARP) {
     tc::tmem_alloc(tmem_slot, 512);
     tc::tmem_relinquish();
   }
@@ -900,305 +905,260 @@ __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const int total = p.total[0];
   const bool sym = p.asym != nullptr && *p.asym == 0;
-  // item n of this CTA (total when there are no more), read from the ring by
-  // lane 0 of the calling warp and broadcast; every warp calls it for n = 0, 1, ...
-  auto item_of = [&](uint32_t n, bool whole_warp) -> int {
-    int t = total;
-    if (!whole_warp || lane == 0) {
-      if (tc::mbar_wait(&ifull[n % kRing], (n / kRing) & 1, err, 40, false, lim))
-        t = *reinterpret_cast<volatile int*>(&ring[n % kRing]);
-      tc::mbar_arrive(&iempty[n % kRing]);
+  // item n of this CTA, read by the whole warp (or by its lane 0 alone); false
+  // when there are no more.  Every warp calls it for n = 0, 1, ...
+  auto item_of = [&](uint32_t n, bool whole_warp, RingItem& it) -> bool {
+    int got = 0;
+    if (!whole_warp || lane == 0)
+      got = tc::mbar_wait(&ifull[n % kRing], (n / kRing) & 1, err, 40, false, lim);
+    if (whole_warp) {
+      got = __shfl_sync(0xffffffffu, got, 0);
+      __syncwarp();
     }
-    if (whole_warp) t = __shfl_sync(0xffffffffu, t, 0);
-    return t;
+    if (!got) return false;
+    it = *(ring + n % kRing);
+    if (whole_warp) __syncwarp();
+    if (!whole_warp || lane == 0) tc::mbar_arrive(&iempty[n % kRing]);
+    return it.live != 0;
   };
 
   if (warp < GW) {
-    // ---------------- gather D digits, then the epilogue ----------------
-    // Group grp takes the chunks c = kc0 + grp, + NG, ... of every item; warp
-    // wq of the group fills D rows WROWS*wq .. of the tile, four rows per step.
-    // Lane (qd, ri, hh) = lane bits (4:3, 2:1, 0) loads, for row 4*step+ri,
-    // the union columns 16hh + 4k + qd (k = 0..3) and ends up holding digit
-    // planes 2qd and 2qd+1 of the 16-byte half hh of that row.
+    // ---------------- gather D digits ----------------
+    // Group grp fills every NG-th chunk of the CTA's stream of chunks (its
+    // items' chunks one after another), so always the same stage; warp wq of the
+    // group fills D rows WROWS*wq .. of the tile, four rows per step.  Lane (ri, x)
+    // = lane bits (4:3, 2:0) takes K slots 4x .. 4x+3 of row 4*step + ri: slot
+    // 4x + k of a chunk is union column 8k + x, in the phi tiles too, so that one
+    // load instruction reads 8 columns (64 bytes) of each row and the lane's four
+    // digit strings transpose into one word per plane within the lane, stored
+    // free of bank conflicts (8 words x 4 rows = 128 consecutive bytes).  The
+    // loads of step st of the group's next chunk are issued as soon as step st of
+    // this one is in its stage, and the indices of the chunk after that a chunk
+    // earlier, over the ends of items.
     const int grp = warp >> 2, wq = warp & 3;
-    const int qd = lane >> 3, ri = (lane >> 1) & 3, hh = lane & 1;
-    const bool b1 = (qd & 2) != 0, b0 = (qd & 1) != 0;
-    const uint32_t sel_a = gather_selector(qd), sel_b = sel_a + 0x1111u;
-    // this warp's phi_lhs values for the epilogue: [group column][lane]
-    double* phl = phl_all + size_t(warp) * (4 * C::MAXQ * 32);
-    struct Item {
-      int t, pi, ut, s, w, nu, kc, kc0;
-      int iu[C::STEPS];  // AO of the D row this lane loads at each step (-1: none)
-    };
-    auto setup = [&](int t, Item& g) {
-      g.t = t;
-      if (t >= total) return;
-      const int4 it = p.items[t];
-      g.pi = it.x;
-      g.ut = it.y;
-      g.s = it.z;
-      g.w = it.w;
-      g.nu = p.ucount[g.pi];
-      g.kc = (g.nu + TK - 1) / TK;
-      g.kc0 = sym ? (g.ut * TN) / TK : 0;
-      const int* U = p.ulist + size_t(g.pi) * p.nao;
+    const int ri = lane >> 3, x = lane & 7;
+    // the chunk whose indices are held
+    uint32_t nitem = 0, base = 0, nch = 0;  // items read, first chunk of the last one, its chunks
+    int row0 = 0, kc0 = 0, col0 = 0;
+    bool more = true, diag = false, whole = false;
+    RingItem it;
+    it.s = 0;
+    int iu[C::STEPS];  // AO of the D row this lane loads at each step (-1: none)
+    int iv[4];         // AO of the column (-1: past the list)
 #pragma unroll
-      for (int st = 0; st < C::STEPS; ++st) {
-        const int prow = g.ut * TN + C::WROWS * wq + 4 * st + ri;
-        g.iu[st] = prow < g.nu ? __ldg(U + prow) : -1;
+    for (int st = 0; st < C::STEPS; ++st) iu[st] = -1;
+    auto advance = [&](uint32_t q) {  // to chunk q of the stream
+      bool fresh = false;
+      while (q >= base + nch) {
+        base += nch;
+        more = item_of(nitem++, true, it);
+        if (!more) return;
+        row0 = it.ut * TN;
+        kc0 = sym ? row0 / TK : 0;
+        nch = uint32_t((it.nu + TK - 1) / TK - kc0);
+        fresh = true;
       }
-    };
-    // the union columns this lane loads in chunk c (-1: past the list)
-    auto columns = [&](const Item& g, int c, int (&iv)[4]) {
-      const int* U = p.ulist + size_t(g.pi) * p.nao;
+      const int* U = p.ulist + size_t(it.pi) * p.nao;
+      col0 = (kc0 + int(q - base)) * TK;
+      diag = sym && col0 < row0 + TN;
+      whole = !diag && col0 + TK <= it.nu && row0 + TN <= it.nu;
+      if (fresh) {
+#pragma unroll
+        for (int st = 0; st < C::STEPS; ++st) {
+          const int prow = row0 + C::WROWS * wq + 4 * st + ri;
+          iu[st] = prow < it.nu ? __ldg(U + prow) : -1;
+        }
+      }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int pc = c * TK + 16 * hh + 4 * k + qd;
-        iv[k] = pc < g.nu ? __ldg(U + pc) : -1;
+        const int pc = col0 + 8 * k + x;
+        iv[k] = pc < it.nu ? __ldg(U + pc) : -1;
       }
     };
-    // The MMAs of every chunk up to `done` (stage sequence number) are known
-    // to have completed.  A parity wait names a phase only while the phase
-    // before it has completed, so stage_free steps through the completions
-    // in order: waiting for chunk y is safe once chunk y - STAGES is done.
-    long long done = -1;
-    auto stage_free = [&](uint32_t seq) -> bool {
-      const long long need = static_cast<long long>(seq) - STAGES;
-      while (done < need) {
-        const long long y = done + STAGES < need ? done + STAGES : need;
-        if (!tc::mbar_wait(&empty[y % STAGES], uint32_t((y / STAGES) & 1), err, 31, false, lim))
-          return false;
-        done = y;
-      }
-      return true;
-    };
-    // D digits of chunk c of item g at this lane's positions (no waits)
-    auto load_chunk = [&](const Item& g, int c, const int (&iv)[4], uint2 (&w)[C::STEPS][4]) {
-      const uint2* dset = p.dsl + size_t(g.s) * p.nao * p.nao;
-      const uint2* dh = p.dhalf + size_t(g.s) * p.nao;
-      // symmetric D: only columns from the row's own position on, the
-      // diagonal with the digits of D_uu / 2
+    uint2 w[C::STEPS][4];
+    // symmetric D: only columns from the row's own position on, the diagonal
+    // with the digits of D_uu / 2
+    auto load_step = [&](int st) {
+      const size_t rowi = size_t(it.s) * p.nao + (iu[st] >= 0 ? iu[st] : 0);
+      const uint2* row = p.dsl + rowi * p.nao;
+      if (whole) {
 #pragma unroll
-      for (int st = 0; st < C::STEPS; ++st) {
-        const int prow = g.ut * TN + C::WROWS * wq + 4 * st + ri;
+        for (int k = 0; k < 4; ++k) w[st][k] = __ldg(row + iv[k]);
+      } else if (!diag) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          w[st][k] = iu[st] >= 0 && iv[k] >= 0 ? __ldg(row + iv[k]) : make_uint2(0u, 0u);
+      } else {
+        const int prow = row0 + C::WROWS * wq + 4 * st + ri;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const int pc = c * TK + 16 * hh + 4 * k + qd;
-          w[st][k] = (g.iu[st] >= 0 && iv[k] >= 0 && (!sym || pc >= prow))
-                         ? __ldg(sym && pc == prow ? dh + g.iu[st]
-                                                   : dset + size_t(g.iu[st]) * p.nao + iv[k])
+          const int pc = col0 + 8 * k + x;
+          w[st][k] = iu[st] >= 0 && iv[k] >= 0 && pc >= prow
+                         ? __ldg(pc == prow ? p.dhalf + rowi : row + iv[k])
                          : make_uint2(0u, 0u);
         }
       }
     };
-    // the loaded digits into stage seq % STAGES as digit planes (false: a wait ran out)
-    auto store_chunk = [&](uint32_t seq, const uint2 (&w)[C::STEPS][4]) -> bool {
-      if (!stage_free(seq)) return false;
-      const int stg = int(seq % STAGES);
+    // the loaded digits of a step into the stage as digit planes
+    auto store_step = [&](uint8_t* Bs, int st) {
+      uint32_t o[8];
+      transpose4(w[st][0].x, w[st][1].x, w[st][2].x, w[st][3].x, o[0], o[1], o[2], o[3]);
+      transpose4(w[st][0].y, w[st][1].y, w[st][2].y, w[st][3].y, o[4], o[5], o[6], o[7]);
+      uint8_t* dst = Bs + 4 * (x & 3) +
+                     tc::sw32_offset(uint32_t(C::WROWS * wq + 4 * st + ri), uint32_t(x >> 2));
+#pragma unroll
+      for (int j = 0; j < NSL; ++j) *reinterpret_cast<uint32_t*>(dst + j * C::B_SLICE) = o[j];
+    };
+
+    uint32_t q = uint32_t(grp);
+    advance(q);
+    bool live = more;
+    if (live) {
+#pragma unroll
+      for (int st = 0; st < C::STEPS; ++st) load_step(st);
+      advance(q + NG);
+    }
+    while (live) {
+      const uint32_t stg = q % STAGES;
+      if (q >= STAGES &&
+          !__all_sync(0xffffffffu, tc::mbar_wait(&empty[stg], (q / STAGES - 1) & 1, err, 31,
+                                                 false, lim)))
+        break;
       uint8_t* Bs = smem + stg * C::STAGE + C::A_STAGE;
+      live = more;
 #pragma unroll
       for (int st = 0; st < C::STEPS; ++st) {
-        uint32_t wa[4], wb[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          // round 1 (lanes qd, qd^2): keep digits 0-3 (b1 = 0) or 4-7 (b1 = 1)
-          const uint32_t x = b1 ? w[st][k].y : w[st][k].x;
-          const uint32_t y = __shfl_xor_sync(0xffffffffu, b1 ? w[st][k].x : w[st][k].y, 16);
-          // round 2 (lanes qd, qd^1): keep two of those four digits
-          const uint32_t lo = __byte_perm(x, y, 0x5410), hi = __byte_perm(x, y, 0x7632);
-          const uint32_t keep = b0 ? hi : lo;
-          const uint32_t recv = __shfl_xor_sync(0xffffffffu, b0 ? lo : hi, 8);
-          wa[k] = __byte_perm(keep, recv, sel_a);
-          wb[k] = __byte_perm(keep, recv, sel_b);
-        }
-        const uint32_t off =
-            tc::sw32_offset(uint32_t(C::WROWS * wq + 4 * st + ri), uint32_t(hh));
-        if (2 * qd < NSL)
-          *reinterpret_cast<uint4*>(Bs + (2 * qd) * C::B_SLICE + off) =
-              make_uint4(wa[0], wa[1], wa[2], wa[3]);
-        if (2 * qd + 1 < NSL)
-          *reinterpret_cast<uint4*>(Bs + (2 * qd + 1) * C::B_SLICE + off) =
-              make_uint4(wb[0], wb[1], wb[2], wb[3]);
+        store_step(Bs, st);
+        if (live) load_step(st);
       }
       tc::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&full_d[stg]);
-      return true;
-    };
-
-    const int h = wq >> 1;           // the warp's block tile: lo (0) or hi (1)
-    const int r = 32 * wq + lane;    // TMEM lane = point row
-    const uint32_t trow = tmem + (uint32_t(32 * wq) << 16);
-    uint32_t seq0 = 0;  // stage sequence number of the current item's first chunk
-    bool ok = true, ahead = false;
-    Item cur, nxt;
-    setup(item_of(0, true), cur);
-    for (uint32_t nitem = 0; ok && cur.t < total; ++nitem) {
-      // ---- what the epilogue needs, requested first: lane l holds column l
-      // of the group's columns (octets grp, grp+NG, ...): its AO, membership
-      // flags and row scale; phi_lhs of every group column at this lane's
-      // point, for AOs active in its block (zero-filled elsewhere), is copied
-      // to shared memory while the item's chunks run; bit 4qi+j of `on`
-      // marks column j of quartet qi ----
-      const PairBatch& B = batch_of(p, cur.w);
-      int gpt, sg, nq, eg;
-      // 2^(-tau - eg) of this lane's column, eg the largest -tau of the
-      // group's columns (so every factor is at most 1 and the group's sum
-      // is scaled by 2^eg once); 0 for a row holding Inf or NaN
-      double s_l;
-      uint32_t badbits;  // lanes whose column's D row holds Inf or NaN
-      bool gval;
-      uint32_t on = 0;
-      {
-        const int4 pr = p.pairs[cur.pi];
-        const int tile = h ? pr.y : pr.x;
-        int g0 = 0, gend = 0;
-        if (tile >= 0) tile_points(tile, p.blk, p.gsub, B.ngrid, &g0, &gend);
-        gpt = g0 + (r & (HT - 1));
-        gval = tile >= 0 && gpt < gend;
-        // the group's columns of this tile, in quartets (warp-uniform):
-        // octets grp, grp+NG, ... below OCTETS whose first column lies inside U
-        int nocts = 0;
-        while (grp + NG * nocts < C::OCTETS && cur.ut * TN + (grp + NG * nocts) * 8 < cur.nu)
-          ++nocts;
-        nq = 2 * nocts;
-        const int col_l = (grp + NG * (lane >> 3)) * 8 + (lane & 7);
-        const int kpos_l = cur.ut * TN + col_l;
-        const bool cval_l = col_l < TN && kpos_l < cur.nu;
-        const int u_l = cval_l ? __ldg(p.ulist + size_t(cur.pi) * p.nao + kpos_l) : 0;
-        const int f_l = cval_l ? int(p.uflag[size_t(cur.pi) * p.nao + kpos_l]) : 0;
-        const int tu_l = cval_l ? p.tau[size_t(cur.s) * p.nao + u_l] : kBadExp;
-        const bool bad_l = cval_l && tu_l == kBadExp;
-        eg = __reduce_max_sync(0xffffffffu, tu_l != kBadExp ? -tu_l : INT_MIN);
-        if (eg == INT_MIN) eg = 0;
-        s_l = tu_l != kBadExp ? ldexp(1.0, -tu_l - eg) : 0.0;
-        badbits = __ballot_sync(0xffffffffu, bad_l);
-        sg = gval ? B.sigma[gpt] : 0;
+      q += NG;
+      if (live) advance(q + NG);
+    }
+  } else if (warp < GW + EW) {
+    // ---------------- epilogue ----------------
+    // Warp (eg, wq) takes TMEM lanes 32wq .. (points) and columns CW*eg .. of
+    // the item.  What it needs -- the columns' AOs, flags and row scales, and
+    // phi_lhs of every column at this lane's point for AOs active in its block
+    // (zero elsewhere), copied to shared memory -- is fetched while the item's
+    // chunks run.
+    const int ew = warp - GW, eg = ew >> 2, wq = warp & 3;
+    static_assert(GW % 4 == 0, "warp index modulo 4 names the TMEM lanes");
+    const int h = wq >> 1;         // the warp's block tile: lo (0) or hi (1)
+    const int r = 32 * wq + lane;  // TMEM lane = point row
+    const uint32_t trow = tmem + (uint32_t(32 * wq) << 16) + uint32_t(eg * C::CW);
+    double* phl = phl_all + size_t(ew) * (C::CW * 32) + lane;
+    double* scale = scale_all + ew * C::CW;
+    RingItem it;
+    for (uint32_t n = 0; item_of(n, true, it); ++n) {
+      const PairBatch& B = batch_of(p, it.w);
+      const int4 pr = p.pairs[it.pi];
+      const int tile = h ? pr.y : pr.x;
+      int g0 = 0, gend = 0;
+      if (tile >= 0) tile_points(tile, p.blk, p.gsub, B.ngrid, &g0, &gend);
+      const int gpt = g0 + (r & (HT - 1));
+      const bool gval = tile >= 0 && gpt < gend;
+      const int first = it.ut * TN + eg * C::CW;          // union position of column 0
+      const int ncol = max(0, min(C::CW, it.nu - first));
+      const int nq = (ncol + 3) / 4;                      // quartets of columns
+      const int* U = p.ulist + size_t(it.pi) * p.nao + first;
+      const uint8_t* F = p.uflag + size_t(it.pi) * p.nao + first;
+      const int sg = gval ? B.sigma[gpt] : 0;
+      bool badrow = false;  // an active column whose D row holds Inf or NaN
+      int tu[C::ROUNDS];
+      int ebase = INT_MIN;  // largest -tau of the warp's columns
 #pragma unroll
-        for (int qi = 0; qi < C::MAXQ; ++qi) {
-          if (qi < nq) {
-            const int col0 = (grp + NG * (qi >> 1)) * 8 + 4 * (qi & 1);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int src = qi * 4 + j;  // lane holding the column
-              const int uj = __shfl_sync(0xffffffffu, u_l, src);
-              const int fj = __shfl_sync(0xffffffffu, f_l, src);
-              const bool o = gval && cur.ut * TN + col0 + j < cur.nu && ((fj >> h) & 1);
-              on |= uint32_t(o) << src;
-              cp_async_8(phl + src * 32 + lane,
-                         B.ao_lhs + (o ? size_t(uj) * B.stride_grid + gpt : 0), o);
-            }
-          }
+      for (int rd = 0; rd < C::ROUNDS; ++rd) {
+        const int cl = 32 * rd + lane;  // this lane's column
+        const int u_l = cl < ncol ? __ldg(U + cl) : 0;
+        const int f_l = cl < ncol ? int(F[cl]) : 0;
+        tu[rd] = cl < ncol ? p.tau[size_t(it.s) * p.nao + u_l] : kBadExp;
+        const int cend = min(32, 4 * nq - 32 * rd);
+        const uint32_t badbits = __ballot_sync(0xffffffffu, cl < ncol && tu[rd] == kBadExp);
+#pragma unroll 4
+        for (int j = 0; j < cend; ++j) {
+          const int uj = __shfl_sync(0xffffffffu, u_l, j);
+          const int fj = __shfl_sync(0xffffffffu, f_l, j);
+          const bool o = gval && ((fj >> h) & 1);
+          badrow |= o && ((badbits >> j) & 1);
+          cp_async_8(phl + (32 * rd + j) * 32,
+                     B.ao_lhs + (o ? size_t(uj) * B.stride_grid + gpt : 0), o);
         }
-        cp_async_commit();
+        ebase = max(ebase, __reduce_max_sync(0xffffffffu, tu[rd] != kBadExp ? -tu[rd] : INT_MIN));
       }
-      // ---- the group's chunks of the item (the first one already in its
-      // stage when `ahead`), the union columns of the next one loaded a
-      // chunk ahead ----
-      int c = cur.kc0 + grp + (ahead ? NG : 0);
-      int ivn[4];
-      columns(cur, c, ivn);
-      for (; c < cur.kc; c += NG) {
-        int iv[4];
+      cp_async_commit();
+      if (ebase == INT_MIN) ebase = 0;
+      // 2^(-tau - ebase): at most 1, so the warp's sum is scaled by 2^ebase
+      // once; 0 for a row holding Inf or NaN
 #pragma unroll
-        for (int k = 0; k < 4; ++k) iv[k] = ivn[k];
-        columns(cur, c + NG, ivn);
-        uint2 w[C::STEPS][4];
-        load_chunk(cur, c, iv, w);
-        if (!store_chunk(seq0 + uint32_t(c - cur.kc0), w)) {
-          ok = false;
-          break;
-        }
-      }
-      if (!ok) break;
-      const uint32_t seq1 = seq0 + uint32_t(cur.kc - cur.kc0);
-      // ---- the next item's first chunk of this group: loaded now, stored
-      // as soon as the accumulators are read, so the MMAs go on at once.
-      // Its stage was last used by chunk seq1 + grp - STAGES < seq1
-      // (NG <= STAGES): a chunk of this item or before, done once the
-      // accumulators are full ----
-      setup(item_of(nitem + 1, true), nxt);
-      ahead = nxt.t < total && nxt.kc0 + grp < nxt.kc;
-      uint2 wn[C::STEPS][4];
-      if (ahead) {
-        int iv[4];
-        columns(nxt, nxt.kc0 + grp, iv);
-        load_chunk(nxt, nxt.kc0 + grp, iv, wn);
-      }
-      // ---- epilogue: this warp's 32 points (TMEM lanes 32wq ..) over the
-      // group's column octets ----
-      const bool acc_ok = tc::mbar_wait(acc_full, nitem & 1, err, 32, false, lim);
+      for (int rd = 0; rd < C::ROUNDS; ++rd)
+        if (32 * rd + lane < C::CW)
+          scale[32 * rd + lane] = tu[rd] != kBadExp ? ldexp(1.0, -tu[rd] - ebase) : 0.0;
+      __syncwarp();
+      const bool acc_ok =
+          __all_sync(0xffffffffu, tc::mbar_wait(acc_full, n & 1, err, 32, false, lim));
       cp_async_wait<0>();
       if (!acc_ok) break;
       tc::fence_after_sync();
-      if (done < static_cast<long long>(seq1) - 1) done = static_cast<long long>(seq1) - 1;
-      double acc = 0.0;
-      // an active column whose D row holds Inf or NaN makes the point's value NaN
-      const bool badrow = (on & badbits) != 0;
+      // phi_lhs is zero where the AO is inactive in this point's block and the
+      // scale is zero for a row holding Inf or NaN (flagged above), so every
+      // column goes through the same branch-free update, each of a quartet in a
+      // sum of its own
+      double acc4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+      for (int qi = 0; qi < nq; ++qi) {
+        uint32_t v[NSL][4];
 #pragma unroll
-      for (int qi = 0; qi < C::MAXQ; ++qi) {
-        if (qi < nq) {
-          const int col0 = (grp + NG * (qi >> 1)) * 8 + 4 * (qi & 1);
-          uint32_t v[NSL][4];
+        for (int L = 0; L < NSL; ++L)
+          tc::tmem_ld_32x32b_x4(trow + uint32_t(L * TN + 4 * qi), v[L]);
+        tc::tmem_ld_wait();
+        if (qi + 1 == nq) {  // the accumulators are read: the MMA warp may go on
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(acc_empty);
+        }
 #pragma unroll
-          for (int L = 0; L < NSL; ++L)
-            tc::tmem_ld_32x32b_x4(trow + uint32_t(L * TN + col0), v[L]);
-          tc::tmem_ld_wait();
-          if (qi + 1 == nq) {  // the accumulators are read: the MMA warp may go on
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(acc_empty);
-          }
-          // phi_lhs is zero where the AO is inactive in this point's block
-          // and s is zero for a row holding Inf or NaN (flagged above), so
-          // every column goes through the same branch-free update
+        for (int j = 0; j < 4; ++j) {
+          uint32_t lv[NSL];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int src = qi * 4 + j;
-            const double sj = __shfl_sync(0xffffffffu, s_l, src);
-            uint32_t lv[NSL];
-#pragma unroll
-            for (int L = 0; L < NSL; ++L) lv[L] = v[L][j];
-            acc = fma(phl[src * 32 + lane], combine_levels<NSL>(lv) * sj, acc);
-          }
+          for (int L = 0; L < NSL; ++L) lv[L] = v[L][j];
+          acc4[j] = fma(phl[(4 * qi + j) * 32], combine_levels<NSL>(lv) * scale[4 * qi + j], acc4[j]);
         }
       }
+      const double acc = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
       if (nq == 0) {
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(acc_empty);
       }
-      if (ahead && !store_chunk(seq1 + uint32_t(grp), wn)) break;
+      __syncwarp();  // the scales are read
       double res = 0.0;
       if (gval) {
-        const int e = eg - sg;
+        const int e = ebase - sg;
         res = (sg == kBadExp || badrow) ? __longlong_as_double(0x7ff8000000000000LL)
               : (e >= -1022 && e <= 1023) ? acc * pow2(e)
                                           : ldexp(acc, e);
         if (sym) res *= 2.0;
       }
-      // each group's own partial sum (the reduction adds the groups and the
-      // row tiles in a fixed order), so no group waits for another here
-      const size_t pbase = p.poff ? size_t(p.poff[cur.pi]) : size_t(cur.pi) * p.max_t;
-      p.partial[(((pbase + cur.ut) * p.nset_max + cur.s) * NG + grp) * PT + r] = res;
-      seq0 = seq1;
-      cur = nxt;
+      // each warp's own partial sum (the reduction adds the column parts and
+      // the row tiles in a fixed order)
+      const size_t pbase = p.poff ? size_t(p.poff[it.pi]) : size_t(it.pi) * p.max_t;
+      p.partial[(((pbase + it.ut) * p.nset_max + it.s) * EG + eg) * PT + r] = res;
     }
-  } else if (warp == GW) {
+    cp_async_wait<0>();
+  } else if (warp == MMA_WARP) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      uint32_t seq = 0, nitem = 0;
+      uint32_t seq = 0;
       bool ok = true;
-      for (;; ++nitem) {
-        const int t = item_of(nitem, false);
-        if (t >= total || !ok) break;
-        const int4 it = p.items[t];
-        const int nu = p.ucount[it.x];
-        const int kc = (nu + TK - 1) / TK;
-        const int kc0 = sym ? (it.y * TN) / TK : 0;
-        if (nitem > 0 && !tc::mbar_wait(acc_empty, (nitem - 1) & 1, err, 33, false, lim)) break;
+      RingItem it;
+      for (uint32_t n = 0; ok && item_of(n, false, it); ++n) {
+        const int kc = (it.nu + TK - 1) / TK;
+        const int kc0 = sym ? (it.ut * TN) / TK : 0;
+        if (n > 0 && !tc::mbar_wait(acc_empty, (n - 1) & 1, err, 33, false, lim)) break;
         tc::fence_after_sync();
         for (int c = kc0; c < kc; ++c, ++seq) {
           const int stg = int(seq % STAGES);
@@ -1221,45 +1181,17 @@ __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
       tc::mma_commit(drain);
       tc::mbar_wait(drain, 0, err, 36, true, lim);
     }
-  } else {
+  } else if (warp == LOAD_WARP) {
     // ---------------- phi digit tiles: bulk loads ----------------
     if (lane == 0) {
       uint32_t seq = 0;
-      uint32_t issued[STAGES];
-#pragma unroll
-      for (int s = 0; s < STAGES; ++s) issued[s] = 0;
       bool ok = true;
-      // Items are drawn kAhead ahead of the one whose tiles are loaded, so a
-      // gather group finds the next item in the ring when it reaches it.  A
-      // draw waits until every warp has read the slot's previous item; after
-      // a failed wait the terminal item goes in, so every role stops.
-      int tq[kRing];  // the drawn items by ring slot
-      uint32_t ndrawn = 0;
-      bool ended = false;
-      auto draw = [&]() {
-        const uint32_t n = ndrawn++;
-        const int slot = int(n % kRing);
-        int t = total;
-        if (ok && (n < kRing || tc::mbar_wait(&iempty[slot], ((n / kRing) - 1) & 1, err, 41,
-                                              false, lim))) {
-          t = atomicAdd(p.counter, 1);
-          if (t > total) t = total;
-        }
-        ring[slot] = t;
-        tq[slot] = t;
-        tc::mbar_arrive(&ifull[slot]);   // release: the slot's value is visible to the waiters
-        tc::mbar_arrive(&iempty[slot]);  // this warp's own read
-        ended = t >= total;
-      };
-      for (uint32_t n = 0;; ++n) {
-        while (!ended && ndrawn <= n + kAhead) draw();
-        const int t = tq[n % kRing];
-        if (t >= total) break;
-        const int4 it = p.items[t];
-        const int nu = p.ucount[it.x];
-        const int kc = (nu + TK - 1) / TK;
-        const int kc0 = sym ? (it.y * TN) / TK : 0;
-        const uint8_t* src = p.phisl + size_t(p.cbase[it.x]) * C::A_STAGE;
+      RingItem it;
+      for (uint32_t n = 0; ok && item_of(n, false, it); ++n) {
+        tc::mbar_arrive(&started[n % kRing]);
+        const int kc = (it.nu + TK - 1) / TK;
+        const int kc0 = sym ? (it.ut * TN) / TK : 0;
+        const uint8_t* src = p.phisl + size_t(p.cbase[it.pi]) * C::A_STAGE;
         for (int c = kc0; c < kc; ++c, ++seq) {
           const int stg = int(seq % STAGES);
           const uint32_t use = seq / STAGES;
@@ -1273,25 +1205,44 @@ __global__ void __launch_bounds__(THREADS, 1) pair_main(PairArgs p) {
           tc::mbar_arrive_expect_tx(&full_phi[stg], C::A_STAGE);
           tc::bulk_load(smem + stg * C::STAGE, src + size_t(c) * C::A_STAGE, C::A_STAGE,
                         &full_phi[stg]);
-#pragma unroll
-          for (int s = 0; s < STAGES; ++s) issued[s] += s == stg;
-        }
-        if (!ok) {
-          while (!ended) draw();
-          break;
         }
       }
       // copies still in flight complete before the CTA exits
-#pragma unroll
-      for (int s = 0; s < STAGES; ++s)
-        if (issued[s] > 0) tc::mbar_wait(&full_phi[s], (issued[s] - 1) & 1, err, 38, true, lim);
+      for (uint32_t x = seq > STAGES ? seq - STAGES : 0; x < seq; ++x)
+        if (!(p.inject && x == 0))
+          tc::mbar_wait(&full_phi[x % STAGES], (x / STAGES) & 1, err, 38, true, lim);
+    }
+  } else if (lane == 0) {
+    // ---------------- the item drawer ----------------
+    // Items are drawn kAhead ahead of the one whose tiles are loaded: far enough
+    // for the roles to fetch indices over an item's end, near enough that the
+    // last items still go to the CTAs that are free.  After a failed wait it
+    // stops, and so does every role in turn (their waits see the error).
+    const int total = p.total[0];
+    bool ended = false;
+    for (uint32_t n = 0; !ended; ++n) {
+      if (n >= kAhead && !tc::mbar_wait(&started[(n - kAhead) % kRing],
+                                        ((n - kAhead) / kRing) & 1, err, 39, false, lim))
+        break;
+      if (n >= kRing && !tc::mbar_wait(&iempty[n % kRing], ((n / kRing) - 1) & 1, err, 41, false,
+                                       lim))
+        break;
+      const int t = atomicAdd(p.counter, 1);
+      ended = t >= total;
+      RingItem it{};
+      if (!ended) {
+        const int4 v = p.items[t];
+        it = RingItem{v.x, v.y, v.z, v.w, p.ucount[v.x], 1, {0, 0}};
+      }
+      ring[n % kRing] = it;
+      tc::mbar_arrive(&ifull[n % kRing]);  // release: the item is visible to the waiters
     }
   }
 
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (warp == GW) tc::tmem_dealloc(tmem, 512);
+  if (warp == MMA_WARP) tc::tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -1320,8 +1271,8 @@ pair_reduce(PairArgs p, const int* __restrict__ npairs, int pair0) {
     double acc = 0.0;
     for (int t = 0; t < nt; ++t)
 #pragma unroll
-      for (int gq = 0; gq < NG; ++gq)
-        acc += p.partial[(((pbase + t) * p.nset_max + s) * NG + gq) * PT + r];
+      for (int gq = 0; gq < EG; ++gq)
+        acc += p.partial[(((pbase + t) * p.nset_max + s) * EG + gq) * PT + r];
     double* out = B.rhos + size_t(s) * B.stride_grid + g;
     *out = acc + *out;
   }
@@ -1383,7 +1334,7 @@ Layout layout(size_t nao, size_t ngrid, size_t nset, size_t blk, int nsl) {
   L.pmax = L.sigma + a256(ngrid * sizeof(int));
   L.phisl = L.pmax + a256(ngrid * sizeof(unsigned long long));
   L.partial = L.phisl + a256(nbg * max_kc * a_stage);
-  L.bytes = L.partial + nbg * max_t * nset * NG * PT * sizeof(double);
+  L.bytes = L.partial + nbg * max_t * nset * EG * PT * sizeof(double);
   return L;
 }
 
@@ -1406,7 +1357,7 @@ int split_pair_stages() {  // fixed: with the epilogue's phi_lhs values three st
   return kStages;
 }
 
-int split_pair_partial_points() { return NG * PT; }
+int split_pair_partial_points() { return EG * PT; }
 
 cudaError_t split_pair_launch_main(const PairArgs& a, int nsl, cudaStream_t stream,
                                    bool attrs_only, int /*stages*/) {

@@ -67,6 +67,29 @@ def test_split_aodm_ragged_sets_masked_entries(cm, wl, blk, nset):
     assert np.array_equal(rho[:, g0:g1], rho0[:, g0:g1])
 
 
+@pytest.mark.parametrize("sym", [False, True])
+@pytest.mark.parametrize("nao,ngrid,nset,density", [
+    (31, 20011, 40, 0.9),    # many items of one chunk per CTA
+    (64, 15000, 30, 1.0),    # full tiles of rows and columns
+    (301, 9003, 17, 0.4),    # many items of several chunks, ragged ends
+])
+def test_split_aodm_many_items(cm, wl, nao, ngrid, nset, density, sym):
+    """More items than CTAs: the rings of items and of stages wrap many times,
+    the groups' chunks run on over the ends of items."""
+    rng = np.random.default_rng(nao + nset)
+    blk = 64
+    nblk = -(-ngrid // blk)
+    lhs = rng.standard_normal((nao, ngrid))
+    rhs = lhs if sym else rng.standard_normal((nao, ngrid))
+    dms = rng.uniform(-1, 1, (nset, nao, nao))
+    if sym:
+        dms = dms + dms.transpose(0, 2, 1)
+    tab = (rng.random((nao, nblk)) < density).astype(np.uint8)
+    rho = np.zeros((nset, ngrid))
+    split(cm, rho, dms, lhs, rhs, (nao, ngrid), (nao, ngrid), nset, tab, nblk, blk)
+    assert normwise(rho, wl.dense_rho(lhs, rhs, dms, tab, blk)) < TOL
+
+
 def test_split_aodm_wide_range_and_nonfinite(cm, wl):
     rng = np.random.default_rng(5)
     nao, ngrid, blk = 96, 640, 64
