@@ -807,7 +807,7 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
     size_t points = 0;
     for (size_t i = 0; i < nbatch; ++i) points += batches[i].ngrid;
     const int rc =
-        cfgmm::split_pair_form(nao, points)
+        cfgmm::split_pair_form(nao, points, 0)
             ? build_split_pair(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize,
                                flags, d_lists, d_counts, list_off, cnt_off, nblk, counts, s)
             : build_split(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize, flags,
