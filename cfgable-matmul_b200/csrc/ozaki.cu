@@ -11,9 +11,10 @@
 //      reduced to r_l = C_l mods m_l in its epilogue;
 //   4. reconstruction: C' = A'B' is the unique integer with |C'| < M/2 and
 //      C' = r_l (mod m_l): C' = sum_l r_l w_l - q M with the CRT weights w_l and
-//      q = round(sum_l r_l w_l / M).  Evaluated in FP64 with each w_l and M
-//      split at 2^T into a high part (exact products and sums, < 2^53) and a
-//      low part, so C' comes out with one rounding; C = C' 2^-(e_i + f_j).
+//      q = round(sum_l r_l w_l / M).  Evaluated by pairs of moduli: two
+//      residues make one 24-bit integer t_p (one two-way dot product), and
+//      C' = sum_p t_p W_p - q M in FP64 with W_p and M in three parts, the upper
+//      two with exact products and sums (< 2^53); C = C' 2^-(e_i + f_j).
 //
 // The only error is the rounding of A and B to alpha / beta bits relative to
 // their row / column maxima; the number of moduli sets alpha and beta.
@@ -28,6 +29,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <tuple>
 
 #include <cooperative_groups.h>
 
@@ -100,26 +102,44 @@ OzakiPlan ozaki_plan(int k, int nmod, int min_bits) {
   // three-digit form (the headline shape has the larger B)
   p.beta = std::min(P / 2, kOzakiMaxBits);
   p.alpha = std::min(P - P / 2, kOzakiMaxBits);
-  // split point T: sum_l |r_l| hi_l + |q| H < 2^53 with |r_l| <= 128, |q| <= 128 N
-  const int T = std::max(0, logM + 1 + 7 + ceil_log2(nmod + 1) + 1 - 52);
-  p.two_T = std::ldexp(1.0, T);
-  const u128 lo_mask = (T >= 128) ? ~u128(0) : ((u128(1) << T) - 1);
-  const double Md = double(M);
   for (int l = 0; l < nmod; ++l) {
-    const long long m = kModuli[l];
-    const u128 Ml = M / u128(m);
-    const long long inv = mod_inverse(static_cast<long long>(Ml % u128(m)), m);
-    const u128 w = Ml * u128(inv);  // < M
-    p.mod[l] = int(m);
-    p.inv_f[l] = 1.0f / float(m);
-    p.inv_d[l] = 1.0 / double(m);
-    p.w_hi[l] = double(w >> T);
-    p.w_lo[l] = double(w & lo_mask);
+    p.mod[l] = kModuli[l];
+    p.inv_f[l] = 1.0f / float(kModuli[l]);
+    p.inv_d[l] = 1.0 / double(kModuli[l]);
   }
-  p.M_hi = double(M >> T);
-  p.M_lo = double(M & lo_mask);
-  p.t_x = std::ldexp(1.0, T) / Md;
-  p.t_y = 1.0 / Md;
+  // parts of W_p (the largest: the last pair's, or the last modulus alone) and M:
+  // sum_p |t_p| (W_p >> T1) <= 8 2^23 2^26 = 2^52, and the same of the middle parts
+  int wbits = 0;
+  for (int l = 0; l < nmod; l += 2)
+    wbits = std::max(wbits, bit_length(M / u128(kModuli[l] * (l + 1 < nmod ? kModuli[l + 1] : 1))));
+  const int T1 = std::max(0, wbits - 26), T2 = std::max(0, T1 - 26);
+  auto part = [](u128 v, int from, int to) {  // bits [from, to) of v, from `from` on
+    return double((v >> from) & ((u128(1) << (to - from)) - 1));
+  };
+  for (int l = 0; l < nmod; l += 2) {
+    const long long m = kModuli[l], m2 = l + 1 < nmod ? kModuli[l + 1] : 1;
+    const u128 W = M / u128(m * m2);
+    // r (M / m) inv(M / m) + r' (M / m') inv(M / m') = W (m2 inv r + m inv' r') mod M
+    auto coef = [&](long long mm, long long other) -> short {
+      const long long inv = mod_inverse(static_cast<long long>((M / u128(mm)) % u128(mm)), mm);
+      long long v = other * inv % (m * m2);
+      if (2 * v > m * m2) v -= m * m2;  // least magnitude: at most m m2 / 2 < 2^15
+      return short(v);
+    };
+    p.c[l / 2][0] = coef(m, m2);
+    p.c[l / 2][1] = l + 1 < nmod ? coef(m2, m) : short(0);
+    p.w1[l / 2] = double(W >> T1);
+    p.w2[l / 2] = part(W, T2, T1);
+    p.w3[l / 2] = part(W, 0, T2);
+  }
+  p.M1 = double(M >> T1);
+  p.M2 = part(M, T2, T1);
+  p.M3 = part(M, 0, T2);
+  p.two_T1 = std::ldexp(1.0, T1);
+  p.two_T12 = std::ldexp(1.0, T1 - T2);
+  p.two_T21 = std::ldexp(1.0, T2 - T1);
+  p.two_T2 = std::ldexp(1.0, T2);
+  p.t_x = std::ldexp(1.0, T1) / double(M);
   return p;
 }
 
@@ -548,21 +568,29 @@ residues_cols(const T* __restrict__ x, size_t ld, int rows, int k, size_t kpad, 
 // ---------------------------------------------------------------------------
 struct ReconArgs {
   int nmod;
-  double w_hi[kMaxModuli], w_lo[kMaxModuli];
-  double M_hi, M_lo, two_T;
-  double t_x, t_y;  // 2^T / M and 1 / M (the quotient estimate)
+  int vec;                      // 4 consecutive elements of C at 16-byte boundaries
+  int c[kMaxModuli / 2];        // the pair's two coefficients, 16 bits each
+  double w1[kMaxModuli / 2], w2[kMaxModuli / 2], w3[kMaxModuli / 2];
+  double M1, M2, M3, two_T1, two_T2, two_T12, two_T21;
+  double t_x;                   // 2^T1 / M (the quotient estimate)
 };
 
 // A thread rebuilds 4 consecutive C[i][j]: its residue loads (4 bytes per
-// modulus plane) are all issued before the arithmetic.  A residue byte becomes
-// an exact double without a conversion instruction: with its sign bit flipped
-// it is r + 128 in [0, 255], placed in the low word of 2^52 and the 2^52 + 128
-// subtracted again.  X = sum_l r_l w_hi[l] is exact (every partial sum is
-// below 2^53) and Y = sum_l r_l w_lo[l] rounded, so t = X 2^T / M + Y / M, two
-// operations, is within ~1e-12 of sum_l r_l w_l / M (|X 2^T / M| <= 128 N);
-// |C'| <= M/8 keeps that exact value within 1/8 of the integer q, so
-// q = rint(t) is the one of exact arithmetic.
-template <class T>
+// modulus plane) are all issued before the arithmetic.  Two planes' bytes of an
+// element and the pair's two coefficients go through one two-way dot product,
+// whose 2^23 start makes it t + 2^23 in [0, 2^24): placed in the low word of 2^52
+// it is an exact double after one subtraction.  X1 = sum_p t_p w1[p] and X2 are
+// exact (every partial sum at most 2^52), X3 is rounded, at 2^-53 of 2^70 for M
+// near 2^111.  X1 2^T1 / M is within 2^-15 of sum_p t_p W_p / M (2^T1 / M is near
+// 2^-42 and what lies below T1 adds less than 2^27 2^T1), and |C'| <= M/8 keeps
+// that within 1/8 of the integer q, so q = rint of the estimate is the one of
+// exact arithmetic.
+//
+// What it costs is instructions and the latency of the one round trip.  14 moduli,
+// one conversion and two FMAs per residue -> by pairs (32 in place of 42 FP64
+// operations, C in 16-byte pieces where its rows allow): 3527 x 5000 156 -> 94 us
+// (0.53 GB, 81 us at the copy rate), 3527 x 9583 (odd rows of C) 287 -> 212 us.
+template <int NP, class T>
 __global__ void __launch_bounds__(256)
 reconstruct(T* __restrict__ c, size_t ldc, int m, int n, const int8_t* __restrict__ R,
             size_t ldr, const int* __restrict__ ea, const int* __restrict__ eb,
@@ -574,53 +602,108 @@ reconstruct(T* __restrict__ c, size_t ldc, int m, int n, const int8_t* __restric
   const size_t plane = size_t(m) * ldr;
   // ldr is a multiple of 16 and j0 of 4: the 4 bytes at j0 lie inside row i
   const int8_t* Ri = R + size_t(i) * ldr + j0;
-  uint32_t rv[kMaxModuli];
+  uint32_t rv[2 * NP];
 #pragma unroll
-  for (int l = 0; l < kMaxModuli; ++l)
-    if (l < a.nmod) rv[l] = __ldg(reinterpret_cast<const uint32_t*>(Ri + size_t(l) * plane));
-  // C and the column scales are requested with the residues (one round trip)
-  T* ci = c + size_t(i) * ldc;
-  double c_old[4];
-  int fj[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const bool in = j0 + u < n;
-    c_old[u] = in ? double(ci[j0 + u]) : 0.0;
-    fj[u] = in ? __ldg(eb + j0 + u) : 0;
-  }
-  constexpr double kBias = 4503599627370624.0;  // 2^52 + 128
-  double X[4], Y[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) X[u] = Y[u] = 0.0;
-#pragma unroll
-  for (int l = 0; l < kMaxModuli; ++l) {
-    if (l >= a.nmod) break;
-    const uint32_t wb = rv[l] ^ 0x80808080u;  // r + 128 in every byte
+  for (int l = 0; l < 2 * NP; ++l)
+    rv[l] = l < 2 * NP - 1 || l < a.nmod  // the last pair may be one modulus
+                ? __ldg(reinterpret_cast<const uint32_t*>(Ri + size_t(l) * plane))
+                : 0u;
+  // C and the scales are requested with the residues (one round trip)
+  T* ci = c + size_t(i) * ldc + j0;
+  const bool whole = a.vec && j0 + 4 <= n;
+  T c_old[4];
+  int sc[4];
+  if (whole) {
+    if constexpr (sizeof(T) == 8) {
+      *reinterpret_cast<double2*>(c_old) = *reinterpret_cast<const double2*>(ci);
+      *reinterpret_cast<double2*>(c_old + 2) = *reinterpret_cast<const double2*>(ci + 2);
+    } else {
+      *reinterpret_cast<float4*>(c_old) = *reinterpret_cast<const float4*>(ci);
+    }
+    *reinterpret_cast<int4*>(sc) = __ldg(reinterpret_cast<const int4*>(eb + j0));
+  } else {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const double r = __hiloint2double(0x43300000, int(__byte_perm(wb, 0u, 0x4440u + u))) - kBias;
-      X[u] = fma(r, a.w_hi[l], X[u]);  // exact
-      Y[u] = fma(r, a.w_lo[l], Y[u]);
+      c_old[u] = j0 + u < n ? ci[u] : T(0);
+      sc[u] = j0 + u < n ? __ldg(eb + j0 + u) : 0;
     }
   }
-  const int ei = ea[i];
+  const int ei = __ldg(ea + i);
+  bool plain = ei != kNonFinite;  // every scale is a normal power of two
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int j = j0 + u;
-    if (j >= n) break;
-    const double q = rint(fma(X[u], a.t_x, Y[u] * a.t_y));
-    const double hi = fma(-q, a.M_hi, X[u]);  // exact
-    const double lo = fma(-q, a.M_lo, Y[u]);
-    const double cp = fma(hi, a.two_T, lo);   // C' with one rounding
-    const int sc = -(ei + fj[u]);
+    const bool fin = ei != kNonFinite && sc[u] != kNonFinite;
+    sc[u] = fin ? -(ei + sc[u]) : kNonFinite;
+    plain = plain && sc[u] >= -1022 && sc[u] <= 1023;
+  }
+  constexpr double kBias = 4503599635759104.0;    // 2^52 + 2^23
+  constexpr double kRound = 6755399441055744.0;   // 1.5 2^52: adding it rounds to an integer
+  double X1[4], X2[4], X3[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) X1[u] = X2[u] = X3[u] = 0.0;
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const uint32_t ab = __byte_perm(rv[2 * q], rv[2 * q + 1], 0x5140);  // elements 0, 1
+    const uint32_t cd = __byte_perm(rv[2 * q], rv[2 * q + 1], 0x7362);  // elements 2, 3
+    const int t[4] = {
+        __dp2a_lo(a.c[q], int(ab), 1 << 23), __dp2a_hi(a.c[q], int(ab), 1 << 23),
+        __dp2a_lo(a.c[q], int(cd), 1 << 23), __dp2a_hi(a.c[q], int(cd), 1 << 23)};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double td = __hiloint2double(0x43300000, t[u]) - kBias;
+      X1[u] = fma(td, a.w1[q], X1[u]);  // exact
+      X2[u] = fma(td, a.w2[q], X2[u]);  // exact
+      X3[u] = fma(td, a.w3[q], X3[u]);
+    }
+  }
+  T out[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const double q = __dsub_rn(__dadd_rn(X1[u] * a.t_x, kRound), kRound);
+    double h1 = fma(-q, a.M1, X1[u]);  // exact
+    double h2 = fma(-q, a.M2, X2[u]);  // exact
+    const double h3 = fma(-q, a.M3, X3[u]);
+    // the middle part's carry goes to the upper one (exact), so that the lower two
+    // are small and C' has one rounding
+    const double k = __dsub_rn(__fma_rn(h2, a.two_T21, kRound), kRound);
+    h1 += k;
+    h2 = fma(-k, a.two_T12, h2);
+    const double cp = fma(h1, a.two_T1, fma(h2, a.two_T2, h3));
     double val;
-    if (ei == kNonFinite || fj[u] == kNonFinite)
+    if (plain || (sc[u] >= -1022 && sc[u] <= 1023))  // exact scaling by a normal power of two
+      val = cp * __longlong_as_double(static_cast<long long>(sc[u] + 1023) << 52);
+    else if (sc[u] == kNonFinite)
       val = __longlong_as_double(0x7ff8000000000000LL);
-    else if (sc >= -1022 && sc <= 1023)  // exact scaling by a normal power of two
-      val = cp * __longlong_as_double(static_cast<long long>(sc + 1023) << 52);
     else
-      val = ldexp(cp, sc);
-    ci[j] = T(c_old[u] + val);  // f32: rounded once
+      val = ldexp(cp, sc[u]);
+    out[u] = T(double(c_old[u]) + val);  // f32: rounded once
+  }
+  if (whole) {
+    if constexpr (sizeof(T) == 8) {
+      *reinterpret_cast<double2*>(ci) = *reinterpret_cast<const double2*>(out);
+      *reinterpret_cast<double2*>(ci + 2) = *reinterpret_cast<const double2*>(out + 2);
+    } else {
+      *reinterpret_cast<float4*>(ci) = *reinterpret_cast<const float4*>(out);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (j0 + u < n) ci[u] = out[u];
+  }
+}
+
+template <class T, class... Args>
+void launch_reconstruct(unsigned grid, cudaStream_t stream, T* c, Args... args) {
+  const ReconArgs& rc = std::get<sizeof...(Args) - 1>(std::tie(args...));
+  switch ((rc.nmod + 1) / 2) {
+    case 1: reconstruct<1><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 2: reconstruct<2><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 3: reconstruct<3><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 4: reconstruct<4><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 5: reconstruct<5><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 6: reconstruct<6><<<grid, 256, 0, stream>>>(c, args...); break;
+    case 7: reconstruct<7><<<grid, 256, 0, stream>>>(c, args...); break;
+    default: reconstruct<8><<<grid, 256, 0, stream>>>(c, args...); break;
   }
 }
 
@@ -882,19 +965,25 @@ cudaError_t ozaki_dgemm(T* c, const T* a, const T* b, int m, int n, int k,
 
   ReconArgs rc{};
   rc.nmod = plan.nmod;
-  for (int l = 0; l < plan.nmod; ++l) {
-    rc.w_hi[l] = plan.w_hi[l];
-    rc.w_lo[l] = plan.w_lo[l];
+  for (int q = 0; q < (plan.nmod + 1) / 2; ++q) {
+    rc.c[q] = int(uint32_t(uint16_t(plan.c[q][0])) | uint32_t(uint16_t(plan.c[q][1])) << 16);
+    rc.w1[q] = plan.w1[q];
+    rc.w2[q] = plan.w2[q];
+    rc.w3[q] = plan.w3[q];
   }
-  rc.M_hi = plan.M_hi;
-  rc.M_lo = plan.M_lo;
-  rc.two_T = plan.two_T;
+  rc.M1 = plan.M1;
+  rc.M2 = plan.M2;
+  rc.M3 = plan.M3;
+  rc.two_T1 = plan.two_T1;
+  rc.two_T12 = plan.two_T12;
+  rc.two_T21 = plan.two_T21;
+  rc.two_T2 = plan.two_T2;
   rc.t_x = plan.t_x;
-  rc.t_y = plan.t_y;
+  rc.vec = reinterpret_cast<uintptr_t>(c) % 16 == 0 && ldc * sizeof(T) % 16 == 0;
   const long long rgrid = (long long)((n + 1023) / 1024) * m;
   if (rgrid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   if (c_ready && (err = cudaStreamWaitEvent(stream, c_ready, 0)) != cudaSuccess) return err;
-  reconstruct<<<unsigned(rgrid), 256, 0, stream>>>(c, ldc, m, n, r, L.ldr, ea, eb, rc);
+  launch_reconstruct(unsigned(rgrid), stream, c, ldc, m, n, r, L.ldr, ea, eb, rc);
   mark(3);
   return cudaGetLastError();
 }

@@ -22,11 +22,15 @@ struct OzakiPlan {
   int mod[kMaxModuli];  // moduli, 256 first
   float inv_f[kMaxModuli];
   double inv_d[kMaxModuli];
-  // CRT weights w_l (sum_l r_l w_l = C' mod M), split at 2^T:
-  double w_hi[kMaxModuli];    // w_l >> T (exact)
-  double w_lo[kMaxModuli];    // w_l mod 2^T (rounded)
-  double M_hi, M_lo, two_T;   // M >> T, M mod 2^T, 2^T
-  double t_x, t_y;            // 2^T / M, 1 / M: the quotient from the hi / lo sums
+  // CRT by pairs of moduli (the last one alone when N is odd, with m = 1):
+  // C' = sum_p t_p W_p mod M with W_p = M / (m m') and t_p = c[0] r + c[1] r',
+  // |t_p| < 2^23.  W_p and M are split at 2^T1 and 2^T2.
+  short c[kMaxModuli / 2][2];
+  double w1[kMaxModuli / 2];  // W >> T1 (26 bits)
+  double w2[kMaxModuli / 2];  // the 26 bits below
+  double w3[kMaxModuli / 2];  // W mod 2^T2 (rounded)
+  double M1, M2, M3;
+  double two_T1, two_T2, two_T12, two_T21, t_x;  // 2^T1, 2^T2, 2^(T1 - T2), its inverse, 2^T1 / M
 };
 
 // Plan for contraction length k with `nmod` moduli (<= 0: the fewest moduli
