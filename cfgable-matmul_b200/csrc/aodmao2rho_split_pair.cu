@@ -33,9 +33,13 @@
 // candidates paired; tiles without a profitable partner run alone (the other
 // half of the lanes idle).
 //
-// Kernels (one call):
+// Kernels (one call).  The pairing kernels are a chain of latencies on few CTAs
+// beside the phi kernels' reads; kernel times at nao 2228, 16384 points, before ->
+// now: lists and signatures 13 -> 10 us, rank 11 -> 3 (was a sort in one CTA), scores
+// 13 -> 10, matching 25 -> 18, unions 12 -> 5, phi tiles 67 -> 48; the whole call
+// 621 -> 588 us, nao 3000 on 10000 points 367 -> 321.
 //   pair_sig      per block tile: bit set of I(b) and a 64-bit min-hash key
-//   pair_sort     one CTA: tiles in key order (bitonic sort in shared memory)
+//   pair_rank     tiles in key order (each tile counts the keys before its own)
 //   pair_scores   per tile: the profitable neighbours, best first
 //   pair_match    one CTA: mutual-best rounds -> pairs and singles
 //   pair_union    per pair: the union list U and per-AO membership flags
@@ -95,7 +99,8 @@ constexpr int THREADS = 32 * (DRAW_WARP + 1);
 constexpr int kStages = 3;        // pipeline depth
 constexpr int kBadExp = INT_MAX;  // scale of a row / point holding Inf or NaN
 constexpr int kWin = 32;          // pairing candidates on each side in key order
-constexpr int kSortMax = 4096;    // tiles sorted in shared memory (more: caller's order)
+constexpr int kSortMax = 4096;    // tiles sorted (more: caller's order)
+constexpr int kTileCtas = 6;      // CTAs of pair_phi_tiles per SM (4, 5 and 6: 592, 590, 586 us the call)
 constexpr int kRounds = 8;        // mutual-best matching rounds
 constexpr int kMatchCandMax = 600;  // tiles whose candidate lists the matching stages in shared memory
 constexpr int kRing = 4;          // work items in flight between the kernel's roles
@@ -274,45 +279,66 @@ pair_sig(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nbg, int gs
 
 // The block lists (as aodm_block_lists: ascending active AOs of block b,
 // counts[b]) and the signatures of the block's tiles (as pair_sig) from one
-// read of the mask column; CTA per block.
+// read of the mask column; CTA per block.  The column's bytes are a row apart, so
+// what counts is the reads in flight: 2048 of them between two barriers (256 at a
+// time took 13 us at 2228 AOs, this 5).
 __global__ void __launch_bounds__(256)
 pair_lists_sig(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nblk, int gsub,
                int nwords, int* __restrict__ lists, int* __restrict__ counts,
                uint32_t* __restrict__ bits, int* __restrict__ cnt,
                unsigned long long* __restrict__ key) {
+  constexpr int kPer = 8;
   const int b = blockIdx.x;
   if (b >= nblk) return;
-  __shared__ int warp_tot[8];
-  __shared__ int base_s;
+  __shared__ int tot[kPer * 8];  // of 32 AOs each, then the AOs before them
+  __shared__ int sum_s;
   __shared__ uint32_t s1[8], s2[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) base_s = 0;
-  __syncthreads();
   int* out = lists + size_t(b) * nao;
   uint32_t h1 = 0xffffffffu, h2 = 0xffffffffu;
-  for (int u0 = 0; u0 < nao; u0 += 256) {
-    const int u = u0 + tid;
-    const bool on = u < nao && tab[size_t(u) * ldtab + b] != 0;
-    const uint32_t bal = __ballot_sync(0xffffffffu, on);
-    const int wbase = u0 + (tid & ~31);
-    if (lane == 0 && wbase < nao)
-      for (int t = 0; t < gsub; ++t) bits[size_t(b * gsub + t) * nwords + wbase / 32] = bal;
-    if (on) {
-      h1 = min(h1, mix32(uint32_t(u), 0x2545F491u));
-      h2 = min(h2, mix32(uint32_t(u), 0x6C8E9CF5u));
+  int base = 0;
+  for (int v0 = 0; v0 < nao; v0 += 256 * kPer) {
+    bool on[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int u = v0 + 256 * i + tid;
+      on[i] = u < nao && tab[size_t(u) * ldtab + b] != 0;
     }
-    if (lane == 0) warp_tot[warp] = __popc(bal);
-    __syncthreads();
-    int before = base_s;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (on) out[before + __popc(bal & ((1u << lane) - 1u))] = u;
-    __syncthreads();
-    if (tid == 0) {
-      int t = 0;
-      for (int w = 0; w < 8; ++w) t += warp_tot[w];
-      base_s += t;
+    uint32_t bal[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int u = v0 + 256 * i + tid, wbase = u & ~31;
+      bal[i] = __ballot_sync(0xffffffffu, on[i]);
+      if (lane == 0) {
+        tot[8 * i + warp] = __popc(bal[i]);
+        if (wbase < nao)
+          for (int t = 0; t < gsub; ++t) bits[size_t(b * gsub + t) * nwords + wbase / 32] = bal[i];
+      }
+      if (on[i]) {
+        h1 = min(h1, mix32(uint32_t(u), 0x2545F491u));
+        h2 = min(h2, mix32(uint32_t(u), 0x6C8E9CF5u));
+      }
     }
     __syncthreads();
+    if (warp == 0) {  // exclusive sums of the 64 counts, two to a lane
+      const int x = tot[2 * lane], y = tot[2 * lane + 1];
+      int ic = x + y;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, ic, o);
+        if (lane >= o) ic += t;
+      }
+      tot[2 * lane] = ic - x - y;
+      tot[2 * lane + 1] = ic - y;
+      if (lane == 31) sum_s = ic;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      if (on[i])
+        out[base + tot[8 * i + warp] + __popc(bal[i] & ((1u << lane) - 1u))] = v0 + 256 * i + tid;
+    base += sum_s;
+    __syncthreads();  // the counts are read
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -330,89 +356,93 @@ pair_lists_sig(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int nblk,
       a = min(a, s1[w]);
       c = min(c, s2[w]);
     }
-    const int n = base_s;
-    counts[b] = n;
+    counts[b] = base;
     for (int t = 0; t < gsub; ++t) {
-      cnt[b * gsub + t] = n;
-      key[b * gsub + t] = n == 0 ? ~0ull : (static_cast<unsigned long long>(a) << 32) | c;
+      cnt[b * gsub + t] = base;
+      key[b * gsub + t] = base == 0 ? ~0ull : (static_cast<unsigned long long>(a) << 32) | c;
     }
   }
 }
 
-// order[q] = tile at sorted position q (keys ascending, ties by index); above
+// order[q] = tile at sorted position q (keys ascending, ties by index): each
+// tile's position is the number of keys before its own, a warp per tile.  Above
 // kSortMax tiles the caller's order.
-__global__ void __launch_bounds__(1024)
-pair_sort(const unsigned long long* __restrict__ key, int nbg, int* __restrict__ order) {
-  extern __shared__ unsigned long long sk[];  // kSortMax keys, then kSortMax indices
-  int* id = reinterpret_cast<int*>(sk + kSortMax);
-  const int tid = threadIdx.x;
+__global__ void __launch_bounds__(256)
+pair_rank(const unsigned long long* __restrict__ key, int nbg, int* __restrict__ order) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= nbg) return;
   if (nbg > kSortMax) {
-    for (int i = tid; i < nbg; i += 1024) order[i] = i;
+    if (lane == 0) order[t] = t;
     return;
   }
-  int n2 = 1;
-  while (n2 < nbg) n2 <<= 1;
-  for (int i = tid; i < n2; i += 1024) {
-    sk[i] = i < nbg ? key[i] : ~0ull;
-    id[i] = i < nbg ? i : INT_MAX;
+  const unsigned long long k = key[t];
+  int before = 0;
+#pragma unroll 8
+  for (int j = lane; j < nbg; j += 32) {
+    const unsigned long long kj = key[j];
+    before += kj < k || (kj == k && j < t);
   }
-  __syncthreads();
-  for (int size = 2; size <= n2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < n2; i += 1024) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const bool gt = sk[i] > sk[j] || (sk[i] == sk[j] && id[i] > id[j]);
-          if (gt == up) {
-            const unsigned long long tk = sk[i];
-            sk[i] = sk[j];
-            sk[j] = tk;
-            const int ti = id[i];
-            id[i] = id[j];
-            id[j] = ti;
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  for (int i = tid; i < nbg; i += 1024) order[i] = id[i];
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) order[before] = t;
 }
 
 // Per sorted position q: the neighbours within kWin positions whose pairing
 // with tile order[q] saves MMA work (|I_a|^2 + |I_b|^2 > |I_a u I_b|^2), best
-// first: cand[q][0 .. ncand[q]).  CTA per position, thread per candidate.
-__global__ void __launch_bounds__(2 * kWin)
+// first: cand[q][0 .. ncand[q]).  CTA per position; a warp counts the common AOs
+// of eight candidates at a time, lanes over the words of the bit sets.
+__global__ void __launch_bounds__(256)
 pair_scores(const uint32_t* __restrict__ bits, const int* __restrict__ cnt,
             const int* __restrict__ order, int nbg, int nwords, int* __restrict__ cand,
             int* __restrict__ ncand) {
   const int q = blockIdx.x;
   if (q >= nbg) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  constexpr int PER = 2 * kWin / 8;  // candidates of a warp
   __shared__ long long sc[2 * kWin];
-  __shared__ int who[2 * kWin];
+  __shared__ int who[2 * kWin], common[2 * kWin];
   const int a = order[q];
   const int na = cnt[a];
-  const int off = tid < kWin ? tid - kWin : tid - kWin + 1;  // -kWin..-1, 1..kWin
-  const int qb = q + off;
-  long long score = LLONG_MIN;
-  int b = -1;
-  if (na > 0 && qb >= 0 && qb < nbg) {
-    b = order[qb];
-    const int nb = cnt[b];
-    if (nb > 0) {
-      int inter = 0;
-      const uint32_t* x = bits + size_t(a) * nwords;
-      const uint32_t* y = bits + size_t(b) * nwords;
-      for (int w = 0; w < nwords; ++w) inter += __popc(x[w] & y[w]);
-      const long long un = na + nb - inter;
-      score = static_cast<long long>(na) * na + static_cast<long long>(nb) * nb - un * un;
+  // candidate i: position q - kWin + i, q itself left out
+  auto position = [&](int i) { return q + (i < kWin ? i - kWin : i - kWin + 1); };
+  if (na > 0) {
+    const uint32_t* x = bits + size_t(a) * nwords;
+    const uint32_t* y[PER];
+    int inter[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int qb = position((tid >> 5) * PER + i);
+      y[i] = qb >= 0 && qb < nbg ? bits + size_t(order[qb]) * nwords : nullptr;
+      inter[i] = 0;
+    }
+    for (int w = lane; w < nwords; w += 32) {
+      const uint32_t xw = x[w];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) inter[i] += y[i] ? __popc(xw & y[i][w]) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int n = __reduce_add_sync(0xffffffffu, inter[i]);
+      if (lane == 0) common[(tid >> 5) * PER + i] = n;
     }
   }
-  sc[tid] = score;
-  who[tid] = b;
   __syncthreads();
+  long long score = LLONG_MIN;
+  int b = -1;
+  if (tid < 2 * kWin) {
+    const int qb = position(tid);
+    if (na > 0 && qb >= 0 && qb < nbg) {
+      b = order[qb];
+      const int nb = cnt[b];
+      if (nb > 0) {
+        const long long un = na + nb - common[tid];
+        score = static_cast<long long>(na) * na + static_cast<long long>(nb) * nb - un * un;
+      }
+    }
+    sc[tid] = score;
+    who[tid] = b;
+  }
+  __syncthreads();
+  if (tid >= 2 * kWin) return;
   // the profitable candidates (score > 0), best first, ties by tile index: each
   // thread's rank is the number of candidates ordered before its own
   if (score > 0) {
@@ -423,8 +453,8 @@ pair_scores(const uint32_t* __restrict__ bits, const int* __restrict__ cnt,
   }
   const unsigned pos_w = __ballot_sync(0xffffffffu, score > 0);
   __shared__ int npos[2];
-  if ((tid & 31) == 0) npos[tid >> 5] = __popc(pos_w);
-  __syncthreads();
+  if (lane == 0) npos[tid >> 5] = __popc(pos_w);
+  asm volatile("bar.sync 1, %0;" ::"n"(2 * kWin) : "memory");  // the two warps left
   if (tid == 0) ncand[q] = npos[0] + npos[1];
 }
 
@@ -438,19 +468,29 @@ pair_match(const int* __restrict__ order, const int* __restrict__ cand,
            const int* __restrict__ ncand, const int* __restrict__ cnt, int nbg, int batch,
            int* __restrict__ partner_g, int* __restrict__ pos_g, int* __restrict__ choice_g,
            int4* __restrict__ pairs, int* __restrict__ npairs) {
-  // 3 * kSortMax ints when nbg <= kSortMax, then the candidate lists when
-  // nbg <= kMatchCandMax
-  extern __shared__ int match_s[];
+  // 3 * nbg ints when nbg <= kSortMax, then the candidate lists (16-bit tiles)
+  // when nbg <= kMatchCandMax
+  extern __shared__ __align__(16) int match_s[];
   const bool in_smem = nbg <= kSortMax;
   int* partner = in_smem ? match_s : partner_g;
-  int* pos = in_smem ? match_s + kSortMax : pos_g;
-  int* choice = in_smem ? match_s + 2 * kSortMax : choice_g;
+  int* pos = in_smem ? match_s + nbg : pos_g;
+  int* choice = in_smem ? match_s + 2 * nbg : choice_g;
   const int tid = threadIdx.x;
-  const int* cl = cand;  // candidate lists, staged in shared memory when they fit
-  if (nbg <= kMatchCandMax) {
-    int* cs = match_s + 3 * kSortMax;
-    for (int i = tid; i < nbg * 2 * kWin; i += 1024) cs[i] = cand[i];
-    cl = cs;
+  const int lane = tid & 31, warp = tid >> 5;
+  // candidate lists, their lengths and the order, staged in shared memory when they fit
+  const bool staged = nbg <= kMatchCandMax;
+  __shared__ int ord_s[kMatchCandMax], len_s[kMatchCandMax];
+  ushort4* cs4 = reinterpret_cast<ushort4*>(match_s + (3 * nbg + 3) / 4 * 4);
+  const unsigned short* cs = reinterpret_cast<const unsigned short*>(cs4);
+  if (staged) {
+    for (int i = tid; i < nbg * 2 * kWin / 4; i += 1024) {
+      const int4 v = reinterpret_cast<const int4*>(cand)[i];
+      cs4[i] = make_ushort4(v.x, v.y, v.z, v.w);
+    }
+    for (int q = tid; q < nbg; q += 1024) {
+      ord_s[q] = order[q];
+      len_s[q] = ncand[q];
+    }
   }
   __shared__ int changed;
   __shared__ int warp_tot[32];
@@ -462,28 +502,35 @@ pair_match(const int* __restrict__ order, const int* __restrict__ cand,
     partner[t] = cnt[t] > 0 ? -2 : -3;
   }
   __syncthreads();
+  constexpr int kPer = kSortMax / 1024;  // tiles of a thread
+  int from[kPer] = {};
   for (int r = 0; r < kRounds; ++r) {
     if (tid == 0) changed = 0;
-    // every free tile picks its best free candidate
-    for (int q = tid; q < nbg; q += 1024) {
-      const int t = order[q];
-      int pick = -1;
+    // every free tile picks its best free candidate; a candidate once taken stays
+    // taken, so a tile's search goes on where it stopped the round before
+    auto pick = [&](int q, int& from) {
+      const int t = staged ? ord_s[q] : order[q];
+      int c = -1;
       if (partner[t] == -2) {
-        const int n = ncand[q];
-        for (int i = 0; i < n; ++i) {
-          const int c = cl[size_t(q) * 2 * kWin + i];
-          if (partner[c] == -2) {
-            pick = c;
-            break;
-          }
+        const int n = staged ? len_s[q] : ncand[q];
+        for (; from < n && c < 0; ++from) {
+          const int x = staged ? int(cs[q * 2 * kWin + from]) : cand[size_t(q) * 2 * kWin + from];
+          if (partner[x] == -2) c = x;
         }
+        if (c >= 0) --from;
       }
-      choice[t] = pick;
+      choice[t] = c;
+    };
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (tid + 1024 * k < nbg) pick(tid + 1024 * k, from[k]);
+    for (int q = tid + 1024 * kPer; q < nbg; q += 1024) {
+      int at = 0;
+      pick(q, at);
     }
     __syncthreads();
     // mutual choices become pairs (written by the member with the lower index)
-    for (int q = tid; q < nbg; q += 1024) {
-      const int t = order[q];
+    for (int t = tid; t < nbg; t += 1024) {
       const int c = choice[t];
       if (c >= 0 && t < c && choice[c] == t) {
         partner[t] = c;
@@ -496,20 +543,17 @@ pair_match(const int* __restrict__ order, const int* __restrict__ cand,
     __syncthreads();
     if (!ch) break;
   }
-  for (int q = tid; q < nbg; q += 1024) {
-    const int t = order[q];
+  for (int t = tid; t < nbg; t += 1024)
     if (partner[t] == -2) partner[t] = -1;
-  }
   if (tid == 0) base_s = 0;
   __syncthreads();
   // one entry per leader (a single, or the member at the lower position)
-  const int lane = tid & 31, warp = tid >> 5;
   for (int q0 = 0; q0 < nbg; q0 += 1024) {
     const int q = q0 + tid;
     int t = -1, c = -3;
     bool lead = false;
     if (q < nbg) {
-      t = order[q];
+      t = staged ? ord_s[q] : order[q];
       c = partner[t];
       lead = c == -1 || (c >= 0 && pos[c] > q);
     }
@@ -529,46 +573,60 @@ pair_match(const int* __restrict__ order, const int* __restrict__ cand,
 }
 
 // Per pair: U = ascending union of the two tiles' active lists, flags bit 0 /
-// bit 1 = active in the lo / hi tile's block; ucount.
+// bit 1 = active in the lo / hi tile's block; ucount.  From the tiles' bit sets:
+// a thread counts a word, a warp writes a word's AOs.
 __global__ void __launch_bounds__(256)
-pair_union(const uint8_t* __restrict__ tab, size_t ldtab, int nao, int gsub,
+pair_union(const uint32_t* __restrict__ bits, int nwords, int nao,
            const int4* __restrict__ pairs, const int* __restrict__ npairs, int pair0,
            int* __restrict__ ulist, uint8_t* __restrict__ uflag, int* __restrict__ ucount) {
   const int pl = blockIdx.x;
   if (pl >= npairs[0]) return;
   const int pi = pair0 + pl;
   const int4 pr = pairs[pi];
-  const int b0 = pr.x / gsub, b1 = pr.y >= 0 ? pr.y / gsub : -1;
-  __shared__ int warp_tot[8];
-  __shared__ int base_s;
+  const uint32_t* x = bits + size_t(pr.x) * nwords;
+  const uint32_t* y = pr.y >= 0 ? bits + size_t(pr.y) * nwords : nullptr;
+  __shared__ uint32_t sx[256], sy[256];
+  __shared__ int before[256], warp_tot[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) base_s = 0;
-  __syncthreads();
   int* U = ulist + size_t(pi) * nao;
   uint8_t* F = uflag + size_t(pi) * nao;
-  for (int u0 = 0; u0 < nao; u0 += 256) {
-    const int u = u0 + tid;
-    uint32_t f = 0;
-    if (u < nao) {
-      f = tab[size_t(u) * ldtab + b0] != 0 ? 1u : 0u;
-      if (b1 >= 0 && tab[size_t(u) * ldtab + b1] != 0) f |= 2u;
+  int base = 0;
+  for (int w0 = 0; w0 < nwords; w0 += 256) {
+    const uint32_t xw = w0 + tid < nwords ? x[w0 + tid] : 0u;
+    const uint32_t yw = y && w0 + tid < nwords ? y[w0 + tid] : 0u;
+    const int n = __popc(xw | yw);
+    int ic = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, ic, o);
+      if (lane >= o) ic += t;
     }
-    const unsigned bal = __ballot_sync(0xffffffffu, f != 0);
-    if (lane == 0) warp_tot[warp] = __popc(bal);
+    if (lane == 31) warp_tot[warp] = ic;
+    sx[tid] = xw;
+    sy[tid] = yw;
     __syncthreads();
-    int before = base_s;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (f) {
-      const int at = before + __popc(bal & ((1u << lane) - 1u));
-      U[at] = u;
-      F[at] = uint8_t(f);
+    int bw = base, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      bw += w < warp ? warp_tot[w] : 0;
+      all += warp_tot[w];
     }
+    before[tid] = bw + ic - n;
     __syncthreads();
-    if (tid == 0)
-      for (int w = 0; w < 8; ++w) base_s += warp_tot[w];
+    const int wend = min(256, nwords - w0);
+#pragma unroll 4
+    for (int j = warp; j < wend; j += 8) {
+      const uint32_t a = sx[j], c = sy[j];
+      if (((a | c) >> lane) & 1u) {
+        const int at = before[j] + __popc((a | c) & ((1u << lane) - 1u));
+        U[at] = 32 * (w0 + j) + lane;
+        F[at] = uint8_t(((a >> lane) & 1u) | (((c >> lane) & 1u) << 1));
+      }
+    }
+    base += all;
     __syncthreads();
   }
-  if (tid == 0) ucount[pi] = base_s;
+  if (tid == 0) ucount[pi] = base;
 }
 
 // cbase[pi] (first phi chunk of each pair, from chunk0), and the items
@@ -585,15 +643,18 @@ pair_build(const int* __restrict__ ucount, const int* __restrict__ npairs_d, int
   extern __shared__ int hist[];  // max_kc + 2 counters
   __shared__ int warp_c[32];
   __shared__ int base_c;
+  __shared__ int first_s[1024], nu_s[1024];  // of 1024 pairs: first chunk, union size
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int np = npairs_d[0];
   for (int i = tid; i <= max_kc + 1; i += 1024) hist[i] = 0;
   if (tid == 0) base_c = chunk0;
   __syncthreads();
-  // chunk offsets
+  // chunk offsets, and the items per chunk-count class of the pairs
   for (int p0 = 0; p0 < np; p0 += 1024) {
     const int pl = p0 + tid;
-    const int kc = pl < np ? (ucount[pair0 + pl] + TK - 1) / TK : 0;
+    const int nu = pl < np ? ucount[pair0 + pl] : 0;
+    const int kc = (nu + TK - 1) / TK;
+    if (pl < np) atomicAdd(&hist[kc], (nu + tn - 1) / tn * nset);
     int ic = kc;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -604,39 +665,44 @@ pair_build(const int* __restrict__ ucount, const int* __restrict__ npairs_d, int
     __syncthreads();
     int bc = base_c;
     for (int w = 0; w < warp; ++w) bc += warp_c[w];
-    if (pl < np) {
-      cbase[pair0 + pl] = bc + ic - kc;
-      for (int c = 0; c < kc; ++c) cpair[bc + ic - kc - chunk0 + c] = pair0 + pl;
-    }
+    if (pl < np) cbase[pair0 + pl] = bc + ic - kc;
+    first_s[tid] = bc + ic - kc - chunk0;
+    nu_s[tid] = nu;
     __syncthreads();
+    for (int i = warp; i < min(1024, np - p0); i += 32) {  // the chunks' pair, a warp per pair
+      const int c0 = first_s[i], nc = (nu_s[i] + TK - 1) / TK;
+      for (int c = lane; c < nc; c += 32) cpair[c0 + c] = pair0 + p0 + i;
+    }
     if (tid == 0)
       for (int w = 0; w < 32; ++w) base_c += warp_c[w];
     __syncthreads();
   }
-  // items per chunk-count class of the pairs
-  for (int pl = tid; pl < np; pl += 1024) {
-    const int nu = ucount[pair0 + pl];
-    const int kc = (nu + TK - 1) / TK, nt = (nu + tn - 1) / tn;
-    atomicAdd(&hist[kc], nt * nset);
-  }
-  __syncthreads();
-  if (tid == 0) {  // heaviest first: cursor[w] = items of pairs with more chunks than w
+  if (warp == 0) {  // heaviest first: cursor[w] = items of pairs with more chunks than w
     int run = 0;
-    for (int w = max_kc; w >= 0; --w) {
-      const int c = hist[w];
-      hist[w] = run;
-      run += c;
+    for (int w0 = max_kc; w0 >= 0; w0 -= 32) {
+      const int w = w0 - lane;
+      const int c = w >= 0 ? hist[w] : 0;
+      int ic = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, ic, o);
+        if (lane >= o) ic += t;
+      }
+      if (w >= 0) hist[w] = run + ic - c;
+      run += __shfl_sync(0xffffffffu, ic, 31);
     }
-    hist[max_kc + 1] = run;
+    if (lane == 0) hist[max_kc + 1] = run;
   }
   __syncthreads();
   const int start = total[0];
-  for (int pl = tid; pl < np; pl += 1024) {
-    const int nu = ucount[pair0 + pl];
-    const int kc = (nu + TK - 1) / TK, nt = (nu + tn - 1) / tn;
-    int at = start + atomicAdd(&hist[kc], nt * nset);
-    for (int t = 0; t < nt; ++t)
-      for (int s = 0; s < nset; ++s) items[at++] = make_int4(pair0 + pl, t, s, batch);
+  for (int pl = warp; pl < np; pl += 32) {  // a warp per pair
+    const int nu = np <= 1024 ? nu_s[pl] : ucount[pair0 + pl];
+    const int kc = (nu + TK - 1) / TK, n = (nu + tn - 1) / tn * nset;
+    int at = 0;
+    if (lane == 0) at = start + atomicAdd(&hist[kc], n);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int e = lane; e < n; e += 32)
+      items[at + e] = make_int4(pair0 + pl, e / nset, e % nset, batch);
   }
   __syncthreads();
   if (tid == 0) {
@@ -666,10 +732,15 @@ pair_phi_max(const double* __restrict__ ao, size_t stride_grid, const int* __res
   if (g < gend) {
     bool bad = false;
     const int iend = min(nb, i0 + 64);
-    for (int i = i0 + rg; i < iend; i += 4) {
-      const double a = fabs(ao[size_t(__ldg(I + i)) * stride_grid + g]);
-      bad |= !(a <= 1.7976931348623157e308);
-      mx = fmax(mx, a);
+    // 16 reads a thread, all under way at once (the last AO's again past the end)
+    double a[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      a[j] = fabs(ao[size_t(__ldg(I + min(i0 + rg + 4 * j, iend - 1))) * stride_grid + g]);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      bad |= !(a[j] <= 1.7976931348623157e308);
+      mx = fmax(mx, a[j]);
     }
     if (bad) mx = __longlong_as_double(0x7ff0000000000000LL);
   }
@@ -687,7 +758,7 @@ pair_phi_max(const double* __restrict__ ao, size_t stride_grid, const int* __res
 // + c) * A_STAGE; sigma[g] from pmax.  Persistent CTAs take contiguous runs
 // of the batch's chunks [chunk0, chunks_end) through the chunk -> pair map.
 template <int NSL>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kTileCtas)
 pair_phi_tiles(const double* __restrict__ ao, size_t stride_grid,
                const unsigned long long* __restrict__ pmax, const int4* __restrict__ pairs,
                const int* __restrict__ cpair, int chunk0, const int* __restrict__ chunks_end,
@@ -721,17 +792,25 @@ pair_phi_tiles(const double* __restrict__ ao, size_t stride_grid,
       }
       const int e = g >= 0 ? exp_for(__longlong_as_double(static_cast<long long>(pmax[g]))) : 0;
       if (c == 0 && hq == 0 && g >= 0) sigma[g] = e;
+      const bool gon = g >= 0 && e != kBadExp;
+      const int ex = gon ? e : 0;
+      // all 16 elements requested before the arithmetic; zero (whose digits are
+      // zero) where the AO is inactive, past the list or the point is not finite
+      double x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int k = c * TK + 8 * (i & 3) + hq * 4 + (i >> 2);  // K slot 4q + t (see pair_main)
+        const int kk = min(k, nu - 1);
+        const bool on = gon && k < nu && ((__ldg(F + kk) >> h) & 1u);
+        const double* src = ao + size_t(__ldg(U + kk)) * stride_grid + (on ? g : 0);
+        x[i] = on ? *src : 0.0;
+      }
 #pragma unroll
       for (int qq = 0; qq < 4; ++qq) {
         const int q = hq * 4 + qq;
         uint2 w[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int k = c * TK + 8 * t + q;  // K slot 4q + t (see pair_main)
-          const bool on = g >= 0 && k < nu && e != kBadExp && ((__ldg(F + k) >> h) & 1u);
-          w[t] = on ? digits_of<NSL>(ao[size_t(__ldg(U + k)) * stride_grid + g], e)
-                    : make_uint2(0u, 0u);
-        }
+        for (int t = 0; t < 4; ++t) w[t] = digits_of<NSL>(x[4 * qq + t], ex);
         uint32_t o[8];
         transpose4(w[0].x, w[1].x, w[2].x, w[3].x, o[0], o[1], o[2], o[3]);
         transpose4(w[0].y, w[1].y, w[2].y, w[3].y, o[4], o[5], o[6], o[7]);
@@ -1426,27 +1505,26 @@ cudaError_t split_pair_lists_and_signatures(const PairPrep& q, int* lists, int* 
 cudaError_t split_pair_prepare_pairs(const PairPrep& q, cudaStream_t stream, bool signatures) {
   const BatchDims d = batch_dims(q);
   if (d.nbg <= 0) return cudaSuccess;
-  constexpr size_t sort_smem = size_t(kSortMax) * (sizeof(unsigned long long) + sizeof(int));
-  static const cudaError_t sort_attr = cudaFuncSetAttribute(
-      pair_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sort_smem));
-  if (sort_attr != cudaSuccess) return sort_attr;
   if (signatures)
     pair_sig<<<d.nbg, 256, 0, stream>>>(q.tab, q.ldtab, q.nao, d.nbg, d.gsub, d.nwords, q.bits,
                                         q.cnt, q.key);
-  pair_sort<<<1, 1024, sort_smem, stream>>>(q.key, d.nbg, q.order);
-  pair_scores<<<d.nbg, 2 * kWin, 0, stream>>>(q.bits, q.cnt, q.order, d.nbg, d.nwords, q.cand,
+  pair_rank<<<(d.nbg + 7) / 8, 256, 0, stream>>>(q.key, d.nbg, q.order);
+  pair_scores<<<d.nbg, 256, 0, stream>>>(q.bits, q.cnt, q.order, d.nbg, d.nwords, q.cand,
                                               q.ncand);
-  constexpr size_t match_base = size_t(3) * kSortMax * sizeof(int);
-  constexpr size_t match_cands = size_t(kMatchCandMax) * 2 * kWin * sizeof(int);
+  constexpr size_t match_cand = 2 * kWin * sizeof(unsigned short);  // bytes of a tile's list
+  constexpr size_t match_most = std::max(
+      size_t(3) * kSortMax * sizeof(int), kMatchCandMax * (3 * sizeof(int) + match_cand) + 16);
   static const cudaError_t match_attr = cudaFuncSetAttribute(
-      pair_match, cudaFuncAttributeMaxDynamicSharedMemorySize, int(match_base + match_cands));
+      pair_match, cudaFuncAttributeMaxDynamicSharedMemorySize, int(match_most));
   if (match_attr != cudaSuccess) return match_attr;
   const size_t match_smem =
-      match_base + (d.nbg <= kMatchCandMax ? size_t(d.nbg) * 2 * kWin * sizeof(int) : 0);
+      d.nbg > kSortMax ? 0
+                       : size_t(d.nbg) * (3 * sizeof(int) +
+                                          (d.nbg <= kMatchCandMax ? match_cand : 0)) + 16;
   pair_match<<<1, 1024, match_smem, stream>>>(q.order, q.cand, q.ncand, q.cnt, d.nbg, q.batch,
                                               q.partner, q.pos, q.choice, q.pairs + q.pair0,
                                               q.npairs);
-  pair_union<<<d.nbg, 256, 0, stream>>>(q.tab, q.ldtab, q.nao, d.gsub, q.pairs, q.npairs, q.pair0,
+  pair_union<<<d.nbg, 256, 0, stream>>>(q.bits, d.nwords, q.nao, q.pairs, q.npairs, q.pair0,
                                         q.ulist, q.uflag, q.ucount);
   const size_t hist = size_t(d.max_kc + 2) * sizeof(int);
   pair_build<<<1, 1024, hist, stream>>>(q.ucount, q.npairs, q.pair0, q.nset, q.batch, d.tn,
@@ -1473,8 +1551,8 @@ cudaError_t split_pair_prepare_tiles(const PairPrep& q, cudaStream_t stream) {
   cudaError_t err = cudaGetDevice(&dev);
   if (err == cudaSuccess) err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (err != cudaSuccess) return err;
-  // persistent: as many CTAs as fit beside one another (30 KB of shared memory each)
-  const unsigned grid = unsigned(std::min<long long>((long long)nsm * 6,
+  // persistent: as many CTAs as fit beside one another
+  const unsigned grid = unsigned(std::min<long long>((long long)nsm * kTileCtas,
                                                      (long long)d.nbg * d.max_kc));
   if (q.nsl == 6)
     pair_phi_tiles<6><<<grid, 256, 0, stream>>>(q.ao_rhs, q.stride_grid, q.pmax, q.pairs, q.cpair,
