@@ -241,16 +241,23 @@ split_phi_digits(const double* __restrict__ ao, size_t stride_grid, const int* _
   const bool gok = g < gend;
   const int e = gok ? exp_for(__longlong_as_double(static_cast<long long>(pmax[g]))) : 0;
   if (c == 0 && rg == 0 && gok) sigma[g] = e;
+  // all eight elements requested before the arithmetic; zero (whose digits are zero)
+  // past the list and where the point is not finite
+  double v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = c * TK + 8 * (i & 3) + rg + 4 * (i >> 2);  // K slot 4q + t (see split_main)
+    const bool on = gok && k < nb && e != kBadExp;
+    const double* src = ao + size_t(__ldg(I + min(k, nb - 1))) * stride_grid + (on ? g : 0);
+    v[i] = on ? *src : 0.0;
+  }
 #pragma unroll
   for (int hq = 0; hq < 2; ++hq) {
     const int q = rg + 4 * hq;  // quad of 4 compacted AOs
     uint2 w[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const int i = c * TK + q * 4 + t;
-      w[t] = (gok && i < nb && e != kBadExp)
-                 ? digits_packed(ao[size_t(__ldg(I + i)) * stride_grid + g], e)
-                 : make_uint2(0u, 0u);
+      w[t] = digits_packed(v[4 * hq + t], gok && e != kBadExp ? e : 0);
     }
     uint32_t o[8];
     transpose4(w[0].x, w[1].x, w[2].x, w[3].x, o[0], o[1], o[2], o[3]);
@@ -345,20 +352,6 @@ __device__ __forceinline__ const SplitBatch& batch_of(const SplitArgs& p, int w)
   return p.batches ? p.batches[w] : p.one;
 }
 
-// Byte selector that assembles, from `keep` (bytes 0..3) and `recv` (4..7) of
-// the gather's second shuffle round, the digit word of 4 consecutive columns:
-// column qd comes from keep.b0, qd^2 from keep.b2, qd^1 from recv.b0 and qd^3
-// from recv.b2 (the second digit plane of the lane: +1 on every nibble).
-__device__ __forceinline__ uint32_t gather_selector(int qd) {
-  uint32_t sel = 0;
-#pragma unroll
-  for (int col = 0; col < 4; ++col) {
-    const uint32_t src = col == qd ? 0u : col == (qd ^ 2) ? 2u : col == (qd ^ 1) ? 4u : 6u;
-    sel |= src << (4 * col);
-  }
-  return sel;
-}
-
 template <int STAGES>
 __global__ void __launch_bounds__(THREADS, 1) split_main(SplitArgs p) {
   extern __shared__ uint8_t smem_raw[];
@@ -401,14 +394,15 @@ __global__ void __launch_bounds__(THREADS, 1) split_main(SplitArgs p) {
     // ---------------- gather D digits, then the epilogue ----------------
     // Group grp takes the chunks c = grp, grp+NGROUPS, ... of every item; warp wq
     // of the group fills tile rows 32wq .. 32wq+31, four rows per step.
-    // Lane (qd, ri, hh) = lane bits (4:3, 2:1, 0) loads, for row 4*step+ri,
-    // the columns 16hh + 4k + qd (k = 0..3) and ends up holding digit planes
-    // 2qd and 2qd+1 of the 16-byte half hh of that row (plane 7 is the zero
-    // padding byte and is not stored).
+    // Lane (ri, x) = lane bits (4:3, 2:0) takes K slots 4x .. 4x+3 of row 4*step+ri:
+    // slot 4x + k of a chunk is column 8k + x, in the phi tiles too, so that a load
+    // instruction reads 8 columns (64 bytes) of each row and the lane's four digit
+    // strings transpose into one word per plane within the lane (plane 7 is the
+    // zero padding byte and is not stored).  Against a transposition by shuffles
+    // between lanes that hold every fourth column: nao 2071, 4036 points, 2
+    // matrices 297 -> 272 us, nao 319, 15981 points 88 -> 86.
     const int grp = warp >> 2, wq = warp & 3;
-    const int qd = lane >> 3, ri = (lane >> 1) & 3, hh = lane & 1;
-    const bool b1 = (qd & 2) != 0, b0 = (qd & 1) != 0;
-    const uint32_t sel_a = gather_selector(qd), sel_b = sel_a + 0x1111u;
+    const int ri = lane >> 3, x = lane & 7;
     // 16-byte loads of phi_lhs when every row segment starts 16-byte aligned
     uint32_t seq0 = 0;  // CTA-wide sequence number of the item's first chunk
     uint32_t nitem = 0;
@@ -449,55 +443,51 @@ __global__ void __launch_bounds__(THREADS, 1) split_main(SplitArgs p) {
           asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(pe - 8));
       }
+      uint2 w[8][4];
+      int iv[4];
+      auto columns = [&](int c) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int kk = c * TK + 8 * k + x;
+          iv[k] = kk < nb ? __ldg(I + kk) : -1;
+        }
+      };
+      // the digits of step st in chunk c, whose columns iv holds; symmetric D,
+      // diagonal tile: the strict lower triangle (column before row in the compacted
+      // order) is left out
+      auto load_step = [&](int c, int st) {
+        const uint2* row = dset + size_t(iu[st] >= 0 ? iu[st] : 0) * p.nao;
+        const int row_in = 32 * wq + 4 * st + ri;
+        const int lower = sym && c < kc0 + TU / TK ? c * TK - ut * TU : TU;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          w[st][k] = iu[st] >= 0 && iv[k] >= 0 && lower + 8 * k + x >= row_in
+                         ? __ldg(row + iv[k])
+                         : make_uint2(0u, 0u);
+      };
+      if (kc0 + grp < kc) columns(kc0 + grp);
       for (int c = kc0 + grp; c < kc; c += NGROUPS) {
         const uint32_t seq = seq0 + uint32_t(c - kc0);
         const int stg = int(seq % STAGES);
         const uint32_t use = seq / STAGES;
-        // the loads go out first; the stage has to be free only for the stores
-        int iv[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int kk = c * TK + 16 * hh + 4 * k + qd;
-          iv[k] = kk < nb ? __ldg(I + kk) : -1;
-        }
-        // symmetric D, diagonal tile: the strict lower triangle (column before
-        // row in the compacted order) is left out; elsewhere nothing is
-        const int lower_lim = sym && c < kc0 + TU / TK ? c * TK - ut * TU : TU;
-        uint2 w[8][4];
-#pragma unroll
-        for (int st = 0; st < 8; ++st)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            w[st][k] = (iu[st] >= 0 && iv[k] >= 0 &&
-                        lower_lim + 16 * hh + 4 * k + qd >= 32 * wq + 4 * st + ri)
-                           ? __ldg(dset + size_t(iu[st]) * p.nao + iv[k])
-                           : make_uint2(0u, 0u);
+        for (int st = 0; st < 8; ++st) load_step(c, st);
+        columns(c + NGROUPS);
         if (use > 0 && !tc::mbar_wait(&empty[stg], (use - 1) & 1, err, 11)) {
           ok = false;
           break;
         }
         uint8_t* As = smem + stg * STAGE;
+        // each step's digits into the stage, the next chunk's requested in their place
 #pragma unroll
         for (int st = 0; st < 8; ++st) {
-          uint32_t wa[4], wb[4];
+          uint32_t o[8];
+          transpose4(w[st][0].x, w[st][1].x, w[st][2].x, w[st][3].x, o[0], o[1], o[2], o[3]);
+          transpose4(w[st][0].y, w[st][1].y, w[st][2].y, w[st][3].y, o[4], o[5], o[6], o[7]);
+          uint8_t* dst =
+              As + 4 * (x & 3) + tc::sw32_offset(uint32_t(32 * wq + 4 * st + ri), uint32_t(x >> 2));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            // round 1 (lanes qd, qd^2): keep digits 0-3 (b1 = 0) or 4-7 (b1 = 1)
-            const uint32_t x = b1 ? w[st][k].y : w[st][k].x;
-            const uint32_t y = __shfl_xor_sync(0xffffffffu, b1 ? w[st][k].x : w[st][k].y, 16);
-            // round 2 (lanes qd, qd^1): keep two of those four digits
-            const uint32_t lo = __byte_perm(x, y, 0x5410), hi = __byte_perm(x, y, 0x7632);
-            const uint32_t keep = b0 ? hi : lo;
-            const uint32_t recv = __shfl_xor_sync(0xffffffffu, b0 ? lo : hi, 8);
-            wa[k] = __byte_perm(keep, recv, sel_a);
-            wb[k] = __byte_perm(keep, recv, sel_b);
-          }
-          const uint32_t off = tc::sw32_offset(uint32_t(32 * wq + 4 * st + ri), uint32_t(hh));
-          *reinterpret_cast<uint4*>(As + (2 * qd) * A_SLICE + off) =
-              make_uint4(wa[0], wa[1], wa[2], wa[3]);
-          if (qd < 3)
-            *reinterpret_cast<uint4*>(As + (2 * qd + 1) * A_SLICE + off) =
-                make_uint4(wb[0], wb[1], wb[2], wb[3]);
+          for (int j = 0; j < NSL; ++j) *reinterpret_cast<uint32_t*>(dst + j * A_SLICE) = o[j];
         }
         tc::fence_proxy_async_smem();
         __syncwarp();
