@@ -733,9 +733,9 @@ def run_ours(args, ranks: Ranks):
                      "executed_tflops": xflops / (atot / args.steps * 1e-3) / 1e12,
                      "frac_of_dmma_peak": (xflops / (atot / args.steps * 1e-3) / 1e12) / dmma_sust,
                      "frac_of_dmma_burst": (xflops / (atot / args.steps * 1e-3) / 1e12) / dmma_peak,
-                     "kernel": "aodm_fp64_pipe_kernel (producer warps: cp.async D gather + TMA "
-                               "gather4 of phi rows; consumer warps: DMMA m16n8k8)",
-                     "launches_per_step": 5 if sym else 4},
+                     "kernel": "aodm_fp64_pipe_kernel (producer warps: cp.async D gather + bulk "
+                               "copies of phi rows; consumer warps: DMMA m16n8k8)",
+                     "launches_per_step": 4},
             "split": {"value": ranks.world * aflops * args.steps / (stot * 1e-3) / 1e9,
                       "unit": "GFLOP/s", "ms_per_step": stot / args.steps,
                       "error_vs_fp64": aodm_err, "form": split_form, "digits": split_digits,
@@ -743,7 +743,7 @@ def run_ours(args, ranks: Ranks):
                                 f"{split_digits * (split_digits + 1) // 2} INT8 products per "
                                 "chunk" + ("; two alike grid blocks per work item"
                                            if split_form == "pair" else ""),
-                      "launches_per_step": 14 if split_form == "pair" else 8},
+                      "launches_per_step": 11 if split_form == "pair" else 8},
             "speedup_split_vs_fp64": atot / stot}
     # the drop-in host-pointer call (cfgmm_aodmao2rho_ex, aodmao2rho_loop_parallel's
     # form) end to end on pinned host buffers: phi, D and the mask up, rho up and back
@@ -856,7 +856,7 @@ def run_ours(args, ranks: Ranks):
                               "traffic_source": "ncu capture summarised in "
                                                 "profiles/dgemm_fp64_3527x9583x6581.md, not "
                                                 "measured in this run",
-                              "kernel": "dgemm_tma_kernel (+ packing, tail reduce)",
+                              "kernel": "dgemm_kernel (+ copies of unaligned operands)",
                               "peak_source": "measured in this run: DMMA m16n8k4 register loop on "
                                              "every SM, sustained (1.5 s of back-to-back "
                                              "launches, second half) for a kernel timed over "
@@ -869,9 +869,9 @@ def run_ours(args, ranks: Ranks):
                 "d2h_bytes_per_step": 8 * M * N,
                 "path": "cfgmm_matmul_ex(CFGMM_PREC_OZAKI_INT8) on pinned host buffers "
                         "(synchronous)"},
-        # per split step: emax, exponents and residues of A (3) and of B (4, with
-        # the fill of the column maxima), the INT8 GEMM, the reconstruction
-        "gpu_launches": 9 * args.steps,
+        # per split step: maxima and residues of A (2) and of B (2), the INT8 GEMM, the
+        # reconstruction
+        "gpu_launches": 6 * args.steps,
         "clocks": clk,
         "aodmao2rho": aodm,
     }
