@@ -259,11 +259,24 @@ constexpr double kRoundBias = 6755399441055744.0 + double(kDigitBias);
 // (|s| 2^-24 / m, the error of s * fl(1/m), stays below 1/(2m)).
 constexpr long long kDigitBias16 = 32768LL * (1 + (1LL << 16) + (1LL << 32));
 constexpr double kRoundBias16 = 6755399441055744.0 + double(kDigitBias16);
+// The same with two digits, for |v| <= 2^30 (f32 data): w = v + 2^15 (1 + 2^16) in
+// [0, 2^32) is the double's low word; s = b_0 + b_1 c_16, one FMA per modulus (f32,
+// 2000 x 2000 x 3000: 173 -> 164 us the call).
+constexpr double kRoundBias2x16 = 6755399441055744.0 + 32768.0 * 65537.0;
 
 // Digit forms of write_residues8: plain (integers up to 2^52, four 14-bit
-// digits), biased (up to 2^50, four 14-bit digits read off the double's bits)
-// and biased16 (up to 2^47, three 16-bit digits).
-enum : int { kPlain = 0, kBiased14 = 1, kBiased16 = 2 };
+// digits), biased (up to 2^50, four 14-bit digits read off the double's bits),
+// biased16 (up to 2^47, three 16-bit digits) and biased2x16 (up to 2^30, two).
+enum : int { kPlain = 0, kBiased14 = 1, kBiased16 = 2, kBiased2x16 = 3 };
+
+// The round bias of a form (0: the plain form's).
+template <int kForm>
+__device__ __forceinline__ constexpr double round_bias() {
+  return kForm == kBiased2x16 ? kRoundBias2x16
+         : kForm == kBiased16 ? kRoundBias16
+         : kForm == kBiased14 ? kRoundBias
+                              : 0.0;
+}
 
 // The operand element x(r, p) 2^e as the input of write_residues8: rint(x 2^e)
 // (the plain form), or that integer plus the form's round bias, rounded once by
@@ -271,7 +284,7 @@ enum : int { kPlain = 0, kBiased14 = 1, kBiased16 = 2 };
 template <int kForm>
 __device__ __forceinline__ double scaled(double x, int e) {
   if constexpr (kForm != kPlain) {
-    constexpr double bias = kForm == kBiased16 ? kRoundBias16 : kRoundBias;
+    constexpr double bias = round_bias<kForm>();
     if (e == kNonFinite) return bias;
     if (e >= -1022 && e <= 1023)
       return fma(x, __longlong_as_double(static_cast<long long>(e + 1023) << 52), bias);
@@ -282,12 +295,12 @@ __device__ __forceinline__ double scaled(double x, int e) {
 }
 template <int kForm>
 __device__ __forceinline__ double scaled_zero() {
-  return kForm == kBiased16 ? kRoundBias16 : (kForm == kBiased14 ? kRoundBias : 0.0);
+  return round_bias<kForm>();
 }
 
 // The residues of 8 consecutive elements for every modulus, 8 bytes per modulus
 // plane at Y + l * plane + off (8-byte aligned).  v[] holds integers |v| <= 2^52
-// (plain form) or |v| <= 2^50 (2^47) plus the form's round bias (biased forms:
+// (plain form) or |v| <= 2^50 (2^47, 2^30) plus the form's round bias (biased forms:
 // the digits are bit fields of the double, with no conversion to a 64-bit
 // integer).  The low byte of w is v's (both digit biases are multiples of 256).
 template <int kForm>
@@ -301,7 +314,14 @@ __device__ __forceinline__ void write_residues8(const ResidueArgs& a, int8_t* Y,
     float u[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      if constexpr (kForm == kBiased16) {
+      if constexpr (kForm == kBiased2x16) {
+        // mantissa field = w + 2^51: the low word is w
+        const uint32_t lo = __double2loint(v[j + h]);
+        lowb[(j + h) >> 2] |= (lo & 0xffu) << (8 * ((j + h) & 3));  // modulus 256
+        u[h][0] = float(int(lo & 0xffffu) - 32768);
+        u[h][1] = float(int(lo >> 16) - 32768);
+        u[h][2] = u[h][3] = 0.0f;
+      } else if constexpr (kForm == kBiased16) {
         // mantissa field = w + 2^51: bits 0..31 are w's, bits 32..51 are (w >> 32) + 2^19
         const uint32_t lo = __double2loint(v[j + h]), hi = __double2hiint(v[j + h]);
         lowb[(j + h) >> 2] |= (lo & 0xffu) << (8 * ((j + h) & 3));  // modulus 256
@@ -343,7 +363,9 @@ __device__ __forceinline__ void write_residues8(const ResidueArgs& a, int8_t* Y,
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       f32x2 S;
-      if constexpr (kForm == kBiased16) {
+      if constexpr (kForm == kBiased2x16) {
+        S = fma2(P1[q], a.c16[l], P0[q]);             // s, exact
+      } else if constexpr (kForm == kBiased16) {
         S = fma2(P1[q], a.c16[l], P0[q]);
         S = fma2(P2[q], a.c32[l], S);                 // s, exact
       } else {
@@ -844,8 +866,11 @@ template <class T>
 cudaError_t prepare(const T* x, size_t ld, bool rows_contig, int rows, int k, size_t kpad,
                     int bits, void* top, int* e, int8_t* Y, const ResidueArgs& ra, cudaStream_t s,
                     Mask mask = Mask{nullptr, 0, 1}) {
-  // scaled elements up to 2^47 take three 16-bit digits, up to 2^50 the
-  // biased form of four 14-bit digits, the rest the plain form
+  // scaled elements up to 2^30 take two 16-bit digits, up to 2^47 three, up to
+  // 2^50 the biased form of four 14-bit digits, the rest the plain form
+  if (bits <= 30)
+    return prepare_form<kBiased2x16>(x, ld, rows_contig, rows, k, kpad, bits, top, e, Y, ra, s,
+                                     mask);
   if (bits <= 47)
     return prepare_form<kBiased16>(x, ld, rows_contig, rows, k, kpad, bits, top, e, Y, ra, s, mask);
   if (bits <= 50)
