@@ -9,7 +9,7 @@
 // mma.sync m16n8k8 f64), fed from shared memory.  CTA = 64 x 64 of C, four warps
 // of 32 x 32, K steps of 16 in a ring of three (cp.async), four CTAs per SM.
 //   * Why small tiles, four to an SM: each CTA's barriers and copy latency are
-//     hidden by the other three.  3000 x 3000 x 3000: 1.67 ms (32.3 TFLOP/s, 87 %
+//     hidden by the other three.  3000 x 3000 x 3000: 1.65 ms (32.8 TFLOP/s, 89 %
 //     of the measured DMMA peak); one 128 x 128 CTA of eight warps per SM, staged
 //     by TMA from operands packed K-contiguous, took 1.86 ms with its packing.
 //   * Copies of 16 bytes where an operand's rows are 16-byte aligned, of 8 bytes
@@ -273,15 +273,34 @@ dgemm_kernel(const __grid_constant__ GemmArgs<T> p) {
         for (int e = 0; e < 2; ++e)
           gemm_smem[row_of(mt, h) * CP + col_of(j, e)] = acc[mt][j][2 * h + e];
   cluster.sync();
-  const int rows = TILE / p.splits;  // of each CTA
-  for (int i = tid; i < rows * TILE; i += THREADS) {
-    const int r = part * rows + i / TILE, cc = i % TILE;
-    if (m0 + r >= p.m || n0 + cc >= p.n) continue;
-    double v = 0.0;
-    for (int s = 0; s < p.splits; ++s)
-      v += *cluster.map_shared_rank(gemm_smem + r * CP + cc, s);
-    T* dst = p.c + size_t(m0 + r) * p.ldc + n0 + cc;
-    *dst = T(double(*dst) + v);
+  // each CTA adds its rows over the parts, in their order; a thread's reads of the
+  // other CTAs' memory are all under way at once (in a loop over the parts, one after another, whose
+  // registers also spilled in the main loop: 1000^3 91 -> 87 us, 3000 x 3000 x 300 196
+  // -> 185, 3000^3 1.669 -> 1.648 ms; calls of a few tiles are bound by their launch)
+  const int rows = TILE / p.splits;
+  double v[2][8];
+#pragma unroll 1
+  for (int i0 = 0; i0 < rows * TILE / THREADS; i0 += 2) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = (i0 + u) * THREADS + tid;
+      const int r = part * rows + i / TILE, cc = i % TILE;
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        v[u][s] = s < p.splits ? *cluster.map_shared_rank(gemm_smem + r * CP + cc, s) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = (i0 + u) * THREADS + tid;
+      const int r = part * rows + i / TILE, cc = i % TILE;
+      double sum = 0.0;
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < p.splits) sum += v[u][s];
+      if (m0 + r >= p.m || n0 + cc >= p.n) continue;
+      T* dst = p.c + size_t(m0 + r) * p.ldc + n0 + cc;
+      *dst = T(double(*dst) + sum);
+    }
   }
   cluster.sync();  // a CTA's partial tile is read until here
 }
