@@ -806,12 +806,25 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   if (precision == CFGMM_PREC_OZAKI_INT8) {
     size_t points = 0;
     for (size_t i = 0; i < nbatch; ++i) points += batches[i].ngrid;
-    const int rc =
-        cfgmm::split_pair_form(nao, points, 0)
-            ? build_split_pair(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize,
-                               flags, d_lists, d_counts, list_off, cnt_off, nblk, counts, s)
-            : build_split(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize, flags,
-                          d_lists, d_counts, list_off, cnt_off, nblk, counts, s);
+    bool pair = cfgmm::split_pair_form(nao, points, nset_max);
+    int rc = CFGMM_OK;
+    if (pair) {
+      rc = build_split_pair(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize, flags,
+                            d_lists, d_counts, list_off, cnt_off, nblk, counts, s);
+      if (rc == CFGMM_ERR_OUT_OF_MEMORY) {
+        // the row form's phi tiles take up to half of the memory
+        cudaGetLastError();
+        if (plan->mem2) cudaFree(plan->mem2);
+        if (plan->mem3) cudaFree(plan->mem3);
+        plan->mem2 = plan->mem3 = nullptr;
+        plan->split = plan->pair = false;
+        cfgmm::set_last_error("");
+        pair = false;
+      }
+    }
+    if (!pair)
+      rc = build_split(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize, flags,
+                       d_lists, d_counts, list_off, cnt_off, nblk, counts, s);
     if (rc != CFGMM_OK) return cleanup(rc);
     *out = plan;
     return CFGMM_OK;

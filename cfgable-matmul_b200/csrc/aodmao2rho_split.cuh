@@ -183,16 +183,19 @@ cudaError_t split_pair_launch_main(const PairArgs& a, int nsl, cudaStream_t stre
                                    bool attrs_only = false, int stages = 0);
 cudaError_t split_pair_launch_reduce(const PairArgs& a, int nsl, const int* npairs, int pair0,
                                      int max_pairs, cudaStream_t stream);
-// Whether a single call (points = ngrid, nset matrices) or a plan (points = all
-// batches' points, nset 0) runs the pair form: CFGMM_SPLIT_FORM=pair / =row, else
-// the pair form from kPairMinAos AOs and kPairMinPoints points on, and for a single
-// call from nao^2 points nset = kPairMinWork on (below that the pairing and tile
+// Whether a call of nset matrices on ngrid points, or a plan of up to nset matrices
+// on so many points in all, runs the pair form: CFGMM_SPLIT_FORM=pair / =row, else
+// the pair form from kPairMinAos AOs and kPairMinPoints points on, and from nao^2
+// points nset = kPairMinWork on (below that the pairing and tile
 // building, 35 us and more, cost more than the pairs save; the share of active AOs
 // is known on the device only).  Row / pair form, us: nao 6000, 1000 points, 1
 // matrix (3.6e10) 461 / 321; 3000, 2000, 2 273 / 226; 200, 250000, 4 1347 / 1305;
 // 2522, 2800, 4 661 / 438; 2782, 2293, 1 (1.8e10) 176 / 187; 891, 3998, 4 (1.3e10)
-// 197 / 210.  A plan keeps the narrower rule: the pair form's preparation takes
-// longer and its phi tiles up to twice the memory.
+// 197 / 210.  A plan of one batch runs the single call's form (the same bits); its
+// runs gain at every size measured (508 AOs, 84 batches, 2 matrices 269 / 154, 312
+// AOs, 25 batches 67 / 49), but its creation takes longer and its phi tiles up to
+// twice the memory, so the line is the same (a plan that does not fit takes the row
+// form).
 constexpr size_t kPairMinAos = 1024, kPairMinPoints = 8192;
 constexpr double kPairMinWork = 3.5e10;
 bool split_pair_form(size_t nao, size_t points, size_t nset);
