@@ -81,6 +81,15 @@ int cuda_fail(cudaError_t err, const char* where) {
 
 size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 
+// Gives the plan's memory back behind the work enqueued on `s` so far.  (cudaFree would
+// not wait for it: the memory comes from cudaMallocAsync.)
+void free_on(cfgmm_aodm_plan* plan, cudaStream_t s) {
+  for (void** m : {&plan->mem, &plan->mem2, &plan->mem3}) {
+    if (*m) cudaFreeAsync(*m, s);
+    *m = nullptr;
+  }
+}
+
 // ---- autotune cache: one "key ns tk ms" line per entry -------------------
 std::mutex g_cache_mu;
 
@@ -748,9 +757,7 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
   cfgmm_aodm_plan* plan = new cfgmm_aodm_plan;
   plan->dev = dev;
   auto cleanup = [&](int rc) {
-    if (plan->mem) cudaFree(plan->mem);
-    if (plan->mem2) cudaFree(plan->mem2);
-    if (plan->mem3) cudaFree(plan->mem3);
+    free_on(plan, s);  // behind the work that is enqueued there
     delete plan;
     return rc;
   };
@@ -814,10 +821,12 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
       if (rc == CFGMM_ERR_OUT_OF_MEMORY) {
         // the row form's phi tiles take up to half of the memory
         cudaGetLastError();
-        if (plan->mem2) cudaFree(plan->mem2);
-        if (plan->mem3) cudaFree(plan->mem3);
-        plan->mem2 = plan->mem3 = nullptr;
+        void* lists = plan->mem;
+        plan->mem = nullptr;
+        free_on(plan, s);  // the pairing kernels may still run there
+        plan->mem = lists;
         plan->split = plan->pair = false;
+        plan->stages = 0;
         cfgmm::set_last_error("");
         pair = false;
       }
@@ -1025,11 +1034,21 @@ const char* cfgmm_aodm_plan_info(const cfgmm_aodm_plan* plan) {
 
 int cfgmm_aodm_plan_destroy(cfgmm_aodm_plan* plan) {
   if (!plan) return CFGMM_OK;
+  // Runs may be in flight on any stream, and cudaFree does not wait for work on memory
+  // that comes from cudaMallocAsync.
+  int dev = plan->dev;
+  cudaGetDevice(&dev);
+  if (dev != plan->dev) cudaSetDevice(plan->dev);
+  const cudaError_t err = cudaDeviceSynchronize();
+  if (err == cudaErrorStreamCaptureUnsupported) {  // no wait is possible: the plan stays
+    cudaGetLastError();
+    if (dev != plan->dev) cudaSetDevice(dev);
+    return cuda_fail(err, "plan_destroy during a stream capture");
+  }
   if (plan->exec) cudaGraphExecDestroy(plan->exec);
-  // cudaFree waits for work still using the memory
-  if (plan->mem) cudaFree(plan->mem);
-  if (plan->mem2) cudaFree(plan->mem2);
-  if (plan->mem3) cudaFree(plan->mem3);
+  for (void* m : {plan->mem, plan->mem2, plan->mem3})
+    if (m) cudaFree(m);
+  if (dev != plan->dev) cudaSetDevice(dev);
   delete plan;
   return CFGMM_OK;
 }
@@ -1043,9 +1062,7 @@ namespace cfgmm {
 int aodm_plan_release_idle(cfgmm_aodm_plan* plan, cudaStream_t stream) {
   if (!plan) return CFGMM_OK;
   if (plan->exec) cudaGraphExecDestroy(plan->exec);
-  if (plan->mem) cudaFreeAsync(plan->mem, stream);
-  if (plan->mem2) cudaFreeAsync(plan->mem2, stream);
-  if (plan->mem3) cudaFreeAsync(plan->mem3, stream);
+  free_on(plan, stream);
   delete plan;
   return CFGMM_OK;
 }

@@ -1,0 +1,38 @@
+"""The library's host side on the CPU: all of its objects linked with a stand-in for the
+CUDA runtime (host_side/fake_cuda.cpp: two devices, kernels that do nothing, and a record
+of what the library asks for), one driver program per property."""
+import importlib
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SIDE = os.path.join(HERE, "host_side")
+
+
+@pytest.fixture(scope="module")
+def objects(tmp_path_factory):
+    b = importlib.import_module("cfgable-matmul_b200.build")
+    b.build()
+    tmp = tmp_path_factory.mktemp("host_side")
+    inc = os.path.join(os.path.dirname(os.path.dirname(b.nvcc())), "include")
+    fake = str(tmp / "fake_cuda.o")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", inc, "-c", os.path.join(SIDE, "fake_cuda.cpp"),
+                    "-o", fake], check=True)
+    objs = [os.path.join(b.BUILD, f[:-3] + ".o") for f in sorted(os.listdir(b.CSRC))
+            if f.endswith(".cu")]
+    return tmp, inc, [fake] + objs
+
+
+def drive(objects, name, timeout=120):
+    tmp, inc, objs = objects
+    exe = str(tmp / name)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", inc, os.path.join(SIDE, name + ".cpp"),
+                    "-o", exe] + objs + ["-lpthread"], check=True)
+    r = subprocess.run([exe], timeout=timeout, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_plan_memory_is_not_freed_under_running_work(objects):
+    drive(objects, "plan_memory")
