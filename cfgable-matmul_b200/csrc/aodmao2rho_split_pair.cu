@@ -1514,9 +1514,10 @@ cudaError_t split_pair_prepare_pairs(const PairPrep& q, cudaStream_t stream, boo
   constexpr size_t match_cand = 2 * kWin * sizeof(unsigned short);  // bytes of a tile's list
   constexpr size_t match_most = std::max(
       size_t(3) * kSortMax * sizeof(int), kMatchCandMax * (3 * sizeof(int) + match_cand) + 16);
-  static const cudaError_t match_attr = cudaFuncSetAttribute(
-      pair_match, cudaFuncAttributeMaxDynamicSharedMemorySize, int(match_most));
-  if (match_attr != cudaSuccess) return match_attr;
+  // on every call: the attribute belongs to the device that is current
+  cudaError_t err = cudaFuncSetAttribute(pair_match, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(match_most));
+  if (err != cudaSuccess) return err;
   const size_t match_smem =
       d.nbg > kSortMax ? 0
                        : size_t(d.nbg) * (3 * sizeof(int) +

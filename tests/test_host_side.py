@@ -36,3 +36,7 @@ def drive(objects, name, timeout=120):
 
 def test_plan_memory_is_not_freed_under_running_work(objects):
     drive(objects, "plan_memory")
+
+
+def test_each_device_grants_the_matching_its_shared_memory(objects):
+    drive(objects, "pair_device")
