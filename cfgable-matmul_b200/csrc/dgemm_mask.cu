@@ -339,7 +339,7 @@ MaskPlan mask_plan(const double* a, const double* b, int m, int n, int k, size_t
   MaskPlan P{};
   P.a_inplace = transa && al16(a, lda) && m % 2 == 0;
   P.b_inplace = al16(b, ldb) && blk % 2 == 0 && n % 2 == 0;
-  P.nblk = (n + blk - 1) / blk;
+  P.nblk = int(((long long)n + blk - 1) / blk);
   const int width = std::min(blk, n);  // a block wider than C has only n columns
   P.nsub = pieces(width);
   P.sw = ((width + P.nsub - 1) / P.nsub + 1) / 2 * 2;

@@ -40,3 +40,7 @@ def test_plan_memory_is_not_freed_under_running_work(objects):
 
 def test_each_device_grants_the_matching_its_shared_memory(objects):
     drive(objects, "pair_device")
+
+
+def test_masked_gemm_takes_the_widest_block(objects):
+    drive(objects, "wide_block")
