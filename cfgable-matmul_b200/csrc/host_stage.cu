@@ -5,7 +5,6 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
-#include <functional>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -27,11 +26,14 @@ class Workers {
   }
   int count() const { return 1 + int(threads_); }
   // fn(worker) on every thread, worker 0 being the caller; returns when all are done.
-  void run(const std::function<void(int)>& fn) {
+  // (By address, without a std::function: nothing is allocated that could fail.)
+  template <class F>
+  void run(F& fn) {
     std::lock_guard<std::mutex> one(job_mu_);
     {
       std::lock_guard<std::mutex> lk(mu_);
-      fn_ = &fn;
+      call_ = [](void* f, int worker) { (*static_cast<F*>(f))(worker); };
+      arg_ = &fn;
       running_ = int(threads_);
       ++round_;
     }
@@ -39,7 +41,6 @@ class Workers {
     fn(0);
     std::unique_lock<std::mutex> lk(mu_);
     done_.wait(lk, [&] { return running_ == 0; });
-    fn_ = nullptr;
   }
 
  private:
@@ -58,21 +59,24 @@ class Workers {
   void loop(int worker) {
     unsigned long long seen = 0;
     for (;;) {
-      const std::function<void(int)>* fn;
+      void (*call)(void*, int);
+      void* arg;
       {
         std::unique_lock<std::mutex> lk(mu_);
         start_.wait(lk, [&] { return round_ != seen; });
         seen = round_;
-        fn = fn_;
+        call = call_;
+        arg = arg_;
       }
-      (*fn)(worker);
+      call(arg, worker);
       std::lock_guard<std::mutex> lk(mu_);
       if (--running_ == 0) done_.notify_one();
     }
   }
   std::mutex job_mu_, mu_;
   std::condition_variable start_, done_;
-  const std::function<void(int)>* fn_ = nullptr;
+  void (*call_)(void*, int) = nullptr;
+  void* arg_ = nullptr;
   int running_ = 0;
   unsigned long long round_ = 0;
   size_t threads_ = 0;
@@ -157,15 +161,15 @@ namespace {
 // Runs piece(i, slot) for i < n on the copying threads, with the device current on
 // each and a free pinned buffer; `piece` fills it and enqueues its copy on `stream`,
 // behind which the buffer's event is recorded.
+template <class P>
 cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, size_t n,
-                       cudaStream_t stream,
-                       const std::function<cudaError_t(size_t, char*)>& piece) {
+                       cudaStream_t stream, const P& piece) {
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
   std::atomic<size_t> next{0};
   std::atomic<int> failed{0};
-  Workers::get().run([&](int worker) {
+  auto copy = [&](int worker) {
     cudaError_t e = worker > 0 ? cudaSetDevice(dev) : cudaSuccess;
     for (int turn = 0; e == cudaSuccess && failed.load() == 0; turn ^= 1) {
       const size_t i = next.fetch_add(1);
@@ -179,7 +183,8 @@ cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, siz
       int none = 0;
       failed.compare_exchange_strong(none, int(e));
     }
-  });
+  };
+  Workers::get().run(copy);
   return cudaError_t(failed.load());
 }
 
@@ -240,7 +245,7 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
   if (err != cudaSuccess) return err;
   std::atomic<size_t> next{0};
   std::atomic<int> failed{0};
-  Workers::get().run([&](int worker) {
+  auto copy = [&](int worker) {
     cudaError_t e = worker > 0 ? cudaSetDevice(dev) : cudaSuccess;
     size_t held[2] = {n, n};  // the pieces in this thread's buffers
     bool more = true;
@@ -270,7 +275,8 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
       int none = 0;
       failed.compare_exchange_strong(none, int(e));
     }
-  });
+  };
+  Workers::get().run(copy);
   return cudaError_t(failed.load());
 }
 

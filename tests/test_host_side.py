@@ -44,3 +44,7 @@ def test_each_device_grants_the_matching_its_shared_memory(objects):
 
 def test_masked_gemm_takes_the_widest_block(objects):
     drive(objects, "wide_block")
+
+
+def test_no_exception_leaves_a_host_call(objects):
+    drive(objects, "no_memory")
