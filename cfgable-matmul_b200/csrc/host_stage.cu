@@ -26,10 +26,12 @@ class Workers {
   }
   int count() const { return 1 + int(threads_); }
   // fn(worker) on every thread, worker 0 being the caller; returns when all are done.
-  // (By address, without a std::function: nothing is allocated that could fail.)
+  // While another device's copy has the threads, on the caller alone, so that no
+  // device waits for another.  (By address, without a std::function: nothing is allocated that could fail.)
   template <class F>
   void run(F& fn) {
-    std::lock_guard<std::mutex> one(job_mu_);
+    std::unique_lock<std::mutex> one(job_mu_, std::try_to_lock);
+    if (!one) return fn(0);
     {
       std::lock_guard<std::mutex> lk(mu_);
       call_ = [](void* f, int worker) { (*static_cast<F*>(f))(worker); };
@@ -236,18 +238,30 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
   }
   // A thread copies a piece out of one of its buffers while the next piece arrives in
-  // the other.
+  // the other.  The caller requests its first two here and waits for the first, that is
+  // for all earlier work on the stream, before it takes the threads.
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
   const size_t most = piece_bytes(bytes), n = (bytes + most - 1) / most;
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
-  std::atomic<size_t> next{0};
+  auto request = [&](size_t i, size_t slot) {
+    const size_t off = i * most;
+    cudaError_t e = cudaMemcpyAsync(pinned_ + slot * kSlot, s + off, std::min(most, bytes - off),
+                                    cudaMemcpyDeviceToHost, stream);
+    return e == cudaSuccess ? cudaEventRecord(events_[slot], stream) : e;
+  };
+  const size_t first = std::min<size_t>(n, 2);
+  for (size_t i = 0; err == cudaSuccess && i < first; ++i) err = request(i, i);
+  if (err == cudaSuccess) err = cudaEventSynchronize(events_[0]);
+  if (err != cudaSuccess) return err;
+  std::atomic<size_t> next{first};
   std::atomic<int> failed{0};
   auto copy = [&](int worker) {
     cudaError_t e = worker > 0 ? cudaSetDevice(dev) : cudaSuccess;
     size_t held[2] = {n, n};  // the pieces in this thread's buffers
+    for (size_t i = 0; worker == 0 && i < first; ++i) held[i] = i;
     bool more = true;
     for (int turn = 0; e == cudaSuccess && failed.load() == 0; turn ^= 1) {
       const size_t slot = 2 * size_t(worker) + turn;
@@ -261,10 +275,7 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
       }
       const size_t i = more ? next.fetch_add(1) : n;
       if (i < n) {
-        const size_t off = i * most;
-        e = cudaMemcpyAsync(buf, s + off, std::min(most, bytes - off), cudaMemcpyDeviceToHost,
-                            stream);
-        if (e == cudaSuccess) e = cudaEventRecord(events_[slot], stream);
+        e = request(i, slot);
         held[turn] = i;
       } else {
         more = false;

@@ -48,3 +48,7 @@ def test_masked_gemm_takes_the_widest_block(objects):
 
 def test_no_exception_leaves_a_host_call(objects):
     drive(objects, "no_memory")
+
+
+def test_devices_do_not_wait_for_one_another(objects):
+    drive(objects, "two_devices")
