@@ -40,6 +40,7 @@ int fail(int status, const std::string& msg) {
 }
 
 int cuda_fail(cudaError_t err, const char* where) {
+  cudaGetLastError();  // reported here: a later launch's check does not find it again
   g_last_error = std::string(where) + ": " + cudaGetErrorName(err) + " (" +
                  cudaGetErrorString(err) + ")";
   if (err == cudaErrorMemoryAllocation) return CFGMM_ERR_OUT_OF_MEMORY;

@@ -68,6 +68,7 @@ int fail(int status, const std::string& msg) {
 }
 
 int cuda_fail(cudaError_t err, const char* where) {
+  cudaGetLastError();  // reported here: a later launch's check does not find it again
   return fail(err == cudaErrorMemoryAllocation ? CFGMM_ERR_OUT_OF_MEMORY : CFGMM_ERR_CUDA,
               std::string(where) + ": " + cudaGetErrorName(err) + " (" + cudaGetErrorString(err) +
                   ")");
@@ -820,7 +821,6 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
                             d_lists, d_counts, list_off, cnt_off, nblk, counts, s);
       if (rc == CFGMM_ERR_OUT_OF_MEMORY) {
         // the row form's phi tiles take up to half of the memory
-        cudaGetLastError();
         void* lists = plan->mem;
         plan->mem = nullptr;
         free_on(plan, s);  // the pairing kernels may still run there

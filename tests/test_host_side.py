@@ -52,3 +52,7 @@ def test_no_exception_leaves_a_host_call(objects):
 
 def test_devices_do_not_wait_for_one_another(objects):
     drive(objects, "two_devices")
+
+
+def test_a_failed_allocation_does_not_fail_the_next_call(objects):
+    drive(objects, "after_failure")
