@@ -51,7 +51,7 @@ __device__ int g_fock_error;
 constexpr int FT = 64;        // rows per item = columns per chunk = points per tile
 constexpr int CONS = 8;       // consumer warps: 4 along rows (16 each) x 2 along columns (32 each)
 constexpr int THREADS = 32 * (CONS + 1);
-constexpr int NS = 4;         // weight vectors per item at most
+constexpr int NS = kFockVectors;
 constexpr int STAGES = 2;     // chunks of phi_rhs in flight
 // Row pitch of a staged tile (doubles): 33 16-byte groups, so the 8 lanes of a
 // quarter warp's fragment load (rows r and r + 4, point pairs q = 0..3) meet 8
@@ -74,7 +74,7 @@ struct FockArgs {
   int sym;  // ao_lhs == ao_rhs: chunks from the row tile's own on, mirrored
   int vec;  // phi rows and w 16-byte aligned at every tile
   const int4* items;
-  int* counters;  // the work counter, the item total
+  int* counters;  // the work counter (64 bits), the item total
 };
 
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int code) {
@@ -99,11 +99,9 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
   FockItem* item = reinterpret_cast<FockItem*>(empty + STAGES);
 
   // the items once for each group of weight vectors
-  const int items = p.counters[1];
-  const int groups =
-      max((p.nset + NS - 1) / NS, min(p.nset, (8 * int(gridDim.x) + items - 1) / max(items, 1)));
-  const int per_group = (p.nset + groups - 1) / groups;
-  const int total = items * groups;
+  const int items = p.counters[2];
+  const FockShare share = fock_share(items, p.nset, int(gridDim.x));
+  const int per_group = share.per_group;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
     // the producer's 32 lanes and one more arrival: the bulk copies' expect_tx
@@ -119,9 +117,9 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
 
   if (warp == CONS) {
     // ------------------------------- producer -------------------------------
-    int* counter = p.counters;
-    int it = 0;
-    if (lane == 0) it = atomicAdd(counter, 1);
+    auto* counter = reinterpret_cast<unsigned long long*>(p.counters);
+    long long it = 0;
+    if (lane == 0) it = (long long)atomicAdd(counter, 1ull);
     it = __shfl_sync(0xffffffffu, it, 0);
     int fill = 0, n = 0;
     bool ok = true;
@@ -148,11 +146,12 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
         if (lane == 0) tc::mbar_arrive(bar);  // in the expect_tx's place
       }
     };
-    while (ok && it < total) {
-      int next = 0;  // drawn now, needed after this item's copies
-      if (lane == 0) next = atomicAdd(counter, 1);
-      const int4 wi = p.items[it % items];
-      const int set0 = it / items * per_group;
+    while (ok && it < share.total) {
+      long long next = 0;  // drawn now, needed after this item's copies
+      if (lane == 0) next = (long long)atomicAdd(counter, 1ull);
+      const int group = int(it / items);
+      const int4 wi = p.items[it - (long long)group * items];
+      const int set0 = group * per_group;
       const int ns = min(per_group, p.nset - set0);
       const int b = wi.y / p.gsub, gt = wi.y % p.gsub, a = wi.z;
       const int nb = p.counts[b];
@@ -369,7 +368,7 @@ FockLayout fock_layout(size_t nao, size_t ngrid, size_t nset, size_t blk) {
   L.counts = L.lists + a256(nblk * nao * sizeof(int));
   L.items = L.counts + a256(nblk * sizeof(int));
   L.counters = L.items + a256(nblk * gsub * max_ut * sizeof(int4));
-  L.total = L.counters + a256((nset + 2) * sizeof(int));
+  L.total = L.counters + a256(4 * sizeof(int));  // the work counter, the total, a flag
   return L;
 }
 
@@ -396,7 +395,7 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   int* counters = reinterpret_cast<int*>(wsp + L.counters);
   cudaError_t err = aodm_block_lists_launch(tab, ldtab, nao, nblk, lists, counts, stream);
   if (err != cudaSuccess) return err;
-  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, 1, stream)) !=
+  if ((err = aodm_build_items_launch(counts, nblk, gsub, items, counters, 2, stream)) !=
       cudaSuccess)
     return err;
   FockArgs a{};

@@ -6,6 +6,28 @@
 
 namespace cfgmm {
 
+// How the kernel shares out its work: the items (block tiles x row tiles) once for each
+// of `groups` groups of up to `per_group` weight vectors (the last may be empty), `total`
+// in all.  Items take kFockVectors vectors at most, and fewer where `ctas` CTAs would
+// have under 8 items each to draw.  Vectors are many where items are few and the other
+// way round, but both are the caller's: the product takes 64 bits.
+constexpr int kFockVectors = 4;
+struct FockShare {
+  int groups, per_group;
+  long long total;
+};
+__host__ __device__ inline FockShare fock_share(int items, int nset, int ctas) {
+  const long long least = (nset + kFockVectors - 1ll) / kFockVectors;
+  const long long one = items > 0 ? items : 1;
+  const long long wanted = (8ll * ctas + one - 1) / one;
+  const long long most = wanted < nset ? wanted : nset;
+  FockShare s;
+  s.groups = int(least > most ? least : most);
+  s.per_group = int((nset + s.groups - 1ll) / s.groups);
+  s.total = (long long)items * s.groups;
+  return s;
+}
+
 // Device scratch (bytes) of fock_compact_fp64: active lists, work list, counters.
 size_t fock_compact_workspace(size_t nao, size_t ngrid, size_t nset, size_t blk);
 

@@ -123,3 +123,28 @@ def test_fock_compacted_and_dense_forms_agree(cm, oracle):
     oracle.aodm_fock(vs, ws, lhs, rhs, strides, shape, 2, tab, tab.shape[1], 64)
     for o in outs:
         assert normwise(o, vs) < TOL
+
+
+@pytest.mark.parametrize("nao,nblk,blk,nset,groups,pad,same", [
+    (70, 2500, 16, 4, (1, 4), 0, True),    # one group: four vectors to an item
+    (70, 2500, 16, 7, (2, 4), 0, False),   # two groups, the last of three
+    (70, 1300, 24, 3, (2, 2), 1, True),    # odd rows: 8-byte copies of two vectors and one
+    (70, 650, 16, 5, (4, 2), 0, True),     # four groups of two, the last empty
+    (150, 400, 100, 3, (2, 2), 0, False),  # wide blocks, three row tiles in some
+    (70, 2400, 1, 2, (1, 2), 1, True),     # one point to a block
+])
+def test_fock_items_of_several_vectors(cm, oracle, nao, nblk, blk, nset, groups, pad, same):
+    """Items that serve several weight vectors (many items), the last group of vectors
+    short or empty; the groups expected are the kernel's rule on 148 SMs."""
+    ngrid = nblk * blk - (blk // 3)
+    lhs, rhs, ws, tab, vs, strides, shape = _case(nao + nset, nao, ngrid, nset, blk, pad, pad,
+                                                  density=0.5, same=same)
+    tab[0, :] = 1  # no block is empty
+    items = int((-(-tab[:, :nblk].astype(int).sum(0) // 64) * -(-blk // 64)).sum())
+    g = max(-(-nset // 4), min(nset, -(-8 * 2 * 148 // items)))
+    assert (g, -(-nset // g)) == groups
+    ref = vs.copy()
+    oracle.aodm_fock(ref, ws, lhs, rhs, strides, shape, nset, tab, tab.shape[1], blk)
+    cm.aodm_fock(vs, ws, lhs, rhs, strides, shape, nset, tab, tab.shape[1], blk)
+    for s in range(nset):
+        assert normwise(vs[s], ref[s]) < TOL

@@ -56,3 +56,7 @@ def test_devices_do_not_wait_for_one_another(objects):
 
 def test_a_failed_allocation_does_not_fail_the_next_call(objects):
     drive(objects, "after_failure")
+
+
+def test_fock_items_are_counted_in_64_bits(objects):
+    drive(objects, "fock_share")
