@@ -13,8 +13,23 @@ namespace cfgmm {
 namespace {
 
 constexpr size_t kSlot = size_t(1) << 20;      // bytes of a pinned buffer
-constexpr size_t kDirect = size_t(256) << 10;  // smaller copies go the driver's way
 constexpr int kMaxWorkers = 6;  // copying threads, the caller among them
+// Smaller copies go the driver's way.
+constexpr size_t kDirectUp = size_t(1) << 20, kDirectDown = size_t(256) << 10;
+
+// Threads of a contiguous upload.  More of them get in one another's way in the driver
+// unless there is much to copy; us by the driver and with 2, 4 and 6 threads, the source
+// in the caches / not: 1 MB 69 69 73 73 / 121 94 96 97; 4 MB 219 199 502 632 / 406 258 441
+// 708; 16 MB 790 567 777 1289 / 1528 901 773 797; 64 MB 5200 2815 2014 2078 / 6207 3329
+// 2000 1874.
+int upload_threads(size_t bytes) { return bytes < (size_t(48) << 20) ? 2 : 4; }
+size_t upload_piece(size_t bytes) { return bytes < (size_t(16) << 20) ? kSlot / 2 : kSlot; }
+// Of the present tiles of a table, whose packing takes longer than a plain copy.  A density
+// call with so many MB of tiles, ms with 2, 3, 4 and 6 threads: 6 0.66 0.67 0.73 0.90; 16
+// 1.16 1.06 1.11 1.39; 46 4.0 3.0 2.6 2.7; 117 12.8 8.5 7.4 6.5.
+int tiles_threads(size_t bytes) {
+  return bytes < (size_t(12) << 20) ? 3 : bytes < (size_t(64) << 20) ? 4 : kMaxWorkers;
+}
 
 // A few threads that run one job at a time.  They live as long as the process: the
 // object is never destroyed, so none of them meets a destroyed mutex at exit.
@@ -25,21 +40,23 @@ class Workers {
     return *w;
   }
   int count() const { return 1 + int(threads_); }
-  // fn(worker) on every thread, worker 0 being the caller; returns when all are done.
-  // While another device's copy has the threads, on the caller alone, so that no
-  // device waits for another.  (By address, without a std::function: nothing is allocated that could fail.)
+  // fn(worker) on up to `most` threads, worker 0 being the caller; returns when all are
+  // done.  While another device's copy has the threads, on the caller alone, so that no
+  // device waits for another.  (By address, without a std::function: nothing is allocated
+  // that could fail.)
   template <class F>
-  void run(F& fn) {
+  void run(F& fn, int most) {
     std::unique_lock<std::mutex> one(job_mu_, std::try_to_lock);
-    if (!one) return fn(0);
+    const int helpers = std::min(most - 1, int(threads_));
+    if (!one || helpers <= 0) return fn(0);
     {
       std::lock_guard<std::mutex> lk(mu_);
       call_ = [](void* f, int worker) { (*static_cast<F*>(f))(worker); };
       arg_ = &fn;
-      running_ = int(threads_);
-      ++round_;
+      running_ = helpers;
+      for (int i = 1; i <= helpers; ++i) job_[i] = true;
     }
-    start_.notify_all();
+    for (int i = 1; i <= helpers; ++i) start_[i].notify_one();
     fn(0);
     std::unique_lock<std::mutex> lk(mu_);
     done_.wait(lk, [&] { return running_ == 0; });
@@ -59,14 +76,13 @@ class Workers {
     }
   }
   void loop(int worker) {
-    unsigned long long seen = 0;
     for (;;) {
       void (*call)(void*, int);
       void* arg;
       {
         std::unique_lock<std::mutex> lk(mu_);
-        start_.wait(lk, [&] { return round_ != seen; });
-        seen = round_;
+        start_[worker].wait(lk, [&] { return job_[worker]; });
+        job_[worker] = false;
         call = call_;
         arg = arg_;
       }
@@ -76,11 +92,11 @@ class Workers {
     }
   }
   std::mutex job_mu_, mu_;
-  std::condition_variable start_, done_;
+  std::condition_variable start_[kMaxWorkers], done_;
+  bool job_[kMaxWorkers] = {};
   void (*call_)(void*, int) = nullptr;
   void* arg_ = nullptr;
   int running_ = 0;
-  unsigned long long round_ = 0;
   size_t threads_ = 0;
 };
 
@@ -160,12 +176,12 @@ void HostStage::release() {
 
 namespace {
 
-// Runs piece(i, slot) for i < n on the copying threads, with the device current on
+// Runs piece(i, slot) for i < n on up to `threads` copying threads, with the device current on
 // each and a free pinned buffer; `piece` fills it and enqueues its copy on `stream`,
 // behind which the buffer's event is recorded.
 template <class P>
 cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, size_t n,
-                       cudaStream_t stream, const P& piece) {
+                       int threads, cudaStream_t stream, const P& piece) {
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
@@ -186,11 +202,11 @@ cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, siz
       failed.compare_exchange_strong(none, int(e));
     }
   };
-  Workers::get().run(copy);
+  Workers::get().run(copy, threads);
   return cudaError_t(failed.load());
 }
 
-// Bytes of a piece of a contiguous copy: every thread gets two or more.
+// Bytes of a piece where all threads copy: every one gets two or more.
 size_t piece_bytes(size_t total) {
   const size_t each = total / (2 * size_t(Workers::get().count()));
   return std::min(kSlot, std::max(size_t(128) << 10, (each + 4095) / 4096 * 4096));
@@ -205,7 +221,7 @@ cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t 
     dpitch = spitch = width;
     rows = 1;
   }
-  if (width * rows < kDirect || !host_pageable(src) || ensure() != cudaSuccess) {
+  if (width * rows < kDirectUp || !host_pageable(src) || ensure() != cudaSuccess) {
     cudaGetLastError();
     return rows == 1 ? cudaMemcpyAsync(dst, src, width, cudaMemcpyHostToDevice, stream)
                      : cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows,
@@ -213,10 +229,11 @@ cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t 
   }
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
-  const size_t most = piece_bytes(width * rows);
+  const size_t most = upload_piece(width * rows);
+  const int threads = upload_threads(width * rows);
   if (width > most) {  // parts of a row
     const size_t per_row = (width + most - 1) / most;
-    return run_pieces(pinned_, events_, per_row * rows, stream, [&](size_t i, char* slot) {
+    return run_pieces(pinned_, events_, per_row * rows, threads, stream, [&](size_t i, char* slot) {
       const size_t r = i / per_row, off = i % per_row * most;
       const size_t n = std::min(most, width - off);
       std::memcpy(slot, s + r * spitch + off, n);
@@ -224,7 +241,8 @@ cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t 
     });
   }
   const size_t some = most / width;  // rows
-  return run_pieces(pinned_, events_, (rows + some - 1) / some, stream, [&](size_t i, char* slot) {
+  const size_t pieces = (rows + some - 1) / some;
+  return run_pieces(pinned_, events_, pieces, threads, stream, [&](size_t i, char* slot) {
     const size_t r0 = i * some, n = std::min(some, rows - r0);
     for (size_t r = 0; r < n; ++r) std::memcpy(slot + r * width, s + (r0 + r) * spitch, width);
     return cudaMemcpy2DAsync(d + r0 * dpitch, dpitch, slot, width, width, n,
@@ -233,7 +251,7 @@ cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t 
 }
 
 cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-  if (bytes < kDirect || !host_pageable(dst) || ensure() != cudaSuccess) {
+  if (bytes < kDirectDown || !host_pageable(dst) || ensure() != cudaSuccess) {
     cudaGetLastError();
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
   }
@@ -287,7 +305,7 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
       failed.compare_exchange_strong(none, int(e));
     }
   };
-  Workers::get().run(copy);
+  Workers::get().run(copy, kMaxWorkers);
   return cudaError_t(failed.load());
 }
 
@@ -344,7 +362,8 @@ cudaError_t HostStage::upload_tiles(double* dst, double* packed, unsigned long l
   err = cudaMemcpyAsync(d_offsets, offsets.data(), rows * sizeof(unsigned long long),
                         cudaMemcpyHostToDevice, stream);
   if (err != cudaSuccess) return err;
-  err = run_pieces(pinned_, events_, pieces.size(), stream, [&](size_t i, char* slot) {
+  const int threads = tiles_threads(total * 8);
+  err = run_pieces(pinned_, events_, pieces.size(), threads, stream, [&](size_t i, char* slot) {
     const Piece& p = pieces[i];
     double* to = reinterpret_cast<double*>(slot);
     size_t left = p.elems, r = p.row, b = p.b;

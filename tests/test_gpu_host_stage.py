@@ -110,3 +110,16 @@ def test_two_threads_at_once(cm):
         t.join()
     for (a, b), c in zip(jobs, out):
         assert normwise(c, a @ b) < 1e-13
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (128, 6000, 1050),  # A just past 1 MB, B past 48 MB, C of a few MB
+    (2000, 64, 1100),   # A past 16 MB, B by the driver
+    (131, 137, 1000),   # A just short of 1 MB
+])
+def test_products_on_either_side_of_the_upload_rules(cm, m, n, k):
+    rng = np.random.default_rng(m + n)
+    a, b, c0 = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n)), rng.uniform(-1, 1, (m, n))
+    c = c0.copy()
+    cm.matmul_ex(c, a, b, m, n, k, k, n, n, False, False)
+    assert normwise(c, c0 + a @ b) < 1e-13
