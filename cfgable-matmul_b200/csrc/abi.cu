@@ -216,23 +216,42 @@ int check_split_gemm(size_t k) {
   return CFGMM_OK;
 }
 
-// Reads the sticky error words of the tcgen05 kernels after a synchronised call.
-int check_device_waits() {
-  int code = 0, code2 = 0, code3 = 0, code4 = 0, code5 = 0;
-  CFGMM_CUDA(cfgmm::gemm_i8_read_error(&code));
-  CFGMM_CUDA(cfgmm::aodmao2rho_split_read_error(&code2));
-  CFGMM_CUDA(cfgmm::dgemm_read_error(&code3));
-  CFGMM_CUDA(cfgmm::aodm_read_error(&code4));
-  CFGMM_CUDA(cfgmm::fock_read_error(&code5));
-  if (code == 0) code = code2;
-  if (code == 0) code = code3;
-  if (code == 0) code = code4;
-  if (code == 0) code = code5;
+// The compacted form (fock.cu) unless CFGMM_FOCK_DENSE=1 selects the dense
+// product with K-step skipping (fock_dense.cu).
+bool fock_dense() {
+  static const bool on = [] {
+    const char* e = std::getenv("CFGMM_FOCK_DENSE");
+    return e && e[0] == '1';
+  }();
+  return on;
+}
+
+// Kernels whose error words not every call looks at: each read is a copy that the host
+// waits for (10 us), so a host call reads theirs only where they can have run, and that of
+// the dense Fock form only where the environment selects it.
+enum : unsigned { kMaskWaits = 1, kFockWaits = 2, kAllWaits = 3 };
+
+// Reads the sticky error words of the kernels with bounded waits after a synchronised call.
+int check_device_waits(unsigned extra) {
+  int code = 0;
+  auto look = [&](cudaError_t (*read)(int*)) {
+    int c = 0;
+    const cudaError_t e = read(&c);
+    if (code == 0) code = c;
+    return e;
+  };
+  CFGMM_CUDA(look(cfgmm::gemm_i8_read_error));
+  CFGMM_CUDA(look(cfgmm::aodmao2rho_split_read_error));
+  if (fock_dense()) CFGMM_CUDA(look(cfgmm::fock_dense_read_error));
+  CFGMM_CUDA(look(cfgmm::aodm_read_error));
+  if (extra & kMaskWaits) CFGMM_CUDA(look(cfgmm::dgemm_mask_read_error));
+  if (extra & kFockWaits) CFGMM_CUDA(look(cfgmm::fock_read_error));
   if (code != 0) {
     // reported once: the words start over for the next call
     cudaError_t e = cfgmm::gemm_i8_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::aodmao2rho_split_reset_error(nullptr);
-    if (e == cudaSuccess) e = cfgmm::dgemm_reset_error(nullptr);
+    if (e == cudaSuccess) e = cfgmm::fock_dense_reset_error(nullptr);
+    if (e == cudaSuccess) e = cfgmm::dgemm_mask_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::aodm_reset_error(nullptr);
     if (e == cudaSuccess) e = cfgmm::fock_reset_error(nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
@@ -357,7 +376,7 @@ int gemm_host_blocked(DeviceState* st, double* c, const double* a, const double*
   const cudaError_t e3 = cudaStreamSynchronize(st->down);
   if (err == cudaSuccess) err = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
   if (err != cudaSuccess) return cuda_fail(err, "blocked host GEMM");
-  return check_device_waits();
+  return check_device_waits(dt ? kMaskWaits : 0);
 }
 
 int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const double* b,
@@ -432,7 +451,7 @@ int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const doub
   }
   CFGMM_CUDA(st->stage.download(c, dc, ex.c * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
-  return check_device_waits();
+  return check_device_waits(masked ? kMaskWaits : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -481,7 +500,7 @@ int check_aodm(const void* rhos, size_t rhos_len, const void* dms, size_t dms_le
 
 // The status of a finished AO-DM-AO run: a timed-out pipeline wait of either kernel family.
 int aodm_device_status(bool split) {
-  if (split) return check_device_waits();
+  if (split) return check_device_waits(0);
   int code = 0;
   CFGMM_CUDA(cfgmm::aodm_read_error(&code));
   if (code != 0) {
@@ -665,7 +684,7 @@ int aodm_host(double* rhos, size_t rhos_len, const double* dms, size_t dms_len,
   }
   CFGMM_CUDA(st->stage.download(rhos, d_rho, ex.rhos * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
-  if (split) return check_device_waits();
+  if (split) return check_device_waits(0);
   int code = 0;
   CFGMM_CUDA(cfgmm::aodm_read_error(&code));
   if (code != 0) {
@@ -697,16 +716,6 @@ int check_fock(double* vs, size_t vs_len, const double* ws, size_t ws_len, const
   return rc;
 }
 
-// The compacted form (fock.cu) unless CFGMM_FOCK_DENSE=1 selects the dense
-// product with K-step skipping (fock_dense.cu).
-bool fock_dense() {
-  static const bool on = [] {
-    const char* e = std::getenv("CFGMM_FOCK_DENSE");
-    return e && e[0] == '1';
-  }();
-  return on;
-}
-
 size_t fock_workspace(size_t nao, size_t ngrid, size_t nset, size_t blksize) {
   return fock_dense() ? cfgmm::fock_fp64_workspace(int(nao), int(ngrid))
                       : cfgmm::fock_compact_workspace(nao, ngrid, nset, blksize);
@@ -721,7 +730,7 @@ int fock_run(double* d_v, const double* d_w, const double* d_lhs, const double* 
                                         int(blksize), ws, s));
     return CFGMM_OK;
   }
-  CFGMM_CUDA(cfgmm::dgemm_reset_error(s));
+  CFGMM_CUDA(cfgmm::fock_dense_reset_error(s));
   for (size_t set = 0; set < nset; ++set)
     CFGMM_CUDA(cfgmm::fock_fp64(d_v + set * stride_ao * stride_ao, stride_ao,
                                 d_w + set * stride_grid, d_lhs, d_rhs, stride_grid, int(nao),
@@ -771,7 +780,7 @@ int fock_host(double* vs, size_t vs_len, const double* ws, size_t ws_len, const 
     return rc;
   CFGMM_CUDA(st->stage.download(vs, d_v, ex.dms * 8, st->stream));
   CFGMM_CUDA(cudaStreamSynchronize(st->stream));
-  return check_device_waits();
+  return check_device_waits(kFockWaits);
 }
 
 // ---------------------------------------------------------------------------
@@ -1058,7 +1067,7 @@ int cfgmm_device_check(void) {
   int rc = current_device(&dev);
   if (rc != CFGMM_OK) return rc;
   CFGMM_CUDA(cudaDeviceSynchronize());
-  return check_device_waits();
+  return check_device_waits(kAllWaits);
 }
 
 int cfgmm_aodmao2rho_loop_parallel(double* rhos, size_t rhos_len, const double* dms,
@@ -1228,7 +1237,7 @@ int cfgmm_matmul_f32(float* c, size_t c_len, const float* a, size_t a_len, const
     CFGMM_CUDA(st->stage.download(c, dc, ex.c * 4, s));
   }
   CFGMM_CUDA(cudaStreamSynchronize(s));
-  return check_device_waits();
+  return check_device_waits(0);
 }
 
 int cfgmm_matmul_f32_dev(float* c, const float* a, const float* b, size_t m, size_t n, size_t k,
@@ -1292,7 +1301,7 @@ int cfgmm_aodmao2rho_f32(float* rhos, size_t rhos_len, const float* dms, size_t 
     CFGMM_CUDA(st->stage.download(rhos, d_rho, ex.rhos * 4, s));
   }
   CFGMM_CUDA(cudaStreamSynchronize(s));
-  if (split) return check_device_waits();
+  if (split) return check_device_waits(0);
   int code = 0;
   CFGMM_CUDA(cfgmm::aodm_read_error(&code));
   if (code != 0) return fail(CFGMM_ERR_TIMEOUT, "a pipeline wait of the FP64 kernel timed out");

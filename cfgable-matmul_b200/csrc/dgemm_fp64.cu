@@ -591,14 +591,4 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
   return err;
 }
 
-cudaError_t dgemm_reset_error(cudaStream_t stream) {
-  const cudaError_t err = fock_dense_reset_error(stream);
-  return err != cudaSuccess ? err : dgemm_mask_reset_error(stream);
-}
-
-cudaError_t dgemm_read_error(int* code) {
-  const cudaError_t err = fock_dense_read_error(code);
-  return err != cudaSuccess || *code != 0 ? err : dgemm_mask_read_error(code);
-}
-
 }  // namespace cfgmm

@@ -36,6 +36,7 @@ cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int 
                                size_t lda, size_t ldb, size_t ldc, bool transa,
                                const uint8_t* tab, size_t ldtab, int blk, double max_share,
                                int* compact, void* workspace, cudaStream_t stream);
+// Sticky error word of the compacted form's bounded waits (0 = none).
 cudaError_t dgemm_mask_reset_error(cudaStream_t stream);
 cudaError_t dgemm_mask_read_error(int* code);
 
@@ -55,12 +56,8 @@ cudaError_t fock_fp64(double* v, size_t ldv, const double* w, const double* ao_l
                       const uint8_t* tab, size_t ldtab, int blk, bool pack_rhs, void* workspace,
                       cudaStream_t stream);
 
+// Sticky error word of the dense Fock form's bounded waits (0 = none).
 cudaError_t fock_dense_reset_error(cudaStream_t stream);
 cudaError_t fock_dense_read_error(int* code);
-
-// Sticky error words of the bounded waits of the masked GEMM's compacted form and
-// the dense Fock form (0 = none).
-cudaError_t dgemm_reset_error(cudaStream_t stream);
-cudaError_t dgemm_read_error(int* code);
 
 }  // namespace cfgmm

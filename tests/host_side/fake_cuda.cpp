@@ -24,6 +24,7 @@ struct CUevent_st {
 
 namespace fake {
 int fail_async_alloc = 0;
+int word_reads = 0;
 int free_races = 0;
 int long_device = -1;
 int bad_launches = 0;
@@ -269,6 +270,7 @@ cudaError_t cudaMemcpyToSymbolAsync(const void*, const void*, size_t, size_t, cu
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyFromSymbol(void* d, const void*, size_t n, size_t, cudaMemcpyKind) {
+  ++word_reads;
   std::memset(d, 0, n);  // the error words: none
   return cudaSuccess;
 }

@@ -11,6 +11,7 @@ namespace fake {
 // once; kernels do nothing.  Every launch, copy and memset is "in flight" on its stream
 // until a call that waits for it.
 extern int fail_async_alloc;  // the n-th cudaMallocAsync from now on fails (0: none)
+extern int word_reads;        // cudaMemcpyFromSymbol: copies that the host waits for
 extern int free_races;        // cudaFree of cudaMallocAsync memory with work in flight
 // A kernel launched on a stream of this device (-1: none) runs until release() is called.
 extern int long_device;

@@ -60,3 +60,7 @@ def test_a_failed_allocation_does_not_fail_the_next_call(objects):
 
 def test_fock_items_are_counted_in_64_bits(objects):
     drive(objects, "fock_share")
+
+
+def test_host_calls_read_few_error_words(objects):
+    drive(objects, "wait_words")
