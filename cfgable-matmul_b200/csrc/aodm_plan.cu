@@ -813,8 +813,12 @@ int cfgmm_aodm_plan_create(cfgmm_aodm_plan** out, const cfgmm_aodm_batch* batche
     }
   if (precision == CFGMM_PREC_OZAKI_INT8) {
     size_t points = 0;
-    for (size_t i = 0; i < nbatch; ++i) points += batches[i].ngrid;
-    bool pair = cfgmm::split_pair_form(nao, points, nset_max);
+    double work = 0.0;
+    for (size_t i = 0; i < nbatch; ++i) {
+      points += batches[i].ngrid;
+      work += double(nao) * double(nao) * double(batches[i].ngrid) * double(batches[i].nset);
+    }
+    bool pair = cfgmm::split_pair_plan(nao, points, work, nbatch);
     int rc = CFGMM_OK;
     if (pair) {
       rc = build_split_pair(plan, batches, nbatch, dms, stride_ao, nao, nset_max, blksize, flags,

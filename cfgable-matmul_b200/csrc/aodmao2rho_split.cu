@@ -733,12 +733,22 @@ Layout layout(size_t nao, size_t ngrid, size_t nset, size_t blk) {
 // compacted rows per item) or the pair form (two alike block tiles per item,
 // aodmao2rho_split_pair.cu).  CFGMM_SPLIT_FORM is read on every call; the
 // workspace covers both.
-bool split_pair_form(size_t nao, size_t points, size_t nset) {
+static int forced_form() {  // 1: pair, 0: row, -1: by the rule
   const char* e = std::getenv("CFGMM_SPLIT_FORM");
-  if (e && e[0] == 'p') return true;
-  if (e && e[0] == 'r') return false;
+  return e && e[0] == 'p' ? 1 : e && e[0] == 'r' ? 0 : -1;
+}
+
+bool split_pair_form(size_t nao, size_t points, size_t nset) {
+  if (const int f = forced_form(); f >= 0) return f;
+  return nao >= kPairMinAos &&
+         (points >= kPairMinPoints ||
+          double(nao) * double(nao) * double(points) * double(nset) >= kPairMinWork);
+}
+
+bool split_pair_plan(size_t nao, size_t points, double work, size_t nbatch) {
+  if (const int f = forced_form(); f >= 0) return f;
   return (nao >= kPairMinAos && points >= kPairMinPoints) ||
-         double(nao) * double(nao) * double(points) * double(nset) >= kPairMinWork;
+         (work >= kPairMinWork && work >= kPairMinBatchWork * double(nbatch));
 }
 
 size_t aodmao2rho_split_workspace(size_t nao, size_t ngrid, size_t nset, size_t blk) {

@@ -183,22 +183,32 @@ cudaError_t split_pair_launch_main(const PairArgs& a, int nsl, cudaStream_t stre
                                    bool attrs_only = false, int stages = 0);
 cudaError_t split_pair_launch_reduce(const PairArgs& a, int nsl, const int* npairs, int pair0,
                                      int max_pairs, cudaStream_t stream);
-// Whether a call of nset matrices on ngrid points, or a plan of up to nset matrices
-// on so many points in all, runs the pair form: CFGMM_SPLIT_FORM=pair / =row, else
-// the pair form from kPairMinAos AOs and kPairMinPoints points on, and from nao^2
-// points nset = kPairMinWork on (below that the pairing and tile
-// building, 35 us and more, cost more than the pairs save; the share of active AOs
-// is known on the device only).  Row / pair form, us: nao 6000, 1000 points, 1
-// matrix (3.6e10) 461 / 321; 3000, 2000, 2 273 / 226; 200, 250000, 4 1347 / 1305;
-// 2522, 2800, 4 661 / 438; 2782, 2293, 1 (1.8e10) 176 / 187; 891, 3998, 4 (1.3e10)
-// 197 / 210.  A plan of one batch runs the single call's form (the same bits); its
-// runs gain at every size measured (508 AOs, 84 batches, 2 matrices 269 / 154, 312
-// AOs, 25 batches 67 / 49), but its creation takes longer and its phi tiles up to
-// twice the memory, so the line is the same (a plan that does not fit takes the row
-// form).
+// Whether a call of nset matrices on so many points runs the pair form:
+// CFGMM_SPLIT_FORM=pair / =row, else from kPairMinAos AOs on, with kPairMinPoints points
+// or nao^2 points nset = kPairMinWork.  Below, the pairing and tile building (35 us and
+// more) cost more than the pairs save, or the mask decides, which is known on the device
+// only: tiles that find no partner leave half of the MMA rows idle.  Row / pair form, us,
+// atom-centred masks / random ones of the same density: nao 1500, 5185 points, 3 matrices
+// 230/168, 241/224 at 0.3 and 118/104, 125/122 at 0.1; nao 2522, 2800, 4 661/438; but nao
+// 1000, 36000, 1 (3.6e10) 248/226, 255/334 at 0.3 and 106/129, 109/170 at 0.1; nao 600,
+// 97000, 1 410/328, 433/486 and 186/192, 195/246.
+//
+// A plan pays for the pairing and the tiles (twice the row form's memory: 182 against 91
+// MB for 900 AOs, 45000 points at 0.3) when it is created, for each batch anew, and is run
+// several times.  It takes the pair form where a call on all its points would, if that is
+// by the points, and otherwise where nao^2 points nset comes to kPairMinWork over all
+// batches and kPairMinBatchWork per batch: on atom-centred masks its runs then pay for the
+// creation within about ten.  Row / pair form, creation ms and run us: 900 AOs, 1 batch of
+// 45000 points 1.3/1.7, 207/122; 700, 8 of 4000, 3 matrices 1.4/2.0, 326/181; 900, 20 of
+// 2300, 3 1.9/3.5, 578/331 (1 matrix, 1.9e9 per batch: 1.6/3.4, 210/133, 23 runs); 508, 84
+// of 1700, 2 (0.9e9) 4.1/9.8, 794/350; 600, 96 of 1024 (0.4e9) 3.7/10.1, 301/162, 46 runs.
+// On random masks the runs are within 10 % of one another or gain too.  A plan that does
+// not fit in memory takes the row form.  So a plan's last bits can differ from a call's.
 constexpr size_t kPairMinAos = 1024, kPairMinPoints = 8192;
-constexpr double kPairMinWork = 3.5e10;
+constexpr double kPairMinWork = 3.5e10, kPairMinBatchWork = 5e9;
 bool split_pair_form(size_t nao, size_t points, size_t nset);
+// work: the sum of nao^2 points nset over the plan's batches.
+bool split_pair_plan(size_t nao, size_t points, double work, size_t nbatch);
 int split_pair_row_tile(int nsl);  // D rows per item (the MMA N): 80 (6 digits), 64 (7)
 int split_pair_digits();           // digit count (CFGMM_SPLIT_DIGITS, default 7), read per call
 cudaError_t aodmao2rho_split_pair_reset_error(cudaStream_t stream);

@@ -62,5 +62,9 @@ def test_fock_items_are_counted_in_64_bits(objects):
     drive(objects, "fock_share")
 
 
+def test_form_of_split_calls_and_plans(objects):
+    drive(objects, "split_form")
+
+
 def test_host_calls_read_few_error_words(objects):
     drive(objects, "wait_words")
