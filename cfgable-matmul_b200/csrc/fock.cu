@@ -36,6 +36,7 @@
 // weight vector per item and unpermuted atomics; 1.12 ms before the skips.  What
 // bounds it: the FP64 tensor pipe (DMMA; its floor is 0.6 ms), then the L2's atomic
 // units (without the atomics the kernel takes 0.15 ms less).
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -75,6 +76,7 @@ struct FockArgs {
   int vec;  // phi rows and w 16-byte aligned at every tile
   const int4* items;
   int* counters;  // the work counter (64 bits), the item total
+  int ctas;       // that the rule of sharing counts on (the grid may be smaller)
 };
 
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int code) {
@@ -100,7 +102,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
 
   // the items once for each group of weight vectors
   const int items = p.counters[2];
-  const FockShare share = fock_share(items, p.nset, int(gridDim.x));
+  const FockShare share = fock_share(items, p.nset, p.ctas);
   const int per_group = share.per_group;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
@@ -147,8 +149,6 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
       }
     };
     while (ok && it < share.total) {
-      long long next = 0;  // drawn now, needed after this item's copies
-      if (lane == 0) next = (long long)atomicAdd(counter, 1ull);
       const int group = int(it / items);
       const int4 wi = p.items[it - (long long)group * items];
       const int set0 = group * per_group;
@@ -207,7 +207,10 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
           }
         }
       }
-      it = __shfl_sync(0xffffffffu, next, 0);
+      // the next item only now: its chunks are staged two ahead of the products, which
+      // hides the draw, and one drawn earlier would wait behind this one's
+      if (lane == 0) it = (long long)atomicAdd(counter, 1ull);
+      it = __shfl_sync(0xffffffffu, it, 0);
     }
     if (ok && (n == 0 || wait_all(aempty, (n - 1) & 1, 0x6102))) {  // the end mark
       if (lane == 0) {
@@ -429,7 +432,10 @@ cudaError_t fock_compact_fp64(double* vs, const double* ws, const double* ao_lhs
   if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
   if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return err;
-  fock_compact_kernel<<<2 * nsm, THREADS, FOCK_SMEM, stream>>>(a);
+  a.ctas = 2 * nsm;
+  // no more CTAs than there can be items (every one draws from one counter)
+  const double most = double(nblk) * gsub * ((nao + FT - 1) / FT) * nset;
+  fock_compact_kernel<<<int(std::min(most, double(a.ctas))), THREADS, FOCK_SMEM, stream>>>(a);
   return cudaGetLastError();
 }
 
