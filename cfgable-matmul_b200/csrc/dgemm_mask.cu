@@ -80,8 +80,10 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int cod
   return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_mask_error, code));
 }
 
-// NTP: pairs of n8 tiles per item, i.e. 16 * NTP columns.
-template <int NTP>
+// NTP: pairs of n8 tiles per item, i.e. 16 * NTP columns.  kLate: the next item is drawn
+// after this one's copies instead of before them (see draws_late; a template argument,
+// because a branch on it in the kernel cost 3 % of every product).
+template <int NTP, bool kLate>
 __global__ void __launch_bounds__(THREADS, 2)
 dgemm_mask_kernel(const __grid_constant__ MaskArgs p) {
   constexpr int PB = 16 * NTP + 4;
@@ -112,8 +114,8 @@ dgemm_mask_kernel(const __grid_constant__ MaskArgs p) {
     if (lane == 0) it = atomicAdd(p.counter, 1);
     it = __shfl_sync(0xffffffffu, it, 0);
     while (ok && it < total) {
-      int next = 0;  // drawn now, needed after this item's copies
-      if (lane == 0) next = atomicAdd(p.counter, 1);
+      int next = 0;
+      if (!kLate && lane == 0) next = atomicAdd(p.counter, 1);
       const int mt = it % p.tiles_m, piece = it / p.tiles_m;
       const int b = piece / p.nsub, sub = piece % p.nsub;
       const int nb = p.counts[b];
@@ -148,6 +150,7 @@ dgemm_mask_kernel(const __grid_constant__ MaskArgs p) {
           tc::bulk_load(st + TK * PA + r * PB,
                         row >= 0 ? p.b + size_t(row) * p.pitch_b + x0 : p.zero, bb, &full[s]);
       }
+      if (kLate && lane == 0) next = atomicAdd(p.counter, 1);
       it = __shfl_sync(0xffffffffu, next, 0);
     }
     if (ok) {  // the end mark
@@ -292,19 +295,32 @@ int sm_count() {
   return nsm;
 }
 
-template <int NTP>
-cudaError_t launch_mask(const MaskArgs& a, cudaStream_t stream) {
+// Whether the items are so few that up to half of the CTAs get a second one.  Drawn before
+// the first one's copies, the rest went to the CTAs that start first, or both to one SM,
+// while others had none.  16384 columns x 2228, us, drawn before / after the copies: 8 rows
+// (1.2 items to a CTA), 0.3 present 186 / 136, all 550 / 383; 60 rows, 4000 columns (0.3)
+// 160 / 116; but 300 rows (3.5), 0.6 565 / 610, 500 rows, 8000 columns (1.7) 156 / 170.
+bool draws_late(long long items, int ctas) { return items <= ctas + ctas / 2; }
+
+template <int NTP, bool kLate>
+cudaError_t launch_form(const MaskArgs& a, int ctas, cudaStream_t stream) {
   constexpr size_t smem = mask_smem<NTP>();
   static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM");
-  cudaError_t err = cudaFuncSetAttribute(dgemm_mask_kernel<NTP>,
+  cudaError_t err = cudaFuncSetAttribute(dgemm_mask_kernel<NTP, kLate>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (err != cudaSuccess) return err;
+  dgemm_mask_kernel<NTP, kLate><<<ctas, THREADS, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
+template <int NTP>
+cudaError_t launch_mask(const MaskArgs& a, cudaStream_t stream) {
   const int nsm = sm_count();
   if (nsm <= 0) return cudaErrorInvalidDevice;
   const long long total = (long long)a.nblk * a.nsub * a.tiles_m;
-  dgemm_mask_kernel<NTP>
-      <<<unsigned(std::min<long long>(total, 2 * nsm)), THREADS, smem, stream>>>(a);
-  return cudaGetLastError();
+  const int ctas = int(std::min<long long>(total, 2 * nsm));
+  return draws_late(total, ctas) ? launch_form<NTP, true>(a, ctas, stream)
+                                 : launch_form<NTP, false>(a, ctas, stream);
 }
 
 size_t a256(size_t x) { return (x + 255) / 256 * 256; }
@@ -447,8 +463,7 @@ cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int 
   g.cvec = al16(c, ldc) && blk % 2 == 0 && n % 2 == 0;
   g.counter = counter;
   g.compact = compact;
-  switch ((P.sw + 15) / 16) {
-    case 1: return launch_mask<1>(g, stream);
+  switch ((P.sw + 15) / 16) {  // a piece of a block of 32 columns or more has over 16
     case 2: return launch_mask<2>(g, stream);
     case 3: return launch_mask<3>(g, stream);
     default: return launch_mask<4>(g, stream);

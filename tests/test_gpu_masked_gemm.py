@@ -161,3 +161,70 @@ def test_non0tab_compacted_rows_vs_dense(cm, wl, transa, m, n, k, blk, density, 
     assert np.array_equal(c[:, n:], c0[:, n:])
     if density < 1.0:
         assert np.array_equal(c[:, :min(blk, n)], c0[:, :min(blk, n)])
+
+
+@pytest.mark.parametrize("transa,m,n,k,blk,density,pad", [
+    (False, 260, 1400, 600, 200, 0.2, 0),     # five pieces of 40 columns to a block
+    (True, 260, 1450, 600, 145, 0.3, 0),      # odd BLKSIZE: five pieces of 30, B copied
+    (True, 457, 1001, 501, 65, 0.4, 1),       # odd sizes and rows throughout
+    (False, 129, 3200, 500, 32, 0.5, 0),      # two column pairs to an item; one row past a tile
+    (False, 385, 1057, 517, 64, 0.6, 3),      # a last block of 33 columns
+    (True, 384, 1056, 518, 48, 0.6, 2),       # A and B in place
+    (False, 1500, 33, 5000, 48, 1.0, 0),      # one block, wider than C, all of it present
+    (False, 1500, 34, 5000, 2**31 - 1 - 4096, 0.5, 0),  # the widest block there is
+    (False, 300, 2400, 300, 80, 0.0, 0),      # no tile present: C is untouched
+    (False, 128, 96, 20000, 48, 0.3, 0),      # lists of more rows than one pass builds
+    (True, 9, 16384, 1600, 48, 0.4, 1),       # few rows of C
+    (False, 1000, 2000, 640, 40, 0.5, 0),     # both forms enqueued, compacted runs
+    (False, 1000, 2000, 640, 40, 0.97, 0),    # both forms enqueued, dense runs
+])
+def test_non0tab_compacted_form_edges(cm, wl, transa, m, n, k, blk, density, pad):
+    """The compacted form (products of more than 4e8 operations, blocks of 32 columns
+    and more) at the edges of its tiles and in each of its alignment cases.  Absent
+    tiles of B hold NaN, list rows of one, 16 and 17 rows occur, and blocks without a
+    present tile leave C bit for bit."""
+    import torch
+    assert 2.0 * m * n * k > 4e8 and min(blk, n) >= 32
+    rng = np.random.default_rng(m + n)
+    a = rng.uniform(-1, 1, (k, m + pad) if transa else (m, k + pad))
+    b = rng.uniform(-1, 1, (k, n + pad))
+    nblk = -(-n // blk)
+    tab = (rng.random((k, nblk)) < density).astype(np.uint8)
+    if 0.0 < density < 0.9 and nblk > 4:
+        tab[:, 0] = 0
+        for blk_i, rows in zip(range(1, 4), (1, 16, 17)):
+            tab[:, blk_i] = 0
+            tab[rng.choice(k, rows, replace=False), blk_i] = 1
+    on = np.repeat(tab, min(blk, n), axis=1)[:, :n].astype(bool)
+    ref = rng.uniform(-1, 1, (m, n + pad))
+    t = lambda x: torch.from_numpy(x.copy()).cuda()
+    c0, c = ref.copy(), t(ref)
+    ref[:, :n] += (a[:, :m].T if transa else a[:, :k]) @ np.where(on, b[:, :n], 0.0)
+    b[:, :n][~on] = np.nan
+    cm.matmul_non0tab_ex(c, t(a), t(b), m, n, k, a.shape[1], n + pad, n + pad, transa, False,
+                         t(tab), nblk, blk)
+    torch.cuda.synchronize()
+    c = c.cpu().numpy()
+    assert normwise(c, ref) < TOL
+    assert np.array_equal(c[:, n:], c0[:, n:])
+    empty = ~on.any(axis=0)
+    assert np.array_equal(c[:, :n][:, empty], c0[:, :n][:, empty])
+
+
+def test_non0tab_compacted_form_leaves_out_rows_without_a_present_tile(cm):
+    """Row p of op(A)^T meets only the present tiles of row p of B: Inf and NaN there
+    do not reach C when there are none (as in the reference's compaction).  The
+    zero-filled form of smaller products multiplies them with zeros."""
+    import torch
+    rng = np.random.default_rng(4)
+    m, n, k, blk = 300, 1920, 500, 48
+    a, b = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n))
+    tab = (rng.random((k, n // blk)) < 0.3).astype(np.uint8)
+    tab[[3, 77, 499]] = 0
+    ref = a @ np.where(np.repeat(tab, blk, axis=1).astype(bool), b, 0.0)
+    a[:, 3], a[:, 77], a[5, 499] = np.inf, np.nan, -np.inf
+    t = lambda x: torch.from_numpy(x).cuda()
+    c = torch.zeros(m, n, dtype=torch.float64, device="cuda")
+    cm.matmul_non0tab_ex(c, t(a), t(b), m, n, k, k, n, n, False, False, t(tab), n // blk, blk)
+    torch.cuda.synchronize()
+    assert normwise(c.cpu().numpy(), ref) < TOL
