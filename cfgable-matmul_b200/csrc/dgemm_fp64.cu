@@ -560,9 +560,10 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
                 stream);
   // Where the dense form can be the faster one, both are enqueued and the device
   // picks by the share of present tiles: the host does not know it without
-  // waiting for the mask.  Smaller products would pay more for the second form's
-  // launches than it saves.
-  const double share = 2.0 * m * n * k >= 2e9 ? dgemm_mask_max_share(n, blk) : 1.0;
+  // waiting for the mask.  Smaller products (of the dense form's padded rows) would pay
+  // more for the second form's launches than it saves.
+  const double rows = (m + TILE - 1) / TILE * double(TILE);
+  const double share = 2.0 * rows * n * k >= 2e9 ? dgemm_mask_max_share(m, n, blk) : 1.0;
   const size_t wsb = dgemm_mask_workspace(a, b, m, n, k, lda, ldb, transa, blk);
   int* compact = nullptr;  // the choice, outliving the compacted form's scratch
   void* ws = nullptr;

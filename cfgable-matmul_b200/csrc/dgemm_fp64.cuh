@@ -29,7 +29,7 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
 // device word *compact is 0 (the caller then enqueues the dense form gated on
 // it), otherwise it is 1.
 bool dgemm_mask_applies(int m, int n, int k, int blk);
-double dgemm_mask_max_share(int n, int blk);
+double dgemm_mask_max_share(int m, int n, int blk);
 size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,
                             size_t ldb, bool transa, int blk);
 cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int m, int n, int k,

@@ -396,10 +396,20 @@ bool dgemm_mask_applies(int m, int n, int k, int blk) {
 // one up to a share of 0.96 times the used part of the padded width.  Where the
 // whole width is used (BLKSIZE 48, 64) it always runs: with every tile present it
 // loses 1 to 5 %, less than a dense form that is enqueued and mostly not run.
-double dgemm_mask_max_share(int n, int blk) {
-  const int width = std::min(blk, n);
-  const double used = double(width) / padded(width, pieces(width));
-  return used == 1.0 ? 1.0 : 0.96 * used;
+// With few rows of C the other paddings count too: the compacted form's rows go by 128,
+// the dense form's by 64 (three quarters of that is felt: CTAs alone on an SM are faster),
+// and a second round of items that is not full takes as long as the first, unless it is
+// spread (draws_late).  16384 columns x 2228, us at 0.3, 0.6 and 1.0 present against the dense
+// form: 40 rows, BLKSIZE 33 (1.7 rounds) 357, 544, - against 330; 70 rows 362, 550, - against
+// 508; 130 rows 471, 765, - against 690; 40 rows, BLKSIZE 56 141, 240, - against 248.
+double dgemm_mask_max_share(int m, int n, int blk) {
+  const int width = std::min(blk, n), nsub = pieces(width);
+  const double used = double(width) / padded(width, nsub);
+  if (used == 1.0) return 1.0;
+  const double rows = double((m + 63) / 64 * 64) / ((m + 127) / 128 * 128);
+  const double round = double(((long long)n + blk - 1) / blk * nsub * ((m + TM - 1) / TM)) /
+                       (2.0 * std::max(sm_count(), 1));
+  return 0.96 * used * (0.25 + 0.75 * rows) * (round > 1.5 && round < 2.0 ? 0.5 * round : 1.0);
 }
 
 size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,

@@ -177,6 +177,8 @@ def test_non0tab_compacted_rows_vs_dense(cm, wl, transa, m, n, k, blk, density, 
     (True, 9, 16384, 1600, 48, 0.4, 1),       # few rows of C
     (False, 1000, 2000, 640, 40, 0.5, 0),     # both forms enqueued, compacted runs
     (False, 1000, 2000, 640, 40, 0.97, 0),    # both forms enqueued, dense runs
+    (False, 40, 16384, 1000, 40, 0.2, 0),     # both enqueued for few rows, compacted runs
+    (False, 40, 16384, 1000, 40, 0.8, 0),     # and dense
 ])
 def test_non0tab_compacted_form_edges(cm, wl, transa, m, n, k, blk, density, pad):
     """The compacted form (products of more than 4e8 operations, blocks of 32 columns
