@@ -818,7 +818,7 @@ cudaError_t prepare_form(const T* x, size_t ld, bool rows_contig, int rows, int 
                          cudaStream_t s, Mask mask) {
   using Bits = typename Magnitude<T>::Bits;
   Bits* maxima = static_cast<Bits*>(top);
-  const bool scan = size_t(rows) * k * sizeof(T) <= kScanBytes;
+  bool scan = size_t(rows) * k * sizeof(T) <= kScanBytes;
   if (rows_contig) {
     if (!scan) {
       maxima_rows<T><<<rows, 256, 0, s>>>(x, ld, k, maxima);
@@ -833,6 +833,11 @@ cudaError_t prepare_form(const T* x, size_t ld, bool rows_contig, int rows, int 
     }
     return cudaGetLastError();
   }
+  // Few rows over a long k: the scan's clusters are few and walk many tiles each, one
+  // after the other.  Both operands by columns, us the call with the scan / without:
+  // 64 x 64 x 60000 (59 tiles to a CTA) 370 / 220, 200 x 200 x 16000 131 / 118, 30 x 30 x
+  // 13000 (13 tiles) 78 / 61, 500 x 500 x 13000 in f32 126 / 120.
+  if ((rows + 15) / 16 * 8 < 592 && k > 8 * 12 * 128) scan = false;
   int parts = 8;
   while (parts > (k + 127) / 128) parts /= 2;
   cudaLaunchConfig_t cfg{};

@@ -194,3 +194,55 @@ def test_split_device_call_in_cuda_graph(cm):
     torch.cuda.synchronize()
     assert torch.equal(c, 2 * ref)
     del graph
+
+
+def test_one_cta_form_of_the_int8_gemm(cm):
+    """CFGMM_GEMM_PAIR=0 runs every INT8 tile on one CTA: the same residues, so the same
+    bits as the form on pairs of SMs, with ragged rows, columns and K."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    tmp = os.environ.get("TMPDIR", "/tmp")
+    code = ("import importlib,sys,numpy as np,torch; sys.path.insert(0,'.');"
+            "cm=importlib.import_module('cfgable-matmul_b200'); r=np.random.default_rng(9); out=[]\n"
+            "for m,n,k in ((1,1,1),(129,257,131),(300,515,1000)):\n"
+            "  a,b=r.uniform(-1,1,(m,k)),r.uniform(-1,1,(k,n)); c=np.zeros((m,n))\n"
+            "  cm.matmul_ex(c,a,b,m,n,k,k,n,n,False,False,cm.PREC_OZAKI_INT8)\n"
+            "  assert np.abs(c-a@b).max()<1e-12*np.abs(a@b).max(); out.append(c.ravel())\n"
+            "np.save(sys.argv[1],np.concatenate(out))")
+    outs = []
+    for pair in ("0", "1"):
+        path = os.path.join(tmp, f"cfgmm_gemm_pair{pair}.npy")
+        subprocess.run([sys.executable, "-c", code, path], cwd=root, check=True,
+                       env=dict(os.environ, CFGMM_GEMM_PAIR=pair))
+        outs.append(np.load(path))
+    assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("transa,transb", [(False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [
+    (33, 65, 12288),   # the longest k whose columns are scanned in one launch
+    (33, 65, 12289),   # the shortest with the maxima in a kernel of their own
+    (1, 17, 30001),
+])
+def test_small_operands_with_long_contractions(cm, transa, transb, m, n, k):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(k + m)
+    u = lambda *s: torch.rand(*s, generator=g, device="cuda", dtype=torch.float64) * 2 - 1
+    a, b = u(k, m) if transa else u(m, k), u(n, k) if transb else u(k, n)
+    opa, opb = (a.t() if transa else a), (b.t() if transb else b)
+    opa[0].mul_(2.0 ** 60)
+    opb[:, n - 1].zero_()
+    ref = opa @ opb
+    for dtype, tol in ((torch.float64, 1e-12), (torch.float32, 2e-7)):
+        x, y = a.to(dtype).contiguous(), b.to(dtype).contiguous()
+        c = torch.zeros(m, n, device="cuda", dtype=dtype)
+        call = cm.matmul_ex if dtype == torch.float64 else cm.matmul_f32
+        call(c, x, y, m, n, k, x.shape[1], y.shape[1], n, transa, transb, cm.PREC_OZAKI_INT8)
+        want = ref if dtype == torch.float64 else (
+            (x.t() if transa else x).double() @ (y.t() if transb else y).double())
+        torch.cuda.synchronize()
+        for i in range(m):  # row by row: the first is 2^60 times the others
+            assert normwise(c[i].double().cpu().numpy(), want[i].cpu().numpy()) < tol
+        assert not c[:, n - 1].any()
