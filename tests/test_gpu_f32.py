@@ -100,3 +100,35 @@ def test_f32_device_tensors(cm, oracle, wl):
     assert normwise(rho.cpu().numpy().astype(np.float64), ref) < 1e-7
     cref = a.double().cpu().numpy() @ b.double().cpu().numpy()
     assert normwise(c.cpu().numpy().astype(np.float64), cref) < 1e-7
+
+
+@pytest.mark.parametrize("transa,transb,m,n,k", [
+    (False, False, 3301, 67, 3203),   # A past 40 MB by rows
+    (True, False, 67, 3301, 3203),    # B past 40 MB by columns
+    (True, True, 3301, 3259, 3219),   # both, the other way round
+])
+def test_matmul_f32_split_of_large_operands(cm, transa, transb, m, n, k):
+    """f32 operands past 40 MB have their maxima from a kernel of their own; some rows
+    and columns are zero or far larger than the others."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    u = lambda *s: torch.rand(*s, generator=g, device="cuda", dtype=torch.float32) * 2 - 1
+    a = u(k, m) if transa else u(m, k)
+    b = u(n, k) if transb else u(k, n)
+    opa, opb = (a.t() if transa else a), (b.t() if transb else b)
+    opa[5].zero_()
+    opa[m - 1].mul_(2.0 ** 40)
+    opb[:, 7].zero_()
+    opb[:, n - 1].mul_(2.0 ** -50)
+    c = torch.zeros(m, n, device="cuda")
+    cm.matmul_f32(c, a, b, m, n, k, a.shape[1], b.shape[1], n, transa, transb,
+                  precision=cm.PREC_OZAKI_INT8)
+    ref = opa.double() @ opb.double()
+    scale = opa.abs().amax(1, keepdim=True).double() * opb.abs().amax(0, keepdim=True).double()
+    torch.cuda.synchronize()
+    # the output's rounding and 26-bit operands: 2 k 2^-27 of the largest product each
+    bound = ref.abs() * 2.0 ** -24 * 1.001 + scale * (k * 2.0 ** -26)
+    assert bool(((c.double() - ref).abs() <= bound).all())
+    assert normwise((c.double() / scale.clamp_min(1e-300)).cpu().numpy(),
+                    (ref / scale.clamp_min(1e-300)).cpu().numpy()) < 2e-7
+    assert not c[5].any() and not c[:, 7].any()
