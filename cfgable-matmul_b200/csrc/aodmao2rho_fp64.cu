@@ -218,7 +218,9 @@ aodm_build_items(const int* __restrict__ counts, int nblk, int gsub, int4* __res
   }
   if (lane == 31) warp_tot[warp] = blocks;
   __syncthreads();
-  for (int w = 0; w < warp; ++w) blocks += warp_tot[w];  // blocks with >= rank tiles
+  // of the warps before, by lanes (a loop over them took 1 us of the two scans)
+  auto before = [&] { return __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0); };
+  blocks += before();  // blocks with >= rank tiles
   int mine = blocks;
   if (tid == 0)  // rank RANKS: every tile from the RANKS-th on
     for (int b = 0; mine && b < nblk; ++b) mine += max(0, (counts[b] + TU - 1) / TU - RANKS);
@@ -231,7 +233,7 @@ aodm_build_items(const int* __restrict__ counts, int nblk, int gsub, int4* __res
   }
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  for (int w = 0; w < warp; ++w) incl += warp_tot[w];
+  incl += before();
   start[rank] = (incl - mine) * gsub;
   if (tid == 1023) counters[ncounters] = incl * gsub;  // rank 1: the total
   __syncthreads();
