@@ -422,8 +422,9 @@ int gemm_host(double* c, size_t c_len, const double* a, size_t a_len, const doub
   CFGMM_CUDA(st->stage.upload(db, b, ex.b * 8, st->stream));
   if (masked) CFGMM_CUDA(cudaMemcpyAsync(dt, mk.tab, tab_ext, cudaMemcpyHostToDevice, st->stream));
   if (split) {
-    // C goes up on the copy stream once A and B are in, while the residues
-    // and the INT8 GEMM run; the reconstruction waits for it
+    // C goes up on the copy stream once A and B are in and the reconstruction waits for
+    // it: from pinned memory while the residues and the INT8 GEMM run, from pageable
+    // memory before them (the upload returns when C has been read)
     if ((rc = ensure_copy_stream(st)) != CFGMM_OK) return rc;
     CFGMM_CUDA(cudaEventRecord(st->ab_done, st->stream));
     CFGMM_CUDA(cudaStreamWaitEvent(st->copy, st->ab_done, 0));
@@ -514,6 +515,12 @@ int aodm_device_status(bool split) {
 // How the phi tables of a host call go up: from pageable memory only the present
 // tiles, packed by the copying threads (the kernels read no others), when they are at
 // most three quarters of a table of 4 MB or more.  `offsets` empty: whole tables.
+// Tables of 64 MB and more go so too, all of them before the contraction, and not in
+// blocks that overlap it (aodm_host_blocked): fewer bytes win at every size measured.  ms in
+// blocks / tiles at 0.05, 0.3 and 0.7 present: 2228 AOs, 16384 points, 3 matrices (292 MB)
+// 15.9/4.6, 16.5/6.7, 20.0/12.4, split 16.3/4.8, 16.8/6.5, 18.1/10.1; 40000 points (713 MB)
+// 23.4/5.1, 25.2/10.6, 33.3/24.8; 1000 AOs, 100000 points, 1 matrix 22.6/2.8, 23.3/8.0,
+// 25.8/19.1.
 struct PhiUpload {
   size_t elems = 0;  // of a table's present tiles
   std::vector<unsigned long long> offsets;

@@ -17,16 +17,7 @@ __device__ __forceinline__ void cp_async_8(void* smem_dst, const void* gmem_src,
                : "memory");
 }
 
-// 16-byte asynchronous copy (L2 only), zero-filled when `valid` is false.
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src, bool valid) {
-  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  const int src_size = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem_src),
-               "r"(src_size)
-               : "memory");
-}
-
-// 16-byte asynchronous copy of which the first `bytes` (0, 8 or 16) are read
+// 16-byte asynchronous copy (L2 only) of which the first `bytes` (0, 8 or 16) are read
 // from `src`; the rest of the destination is zero-filled.
 __device__ __forceinline__ void cp_async_16_n(void* smem_dst, const void* gmem_src, int bytes) {
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));

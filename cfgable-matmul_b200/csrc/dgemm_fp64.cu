@@ -274,8 +274,8 @@ dgemm_kernel(const __grid_constant__ GemmArgs<T> p) {
           gemm_smem[row_of(mt, h) * CP + col_of(j, e)] = acc[mt][j][2 * h + e];
   cluster.sync();
   // each CTA adds its rows over the parts, in their order; a thread's reads of the
-  // other CTAs' memory are all under way at once (in a loop over the parts, one after another, whose
-  // registers also spilled in the main loop: 1000^3 91 -> 87 us, 3000 x 3000 x 300 196
+  // other CTAs' memory are all under way at once (in a loop over the parts, one after
+  // another, whose registers also spilled in the main loop: 1000^3 91 -> 87 us, 3000 x 3000 x 300 196
   // -> 185, 3000^3 1.669 -> 1.648 ms; calls of a few tiles are bound by their launch)
   const int rows = TILE / p.splits;
   double v[2][8];
@@ -350,11 +350,10 @@ pack_rows(double* __restrict__ dst, const double* __restrict__ src, size_t ld, i
 }
 
 // dst[j][p] = src[p * ld + j] for p < k (0 for k <= p < kpad), j < cols: the
-// transpose into a K-contiguous operand, through a 32 x 32 shared tile.  With
-// a mask, element (p, j) is zero unless tab[p * ldtab + j / blk].
+// transpose into a K-contiguous operand, through a 32 x 32 shared tile.
 __global__ void __launch_bounds__(256)
 pack_transpose(double* __restrict__ dst, const double* __restrict__ src, size_t ld, int cols,
-               int k, int kpad, const uint8_t* __restrict__ tab, size_t ldtab, int blk, Gate gate) {
+               int k, int kpad, Gate gate) {
   if (gate.closed()) return;
   __shared__ double t[32][33];
   const int j0 = blockIdx.x * 32, p0 = blockIdx.y * 32;
@@ -362,12 +361,7 @@ pack_transpose(double* __restrict__ dst, const double* __restrict__ src, size_t 
 #pragma unroll
   for (int i = 0; i < 32; i += 8) {
     const int p = p0 + ty + i, j = j0 + tx;
-    double v = 0.0;
-    if (p < k && j < cols) {
-      v = src[size_t(p) * ld + j];
-      if (tab && !tab[size_t(p) * ldtab + j / blk]) v = 0.0;
-    }
-    t[ty + i][tx] = v;
+    t[ty + i][tx] = p < k && j < cols ? src[size_t(p) * ld + j] : 0.0;
   }
   __syncthreads();
 #pragma unroll
@@ -376,7 +370,6 @@ pack_transpose(double* __restrict__ dst, const double* __restrict__ src, size_t 
     if (j < cols && p < kpad) dst[size_t(j) * kpad + p] = t[tx][ty + i];
   }
 }
-
 
 template <bool TA, bool TB, class T>
 cudaError_t launch_t(const GemmArgs<T>& p, cudaStream_t stream) {
@@ -547,7 +540,7 @@ cudaError_t dgemm_pack_kmajor(double* dst, const double* a, size_t lda, int m, i
                                                                          gate);
   else
     pack_transpose<<<dim3((k + 31) / 32, (pitch + 31) / 32), 256, 0, stream>>>(
-        dst, a, lda, k, m, pitch, nullptr, 0, 1, gate);
+        dst, a, lda, k, m, pitch, gate);
   return cudaGetLastError();
 }
 

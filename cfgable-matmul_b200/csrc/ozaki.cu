@@ -105,7 +105,6 @@ OzakiPlan ozaki_plan(int k, int nmod, int min_bits) {
   for (int l = 0; l < nmod; ++l) {
     p.mod[l] = kModuli[l];
     p.inv_f[l] = 1.0f / float(kModuli[l]);
-    p.inv_d[l] = 1.0 / double(kModuli[l]);
   }
   // parts of W_p (the largest: the last pair's, or the last modulus alone) and M:
   // sum_p |t_p| (W_p >> T1) <= 8 2^23 2^26 = 2^52, and the same of the middle parts

@@ -8,8 +8,8 @@
 
 namespace cfgmm {
 
-// Exact INT32 accumulation needs k * 128 * 128 < 2^31; the epilogue's
-// float-quotient reduction is exact (after two corrections) for |acc| < 2^30.
+// Exact INT32 accumulation needs k * 128 * 128 < 2^31; the epilogue's quotient is exact
+// for |acc| <= 2^30 (gemm_i8.cu, mods32).
 constexpr int kOzakiMaxK = 65536;
 // Default operand precision (bits kept relative to each row / column max).
 constexpr int kOzakiMinBits = 46;
@@ -21,7 +21,6 @@ struct OzakiPlan {
   int alpha, beta;      // bits of the scaled integer operands A', B'
   int mod[kMaxModuli];  // moduli, 256 first
   float inv_f[kMaxModuli];
-  double inv_d[kMaxModuli];
   // CRT by pairs of moduli (the last one alone when N is odd, with m = 1):
   // C' = sum_p t_p W_p mod M with W_p = M / (m m') and t_p = c[0] r + c[1] r',
   // |t_p| < 2^23.  W_p and M are split at 2^T1 and 2^T2.
