@@ -235,3 +235,32 @@ def test_plan_symmetric_d_with_two_phi_arrays(cm, wl, precision):
     for b, d in zip(bs, dev):
         assert normwise(d[0].cpu().numpy(), _single(cm, torch, b, dms, 64, precision)) < 1e-12
     plan.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_plan_destroyed_with_runs_in_flight(cm, wl, tmp_path, monkeypatch, precision):
+    """Destroying a plan waits for its runs, on whatever stream they are: the stream is
+    idle afterwards, and every run has added its density although the memory that the plan
+    gave back is allocated and written at once."""
+    import torch
+    monkeypatch.setenv("CFGMM_AUTOTUNE_CACHE", str(tmp_path / "tune.txt"))
+    rng = np.random.default_rng(7)
+    nao, ngrid, blk, runs = 600, 20000, 64, 20
+    tab = (rng.random((nao, -(-ngrid // blk))) < 0.4).astype(np.uint8)
+    phi = np.where(wl.expand_mask(tab, ngrid, blk), rng.standard_normal((nao, ngrid)), 0.0)
+    dms = wl.sym_dms(rng, 1, nao)
+    b = dict(lhs=phi, rhs=phi, tab=tab, nset=1, rho0=np.zeros((1, ngrid)), ngrid=ngrid)
+    dev, ddms = _device(torch, [b], dms)
+    plan = cm.AodmPlan(dev, ddms, blksize=blk, precision=precision, tune=False)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for _ in range(runs):
+            plan.run()
+    plan.close()
+    assert stream.query()
+    other = cm.AodmPlan(dev, ddms, blksize=blk, precision=1 - precision, tune=False)
+    torch.cuda.synchronize()
+    want = runs * _single(cm, torch, b, dms, blk)
+    assert normwise(dev[0][0].cpu().numpy(), want) < (1e-12 if precision else 1e-13)
+    other.close()
