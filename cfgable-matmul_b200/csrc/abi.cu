@@ -303,8 +303,11 @@ int check_mask(const GemmMask& mk, size_t n, size_t k, uint8_t transb, size_t* t
 // up first and its residues are formed once.  In FP64 the work bounds the
 // call: 8 equal blocks of columns of C and op(B), A going up first (186 MB
 // instead of 505 MB at the headline shape), so that the work starts early and
-// each block's upload takes about as long as the previous block's work.  The device buffers keep the host layouts; every element of C is
-// computed from the same row of op(A) and column of op(B) as in one call.
+// each block's upload takes about as long as the previous block's work.  The device
+// buffers keep the host layouts; every element of C is computed from the same row of
+// op(A) and column of op(B) as in one call.  All of this holds for pinned memory: to and
+// from pageable memory the copies take the host's time, and C's parts come back by the
+// driver's path, which waits for each block.
 int gemm_host_blocked(DeviceState* st, double* c, const double* a, const double* b, size_t m,
                       size_t n, size_t k, size_t lda, size_t ldb, size_t ldc, bool transa,
                       bool transb, bool split, int nmod, double* da, double* db, double* dc,
