@@ -953,20 +953,26 @@ cudaError_t ozaki_dgemm(T* c, const T* a, const T* b, int m, int n, int k,
   // op(A) rows are i (k contiguous unless transa); op(B) "rows" are j
   // (k contiguous only when transb).
   cudaError_t err = cudaSuccess;
-  // With both operands to prepare, A's kernel runs on a side stream beside B's:
+  // With both operands to prepare, one's kernel runs on a side stream beside the other's:
   // their phases are bound by instruction issue (residues) and by memory (the
   // scan for the exponents), so the two overlap.  The side stream joins back before the
-  // GEMM (the fork and join are events, so a stream capture follows them).
+  // GEMM (the fork and join are events, so a stream capture follows them).  The side
+  // stream starts later, and an operand by rows goes there: clusters of an operand by
+  // columns that start behind its CTAs share fewer SMs.  A by columns with B by rows, us
+  // with B / A on the side: 300 x 300 x 6000 63 / 97, 200 x 200 x 3000 36 / 59, 1500 x 700
+  // x 2500 100 / 121, 2000 x 2000 x 2000 in f32 123 / 133; A by rows with B by columns
+  // the other way round; two of one kind alike.
   SideScope side((!reuse_a && !reuse_b) ? side_stream() : nullptr, stream);
   if ((err = side.fork()) != cudaSuccess) return err;
-  const cudaStream_t sa = side.stream();
+  const bool b_aside = transa && transb;
+  const cudaStream_t sa = b_aside ? stream : side.stream(), sb = b_aside ? side.stream() : stream;
   if (!reuse_a) {
     err = prepare(a, lda, !transa, m, k, L.kpad, plan.alpha, ws + L.top_a, ea,
                   a_res, ra, sa);
     if (err != cudaSuccess) return err;
   }
   if (!reuse_b) {
-    err = prepare(b, ldb, transb, n, k, L.kpad, plan.beta, ws + L.top_b, eb, b_res, ra, stream,
+    err = prepare(b, ldb, transb, n, k, L.kpad, plan.beta, ws + L.top_b, eb, b_res, ra, sb,
                   Mask{tab, ldtab, blk > 0 ? blk : 1});
     if (err != cudaSuccess) return err;
   }

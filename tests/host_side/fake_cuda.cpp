@@ -29,6 +29,8 @@ int free_races = 0;
 int long_device = -1;
 int bad_launches = 0;
 std::string last_bad;
+bool record = false;
+std::vector<std::pair<std::string, cudaStream_t>> launches;
 
 namespace {
 std::mutex mu;
@@ -77,6 +79,7 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t smem, cudaStream
     last_bad = names[f];
     return ret(empty ? cudaErrorInvalidConfiguration : cudaErrorInvalidValue);
   }
+  if (record) launches.emplace_back(names[f], stream);
   CUstream_st* s = of(stream);
   s->work = true;
   if (long_device == device) {

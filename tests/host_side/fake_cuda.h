@@ -2,6 +2,8 @@
 #pragma once
 #include <cstddef>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include <cuda_runtime_api.h>
 
@@ -21,6 +23,9 @@ bool running();  // such a kernel has been launched
 // granted on the launching device return an error, as the runtime's do.
 extern int bad_launches;
 extern std::string last_bad;
+// With `record`, every launch: the kernel's (mangled) name and its stream.
+extern bool record;
+extern std::vector<std::pair<std::string, cudaStream_t>> launches;
 
 }  // namespace fake
 

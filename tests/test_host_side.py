@@ -68,3 +68,7 @@ def test_form_of_split_calls_and_plans(objects):
 
 def test_host_calls_read_few_error_words(objects):
     drive(objects, "wait_words")
+
+
+def test_residues_by_rows_are_formed_aside(objects):
+    drive(objects, "residue_streams")
