@@ -400,16 +400,16 @@ cudaError_t launch_t(const GemmArgs<T>& p, cudaStream_t stream) {
 // and 8 parts the choice is within 0.8 % of the fastest on average and 9 % at worst;
 // 130 x 130 x 5000 takes 269, 146, 75, 42 us with 1, 2, 4, 8 parts, 1200 x 1500 x 1000
 // 166, 154, 142, 148, 2000 x 2000 x 500 146, 160, 176, 204.
-int choose_splits(long long tiles, int steps, int nsm) {
-  int best = 1;
-  double least = 0.0;
+struct Splits {
+  int count;
+  double time;  // the model's, in units of 0.56 us
+};
+Splits choose_splits(long long tiles, int steps, int nsm) {
+  Splits best{1, 0.0};
   for (int s = 1; s <= 8 && (s == 1 || steps >= 2 * s); s *= 2) {
     const double mean = double(tiles * s) / nsm, most = double((tiles * s + nsm - 1) / nsm);
     const double t = std::max(0.5 * (most + mean) + 0.5, 3.0) * (double(steps) / s + 2.0);
-    if (s == 1 || t < least) {
-      best = s;
-      least = t;
-    }
+    if (s == 1 || t < best.time) best = Splits{s, t};
   }
   return best;
 }
@@ -460,12 +460,12 @@ cudaError_t gemm(T* c, const T* a, const T* b, int m, int n, int k, size_t lda, 
   p.ldc = ldc;
   p.tiles_m = int(tiles_m);
   p.tiles_n = int(tiles_n);
-  p.splits = choose_splits(tiles_m * tiles_n, (k + TK - 1) / TK, nsm);
+  p.splits = choose_splits(tiles_m * tiles_n, (k + TK - 1) / TK, nsm).count;
   p.gate = gate;
   const int ar = transa ? k : m, ac = transa ? m : k, br = transb ? n : k, bc = transb ? k : n;
   constexpr bool widen = !std::is_same<T, double>::value;
-  const bool pa = widen || (!al16(a, lda) && pack_pays(m, n, k, double(m) * k));
-  const bool pb = widen || ((tab || !al16(b, ldb)) && pack_pays(m, n, k, double(n) * k));
+  bool pa = widen || (!al16(a, lda) && pack_pays(m, n, k, double(m) * k));
+  bool pb = widen || ((tab || !al16(b, ldb)) && pack_pays(m, n, k, double(n) * k));
   const int apitch = (ac + 1) / 2 * 2, bpitch = (bc + 1) / 2 * 2;
   const double *da = nullptr, *db = nullptr;
   if constexpr (!widen) {
@@ -475,17 +475,26 @@ cudaError_t gemm(T* c, const T* a, const T* b, int m, int n, int k, size_t lda, 
   double* ws = nullptr;
   if (pa || pb) {
     const size_t an = pa ? size_t(ar) * apitch : 0, bn = pb ? size_t(br) * bpitch : 0;
-    if ((err = cudaMallocAsync(reinterpret_cast<void**>(&ws), (an + bn) * 8, stream)) !=
-        cudaSuccess)
-      return err;
+    err = cudaMallocAsync(reinterpret_cast<void**>(&ws), (an + bn) * 8, stream);
+    if (err == cudaErrorMemoryAllocation && !widen) {  // it runs without the copies too
+      cudaGetLastError();
+      err = cudaSuccess;
+      ws = nullptr;
+      pa = pb = false;
+    }
+    if (err != cudaSuccess) return err;
+    auto grid = [&](int pitch, int rows) {  // gated: few CTAs, soon over if they do not run
+      const int across = (pitch + 1023) / 1024;
+      return dim3(across, std::min(rows, gate.word ? 1024 / across + 1 : 65535));
+    };
     if (pa) {
-      pack_aligned<<<dim3((apitch + 1023) / 1024, std::min(ar, 65535)), 256, 0, stream>>>(
+      pack_aligned<<<grid(apitch, ar), 256, 0, stream>>>(
           ws, apitch, a, lda, ar, ac, nullptr, 0, 1, gate);
       da = ws;
       lda = apitch;
     }
     if (pb) {
-      pack_aligned<<<dim3((bpitch + 1023) / 1024, std::min(br, 65535)), 256, 0, stream>>>(
+      pack_aligned<<<grid(bpitch, br), 256, 0, stream>>>(
           ws + an, bpitch, b, ldb, br, bc, tab, ldtab, blk, gate);
       db = ws + an;
       ldb = bpitch;
@@ -513,6 +522,22 @@ cudaError_t gemm(T* c, const T* a, const T* b, int m, int n, int k, size_t lda, 
     if (err == cudaSuccess) err = e2;
   }
   return err;
+}
+
+// The dense form of a masked product (in-place copies of B ask for the mask 8 bytes at a
+// time): the model of choose_splits and the copies, within 15 % of 22 shapes of 50 us to 5 ms.
+double masked_dense_us(int m, int n, int k, bool transa) {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      nsm <= 0) {
+    cudaGetLastError();
+    nsm = 148;
+  }
+  const long long tiles = (long long)((m + TILE - 1) / TILE) * ((n + TILE - 1) / TILE);
+  const double us = 0.56 * choose_splits(tiles, (k + TK - 1) / TK, nsm).time;
+  if (pack_pays(m, n, k, double(n) * k)) return 1.03 * us + 16.0 * n * k / 5.5e6 + 6.0;
+  return (transa ? 1.4 : 1.28) * us + 12.0;
 }
 
 }  // namespace
@@ -551,12 +576,21 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
   if (!dgemm_mask_applies(m, n, k, blk))
     return gemm(c, a, b, m, n, k, lda, ldb, ldc, transa, false, tab, ldtab, blk, Gate{nullptr, 0},
                 stream);
-  // Where the dense form can be the faster one, both are enqueued and the device
-  // picks by the share of present tiles: the host does not know it without
-  // waiting for the mask.  Smaller products (of the dense form's padded rows) would pay
-  // more for the second form's launches than it saves.
+  // Where the dense form can be the faster one, both are enqueued and the device picks by
+  // the share of present tiles: the host does not know it without waiting for the mask.
+  // The second form's launches cost 3 to 10 us, so not for smaller products (of the dense
+  // form's padded rows): at 0.05 present 84 -> 95 us at 2228 x 2000 x 2228, with all tiles
+  // present 821 -> 704.  Where the lists and copies leave the compacted form no gain above
+  // a share of 0.15, the dense one runs alone (64 x 16384 x 500, BLKSIZE 33, 0.3 present: 93
+  // -> 59 us).
+  const double dense = masked_dense_us(m, n, k, transa);
+  const MaskTimes t = dgemm_mask_times(a, b, m, n, k, lda, ldb, transa, blk);
+  if (dense <= t.lists + t.copies + 0.15 * t.products)
+    return gemm(c, a, b, m, n, k, lda, ldb, ldc, transa, false, tab, ldtab, blk, Gate{nullptr, 0},
+                stream);
   const double rows = (m + TILE - 1) / TILE * double(TILE);
-  const double share = 2.0 * rows * n * k >= 2e9 ? dgemm_mask_max_share(m, n, blk) : 1.0;
+  double share = (dense - t.copies) / t.products;  // up to which the compacted form is faster
+  if (2.0 * rows * n * k < 2e9) share = 1.0;
   const size_t wsb = dgemm_mask_workspace(a, b, m, n, k, lda, ldb, transa, blk);
   int* compact = nullptr;  // the choice, outliving the compacted form's scratch
   void* ws = nullptr;

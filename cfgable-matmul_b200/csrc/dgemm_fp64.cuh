@@ -22,14 +22,17 @@ cudaError_t dgemm_fp64_non0tab(double* c, const double* a, const double* b, int 
                                const uint8_t* tab, size_t ldtab, int blk, cudaStream_t stream);
 
 // The masked GEMM on each column block's compacted rows (dgemm_mask.cu).
-// dgemm_mask_applies: the shapes it takes; dgemm_mask_max_share: the share of
-// present tiles up to which it is faster than the dense form (>= 1: always).
-// dgemm_mask_compact enqueues the lists, the choice and the kernel: where more
+// dgemm_mask_applies: the shapes it takes; dgemm_mask_times: what it takes, in us (its
+// products with every tile present).  dgemm_mask_compact enqueues the lists, the choice and the kernel: where more
 // than max_share (< 1) of the tiles is present nothing is added to C and the
 // device word *compact is 0 (the caller then enqueues the dense form gated on
 // it), otherwise it is 1.
 bool dgemm_mask_applies(int m, int n, int k, int blk);
-double dgemm_mask_max_share(int m, int n, int blk);
+struct MaskTimes {
+  double lists, copies, products;
+};
+MaskTimes dgemm_mask_times(const double* a, const double* b, int m, int n, int k, size_t lda,
+                           size_t ldb, bool transa, int blk);
 size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,
                             size_t ldb, bool transa, int blk);
 cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int m, int n, int k,

@@ -268,7 +268,8 @@ mask_setup(const int* __restrict__ counts, int nblk, int k, double max_share, in
 }
 
 // The present tiles of B into rows of nblk * blk_pitch columns (blk_pitch = blk
-// rounded up to even): dst[p][b * blk_pitch + j] = src[p*ld + b*blk + j].
+// rounded up to even): dst[p][b * blk_pitch + j] = src[p*ld + b*blk + j].  Four rows at a
+// time (one: 100 x 16384 x 3000, odd rows, 0.3 present 430 us the call, now 257).
 __global__ void __launch_bounds__(256)
 pack_tiles(double* __restrict__ dst, const double* __restrict__ src, size_t ld, int n, int k,
            int blk, int blk_pitch, int nblk, const uint8_t* __restrict__ tab, size_t ldtab,
@@ -280,9 +281,21 @@ pack_tiles(double* __restrict__ dst, const double* __restrict__ src, size_t ld, 
   const int b = int(x / blk_pitch), j = int(x % blk_pitch);
   const int col = b * blk + j;
   const bool in = j < blk && col < n;
-  for (int p = blockIdx.y; p < k; p += gridDim.y)
-    if (tab[size_t(p) * ldtab + b])
-      dst[size_t(p) * cols + x] = in ? src[size_t(p) * ld + col] : 0.0;
+  for (int p0 = blockIdx.y; p0 < k; p0 += 4 * gridDim.y) {
+    bool on[4];
+    double v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int p = p0 + i * gridDim.y;
+      on[i] = p < k && tab[size_t(p) * ldtab + b];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[i] = on[i] && in ? src[size_t(p0 + i * gridDim.y) * ld + col] : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (on[i]) dst[size_t(p0 + i * gridDim.y) * cols + x] = v[i];
+  }
 }
 
 int sm_count() {
@@ -389,27 +402,25 @@ bool dgemm_mask_applies(int m, int n, int k, int blk) {
          nblk * (blk + 1ll) < (1ll << 31) && k <= 500000 && m <= 2000000;
 }
 
-// A piece costs the time of its padded width.  Measured at 2228 x 8000 x 2228 (the
-// dense form takes 2.51 ms there whatever is present): BLKSIZE 33, 33 of 48 columns
-// used, 2.35 ms at 60 % present and 2.89 at 75 %; BLKSIZE 40 (of 48) 2.31 at 75 %
-// and 2.77 at 90 %; 56 (of 64) 2.22 and 2.64.  So the compacted form is the faster
-// one up to a share of 0.96 times the used part of the padded width.  Where the
-// whole width is used (BLKSIZE 48, 64) it always runs: with every tile present it
-// loses 1 to 5 %, less than a dense form that is enqueued and mostly not run.
-// With few rows of C the other paddings count too: the compacted form's rows go by 128,
-// the dense form's by 64 (three quarters of that is felt: CTAs alone on an SM are faster),
-// and a second round of items that is not full takes as long as the first, unless it is
-// spread (draws_late).  16384 columns x 2228, us at 0.3, 0.6 and 1.0 present against the dense
-// form: 40 rows, BLKSIZE 33 (1.7 rounds) 357, 544, - against 330; 70 rows 362, 550, - against
-// 508; 130 rows 471, 765, - against 690; 40 rows, BLKSIZE 56 141, 240, - against 248.
-double dgemm_mask_max_share(int m, int n, int blk) {
-  const int width = std::min(blk, n), nsub = pieces(width);
-  const double used = double(width) / padded(width, nsub);
-  if (used == 1.0) return 1.0;
-  const double rows = double((m + 63) / 64 * 64) / ((m + 127) / 128 * 128);
-  const double round = double(((long long)n + blk - 1) / blk * nsub * ((m + TM - 1) / TM)) /
-                       (2.0 * std::max(sm_count(), 1));
-  return 0.96 * used * (0.25 + 0.75 * rows) * (round > 1.5 && round < 2.0 ? 0.5 * round : 1.0);
+// What the compacted form takes, for the choice between it and the dense one.  An SM's CTAs
+// form 34 TFLOP/s of padded products between them (a piece's columns by 16, rows of C by
+// 128), and the SM with the most items decides: one item alone takes 1.25 times an item's
+// share of a pair of CTAs, two take two.  Before that come the lists with their launches, and
+// the copies of operands that are not used in place.  us in the dense form / this one at 0.5
+// present / at 1.0: 2228 x 2000 x 2228, BLKSIZE 48 683 / 442 / 825; 130 x 8000 x 2228 294 /
+// 209 / 386, A transposed and rows odd 324 / 289 / 482; 70 x 16384 x 2228 404 / 213 / 385, so
+// 452 / 378 / 581; the model is within 12 % of these.
+MaskTimes dgemm_mask_times(const double* a, const double* b, int m, int n, int k, size_t lda,
+                           size_t ldb, bool transa, int blk) {
+  const MaskPlan P = mask_plan(a, b, m, n, k, lda, ldb, transa, blk);
+  const int nsm = std::max(sm_count(), 1);
+  const long long items = (long long)P.nblk * P.nsub * ((m + TM - 1) / TM);
+  const double item = 2.0 * TM * ((P.sw + 15) / 16 * 16) * k / (34e6 / nsm);
+  MaskTimes t;
+  t.lists = 28.0;
+  t.copies = (P.a_inplace ? 0.0 : 16.0 * m * k / 6e6) + (P.b_inplace ? 0.0 : 16.0 * n * k / 3.2e6);
+  t.products = item * (items <= nsm ? 1.25 : double((items + nsm - 1) / nsm));
+  return t;
 }
 
 size_t dgemm_mask_workspace(const double* a, const double* b, int m, int n, int k, size_t lda,
@@ -451,8 +462,10 @@ cudaError_t dgemm_mask_compact(double* c, const double* a, const double* b, int 
   if (!P.b_inplace) {
     double* bp = reinterpret_cast<double*>(ws + P.bp);
     const long long cols = (long long)P.nblk * P.blk_pitch;
-    pack_tiles<<<dim3(unsigned((cols + 255) / 256), unsigned(std::min(k, 4096))), 256, 0,
-                 stream>>>(bp, b, ldb, n, k, blk, P.blk_pitch, P.nblk, tab, ldtab, compact);
+    // a few CTAs per SM's place: those of a form that does not run are soon over
+    const long long across = (cols + 255) / 256;
+    const unsigned down = unsigned(std::min<long long>((k + 3) / 4, 2048 / across + 1));
+    pack_tiles<<<dim3(unsigned(across), down), 256, 0, stream>>>(bp, b, ldb, n, k, blk, P.blk_pitch, P.nblk, tab, ldtab, compact);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     g.b = bp;
     g.pitch_b = size_t(cols);

@@ -106,12 +106,11 @@ int cfgmm_matmul_dev(double* c, const double* a, const double* b, size_t m, size
  * Element (p, j) of B takes part only when its (row, column block) flag is
  * set, whatever B holds there (impl_matmul_non0tab.rs:196-207).
  * An Inf or NaN of opA in a row p of B without a present tile: FP64 products on
- * compacted rows leave it out, as the reference does (more than 4e8 operations
- * and blocks of 32 columns or more; where such blocks do not fill whole pieces
- * and most tiles are present, the device picks the dense form).  The dense form
- * multiplies it with zeros, so its row of C becomes NaN, as in split precision.
- * B cannot be
- * transposed: transb != 0 returns CFGMM_ERR_UNIMPLEMENTED, as the reference's
+ * compacted rows leave it out, as the reference does.  The dense form multiplies
+ * it with zeros, so its row of C becomes NaN, as in split precision.  The dense
+ * form runs up to 4e8 operations, for blocks under 32 columns, and where it is
+ * the faster one by the sizes and the share of present tiles.
+ * B cannot be transposed: transb != 0 returns CFGMM_ERR_UNIMPLEMENTED, as the reference's
  * `unimplemented!` (impl_matmul_non0tab.rs:181-183, 228-230). */
 
 /* Replaces matmul_anyway_full_non0tab (src/impl_matmul_non0tab.rs:308-326): BLKSIZE 48. */

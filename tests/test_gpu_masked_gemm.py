@@ -230,3 +230,35 @@ def test_non0tab_compacted_form_leaves_out_rows_without_a_present_tile(cm):
     cm.matmul_non0tab_ex(c, t(a), t(b), m, n, k, k, n, n, False, False, t(tab), n // blk, blk)
     torch.cuda.synchronize()
     assert normwise(c.cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("transa,m,n,k,blk,density,pad", [
+    (True, 20000, 62, 500, 4096, 0.5, 0),            # a block wider than C, compacted
+    (True, 38000, 64, 200, 2**31 - 1 - 4096, 0.5, 0),  # the widest block there is
+    (True, 129, 8000, 1000, 64, 0.3, 1),             # both forms enqueued, compacted runs
+    (True, 129, 8000, 1000, 64, 0.95, 1),            # and dense
+    (False, 64, 16384, 500, 33, 0.05, 0),            # the dense form alone: few rows, copies
+    (True, 9, 16384, 1600, 48, 0.3, 1),              # and where both operands are copied
+    (False, 60000, 33, 700, 48, 0.95, 0),            # tall A, one narrow block: dense runs
+])
+def test_non0tab_forms_by_the_sizes(cm, transa, m, n, k, blk, density, pad):
+    """Products that take the compacted form, the dense one or the device's choice by the
+    model of both; absent tiles of B hold NaN."""
+    import torch
+    rng = np.random.default_rng(m + n)
+    a = rng.uniform(-1, 1, (k, m + pad) if transa else (m, k + pad))
+    b = rng.uniform(-1, 1, (k, n + pad))
+    nblk = -(-n // blk)
+    tab = (rng.random((k, nblk)) < density).astype(np.uint8)
+    on = np.repeat(tab, min(blk, n), axis=1)[:, :n].astype(bool)
+    ref = rng.uniform(-1, 1, (m, n + pad))
+    t = lambda x: torch.from_numpy(x.copy()).cuda()
+    c0, c = ref.copy(), t(ref)
+    ref[:, :n] += (a[:, :m].T if transa else a[:, :k]) @ np.where(on, b[:, :n], 0.0)
+    b[:, :n][~on] = np.nan
+    cm.matmul_non0tab_ex(c, t(a), t(b), m, n, k, a.shape[1], n + pad, n + pad, transa, False,
+                         t(tab), nblk, blk)
+    torch.cuda.synchronize()
+    c = c.cpu().numpy()
+    assert normwise(c, ref) < TOL
+    assert np.array_equal(c[:, n:], c0[:, n:])

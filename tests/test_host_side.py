@@ -72,3 +72,7 @@ def test_host_calls_read_few_error_words(objects):
 
 def test_residues_by_rows_are_formed_aside(objects):
     drive(objects, "residue_streams")
+
+
+def test_forms_of_the_masked_gemm(objects):
+    drive(objects, "masked_forms")
