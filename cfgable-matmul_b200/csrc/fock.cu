@@ -120,9 +120,10 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
   if (warp == CONS) {
     // ------------------------------- producer -------------------------------
     auto* counter = reinterpret_cast<unsigned long long*>(p.counters);
-    long long it = 0;
-    if (lane == 0) it = (long long)atomicAdd(counter, 1ull);
-    it = __shfl_sync(0xffffffffu, it, 0);
+    // the first item is the CTA's own, the others are drawn: no round trip to L2 at the
+    // start, and the heaviest items one to an SM (1000 AOs, 1000 points, all present 107 ->
+    // 93 us; 100 x 5000 21.8 -> 21.2)
+    long long it = blockIdx.x;
     int fill = 0, n = 0;
     bool ok = true;
     // rows lane and lane + 32 of `rows` table rows (lane r, r + 32: AOs v0, v1)
@@ -149,7 +150,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
       }
     };
     while (ok && it < share.total) {
-      const int group = int(it / items);
+      const int group = it >> 32 ? int(it / items) : int(unsigned(it) / unsigned(items));
       const int4 wi = p.items[it - (long long)group * items];
       const int set0 = group * per_group;
       const int ns = min(per_group, p.nset - set0);
@@ -209,7 +210,7 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
       }
       // the next item only now: its chunks are staged two ahead of the products, which
       // hides the draw, and one drawn earlier would wait behind this one's
-      if (lane == 0) it = (long long)atomicAdd(counter, 1ull);
+      if (lane == 0) it = (long long)(gridDim.x + atomicAdd(counter, 1ull));
       it = __shfl_sync(0xffffffffu, it, 0);
     }
     if (ok && (n == 0 || wait_all(aempty, (n - 1) & 1, 0x6102))) {  // the end mark

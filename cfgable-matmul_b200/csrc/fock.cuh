@@ -17,13 +17,14 @@ struct FockShare {
   long long total;
 };
 __host__ __device__ inline FockShare fock_share(int items, int nset, int ctas) {
-  const long long least = (nset + kFockVectors - 1ll) / kFockVectors;
-  const long long one = items > 0 ? items : 1;
-  const long long wanted = (8ll * ctas + one - 1) / one;
-  const long long most = wanted < nset ? wanted : nset;
+  // in 32 bits as far as that goes: a 64-bit division takes a small call's CTAs 0.1 us
+  const unsigned least = (unsigned(nset) + kFockVectors - 1) / kFockVectors;
+  const unsigned one = items > 0 ? items : 1;
+  const unsigned wanted = (8u * ctas + one - 1) / one;
+  const unsigned most = wanted < unsigned(nset) ? wanted : nset;
   FockShare s;
   s.groups = int(least > most ? least : most);
-  s.per_group = int((nset + s.groups - 1ll) / s.groups);
+  s.per_group = int((unsigned(nset) + s.groups - 1) / s.groups);
   s.total = (long long)items * s.groups;
   return s;
 }
