@@ -879,17 +879,26 @@ aodm_fp64_pipe_kernel(const __grid_constant__ AodmArgs p) {
       // passed the next item's epilogue barrier, i.e. finished reading this one.
       if (!warp_wait(&epi[n & 1], (n >> 1) & 1, err, kErrEpilogue, lim)) break;
       const size_t pslot = t.B->partial_off + size_t(t.bg) * p.max_utiles + t.utile;
+      const int nt = (t.nb + TU - 1) / TU;
+      // a block tile of one item needs no partial sums (and their fence: 50 AOs x 34863
+      // points x 2 67 -> 50 us)
+      const bool alone = p.tickets && nt == 1;
       for (int i = ct; i < t.ns * TG; i += NCONS) {
         const int s = i / TG, j = i % TG;
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < CWM; ++w) v += rb[(s * CWM + w) * TG + j];
-        p.partial[(pslot * p.nset_max + set0 + s) * TG + j] = sym ? 2.0 * v : v;
+        if (sym) v *= 2.0;
+        if (alone) {
+          double* r = t.B->rhos + size_t(set0 + s) * t.B->stride_grid + t.g0 + j;
+          if (j < t.gw) *r = v + *r;
+        } else {
+          p.partial[(pslot * p.nset_max + set0 + s) * TG + j] = v;
+        }
       }
-      if (p.tickets) {
+      if (p.tickets && !alone) {
         // the warp that stores the block tile's last partial sums adds them all into
         // rho, in the fixed order of aodm_reduce
-        const int nt = (t.nb + TU - 1) / TU;
         int ticket = 0;
         __syncwarp();
         if (lane == 0) {

@@ -256,3 +256,26 @@ def test_symmetric_d_with_two_phi_arrays(cm, oracle, prec):
     cm.aodmao2rho_ex(rho, dms, lhs, rhs, (nao, ngrid), (nao, ngrid), nset, tab, nblk, blk, prec)
     oracle.aodmao2rho(ref, dms, lhs, rhs, (nao, ngrid), (nao, ngrid), nset, tab, nblk, blk)
     assert normwise(rho, ref) < (1e-12 if prec else 1e-13)
+
+
+@pytest.mark.parametrize("nset", [1, 3, 4])
+@pytest.mark.parametrize("ngrid,blk", [(701, 100), (515, 64), (33, 48)])
+def test_blocks_of_one_and_of_several_items(cm, wl, nset, ngrid, blk):
+    """Lists of 0, 1, 63, 64, 65 and 130 AOs: a list of up to 64 is one item, whose sums go
+    straight into rho, the others' partial sums are added in order.  Symmetric D, two runs
+    alike bit for bit."""
+    rng = np.random.default_rng(ngrid + nset)
+    nao, nblk = 130, -(-ngrid // blk)
+    tab = np.zeros((nao, nblk), np.uint8)
+    for b in range(nblk):
+        tab[rng.choice(nao, (64, 65, 0, 1, 63, 130)[b % 6], replace=False), b] = 1
+    phi = rng.standard_normal((nao, ngrid))
+    dms = wl.sym_dms(rng, nset, nao)
+    rho0 = rng.standard_normal((nset, ngrid))
+    out = []
+    for _ in range(2):
+        rho = rho0.copy()
+        run_gpu(cm, rho, dms, phi, phi, (nao, ngrid), (nao, ngrid), nset, tab, nblk, blk)
+        out.append(rho)
+    assert np.array_equal(out[0], out[1])
+    assert normwise(out[0], rho0 + wl.dense_rho(phi, phi, dms, tab, blk)) < TOL
