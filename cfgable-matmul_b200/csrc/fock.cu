@@ -83,6 +83,13 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int cod
   return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &g_fock_error, code));
 }
 
+// 8-byte asynchronous copy to a shared address, of which the first `bytes` (0 or 8) are
+// read; zeros for the rest.
+__device__ __forceinline__ void cp_async_8_n(uint32_t dst, const double* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+
 // One item as the producer decodes it for the consumers; bg < 0: no more items.
 struct FockItem {
   int bg, nb, u0, gw, b, set0, ns;
@@ -139,12 +146,17 @@ fock_compact_kernel(const __grid_constant__ FockArgs p) {
           tc::bulk_load(dst + (lane + 32) * PITCH, ao + size_t(v1) * p.stride_grid + g0, gw * 8,
                         bar);
       } else {
-        for (int r = 0; r < rows; ++r) {
+        // copies past gw read nothing; one warp issues them all, so a row takes as few
+        // instructions as it can (193 AOs, 589 points, 2 vectors: 25.2 -> 21.1 us against an
+        // address chosen for each copy)
+        const double* from = ao + g0 + lane;
+        const int lo = lane < gw ? 8 : 0, hi = lane + 32 < gw ? 8 : 0;
+        uint32_t to = tc::smem_u32(dst + lane);
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r, to += PITCH * 8) {
           const int v = __shfl_sync(0xffffffffu, r < 32 ? v0 : v1, r & 31);
-          const double* src = ao + size_t(v) * p.stride_grid + g0;
-#pragma unroll
-          for (int k = lane; k < FT; k += 32)
-            cp_async_8(dst + r * PITCH + k, k < gw ? src + k : ao, k < gw);
+          cp_async_8_n(to, from + size_t(v) * p.stride_grid, lo);
+          cp_async_8_n(to + 256, from + size_t(v) * p.stride_grid + 32, hi);
         }
         if (lane == 0) tc::mbar_arrive(bar);  // in the expect_tx's place
       }
