@@ -582,8 +582,9 @@ cudaError_t upload_phi(DeviceState* st, const PhiUpload& u, void* scratch, doubl
 // the work and the transfers of the others: D, the mask and rho go up first,
 // then each block's columns of phi go up on the copy stream, the block is
 // contracted on the compute stream and its columns of rho come back on the
-// download stream.  Every grid block is contracted exactly as in one call (its
-// rho depends only on its own phi columns, D and its mask column).
+// download stream.  Every grid block is contracted as in one call (its rho depends
+// only on its own phi columns, D and its mask column; in split precision fewer points
+// can select the other form, see split_pair_form).
 int aodm_host_blocked(DeviceState* st, double* rhos, const double* dms, const double* ao_lhs,
                       const double* ao_rhs, size_t stride_ao, size_t stride_grid, size_t nao,
                       size_t ngrid, size_t nset, const uint8_t* tab, size_t ldtab,

@@ -319,6 +319,8 @@ int cfgmm_aodm_plan_run(cfgmm_aodm_plan* plan, void* stream);
  * one run (sum over batches, matrices and blocks of (2|I_b|^2 + 2|I_b|)|b|),
  * chosen tiles, autotuner timings. */
 const char* cfgmm_aodm_plan_info(const cfgmm_aodm_plan* plan);
+/* Waits for the device: runs may be in flight on any stream.  While a stream is being
+ * captured no wait is possible, and the plan stays (CFGMM_ERR_CUDA). */
 int cfgmm_aodm_plan_destroy(cfgmm_aodm_plan* plan);
 
 /* ---- the step before the contraction: AOs on the grid, on the device ------

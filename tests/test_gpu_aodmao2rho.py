@@ -279,3 +279,42 @@ def test_blocks_of_one_and_of_several_items(cm, wl, nset, ngrid, blk):
         out.append(rho)
     assert np.array_equal(out[0], out[1])
     assert normwise(out[0], rho0 + wl.dense_rho(phi, phi, dms, tab, blk)) < TOL
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("pinned,same", [(False, False), (True, False), (True, True)])
+def test_large_host_call_whose_transfers_overlap(cm, wl, prec, pinned, same):
+    """Tables past 64 MB in pinned memory, or with most tiles present, go up in blocks of
+    grid blocks while the earlier ones are contracted.  In FP64 the bits are those of one
+    device call; masked entries hold NaN."""
+    import torch
+    nao, ngrid, nset, blk = 1100, 8001, 2, 48
+    sa, sg = nao + 2, ngrid + 6
+    rng = np.random.default_rng(5 + prec)
+    nblk = -(-ngrid // blk)
+    tab = (rng.random((nao, nblk)) < (0.3 if pinned else 0.9)).astype(np.uint8)
+    host = lambda x: torch.from_numpy(np.ascontiguousarray(x)).pin_memory().numpy() if pinned else x
+    off = ~wl.expand_mask(tab, ngrid, blk).astype(bool)
+    lhs = rng.standard_normal((nao, sg))
+    rhs = lhs if same else rng.standard_normal((nao, sg))
+    a = rng.uniform(-1, 1, (nset, sa, sa))
+    dms = np.ascontiguousarray(0.5 * (a + a.transpose(0, 2, 1)))
+    rho0 = rng.uniform(-1, 1, (nset, sg))
+    ref = rho0[:, :ngrid] + wl.dense_rho(np.where(off, 0.0, lhs[:, :ngrid]),
+                                         np.where(off, 0.0, rhs[:, :ngrid]),
+                                         dms[:, :nao, :nao], tab, blk)
+    lhs[:, :ngrid][off] = np.nan
+    rhs[:, :ngrid][off] = np.nan
+    lhs, dms, rho = host(lhs), host(dms), host(rho0.copy())
+    rhs = lhs if same else host(rhs)
+    cm.aodmao2rho_ex(rho, dms, lhs, rhs, (sa, sg), (nao, ngrid), nset, tab, nblk, blk, prec)
+    assert normwise(rho[:, :ngrid], ref) < (1e-12 if prec else 1e-13)
+    assert np.array_equal(rho[:, ngrid:], rho0[:, ngrid:])
+    if prec == 0:
+        t = lambda x: torch.from_numpy(np.array(x)).cuda()
+        d = dict(rho=t(rho0), dms=t(dms), lhs=t(lhs))
+        d["rhs"] = d["lhs"] if same else t(rhs)
+        cm.aodmao2rho_ex(d["rho"], d["dms"], d["lhs"], d["rhs"], (sa, sg), (nao, ngrid), nset, t(tab),
+                         nblk, blk, prec)
+        torch.cuda.synchronize()
+        assert np.array_equal(d["rho"].cpu().numpy(), rho)
