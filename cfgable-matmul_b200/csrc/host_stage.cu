@@ -9,6 +9,10 @@
 #include <system_error>
 #include <thread>
 
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
+
 namespace cfgmm {
 namespace {
 
@@ -17,18 +21,59 @@ constexpr int kMaxWorkers = 6;  // copying threads, the caller among them
 // Smaller copies go the driver's way.
 constexpr size_t kDirectUp = size_t(1) << 20, kDirectDown = size_t(256) << 10;
 
-// Threads of a contiguous upload.  More of them get in one another's way in the driver
-// unless there is much to copy; us by the driver and with 2, 4 and 6 threads, the source
-// in the caches / not: 1 MB 69 69 73 73 / 121 94 96 97; 4 MB 219 199 502 632 / 406 258 441
-// 708; 16 MB 790 567 777 1289 / 1528 901 773 797; 64 MB 5200 2815 2014 2078 / 6207 3329
-// 2000 1874.
-int upload_threads(size_t bytes) { return bytes < (size_t(48) << 20) ? 2 : 4; }
-size_t upload_piece(size_t bytes) { return bytes < (size_t(16) << 20) ? kSlot / 2 : kSlot; }
-// Of the present tiles of a table, whose packing takes longer than a plain copy.  A density
-// call with so many MB of tiles, ms with 2, 3, 4 and 6 threads: 6 0.66 0.67 0.73 0.90; 16
-// 1.16 1.06 1.11 1.39; 46 4.0 3.0 2.6 2.7; 117 12.8 8.5 7.4 6.5.
-int tiles_threads(size_t bytes) {
-  return bytes < (size_t(12) << 20) ? 3 : bytes < (size_t(64) << 20) ? 4 : kMaxWorkers;
+// The driver takes 9 us for a piece, one after another, and a thread 80 us to fill 1 MB.
+// A contiguous upload: four threads (six are no faster), two pieces or more for each.
+constexpr int kUploadThreads = 4;
+size_t upload_piece(size_t bytes) {
+  const size_t each = bytes / (2 * kUploadThreads);
+  return std::min(kSlot, std::max(size_t(256) << 10, (each + 4095) / 4096 * 4096));
+}
+// The present tiles of a table, whose packing takes longer than a plain copy: all threads,
+// one piece for each where that fits, else four.  A density call with so many MB of tiles,
+// us with 3, 4 and 6 threads: 5.6 928 635 581; 11.3 1195 989 840; 45.8 4391 3556 2888; 110
+// 8575 7112 5889.
+size_t tiles_piece(size_t bytes, int threads) {
+  const size_t one = bytes / threads + bytes / (16 * threads);
+  return one <= kSlot ? std::max(size_t(256) << 10, one)
+                      : std::min(kSlot, std::max(size_t(512) << 10, bytes / (4 * threads)));
+}
+// A download: the caller alone below 1 MB, else four threads.  A product with so many MB of
+// C, us with 1, 2, 4 and 6 threads: 0.7 202 256 281 284; 1.9 560 394 321 334; 7.6 1761 1179
+// 698 772; 30 3750 2435 1841 1801.
+int download_threads(size_t bytes) { return bytes < (size_t(1) << 20) ? 1 : 4; }
+size_t download_piece(size_t bytes) {
+  const size_t each = bytes / 12;
+  return std::min(kSlot, std::max(size_t(128) << 10, (each + 4095) / 4096 * 4096));
+}
+
+// Copies into a pinned buffer past the caches (the piece ends with fill_done): the link's
+// reads of lines that another core has just written go at a fifth of its speed, the more
+// cores the slower, and the device waits for them.  us of a density call with so many MB of
+// phi, a product's with three arrays: 2 threads through the caches, 4 of them, 4 past them:
+// 3.8 365 522 222; 11.4 740 1004 470; 22.9 1235 1405 791; 3 x 3.7 934 755 730; 3 x 7.6 1734
+// 1326 1078.  (The driver alone 315, 764, 1384; 1232, 2081.)
+void fill(void* dst, const void* src, size_t n) {
+#if defined(__x86_64__)
+  char* d = static_cast<char*>(dst);
+  const char* s = static_cast<const char*>(src);
+  const size_t head = size_t(-reinterpret_cast<uintptr_t>(d)) & 15;
+  if (n >= 64 + head) {
+    std::memcpy(d, s, head);
+    for (d += head, s += head, n -= head; n >= 64; d += 64, s += 64, n -= 64) {
+      __m128i x[4];
+      for (int i = 0; i < 4; ++i) x[i] = _mm_loadu_si128(reinterpret_cast<const __m128i*>(s) + i);
+      for (int i = 0; i < 4; ++i) _mm_stream_si128(reinterpret_cast<__m128i*>(d) + i, x[i]);
+    }
+  }
+  std::memcpy(d, s, n);
+#else
+  std::memcpy(dst, src, n);
+#endif
+}
+void fill_done() {
+#if defined(__x86_64__)
+  _mm_sfence();
+#endif
 }
 
 // A few threads that run one job at a time.  They live as long as the process: the
@@ -206,12 +251,6 @@ cudaError_t run_pieces(char* pinned, const std::vector<cudaEvent_t>& events, siz
   return cudaError_t(failed.load());
 }
 
-// Bytes of a piece where all threads copy: every one gets two or more.
-size_t piece_bytes(size_t total) {
-  const size_t each = total / (2 * size_t(Workers::get().count()));
-  return std::min(kSlot, std::max(size_t(128) << 10, (each + 4095) / 4096 * 4096));
-}
-
 }  // namespace
 
 cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t spitch,
@@ -230,21 +269,22 @@ cudaError_t HostStage::upload(void* dst, size_t dpitch, const void* src, size_t 
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
   const size_t most = upload_piece(width * rows);
-  const int threads = upload_threads(width * rows);
   if (width > most) {  // parts of a row
     const size_t per_row = (width + most - 1) / most;
-    return run_pieces(pinned_, events_, per_row * rows, threads, stream, [&](size_t i, char* slot) {
+    return run_pieces(pinned_, events_, per_row * rows, kUploadThreads, stream, [&](size_t i, char* slot) {
       const size_t r = i / per_row, off = i % per_row * most;
       const size_t n = std::min(most, width - off);
-      std::memcpy(slot, s + r * spitch + off, n);
+      fill(slot, s + r * spitch + off, n);
+      fill_done();
       return cudaMemcpyAsync(d + r * dpitch + off, slot, n, cudaMemcpyHostToDevice, stream);
     });
   }
   const size_t some = most / width;  // rows
   const size_t pieces = (rows + some - 1) / some;
-  return run_pieces(pinned_, events_, pieces, threads, stream, [&](size_t i, char* slot) {
+  return run_pieces(pinned_, events_, pieces, kUploadThreads, stream, [&](size_t i, char* slot) {
     const size_t r0 = i * some, n = std::min(some, rows - r0);
-    for (size_t r = 0; r < n; ++r) std::memcpy(slot + r * width, s + (r0 + r) * spitch, width);
+    for (size_t r = 0; r < n; ++r) fill(slot + r * width, s + (r0 + r) * spitch, width);
+    fill_done();
     return cudaMemcpy2DAsync(d + r0 * dpitch, dpitch, slot, width, width, n,
                              cudaMemcpyHostToDevice, stream);
   });
@@ -260,7 +300,7 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
   // for all earlier work on the stream, before it takes the threads.
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
-  const size_t most = piece_bytes(bytes), n = (bytes + most - 1) / most;
+  const size_t most = download_piece(bytes), n = (bytes + most - 1) / most;
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
@@ -305,7 +345,7 @@ cudaError_t HostStage::download(void* dst, const void* src, size_t bytes, cudaSt
       failed.compare_exchange_strong(none, int(e));
     }
   };
-  Workers::get().run(copy, kMaxWorkers);
+  Workers::get().run(copy, download_threads(bytes));
   return cudaError_t(failed.load());
 }
 
@@ -339,7 +379,8 @@ cudaError_t HostStage::upload_tiles(double* dst, double* packed, unsigned long l
     unsigned long long at;
   };
   std::vector<Piece> pieces;
-  const size_t most = std::max(piece_bytes(total * 8) / 8, blk);  // blk * 8 <= kSlot: the caller's
+  const int threads = Workers::get().count();
+  const size_t most = std::max(tiles_piece(total * 8, threads) / 8, blk);  // blk * 8 <= kSlot: the caller's
   for (size_t r = 0; r < rows; ++r) {
     const unsigned long long at = offsets[r];
     const size_t n = size_t((r + 1 < rows ? offsets[r + 1] : total) - at);
@@ -362,7 +403,6 @@ cudaError_t HostStage::upload_tiles(double* dst, double* packed, unsigned long l
   err = cudaMemcpyAsync(d_offsets, offsets.data(), rows * sizeof(unsigned long long),
                         cudaMemcpyHostToDevice, stream);
   if (err != cudaSuccess) return err;
-  const int threads = tiles_threads(total * 8);
   err = run_pieces(pinned_, events_, pieces.size(), threads, stream, [&](size_t i, char* slot) {
     const Piece& p = pieces[i];
     double* to = reinterpret_cast<double*>(slot);
@@ -384,10 +424,11 @@ cudaError_t HostStage::upload_tiles(double* dst, double* packed, unsigned long l
         n += std::min(blk, cols - b * blk);
         ++b;
       }
-      std::memcpy(to, src + r * ld + c0, n * 8);
+      fill(to, src + r * ld + c0, n * 8);
       to += n;
       left -= n;
     }
+    fill_done();
     return cudaMemcpyAsync(packed + p.at, slot, p.elems * 8, cudaMemcpyHostToDevice, stream);
   });
   if (err != cudaSuccess) return err;
