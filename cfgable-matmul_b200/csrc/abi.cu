@@ -519,11 +519,11 @@ int aodm_device_status(bool split) {
 // tiles, packed by the copying threads (the kernels read no others), when they are at
 // most three quarters of a table of 4 MB or more.  `offsets` empty: whole tables.
 // Tables of 64 MB and more go so too, all of them before the contraction, and not in
-// blocks that overlap it (aodm_host_blocked): fewer bytes win at every size measured.  ms in
-// blocks / tiles at 0.05, 0.3 and 0.7 present: 2228 AOs, 16384 points, 3 matrices (292 MB)
-// 15.9/4.6, 16.5/6.7, 20.0/12.4, split 16.3/4.8, 16.8/6.5, 18.1/10.1; 40000 points (713 MB)
-// 23.4/5.1, 25.2/10.6, 33.3/24.8; 1000 AOs, 100000 points, 1 matrix 22.6/2.8, 23.3/8.0,
-// 25.8/19.1.
+// blocks that overlap it (aodm_host_blocked): fewer bytes win at every size measured.  ms
+// whole / tiles at 0.2, 0.5 and 0.75 present: 300 AOs, 5000 points (11 MB) 0.42/0.21,
+// 0.44/0.33, 0.44/0.42; 601, 8191 (38 MB) 1.11/0.80, 1.18/1.16, 1.26/1.31; in blocks / tiles
+// 1000, 20000 (153 MB) 4.9/1.4, 5.4/3.2, 5.9/4.3; 2228, 16384, 3 matrices (278 MB) 12.4/6.4,
+// 14.6/10.4, 18.2/15.0; 1000, 60000 (458 MB) 14.1/4.4, 15.3/8.8, 17.1/12.5.
 struct PhiUpload {
   size_t elems = 0;  // of a table's present tiles
   std::vector<unsigned long long> offsets;
