@@ -525,7 +525,8 @@ cudaError_t gemm(T* c, const T* a, const T* b, int m, int n, int k, size_t lda, 
 }
 
 // The dense form of a masked product (in-place copies of B ask for the mask 8 bytes at a
-// time): the model of choose_splits and the copies, within 15 % of 22 shapes of 50 us to 5 ms.
+// time): the model of choose_splits and the copies, 0.95 to 1.12 of what eight in ten of 22
+// shapes of 50 us to 5 ms take, 0.90 to 1.21 of all.
 double masked_dense_us(int m, int n, int k, bool transa) {
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
